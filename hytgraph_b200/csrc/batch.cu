@@ -31,12 +31,11 @@ enum : uint32_t { kFree = 0, kSSSP = 1, kPPR = 2 };
 
 constexpr uint32_t kMaxSlots = 4096;
 constexpr int kWorkThreads = 256;
-constexpr size_t kSliceFloats = 2 * size_t(kTileCostMax) + 8;  // PPR tile staging per warp
 constexpr int kSplitBlocks = 4;
 constexpr int kInitBlocks = 64;
 constexpr uint32_t kEndBlocks = 16;  // blocks per PPR slot in the end reduction
 constexpr uint32_t kGrab = 4;        // units / hub tasks a warp takes at a time
-constexpr bool kHotGlobal = true;    // hot sources read from the slot's hot_contrib array
+constexpr bool kSmemHot = false;     // hot sources are read from the slot's hot_contrib array, in global memory
 
 struct Slot {
     uint32_t kind;        // kFree / kSSSP / kPPR
@@ -300,16 +299,13 @@ __global__ void __launch_bounds__(kWorkThreads, 3) engine_sssp_kernel(const Engi
 // arguments are read per unit (L1-resident); hot sources come from the
 // slot's hot_contrib array.
 __global__ void __launch_bounds__(kWorkThreads) engine_ppr_kernel(const EngineArgs *__restrict__ eap) {
-    extern __shared__ __align__(16) float s_dyn[];
+    extern __shared__ __align__(16) uint32_t s_base[];
     const EngineArgs ea = *eap;
     const uint32_t n = ea.n;
-    uint32_t *s_base = reinterpret_cast<uint32_t *>(s_dyn + (kWorkThreads / 32) * kSliceFloats);
     for (uint32_t i = threadIdx.x; i <= n; i += blockDim.x) s_base[i] = ea.pr_base[i];
     __syncthreads();
     const uint32_t total = s_base[n];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *sv = s_dyn + warp * kSliceFloats;
-    const uint64_t pol = dev::policy_evict_last();
     const uint32_t nwarps = gridDim.x * (kWorkThreads / 32);
     for (uint32_t u = blockIdx.x * (kWorkThreads / 32) + warp; u < total; u += nwarps) {
         const uint32_t q = find_slot(s_base, n, u);
@@ -320,13 +316,14 @@ __global__ void __launch_bounds__(kWorkThreads) engine_ppr_kernel(const EngineAr
         const PRBuffers b = prc::buffers(a, it);
         const PRState ps = prc::make_state(a, a.dangling[it]);
         const float *hot = x.hot_contrib[it & 1];
+        const prc::TaskSpan span = prc::task_span(a.tasks[t]);
         double res = 0.0, dang = 0.0;
         if (t < x.num_chunks) {
-            const uint32_t li = prc::chunk_task<kHotGlobal>(a, ps, b, a.in_src, hot, t, pol, lane, res, dang);
+            const uint32_t li = prc::chunk_task<kSmemHot>(a, ps, b, a.in_src, hot, span, lane, res, dang);
             if (li != ~0u && lane == 0) x.task_sums[x.num_tiles + li] = make_double2(res, dang);
         } else {
             const uint64_t k = t - x.num_chunks;
-            prc::tile_task<kHotGlobal>(a, ps, b, a.in_src, hot, sv, k, pol, lane, res, dang);
+            prc::tile_task<kSmemHot>(a, ps, b, a.in_src, hot, span, lane, res, dang);
             res = dev::warp_sum(res);
             dang = dev::warp_sum(dang);
             if (lane == 0) x.task_sums[k] = make_double2(res, dang);
@@ -461,7 +458,7 @@ __global__ void engine_status_kernel(const EngineArgs *__restrict__ eap, SlotSta
 uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
 int ppr_kernel_smem(uint32_t cap) {
-    return static_cast<int>((kWorkThreads / 32) * kSliceFloats * sizeof(float) + (cap + 1) * sizeof(uint32_t));
+    return static_cast<int>((cap + 1) * sizeof(uint32_t));
 }
 
 int sssp_kernel_smem(uint32_t cap) { return static_cast<int>((cap + 1) * sizeof(uint32_t)); }
@@ -651,6 +648,7 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
         a.tile_start = g.tile_start.get();
         a.long_rows = g.long_rows.get();
         a.chunk_tasks = g.chunk_tasks.get();
+        a.tasks = g.pull_tasks.get();
         a.hot_vertex = g.hot_vertex.get();
         a.num_hot = g.num_hot;
         a.tile_cost = g.tile_cost;

@@ -303,6 +303,29 @@ struct CSum {
     __device__ __forceinline__ float value() const { return __fsub_rn(s, c); }
 };
 
+// Two compensated accumulators side by side (packed FP32 adds: 4
+// instructions for two elements), merged into one sum at the end.  c holds
+// the low-order parts with their own sign (value = s + c).
+struct CSum2 {
+    float2 s = {0.f, 0.f};
+    float2 c = {0.f, 0.f};
+    __device__ __forceinline__ void add(float x0, float x1) {
+        const float2 y = __fadd2_rn(make_float2(x0, x1), c);
+        const float2 t = __fadd2_rn(s, y);
+        c = __fadd2_rn(y, __ffma2_rn(t, make_float2(-1.f, -1.f), s));  // y - (t - s)
+        s = t;
+    }
+    __device__ __forceinline__ CSum total() const {
+        CSum a, b;
+        a.s = s.x;
+        a.c = -c.x;
+        b.s = s.y;
+        b.c = -c.y;
+        a.merge(b);
+        return a;
+    }
+};
+
 __device__ __forceinline__ CSum warp_reduce(CSum v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

@@ -24,7 +24,7 @@ namespace hyt {
 // so its rows hold fewer than tile_cost edges except for its last row.  A
 // last row with in-degree >= tile_cost is a "long row": it is excluded from
 // the tile and split into kLongChunk-edge chunks.  One warp processes one
-// task (tile or chunk), so a tile's staged contributions fit in a per-warp
+// task (tile or chunk), so a tile's staged SSSP candidates fit in a per-warp
 // shared-memory slice of 2 * tile_cost floats.
 constexpr uint32_t kTileCostDefault = 512;   // merge-path units per tile (tunable: HYT_PR_TILE)
 constexpr uint32_t kTileCostMax = 512;       // register-path tiles; bulk-staged tasks need <= kStageTileMax
@@ -171,9 +171,12 @@ struct GraphImpl {
     size_t device_bytes() const;
 };
 
-// PageRank CTA shape: kPRThreads threads; dynamic shared memory = hot cache
-// + one staging slice (2 * tile_cost + 8 floats) per warp.
+// PageRank CTA shape: kPRThreads threads; dynamic shared memory = hot
+// cache and its zero slot.
 constexpr int kPRThreads = 1024;
+inline size_t pr_hot_bytes(uint32_t num_hot) { return (size_t(num_hot) + 1) * sizeof(float); }
+// SSSP sweeps of the same shape: hot slots + one staging slice (2 * tile_cost
+// + 8 words) per warp.
 inline size_t pr_shared_bytes(uint32_t num_hot, uint32_t tile_cost) {
     return (size_t(num_hot) + size_t(kPRThreads / 32) * (2 * size_t(tile_cost) + 8)) * sizeof(float);
 }

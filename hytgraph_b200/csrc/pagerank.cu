@@ -19,18 +19,18 @@
 //                   last arriving warp of a row merges the partials in chunk
 //                   order;
 //   tile tasks   -- merge-path tiles of consecutive shorter rows (512
-//                   units by default); the tile's contributions are
-//                   gathered, 16 per lane in flight, into the warp's
-//                   shared-memory slice, then summed lane-per-row (in-degree
-//                   < kWarpRowDegree) or warp-per-row.  The first 32 rows'
-//                   bounds, ranks and out-degrees are loaded with the
-//                   gathers, and before its row phase a warp warms L2 with
-//                   its next task's id lines.
-// With HYT_STAGED=1 (256-unit tiles) pr_staged_kernel stages each task's
-// source ids in shared memory by bulk copies (cp.async.bulk, completion on
-// an mbarrier; stage.cuh) instead; on R-MAT graphs it ran slower than the
-// register path.  The out-of-HBM solver, whose ids come from staging slots
-// or mapped host memory, runs the register path over its partitions.
+//                   units by default), 32 rows at a time: groups of 1 to 8
+//                   lanes, or the whole warp, gather a row's contributions
+//                   and sum them in registers (tile_task).
+//
+// What bounds it: random 4-byte gathers cost one 32-byte L2 sector each, and
+// an SM takes at most 1.02 sectors per clock (measured on a 64 MB table), but
+// only with L1 to hold the outstanding misses: 0.85 per clock beside 132 KB of
+// shared memory, 0.60 beside 164 KB, 0.28 beside 196 KB.  So nothing but the
+// hot-source table lives in shared memory.  The former layout staged every
+// tile's contributions in 4 KB per warp (132 KB per CTA) and ran an iteration
+// of R-MAT scale 24 (263 M edges, 8192 hot sources) in 1.16 ms; sums in
+// registers take 1.02 ms.
 //
 // Results are deterministic: every row sum has a fixed association order,
 // and the FP64 residual and dangling mass are summed in a fixed slot order
@@ -42,19 +42,16 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "bulk.cuh"
 #include "common.cuh"
 #include "graph.cuh"
 #include "hybrid.cuh"
 #include "pagerank_core.cuh"
 #include "solvers.cuh"
-#include "stage.cuh"
 
 namespace hyt {
 namespace {
 
 using namespace prc;
-using namespace stage;
 
 // Slot of long row i and of tile k in the fixed-order reduction.
 __device__ __forceinline__ uint32_t long_slot(uint32_t i) { return i; }
@@ -65,6 +62,7 @@ __device__ __forceinline__ uint32_t tile_slot(const PRArgs &a, uint64_t k) {
 // Hot-source contributions of this iteration, loaded once per CTA.
 __device__ __forceinline__ void load_hot(const PRArgs &a, const PRBuffers &b, float *s_hot) {
     const uint32_t nt = blockDim.x;
+    if (threadIdx.x == 0) s_hot[a.num_hot] = 0.0f;  // "no edge"
     for (uint32_t i0 = 0; i0 < a.num_hot; i0 += 8 * nt) {
         uint32_t hv[8];
 #pragma unroll
@@ -83,8 +81,6 @@ __device__ __forceinline__ void load_hot(const PRArgs &a, const PRBuffers &b, fl
     }
 }
 
-// ---- register path (out-of-HBM partitioned solves) ------------------------
-
 // One launch processes chunk tasks [chunk_begin, chunk_end) and tiles
 // [tile_begin, tile_end); in_src is the base of the source ids, addressed by
 // global edge index (a device array, a staging slot offset by its first
@@ -96,163 +92,48 @@ struct PRRange {
     const uint4 *tasks;  // the graph's task descriptors (whole-graph launches; NULL: no prefetch)
 };
 
-__global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs *__restrict__ args, PRRange rg) {
+// a: the solve's arguments as kernel parameters (the constant bank: no
+// registers held across the tasks); its scalars may be of an earlier solve,
+// those of this one are in *args.
+__global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs *__restrict__ args,
+                                                                   const __grid_constant__ PRArgs a,
+                                                                   const __grid_constant__ PRRange rg) {
     extern __shared__ __align__(16) float s_dyn[];
 
-    const PRArgs a = *args;
     const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
     if (*(volatile uint32_t *)&a.hdr->done) return;
 
     const PRBuffers b = buffers(a, it);
-    const PRState ps = make_state(a, a.dangling[it]);
-    const uint64_t pol = dev::policy_evict_last();
+    const PRState ps = make_state(*args, a.dangling[it]);
     const uint64_t n_chunks = rg.chunk_end - rg.chunk_begin;
     const uint64_t total_tasks = n_chunks + (rg.tile_end - rg.tile_begin);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *s_hot = s_dyn;
     load_hot(a, b, s_hot);
     __syncthreads();
-    float *sv = s_dyn + a.num_hot + warp * (2 * a.tile_cost + 8);
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPRThreads / 32);
 
-    for (uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp; task < total_tasks; task += nwarps) {
+    uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp;
+    // whole-graph launches read each task's descriptor while the task before
+    // it runs (one 16-byte load in place of a chain of table reads)
+    uint4 d = (rg.tasks && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
+    for (; task < total_tasks; task += nwarps) {
         double res = 0.0, dang = 0.0;
-        // whole-graph launches index the descriptors like their tasks
         const uint64_t next = task + nwarps;
         const uint4 nd = (rg.tasks && next < total_tasks) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
         const uint4 *pf = rg.tasks ? &nd : nullptr;
         if (task < n_chunks) {
-            const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, rg.chunk_begin + task, pol, lane, res,
-                                                  dang, pf);
+            const TaskSpan t = rg.tasks ? task_span(d) : chunk_span(a, rg.chunk_begin + task);
+            const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
             if (row != ~0u) slot_store(a, long_slot(row), dev::warp_sum(res), dev::warp_sum(dang), lane);
         } else {
             const uint64_t k = rg.tile_begin + (task - n_chunks);
-            tile_task<true>(a, ps, b, rg.in_src, s_hot, sv, k, pol, lane, res, dang, pf);
+            const TaskSpan t = rg.tasks ? task_span(d) : tile_span(a, k);
+            tile_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
             slot_store(a, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
         }
+        d = nd;
     }
-}
-
-// ---- staged path (graph in HBM; pipeline in stage.cuh) ---------------------
-
-__device__ __forceinline__ void stage_failed(const PRArgs &a) {
-    atomicExch(&a.hdr->error, 1u);
-    atomicExch(&a.hdr->done, 1u);
-    if (a.use_cond) cudaGraphSetConditional(a.cond, 0);
-}
-
-// Gathers the contributions of staged edges [lo, hi) (ids at
-// slot[x - a0]): lane l takes edges lo + 32k + l, all kUnitEdges / 32
-// gathers in flight.  sink(i, value) receives edge lo + i.
-template <class Sink>
-__device__ __forceinline__ void gather_staged(const uint32_t *slot, uint64_t a0, uint64_t lo, uint64_t hi,
-                                              const float *ccur, const float *s_hot, uint64_t pol, int lane,
-                                              Sink &&sink) {
-    constexpr int kB = kUnitEdges / 32;
-    const uint32_t n = static_cast<uint32_t>(hi - lo);
-    const uint32_t *ids = slot + (lo - a0);
-    float v[kB];
-#pragma unroll
-    for (int k = 0; k < kB; ++k) {
-        const uint32_t i = 32 * k + lane;
-        const uint32_t id = (i < n) ? ids[i] : 0u;
-        v[k] = (id & kHotTag) ? s_hot[id & ~kHotTag] : dev::ld_keep(ccur + id, pol);
-    }
-#pragma unroll
-    for (int k = 0; k < kB; ++k) {
-        const uint32_t i = 32 * k + lane;
-        if (i < n) sink(i, v[k]);
-    }
-}
-
-__global__ void __launch_bounds__(kStageThreads, 1) pr_staged_kernel(const PRArgs *__restrict__ args) {
-    extern __shared__ __align__(128) unsigned char s_stage[];
-    const PRArgs a = *args;
-    const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
-    if (*(volatile uint32_t *)&a.hdr->done) return;
-
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const WarpStage ws = warp_stage(s_stage, warp, lane);
-    float *s_hot = reinterpret_cast<float *>(s_stage + kStageBytes);
-    const PRBuffers b = buffers(a, it);
-    const PRState ps = make_state(a, a.dangling[it]);
-    const uint64_t pol = dev::policy_evict_last();
-    load_hot(a, b, s_hot);
-    __syncthreads();
-
-    const uint64_t total = a.num_chunks + a.num_tiles;
-    const uint64_t nwarps = uint64_t(gridDim.x) * kStageWarps;
-    dev::CSum acc;  // running sum of the current chunk
-    const bool ok = stage_pipeline(
-        a.tasks, a.in_src, uint64_t(blockIdx.x) * kStageWarps + warp, nwarps, total, ws, lane,
-        [&](uint4 d, uint64_t task, uint32_t j, uint32_t nu, uint32_t *slot, uint64_t a0) {
-            double res = 0.0, dang = 0.0;
-            if (task_is_chunk(d)) {
-                const Unit u = unit_of(d, j);
-                if (j == 0) acc = dev::CSum();
-                gather_staged(slot, a0, u.lo, u.hi, b.ccur, s_hot, pol, lane, [&](uint32_t, float v) { acc.add(v); });
-                if (j + 1 < nu) return;
-                // last piece: publish the chunk's partial; the row's last
-                // arriving chunk merges the partials in chunk order
-                const LongRow L = a.long_rows[d.z];
-                const dev::CSum w = dev::warp_reduce(acc);
-                uint32_t last = 0;
-                if (lane == 0) {
-                    a.partial[L.first_chunk + d.w] = make_float2(w.s, w.c);
-                    __threadfence();
-                    const uint32_t tk = atomicAdd(&a.ticket[d.z], 1u) + 1u;
-                    last = (tk % L.num_chunks == 0) ? 1u : 0u;
-                }
-                if (!__shfl_sync(0xffffffffu, last, 0)) return;
-                __threadfence();
-                dev::CSum row;
-                for (uint32_t c = lane; c < L.num_chunks; c += 32) {
-                    const float2 p = __ldcg(a.partial + L.first_chunk + c);
-                    dev::CSum x;
-                    x.s = p.x;
-                    x.c = p.y;
-                    row.merge(x);
-                }
-                row = dev::warp_reduce(row);
-                if (lane == 0) finalize_row(a, ps, L.row, row.value(), b.cur, b.nxt, b.cnxt, res, dang);
-                slot_store(a, long_slot(d.z), res, dang, lane);  // lane 0 finalized the row
-                return;
-            }
-            // tile: rows [r0, rl), edges [e0, e0 + n); contributions replace
-            // the ids in the slot, then rows are summed in edge order
-            const uint32_t r0 = d.z, rl = d.w;
-            const uint64_t e0 = task_first_edge(d), e1 = e0 + task_edges(d);
-            float *vals = reinterpret_cast<float *>(slot);
-            const uint32_t r = r0 + lane;
-            const uint64_t lo0 = (r < rl) ? a.in_off[r] : 0, hi0 = (r < rl) ? a.in_off[r + 1] : 0;  // in flight
-            gather_staged(slot, a0, e0, e1, b.ccur, s_hot, pol, lane,
-                          [&](uint32_t i, float v) { vals[e0 - a0 + i] = v; });
-            __syncwarp();
-            for (uint32_t rb = r0; rb < rl; rb += 32) {
-                const uint32_t rr = rb + lane;
-                const bool active = rr < rl;
-                const uint64_t lo = (rb == r0) ? lo0 : (active ? a.in_off[rr] : 0);
-                const uint64_t hi = (rb == r0) ? hi0 : (active ? a.in_off[rr + 1] : 0);
-                if (active && hi - lo < kWarpRowDegree) {
-                    dev::CSum s;
-                    for (uint64_t x = lo; x < hi; ++x) s.add(vals[x - a0]);
-                    finalize_row(a, ps, rr, s.value(), b.cur, b.nxt, b.cnxt, res, dang);
-                }
-                uint32_t big = __ballot_sync(0xffffffffu, active && (hi - lo >= kWarpRowDegree));
-                while (big) {
-                    const int src = __ffs(big) - 1;
-                    big &= big - 1;
-                    const uint64_t bb = __shfl_sync(0xffffffffu, lo, src);
-                    const uint64_t ee = __shfl_sync(0xffffffffu, hi, src);
-                    dev::CSum s;
-                    for (uint64_t x = bb + lane; x < ee; x += 32) s.add(vals[x - a0]);
-                    s = dev::warp_reduce(s);
-                    if (lane == 0) finalize_row(a, ps, rb + src, s.value(), b.cur, b.nxt, b.cnxt, res, dang);
-                }
-            }
-            slot_store(a, tile_slot(a, task - a.num_chunks), dev::warp_sum(res), dev::warp_sum(dang), lane);
-        });
-    if (!ok) stage_failed(a);
 }
 
 // Closes an iteration: block b sums slot groups b, b + grid, ... (thread t
@@ -347,8 +228,6 @@ int pr_occupancy_grid() {
         int per_sm = 0;
         HYT_CUDA(cudaFuncSetAttribute(pr_iterate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaFuncSetAttribute(pr_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPRSmemMax)));
         HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_iterate_kernel, kPRThreads, kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
         if (const char *e = std::getenv("HYT_PR_GRID")) {
@@ -357,26 +236,6 @@ int pr_occupancy_grid() {
         }
     }
     return grid;
-}
-
-// Grid of the staged kernel: one CTA per SM, or HYT_PR_GRID CTAs.
-int pr_staged_grid() {
-    static int grid = 0;
-    if (grid == 0) {
-        grid = sm_count();
-        if (const char *e = std::getenv("HYT_PR_GRID")) {
-            const long v = std::strtol(e, nullptr, 10);
-            if (v > 0 && v <= 65535) grid = static_cast<int>(v);
-        }
-    }
-    return grid;
-}
-
-// In-HBM solves use the staged kernel when it was asked for (HYT_STAGED=1)
-// and the graph's tiles fit a staging slot.
-bool pr_use_staged(const GraphImpl &g) {
-    return stage::staged_requested() && g.tile_cost <= kStageTileMax && g.pull_tasks.get() &&
-           staged_shared_bytes(g.num_hot) <= kPRSmemMax;
 }
 
 }  // namespace
@@ -503,20 +362,12 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
     PRHeader *hdr = st0.hdr;
     const bool use_graph = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = pr_occupancy_grid();
-    const bool staged = pr_use_staged(g);
-    const int sgrid = pr_staged_grid();
-    const void *kfunc = staged ? reinterpret_cast<const void *>(pr_staged_kernel)
-                               : reinterpret_cast<const void *>(pr_iterate_kernel);
-    const unsigned smem = static_cast<unsigned>(staged ? staged_shared_bytes(g.num_hot)
-                                                       : pr_shared_bytes(g.num_hot, g.tile_cost));
+    const unsigned smem = static_cast<unsigned>(pr_hot_bytes(g.num_hot));
     PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get()};
-    void *kargs[] = {&d_args, &full};
+    void *kargs[] = {&d_args, &a, &full};
     const unsigned rgrid = pr_reduce_grid(a);
     auto launch = [&] {
-        if (staged)
-            pr_staged_kernel<<<sgrid, kStageThreads, smem, s>>>(d_args);
-        else
-            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(d_args, full);
+        pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(d_args, a, full);
         pr_reduce_kernel<<<rgrid, kReduceThreads, 0, s>>>(d_args);
         HYT_CUDA(cudaGetLastError());
     };
@@ -551,9 +402,9 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
         HYT_CUDA(cudaGraphAddNode(&cnode, graph, nullptr, 0, &cp));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         cudaKernelNodeParams kp = {};
-        kp.func = const_cast<void *>(kfunc);
-        kp.gridDim = dim3(staged ? sgrid : grid);
-        kp.blockDim = dim3(staged ? kStageThreads : kPRThreads);
+        kp.func = reinterpret_cast<void *>(pr_iterate_kernel);
+        kp.gridDim = dim3(grid);
+        kp.blockDim = dim3(kPRThreads);
         kp.sharedMemBytes = smem;
         kp.kernelParams = kargs;
         cudaGraphNode_t knode, rnode;
@@ -641,7 +492,7 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
     PRSolveState st0 = pr_prepare(g, personalized, source, damping, tolerance, max_iter);
     const PRArgs &a = st0.a;
     const int grid = pr_occupancy_grid();
-    const size_t smem = pr_shared_bytes(a.num_hot, a.tile_cost);
+    const size_t smem = pr_hot_bytes(a.num_hot);
 
     EventTimer total;
     total.start(s);
@@ -658,7 +509,7 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
             if (pp.chunk_begin == pp.chunk_end && pp.tile_begin == pp.tile_end) continue;
             const uint32_t *base = src.acquire(p, s);
             const PRRange rg{base, pp.chunk_begin, pp.chunk_end, pp.tile_begin, pp.tile_end};
-            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(st0.d_args, rg);
+            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
             HYT_CUDA(cudaGetLastError());
             src.release(p, s);
             ++launches;

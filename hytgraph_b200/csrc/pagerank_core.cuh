@@ -19,7 +19,8 @@ namespace prc {
 #ifndef HYT_PR_WARP_ROW
 #define HYT_PR_WARP_ROW 64
 #endif
-constexpr uint32_t kWarpRowDegree = HYT_PR_WARP_ROW;  // rows with more in-edges are summed by a whole warp
+constexpr uint32_t kWarpRowDegree = HYT_PR_WARP_ROW;  // rows with this many in-edges are summed by a whole warp
+static_assert(kWarpRowDegree <= 64, "8 lanes of 8 edges sum the other rows");
 
 struct PRHeader {
     uint32_t iter;       // iterations completed
@@ -77,7 +78,7 @@ struct PRArgs {
     cudaGraphConditionalHandle cond;
     uint32_t use_cond;
     PRSlots red;        // fixed-order residual / dangling reduction (single-query solver)
-    const uint4 *tasks; // pull task descriptors (staged solver)
+    const uint4 *tasks; // pull task descriptors
 };
 
 struct PRState {
@@ -123,76 +124,98 @@ __device__ __forceinline__ void finalize_row(const PRArgs &a, const PRState &ps,
     if (od == 0) dang += static_cast<double>(nx);
 }
 
-// Gathers the contributions of edges [lo, hi) of the in-source array.
-// Lane l of the warp takes edges lo + base + 32k + l (k < kBatch): each of
-// the kBatch id loads is one coalesced 128-byte access, and because the
-// sources of an in-row are sorted, the 32 addresses of each gather
-// instruction are ascending and neighbouring lanes often share an L2 sector
-// (dense for hub-heavy rows).  All kBatch gathers of a lane are issued
-// before any is consumed.  Edges past hi yield 0 and read a clamped address.
+// In-edge batches per lane of one gather pass of long and wide rows.
 #ifndef HYT_PR_BATCH
-#define HYT_PR_BATCH 16
+#define HYT_PR_BATCH 8
 #endif
 constexpr int kBatch = HYT_PR_BATCH;
 
-// kSmemHot: hot sources (tagged ids) read their contribution from the
-// CTA's shared-memory copy s_hot; otherwise from ccur[hot_vertex[slot]].
-// One pass of kK = 4 * kG batches (edges src[base + 32k + lane], k < kK).
-template <int kK, bool kSmemHot, class Sink>
-__device__ __forceinline__ void gather_pass(const uint32_t *src, uint32_t base, uint32_t n, const float *ccur,
-                                            const float *s_hot, const uint32_t *hot_vertex, uint64_t pol, int lane,
-                                            Sink &sink) {
+// Where a task reads its contributions: whole-vector array for untagged
+// sources (L2, evict-last), table of the hot sources for tagged ones.  Slot
+// num_hot of the table is 0: `none`, its tagged id, stands for "no edge".
+// kSmemHot: the table is in shared memory (else in global memory).
+struct Sources {
+    const float *ccur;
+    const float *hot;
+    uint32_t none;
+    uint64_t pol;
+};
+
+__device__ __forceinline__ Sources make_sources(const PRArgs &a, const float *ccur, const float *hot) {
+    return Sources{ccur, hot, kHotTag | a.num_hot, dev::policy_evict_last()};
+}
+
+// Loads one source's contribution: its bits end in `g | id`.  The two loads
+// are predicated on the tag and write registers of their own (the hot one
+// its id's), so that neither waits for the other and no branch splits a run
+// of gathers.
+template <bool kSmemHot>
+__device__ __forceinline__ void load_contribution(uint32_t &id, uint32_t &g, const Sources &S) {
+    g = 0;
+    if constexpr (kSmemHot) {
+        const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(S.hot)) + (id << 2);  // drops the tag
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, 0;\n\t"
+            "@!p ld.global.nc.L2::cache_hint.b32 %0, [%2], %3;\n\t"
+            "@!p mov.b32 %1, 0;\n\t"
+            "@p ld.shared.b32 %1, [%4];\n\t}"
+            : "+r"(g), "+r"(id)
+            : "l"(S.ccur + id), "l"(S.pol), "r"(at));
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, 0;\n\t"
+            "@!p ld.global.nc.L2::cache_hint.b32 %0, [%2], %3;\n\t"
+            "@!p mov.b32 %1, 0;\n\t"
+            "@p ld.global.nc.b32 %1, [%4];\n\t}"
+            : "+r"(g), "+r"(id)
+            : "l"(S.ccur + id), "l"(S.pol), "l"(S.hot + (id & ~kHotTag)));
+    }
+}
+
+// Adds the kK contributions loaded by load_contribution.
+template <int kK>
+__device__ __forceinline__ void add_contributions(const uint32_t (&id)[kK], const uint32_t (&g)[kK], dev::CSum2 &acc) {
+#pragma unroll
+    for (int k = 0; k < kK; k += 2) acc.add(__uint_as_float(g[k] | id[k]), __uint_as_float(g[k + 1] | id[k + 1]));
+}
+
+// Adds the contributions of edges src[base + 32k + lane], k < kK, below n
+// (kFull: all of them are).  Each of the kK id loads is one coalesced
+// 128-byte access, and because the sources of an in-row are sorted, the 32
+// addresses of each gather instruction are ascending and neighbouring lanes
+// often share an L2 sector (dense for hub-heavy rows).  All kK gathers of a
+// lane are issued before any is consumed.
+template <int kK, bool kSmemHot, bool kFull>
+__device__ __forceinline__ void gather_pass(const uint32_t *src, uint32_t base, uint32_t n, const Sources &S, int lane,
+                                            dev::CSum2 &acc) {
     uint32_t id[kK];
 #pragma unroll
     for (int k = 0; k < kK; ++k) {
         const uint32_t i = base + 32 * k + lane;
-        id[k] = (i < n) ? dev::ld_stream(src + i) : 0u;
+        id[k] = (kFull || i < n) ? dev::ld_stream(src + i) : S.none;
     }
-    float v[kK];
+    uint32_t g[kK];
 #pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        v[k] = 0.0f;
-        if (!(id[k] & kHotTag)) v[k] = dev::ld_keep(ccur + id[k], pol);
-    }
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        if (id[k] & kHotTag) {
-            if constexpr (kSmemHot) {
-                v[k] = s_hot[id[k] & ~kHotTag];
-            } else {
-                v[k] = ccur[hot_vertex[id[k] & ~kHotTag]];
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        const uint32_t i = base + 32 * k + lane;
-        if (i < n) sink(i, v[k]);
-    }
+    for (int k = 0; k < kK; ++k) load_contribution<kSmemHot>(id[k], g[k], S);
+    add_contributions<kK>(id, g, acc);
 }
 
-// A pass over the last, partial batch group issues only the 4-batch groups
-// that hold edges (a warp-uniform choice), so short tiles do not pay for
-// kBatch gather slots; the edges and their order are the same.
-template <bool kSmemHot, class Sink>
-__device__ __forceinline__ void gather_span(const uint32_t *in_src, const float *ccur, const float *s_hot,
-                                            const uint32_t *hot_vertex, uint64_t lo, uint64_t hi, uint64_t pol,
-                                            int lane, Sink &&sink) {
+// Adds the contributions of edges [0, n) of src.  The last, partial pass
+// issues only the 4-batch groups that hold edges (a warp-uniform choice).
+template <bool kSmemHot>
+__device__ __forceinline__ void gather_span(const uint32_t *src, uint32_t n, const Sources &S, int lane,
+                                            dev::CSum2 &acc) {
     static_assert(kBatch % 4 == 0 && kBatch >= 4, "batches come in groups of 4");
-    const uint32_t n = static_cast<uint32_t>(hi - lo);
-    const uint32_t *src = in_src + lo;
-    for (uint32_t base = 0; base < n; base += 32 * kBatch) {
-        const uint32_t groups = (n - base + 127) / 128;  // 4-batch groups holding edges
-        if (groups >= kBatch / 4)
-            gather_pass<kBatch, kSmemHot>(src, base, n, ccur, s_hot, hot_vertex, pol, lane, sink);
-        else if (groups == 1)
-            gather_pass<4, kSmemHot>(src, base, n, ccur, s_hot, hot_vertex, pol, lane, sink);
-        else if (groups == 2)
-            gather_pass<8, kSmemHot>(src, base, n, ccur, s_hot, hot_vertex, pol, lane, sink);
-        else
-            gather_pass<(kBatch >= 12 ? 12 : kBatch), kSmemHot>(src, base, n, ccur, s_hot, hot_vertex, pol, lane,
-                                                                sink);
-    }
+    uint32_t base = 0;
+    for (; base + 32 * kBatch <= n; base += 32 * kBatch) gather_pass<kBatch, kSmemHot, true>(src, base, n, S, lane, acc);
+    if (base == n) return;
+    const uint32_t groups = (n - base + 127) / 128;  // 4-batch groups holding edges
+    if (groups == 1)
+        gather_pass<4, kSmemHot, false>(src, base, n, S, lane, acc);
+    else if (groups == 2)
+        gather_pass<8, kSmemHot, false>(src, base, n, S, lane, acc);
+    else
+        gather_pass<kBatch, kSmemHot, false>(src, base, n, S, lane, acc);
 }
 
 // Stop rule of iteration `it` (thread 0 of the last CTA, or the separate
@@ -259,32 +282,57 @@ __device__ __forceinline__ PRBuffers buffers(const PRArgs &a, uint32_t it) {
     return b;
 }
 
-// Chunk task `ci` (index into a.chunk_tasks): a kLongChunk-edge slice of a
-// long row.  The warp stores its compensated partial; the last arriving
-// warp of the row merges every partial in chunk order (lane j takes chunks
-// j, j+32, ...) and finalizes the row.  Returns the row's long-row index
-// when this warp finalized it (lane 0 holds res/dang), else ~0u.  Must be
-// called by all 32 lanes.
+// What a pull task works on: edges [e0, e0 + n); a tile's rows [a, b), or a
+// chunk's long-row index a and chunk number b.
+struct TaskSpan {
+    uint64_t e0;
+    uint32_t n, a, b;
+};
+
+__device__ __forceinline__ TaskSpan task_span(uint4 d) {
+    return TaskSpan{task_first_edge(d), task_edges(d), d.z, d.w};
+}
+
+// The same from the graph's tables, for callers that hold no descriptor.
+__device__ __forceinline__ TaskSpan chunk_span(const PRArgs &a, uint64_t ci) {
+    const uint2 t = a.chunk_tasks[ci];
+    const uint32_t row = a.long_rows[t.x].row;
+    const uint64_t lo = a.in_off[row] + uint64_t(t.y) * kLongChunk, re = a.in_off[row + 1];
+    return TaskSpan{lo, static_cast<uint32_t>((lo + kLongChunk < re ? lo + kLongChunk : re) - lo), t.x, t.y};
+}
+
+__device__ __forceinline__ TaskSpan tile_span(const PRArgs &a, uint64_t k) {
+    const uint32_t r0 = a.tile_start[k], r1 = a.tile_start[k + 1];
+    if (r0 == r1) return TaskSpan{0, 0, r0, r0};
+    const uint64_t last_b = a.in_off[r1 - 1], last_e = a.in_off[r1];
+    const bool chunked = last_e - last_b >= a.tile_cost;  // a long last row is chunked
+    const uint64_t e0 = a.in_off[r0];
+    return TaskSpan{e0, static_cast<uint32_t>((chunked ? last_b : last_e) - e0), r0, chunked ? r1 - 1 : r1};
+}
+
+// Chunk task: a kLongChunk-edge slice of a long row.  The warp stores its
+// compensated partial; the last arriving warp of the row merges every partial
+// in chunk order (lane j takes chunks j, j+32, ...) and finalizes the row.
+// Returns the row's long-row index when this warp finalized it (lane 0 holds
+// res/dang), else ~0u.  Must be called by all 32 lanes.
 template <bool kSmemHot>
 __device__ __forceinline__ uint32_t chunk_task(const PRArgs &a, const PRState &ps, const PRBuffers &b,
-                                               const uint32_t *in_src, const float *s_hot, uint64_t ci, uint64_t pol,
-                                               int lane, double &res, double &dang,
-                                               const uint4 *prefetch = nullptr) {
-    const uint2 t = a.chunk_tasks[ci];
-    const LongRow L = a.long_rows[t.x];
-    const uint64_t rb = a.in_off[L.row], re = a.in_off[L.row + 1];
-    const uint64_t lo = rb + uint64_t(t.y) * kLongChunk;
-    const uint64_t hi = (lo + kLongChunk < re) ? lo + kLongChunk : re;
-    dev::CSum acc;
-    gather_span<kSmemHot>(in_src, b.ccur, s_hot, a.hot_vertex, lo, hi, pol, lane,
-                          [&](uint32_t, float v) { acc.add(v); });
+                                               const uint32_t *in_src, const float *s_hot, const TaskSpan &t, int lane,
+                                               double &res, double &dang, const uint4 *prefetch = nullptr) {
+    dev::CSum2 acc2;
+    const LongRow L = a.long_rows[t.a];
     if (prefetch) prefetch_task(*prefetch, in_src, nullptr, lane);
-    acc = dev::warp_reduce(acc);
+    gather_span<kSmemHot>(in_src + t.e0, t.n, make_sources(a, b.ccur, s_hot), lane, acc2);
+    const dev::CSum acc = dev::warp_reduce(acc2.total());
+    if (L.num_chunks == 1) {  // the whole row: nothing to merge
+        if (lane == 0) finalize_row(a, ps, L.row, acc.value(), b.cur, b.nxt, b.cnxt, res, dang);
+        return t.a;
+    }
     uint32_t last = 0;
     if (lane == 0) {
-        a.partial[L.first_chunk + t.y] = make_float2(acc.s, acc.c);
+        a.partial[L.first_chunk + t.b] = make_float2(acc.s, acc.c);
         __threadfence();
-        const uint32_t tk = atomicAdd(&a.ticket[t.x], 1u) + 1u;
+        const uint32_t tk = atomicAdd(&a.ticket[t.a], 1u) + 1u;
         last = (tk % L.num_chunks == 0) ? 1u : 0u;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
@@ -300,73 +348,120 @@ __device__ __forceinline__ uint32_t chunk_task(const PRArgs &a, const PRState &p
     }
     row = dev::warp_reduce(row);
     if (lane == 0) finalize_row(a, ps, L.row, row.value(), b.cur, b.nxt, b.cnxt, res, dang);
-    return t.x;
+    return t.a;
 }
 
-// Tile task k: rows [tile_start[k], tile_start[k+1]) minus a long last row
-// (chunked).  The tile's contributions are gathered into the warp's
-// shared-memory slice sv, then summed lane-per-row (in-degree <
-// kWarpRowDegree) or warp-per-row, in edge order.  Must be called by all 32
-// lanes.
+// One group step of a tile's short rows: kG lanes per row, 32 / kG rows at a
+// time (the step's rows belong to lanes step * 32 / kG ... of the batch).
+// Lane l of a row takes edges lo + l, lo + l + kG, ..., up to kEdges of them,
+// all in flight (rows have at most kG * kEdges in-edges here); the group's compensated sums merge by shuffles.  Returns the
+// row's sum to the lane that owns it (other lanes keep `sum`).
+template <int kG, int kEdges, bool kSmemHot>
+__device__ __forceinline__ float group_step(const uint32_t *src, uint32_t lo, uint32_t hi, int step, const Sources &S,
+                                            int lane, float sum) {
+    constexpr int kRows = 32 / kG;   // rows of one step
+    const int owner = step * kRows + lane / kG;
+    const uint32_t b = __shfl_sync(0xffffffffu, lo, owner) + (lane % kG);
+    const uint32_t e = __shfl_sync(0xffffffffu, hi, owner);
+    uint32_t id[kEdges];
+#pragma unroll
+    for (int j = 0; j < kEdges; ++j) id[j] = (b + j * kG < e) ? dev::ld_stream(src + b + j * kG) : S.none;
+    uint32_t g[kEdges];
+#pragma unroll
+    for (int j = 0; j < kEdges; ++j) load_contribution<kSmemHot>(id[j], g[j], S);
+    dev::CSum2 acc2;
+    add_contributions<kEdges>(id, g, acc2);
+    dev::CSum acc = acc2.total();
+#pragma unroll
+    for (int o = 1; o < kG; o <<= 1) {
+        dev::CSum w;
+        w.s = __shfl_xor_sync(0xffffffffu, acc.s, o);
+        w.c = __shfl_xor_sync(0xffffffffu, acc.c, o);
+        acc.merge(w);
+    }
+    const float t = __shfl_sync(0xffffffffu, acc.value(), (lane % kRows) * kG);
+    return lane / kRows == step ? t : sum;
+}
+
+template <int kG, int kEdges, bool kSmemHot>
+__device__ __forceinline__ float group_rows(const uint32_t *src, uint32_t lo, uint32_t hi, const Sources &S, int lane) {
+    float sum = 0.0f;
+    for (int step = 0; step < kG; ++step) sum = group_step<kG, kEdges, kSmemHot>(src, lo, hi, step, S, lane, sum);
+    return sum;
+}
+
+// Tile task: rows [t.a, t.b), 32 at a time, one per lane: bounds, rank and
+// out-degree are loaded coalesced (the next batch's before this one's
+// gathers), in-edge sums are taken from registers, and every lane finalizes
+// its row.  Rows of kWarpRowDegree or more in-edges are summed by the whole
+// warp one after another; the others by groups of 1, 2, 4 or 8 lanes, the
+// smallest that leaves each lane at most 8 edges of the batch's largest row
+// (one round of loads per row; larger groups leave lanes idle, and 16 lanes
+// for rows of 64 to 127 ran 5 to 15 % slower than the warp on R-MAT scale
+// 24).  Must be called by all 32 lanes.
 // prefetch (optional): the warp's next pull task, whose edge lines are
-// warmed in L2 once this task's gathers are issued.
+// warmed in L2 (warming its rows' offsets and ranks too gained nothing).
 template <bool kSmemHot>
 __device__ __forceinline__ void tile_task(const PRArgs &a, const PRState &ps, const PRBuffers &b,
-                                          const uint32_t *in_src, const float *s_hot, float *sv, uint64_t k,
-                                          uint64_t pol, int lane, double &res, double &dang,
-                                          const uint4 *prefetch = nullptr) {
-    const uint32_t r0 = a.tile_start[k];
-    const uint32_t r1 = a.tile_start[k + 1];
-    if (r0 == r1) return;
-    const uint64_t last_b = a.in_off[r1 - 1], last_e = a.in_off[r1];
-    const uint32_t rl = (last_e - last_b >= a.tile_cost) ? r1 - 1 : r1;  // long last row is chunked
-    const uint64_t e0 = a.in_off[r0];
-    const uint64_t e1 = (rl == r1) ? last_e : last_b;
-    // the first 32 rows' bounds (relative to e0), ranks and out-degrees,
-    // loaded before the gathers so that they arrive with them
-    uint32_t lo_p = 0, hi_p = 0, od_p = 0;
-    float old_p = 0.0f;
-    if (r0 + lane < rl) {
-        lo_p = static_cast<uint32_t>(a.in_off[r0 + lane] - e0);
-        hi_p = static_cast<uint32_t>(a.in_off[r0 + lane + 1] - e0);
-        old_p = b.cur[r0 + lane];
-        od_p = a.out_deg[r0 + lane];
-    }
-    gather_span<kSmemHot>(in_src, b.ccur, s_hot, a.hot_vertex, e0, e1, pol, lane,
-                          [&](uint32_t i, float v) { sv[i] = v; });
+                                          const uint32_t *in_src, const float *s_hot, const TaskSpan &t, int lane,
+                                          double &res, double &dang, const uint4 *prefetch = nullptr) {
+    const uint32_t r0 = t.a, rl = t.b;
+    if (r0 == rl) return;
+    const uint64_t e0 = t.e0;
+    const uint32_t *src = in_src + e0;
+    const Sources S = make_sources(a, b.ccur, s_hot);
+    uint32_t lo = 0, hi = 0, od = 0;  // this lane's row: bounds relative to e0, out-degree, rank
+    float old = 0.0f;
+    auto load_row = [&](uint32_t r, uint32_t &l, uint32_t &h, uint32_t &d, float &o) {
+        l = h = d = 0;
+        o = 0.0f;
+        if (r < rl) {
+            l = static_cast<uint32_t>(a.in_off[r] - e0);
+            h = static_cast<uint32_t>(a.in_off[r + 1] - e0);
+            o = b.cur[r];
+            d = a.out_deg[r];
+        }
+    };
+    load_row(r0 + lane, lo, hi, od, old);
     if (prefetch) prefetch_task(*prefetch, in_src, nullptr, lane);
-    __syncwarp();
     for (uint32_t rb = r0; rb < rl; rb += 32) {
-        const uint32_t r = rb + lane;
-        const bool active = r < rl;
-        uint32_t lo = lo_p, hi = hi_p, od = od_p;
-        float old = old_p;
-        if (rb != r0) {
-            lo = active ? static_cast<uint32_t>(a.in_off[r] - e0) : 0u;
-            hi = active ? static_cast<uint32_t>(a.in_off[r + 1] - e0) : 0u;
-            old = active ? b.cur[r] : 0.0f;
-            od = active ? a.out_deg[r] : 0u;
-        }
-        if (active && hi - lo < kWarpRowDegree) {
-            dev::CSum acc;
-            for (uint32_t x = lo; x < hi; ++x) acc.add(sv[x]);
-            finalize_row_with(ps, r, acc.value(), old, od, b.nxt, b.cnxt, res, dang);
-        }
-        uint32_t big = __ballot_sync(0xffffffffu, active && (hi - lo >= kWarpRowDegree));
+        uint32_t lo_n, hi_n, od_n;
+        float old_n;
+        load_row(rb + 32 + lane, lo_n, hi_n, od_n, old_n);
+        const uint32_t deg = hi - lo;
+        const bool wide = deg >= kWarpRowDegree;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, wide ? 0u : deg);
+        const uint32_t hs = wide ? lo : hi;  // group steps see a wide row as empty
+        float sum = 0.0f;
+        if (most > 32)
+            sum = group_rows<8, 8, kSmemHot>(src, lo, hs, S, lane);
+        else if (most > 16)
+            sum = group_rows<4, 8, kSmemHot>(src, lo, hs, S, lane);
+        else if (most > 8)
+            sum = group_rows<2, 8, kSmemHot>(src, lo, hs, S, lane);
+        else if (most > 4)
+            sum = group_rows<1, 8, kSmemHot>(src, lo, hs, S, lane);
+        else if (most > 2)
+            sum = group_rows<1, 4, kSmemHot>(src, lo, hs, S, lane);
+        else if (most)
+            sum = group_rows<1, 2, kSmemHot>(src, lo, hs, S, lane);
+        uint32_t big = __ballot_sync(0xffffffffu, wide);
         while (big) {
-            const int src = __ffs(big) - 1;
+            const int w = __ffs(big) - 1;
             big &= big - 1;
-            const uint32_t bb = __shfl_sync(0xffffffffu, lo, src);
-            const uint32_t ee = __shfl_sync(0xffffffffu, hi, src);
-            const float o_src = __shfl_sync(0xffffffffu, old, src);
-            const uint32_t d_src = __shfl_sync(0xffffffffu, od, src);
-            dev::CSum acc;
-            for (uint32_t x = bb + lane; x < ee; x += 32) acc.add(sv[x]);
-            acc = dev::warp_reduce(acc);
-            if (lane == 0) finalize_row_with(ps, rb + src, acc.value(), o_src, d_src, b.nxt, b.cnxt, res, dang);
+            const uint32_t bb = __shfl_sync(0xffffffffu, lo, w);
+            const uint32_t ee = __shfl_sync(0xffffffffu, hi, w);
+            dev::CSum2 acc;
+            gather_span<kSmemHot>(src + bb, ee - bb, S, lane, acc);
+            const float t = dev::warp_reduce(acc.total()).value();
+            if (lane == w) sum = t;
         }
+        if (rb + lane < rl) finalize_row_with(ps, rb + lane, sum, old, od, b.nxt, b.cnxt, res, dang);
+        lo = lo_n;
+        hi = hi_n;
+        od = od_n;
+        old = old_n;
     }
-    __syncwarp();
 }
 
 }  // namespace prc

@@ -89,21 +89,20 @@ __global__ void __launch_bounds__(kPRThreads, 1) shard_pr_step_kernel(PRArgs a, 
     __shared__ double s_red[32];
 
     const PRState ps = make_state(a, t.dangling);
-    const uint64_t pol = dev::policy_evict_last();
     const uint64_t n_chunks = t.chunk_end - t.chunk_begin;
     const uint64_t total = n_chunks + (t.tile_end - t.tile_begin);
     double res = 0.0, dang = 0.0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *s_hot = s_dyn;
     for (uint32_t i = threadIdx.x; i < a.num_hot; i += kPRThreads) s_hot[i] = b.ccur[a.hot_vertex[i]];
+    if (threadIdx.x == 0) s_hot[a.num_hot] = 0.0f;  // "no edge"
     __syncthreads();
-    float *sv = s_dyn + a.num_hot + warp * (2 * a.tile_cost + 8);
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPRThreads / 32);
     for (uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp; task < total; task += nwarps) {
         if (task < n_chunks) {
-            chunk_task<true>(a, ps, b, a.in_src, s_hot, t.chunk_begin + task, pol, lane, res, dang);
+            chunk_task<true>(a, ps, b, a.in_src, s_hot, task_span(a.tasks[t.chunk_begin + task]), lane, res, dang);
         } else {
-            tile_task<true>(a, ps, b, a.in_src, s_hot, sv, t.tile_begin + (task - n_chunks), pol, lane, res, dang);
+            tile_task<true>(a, ps, b, a.in_src, s_hot, task_span(a.tasks[a.num_chunks + t.tile_begin + (task - n_chunks)]), lane, res, dang);
         }
     }
     const double bres = dev::block_sum(res, s_red);
@@ -653,6 +652,7 @@ void shard_pagerank_step(ShardImpl &sh, const hyt_shard_pagerank &p, uint32_t it
     a.tile_start = g.tile_start.get();
     a.long_rows = g.long_rows.get();
     a.chunk_tasks = g.chunk_tasks.get();
+    a.tasks = g.pull_tasks.get();
     a.hot_vertex = g.hot_vertex.get();
     a.num_hot = g.num_hot;
     a.tile_cost = g.tile_cost;
@@ -673,7 +673,7 @@ void shard_pagerank_step(ShardImpl &sh, const hyt_shard_pagerank &p, uint32_t it
     const ShardTasks t{sh.chunk_begin, sh.chunk_end, sh.tile_begin, sh.tile_end, dangling, p.sums};
     const uint64_t want = (tasks + kPRThreads / 32 - 1) / (kPRThreads / 32);
     const int grid = static_cast<int>(std::min<uint64_t>(shard_pr_grid(), want));
-    shard_pr_step_kernel<<<grid, kPRThreads, pr_shared_bytes(g.num_hot, g.tile_cost), s>>>(a, b, t);
+    shard_pr_step_kernel<<<grid, kPRThreads, pr_hot_bytes(g.num_hot), s>>>(a, b, t);
     HYT_CUDA(cudaGetLastError());
 }
 
