@@ -41,6 +41,7 @@
 #include "scratch.cuh"
 #include "solvers.cuh"
 #include "sssp_core.cuh"
+#include "sssp_pull.cuh"
 
 namespace hyt {
 
@@ -169,13 +170,13 @@ struct SSPull {
     const uint64_t *in_off;
     const uint32_t *in_src;
     const uint32_t *in_w;
-    const uint32_t *tile_start;
     const LongRow *long_rows;
-    const uint2 *chunk_tasks;
     const uint32_t *hot_vertex;
+    const uint4 *tasks;   // the graph's task descriptors: chunks, then tiles
+    uint64_t num_chunks;  // of the graph
     uint64_t chunk_begin, chunk_end, tile_begin, tile_end;
     uint64_t edges;  // in-edges of the sweep's rows
-    uint32_t num_hot, tile_cost;
+    uint32_t num_hot;
 };
 
 // Same answer in every kernel of a round and on every shard (the count is
@@ -304,106 +305,48 @@ __global__ void __launch_bounds__(256) shard_sssp_expand_kernel(SSShard a) {
     if (lane == 0 && relaxed) atomicAdd(&a.ctr[2], relaxed);
 }
 
-// Candidate labels d[u] + w of in-edges [lo, hi) (infinity from unreached
-// sources), 16 per lane in flight: ids and weights streamed, hot slots
-// mapped to vertex ids through the CTA's table, labels gathered from L2.
-constexpr int kShardPullBatch = 16;
-
-template <int WK, class Sink>
-__device__ __forceinline__ void shard_pull_span(const SSShard &a, const SSPull &p, const uint32_t *s_hot,
-                                                uint64_t lo, uint64_t hi, uint64_t pol, int lane, Sink &&sink) {
-    const uint32_t n = static_cast<uint32_t>(hi - lo);
-    for (uint32_t base = 0; base < n; base += 32 * kShardPullBatch) {
-        uint32_t id[kShardPullBatch], w[kShardPullBatch], du[kShardPullBatch];
-#pragma unroll
-        for (int k = 0; k < kShardPullBatch; ++k) {
-            const uint32_t i = base + 32 * k + lane;
-            id[k] = (i < n) ? dev::ld_stream(p.in_src + lo + i) : 0u;
-            w[k] = (i < n) ? ssc::edge_weight<WK>(p.in_w, lo + i) : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < kShardPullBatch; ++k)
-            if (id[k] & kHotTag) id[k] = s_hot[id[k] & ~kHotTag];
-#pragma unroll
-        for (int k = 0; k < kShardPullBatch; ++k)
-            du[k] = static_cast<uint32_t>(dev::ld_keep_u32(reinterpret_cast<const uint32_t *>(a.keys) + id[k], pol)) ^
-                    kKeyBias;
-#pragma unroll
-        for (int k = 0; k < kShardPullBatch; ++k) {
-            const uint32_t i = base + 32 * k + lane;
-            if (i < n) sink(i, du[k] == a.inf ? a.inf : ssc::extend<WK>(du[k], w[k]));
-        }
-    }
-}
-
 __device__ __forceinline__ void shard_pull_relax(const SSShard &a, uint32_t r, uint32_t c) {
     if (c < (static_cast<uint32_t>(__ldcg(a.keys + r)) ^ kKeyBias))
         atomicMin(a.keys + r, static_cast<int32_t>(c ^ kKeyBias));
 }
 
 // Pull round: every row of the shard's sweep range takes the minimum over
-// its in-edges of d[u] + w (the single-GPU sweep's task decomposition:
-// merge-path tiles of short rows staged per warp, long rows in chunks whose
-// minima meet in an atomic min).  Nothing in a push round.
+// its in-edges of d[u] + w (the single-GPU sweep's task decomposition and row
+// minima, sssp_pull.cuh; the chunks of a long row meet in an atomic min).
+// Nothing in a push round.
 template <int WK>
-__global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(SSShard a, SSPull p) {
-    extern __shared__ __align__(16) uint32_t s_pull[];
+__global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(const __grid_constant__ SSShard a,
+                                                                        const __grid_constant__ SSPull p) {
+    extern __shared__ __align__(16) uint32_t s_hot[];
     if (!shard_pull_round(a)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *s_hot = s_pull;
     for (uint32_t i = threadIdx.x; i < p.num_hot; i += blockDim.x) s_hot[i] = p.hot_vertex[i];
     __syncthreads();
-    uint32_t *sv = s_pull + p.num_hot + warp * (2 * p.tile_cost + 8);
     const uint64_t pol = dev::policy_evict_last();
+    const auto label = [&](uint32_t u) {
+        return dev::ld_keep_u32(reinterpret_cast<const uint32_t *>(a.keys) + u, pol) ^ kKeyBias;
+    };
     const uint64_t n_chunks = p.chunk_end - p.chunk_begin;
     const uint64_t total = n_chunks + (p.tile_end - p.tile_begin);
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPRThreads / 32);
     for (uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp; task < total; task += nwarps) {
+        const uint4 d = p.tasks[task < n_chunks ? p.chunk_begin + task : p.num_chunks + p.tile_begin + (task - n_chunks)];
+        const uint64_t e0 = task_first_edge(d);
+        const ssp::InEdges E{p.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : p.in_w + e0, s_hot};
         if (task < n_chunks) {
-            const uint2 t = p.chunk_tasks[p.chunk_begin + task];
-            const LongRow L = p.long_rows[t.x];
-            const uint64_t rb = p.in_off[L.row], re = p.in_off[L.row + 1];
-            const uint64_t lo = rb + uint64_t(t.y) * kLongChunk;
-            const uint64_t hi = (lo + kLongChunk < re) ? lo + kLongChunk : re;
-            uint32_t best = a.inf;
-            shard_pull_span<WK>(a, p, s_hot, lo, hi, pol, lane, [&](uint32_t, uint32_t c) { best = min(best, c); });
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane == 0) shard_pull_relax(a, L.row, best);
-        } else {
-            const uint64_t k = p.tile_begin + (task - n_chunks);
-            const uint32_t r0 = p.tile_start[k], r1 = p.tile_start[k + 1];
-            if (r0 == r1) continue;
-            const uint64_t last_b = p.in_off[r1 - 1], last_e = p.in_off[r1];
-            const uint32_t rl = (last_e - last_b >= p.tile_cost) ? r1 - 1 : r1;  // long last row is chunked
-            const uint64_t e0 = p.in_off[r0];
-            const uint64_t e1 = (rl == r1) ? last_e : last_b;
-            shard_pull_span<WK>(a, p, s_hot, e0, e1, pol, lane, [&](uint32_t i, uint32_t c) { sv[i] = c; });
-            __syncwarp();
-            for (uint32_t rb = r0; rb < rl; rb += 32) {
-                const uint32_t r = rb + lane;
-                const bool active = r < rl;
-                const uint64_t lo = active ? p.in_off[r] : 0;
-                const uint64_t hi = active ? p.in_off[r + 1] : 0;
-                if (active && hi - lo < 64) {
-                    uint32_t best = a.inf;
-                    for (uint64_t x = lo; x < hi; ++x) best = min(best, sv[x - e0]);
-                    shard_pull_relax(a, r, best);
-                }
-                uint32_t big = __ballot_sync(0xffffffffu, active && (hi - lo >= 64));
-                while (big) {
-                    const int src = __ffs(big) - 1;
-                    big &= big - 1;
-                    const uint64_t bb = __shfl_sync(0xffffffffu, lo, src);
-                    const uint64_t ee = __shfl_sync(0xffffffffu, hi, src);
-                    uint32_t best = a.inf;
-                    for (uint64_t x = bb + lane; x < ee; x += 32) best = min(best, sv[x - e0]);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-                    if (lane == 0) shard_pull_relax(a, rb + src, best);
-                }
+            const uint32_t best = ssp::span_min<WK>(E, 0, task_edges(d), a.inf, label, lane);
+            if (lane == 0) shard_pull_relax(a, p.long_rows[d.z].row, best);
+            continue;
+        }
+        for (uint32_t rb = d.z; rb < d.w; rb += 32) {
+            const uint32_t r = rb + lane;
+            uint32_t lo = 0, hi = 0;
+            if (r < d.w) {
+                lo = static_cast<uint32_t>(p.in_off[r] - e0);
+                hi = static_cast<uint32_t>(p.in_off[r + 1] - e0);
             }
-            __syncwarp();
+            const uint32_t best = ssp::rows_min<WK>(E, lo, hi, a.inf, label, lane);
+            if (r < d.w) shard_pull_relax(a, r, best);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.edges) atomicAdd(&a.ctr[2], static_cast<unsigned long long>(p.edges));
@@ -440,17 +383,16 @@ SSPull pull_view(const ShardImpl &sh) {
     p.in_off = g.in_offsets.get();
     p.in_src = g.in_sources.get();
     p.in_w = g.in_weights.get();
-    p.tile_start = g.tile_start.get();
     p.long_rows = g.long_rows.get();
-    p.chunk_tasks = g.chunk_tasks.get();
     p.hot_vertex = g.hot_vertex.get();
+    p.tasks = g.pull_tasks.get();
+    p.num_chunks = g.num_chunks;
     p.chunk_begin = sh.chunk_begin;
     p.chunk_end = sh.chunk_end;
     p.tile_begin = sh.tile_begin;
     p.tile_end = sh.tile_end;
     p.edges = sh.pull_edges;
     p.num_hot = g.num_hot;
-    p.tile_cost = g.tile_cost;
     return p;
 }
 
@@ -715,7 +657,7 @@ void launch_relax(const ShardImpl &sh, const SSShard &a, cudaStream_t s) {
     static const int full = pull_grid_for(reinterpret_cast<const void *>(shard_sssp_pull_kernel<WK>));
     const uint64_t want = (tasks + kPRThreads / 32 - 1) / (kPRThreads / 32);
     const int grid = static_cast<int>(std::min<uint64_t>(full, want));
-    shard_sssp_pull_kernel<WK><<<grid, kPRThreads, pr_shared_bytes(p.num_hot, p.tile_cost), s>>>(a, p);
+    shard_sssp_pull_kernel<WK><<<grid, kPRThreads, p.num_hot * sizeof(uint32_t), s>>>(a, p);
     HYT_CUDA(cudaGetLastError());
 }
 

@@ -23,17 +23,20 @@
 // a time, finding each edge's owner with a 5-step shuffle binary search.
 // Rows of >= kHubDegree edges become kHubChunk-edge warp tasks for a second
 // grid-wide kernel, so no warp owns more than ~2K edges of a round.  Each
-// lane keeps 4 edges in flight through loads and atomics (relax_batch).  A
+// lane keeps 16 edges in flight through loads and atomics (relax_batch).  A
 // vertex joins a frontier once per round (round stamp) and the far pile once
 // per phase (phase stamp), appended with one warp-aggregated atomic.
 //
 // With one bucket and a CSC, a round whose frontier carries more than
 // E / pull_div out-edges runs as a pull sweep over the CSC instead
-// (sssp_pull_kernel: 512-unit tiles, labels gathered 8 per lane in flight,
-// tile rows written with plain stores).  A sweep skips the rows whose label
+// (sssp_pull_kernel: rows take their minimum from registers, sssp_pull.cuh;
+// tile rows are written with plain stores).  Staging a tile's candidates in
+// 132 KB of shared memory left the label gathers too little L1 for their
+// outstanding misses; without it, and with the next frontier's out-edges and
+// lowest label summed by the kernels that fill it, a solve of R-MAT scale 24
+// went from 4.76 to 4.33 ms.  A sweep skips the rows whose label
 // is at most (lowest frontier label + smallest weight): no in-edge can
-// lower them, so their in-edges are neither read nor gathered (the round
-// close finds the frontier's lowest label).  All round state lives on the
+// lower them, so their in-edges are neither read nor gathered.  All round state lives on the
 // device; inside a CUDA graph the rounds run as a conditional while-loop
 // (expand, hub chunks, pull sweep, round close), instantiated once per
 // graph and launched again by later solves.
@@ -54,7 +57,7 @@
 #include "hybrid.cuh"
 #include "solvers.cuh"
 #include "sssp_core.cuh"
-#include "stage.cuh"
+#include "sssp_pull.cuh"
 
 namespace hyt {
 namespace {
@@ -74,7 +77,9 @@ __global__ void __launch_bounds__(kSSThreads) sssp_split_kernel(const SSArgs *__
 // HYB: the edges of a vertex's partition are reached through a.loc
 // (partitioned solves); compacted partitions are expanded from their packed
 // payload by sssp_expand_packed_kernel instead.
-template <int WK, bool HYB = false>
+// TRACK: pull-capable solves (the kernel also gathers the next frontier's
+// out-edges and lowest label).
+template <int WK, bool HYB = false, bool TRACK = false>
 __global__ void __launch_bounds__(kSSThreads) sssp_expand_kernel(const SSArgs *__restrict__ args) {
     const SSArgs a = *args;
     if (*(volatile uint32_t *)&a.hdr->done || pull_round(a)) return;
@@ -87,15 +92,18 @@ __global__ void __launch_bounds__(kSSThreads) sssp_expand_kernel(const SSArgs *_
         const uint32_t base = atomicAdd(&a.hdr->hub_count, nch);
         for (uint32_t c = 0; c < nch; ++c) a.hubs[base + c] = make_uint2(v, c);
     };
+    Gain gain;
     for (uint32_t w = gwarp; uint64_t(w) * 32 < rv.qn; w += nwarps)
-        expand_warp<WK, HYB, HYB ? kEdgeBatch : 16>(a, rv, w * 32, lane, kHubDegree, relaxed, improved, hub);
+        expand_warp<WK, HYB, HYB ? kEdgeBatch : 16, TRACK>(a, rv, w * 32, lane, kHubDegree, relaxed, improved, hub,
+                                                           &gain);
+    if constexpr (TRACK) flush_gain(a, gain, lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) relaxed += __shfl_xor_sync(0xffffffffu, relaxed, o);
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
 }
 
 // One warp per kHubChunk-edge slice of a long frontier row.
-template <int WK, bool HYB = false>
+template <int WK, bool HYB = false, bool TRACK = false>
 __global__ void __launch_bounds__(kSSThreads) sssp_hub_kernel(const SSArgs *__restrict__ args) {
     const SSArgs a = *args;
     if (*(volatile uint32_t *)&a.hdr->done || pull_round(a)) return;
@@ -105,6 +113,7 @@ __global__ void __launch_bounds__(kSSThreads) sssp_hub_kernel(const SSArgs *__re
     const uint32_t gwarp = (blockIdx.x * kSSThreads + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * kSSThreads) >> 5;
     unsigned long long improved = 0;
+    Gain gain;
     for (uint32_t t = gwarp; t < n; t += nwarps) {
         const uint2 h = a.hubs[t];
         const uint32_t *hc = a.cols, *hw = a.weights;
@@ -113,8 +122,9 @@ __global__ void __launch_bounds__(kSSThreads) sssp_hub_kernel(const SSArgs *__re
             hc = L.cols;
             hw = L.weights;
         }
-        hub_chunk<WK>(a, rv, hc, hw, h.x, h.y, lane, improved);
+        hub_chunk<WK, TRACK>(a, rv, hc, hw, h.x, h.y, lane, improved, &gain);
     }
+    if constexpr (TRACK) flush_gain(a, gain, lane);
 }
 
 // ---- pull sweeps (direction-optimised rounds) ------------------------------
@@ -131,13 +141,10 @@ struct PullGraph {
     const uint64_t *in_off;
     const uint32_t *in_src;   // hot sources tagged kHotTag | slot
     const uint32_t *in_w;     // weights in CSC order (NULL when unweighted)
-    const uint32_t *tile_start;
     const LongRow *long_rows;
-    const uint2 *chunk_tasks;
     const uint32_t *hot_vertex;
-    const uint4 *tasks;       // pull task descriptors (next-task prefetch, staged sweeps)
-    uint64_t num_tiles, num_chunks;
-    uint32_t tile_cost;
+    const uint4 *tasks;       // pull task descriptors: chunks of long rows, then tiles
+    uint64_t num_tasks, num_chunks;
     uint32_t num_hot;
 };
 
@@ -155,82 +162,15 @@ __device__ __forceinline__ bool pull_store(const SSArgs &a, const RoundView &rv,
     return true;
 }
 
-// Lowers row r's label to c if that improves it; returns true when r joins
-// the next frontier for the first time this round.
-__device__ __forceinline__ bool pull_relax(const SSArgs &a, const RoundView &rv, uint32_t r, uint32_t c) {
-    if (c >= __ldcg(a.dist + r)) return false;
-    const uint32_t old = atomicMin(a.dist + r, c);
-    if (c >= old) return false;
-    return atomicExch(a.stamp + r, rv.next_stamp) != rv.next_stamp;
+// Lowers row r's label to c; true when that improved it, `joined` when r
+// joins the next frontier for the first time this round.
+__device__ __forceinline__ bool pull_relax(const SSArgs &a, const RoundView &rv, uint32_t r, uint32_t c, bool &joined) {
+    if (c >= __ldcg(a.dist + r) || c >= atomicMin(a.dist + r, c)) return false;
+    joined = atomicExch(a.stamp + r, rv.next_stamp) != rv.next_stamp;
+    return true;
 }
 
-// Candidate labels d[u] + w of in-edges [lo, hi), kPullBatch per lane in
-// flight: all ids and weights, hot slots mapped to vertex ids through the
-// CTA's shared-memory table, all labels gathered evict-last from L2, then
-// the sink.  Unreached sources give infinity.
-#ifndef HYT_PULL_BATCH
-#define HYT_PULL_BATCH 8  // 16: register spills and 5 % slower sweeps at R-MAT scale 24
-#endif
-constexpr int kPullBatch = HYT_PULL_BATCH;
-
-// One pass of kK batches (edges lo + base + 32k + lane, k < kK).  With
-// kMask, edges whose bit is set in `skip` (bit i of word i / 32) belong to
-// skipped rows: they are neither read nor gathered.
-template <int kK, int WK, bool kMask, class Sink>
-__device__ __forceinline__ void pull_pass(const SSArgs &a, const PullGraph &pg, const uint32_t *s_hot, uint64_t lo,
-                                          uint32_t base, uint32_t n, uint64_t pol, int lane, const uint32_t *skip,
-                                          Sink &sink) {
-    // ids, then the label gathers, then the weights (streamed; issued after
-    // the gathers so that ids and weights are not live together)
-    uint32_t id[kK], w[kK], du[kK];
-    bool live[kK];
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        const uint32_t i = base + 32 * k + lane;
-        live[k] = i < n && !(kMask && ((skip[(base >> 5) + k] >> lane) & 1u));
-        id[k] = live[k] ? dev::ld_stream(pg.in_src + lo + i) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < kK; ++k)
-        if (id[k] & kHotTag) id[k] = s_hot[id[k] & ~kHotTag];  // hot slot -> vertex id
-#pragma unroll
-    for (int k = 0; k < kK; ++k) du[k] = (!kMask || live[k]) ? dev::ld_keep_u32(a.dist + id[k], pol) : a.inf;
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        const uint32_t i = base + 32 * k + lane;
-        w[k] = live[k] ? edge_weight<WK>(pg.in_w, lo + i) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-        const uint32_t i = base + 32 * k + lane;
-        if (live[k]) sink(i, du[k] == a.inf ? a.inf : extend<WK>(du[k], w[k]));
-    }
-}
-
-// The last, partial pass issues only the 4-batch groups that hold edges
-// (a warp-uniform choice); the edges and their order are the same.
-template <int WK, bool kMask, class Sink>
-__device__ __forceinline__ void pull_span(const SSArgs &a, const PullGraph &pg, const uint32_t *s_hot, uint64_t lo,
-                                          uint64_t hi, uint64_t pol, int lane, const uint32_t *skip, Sink &&sink) {
-    static_assert(kPullBatch % 4 == 0 && kPullBatch >= 4, "batches come in groups of 4");
-    const uint32_t n = static_cast<uint32_t>(hi - lo);
-    for (uint32_t base = 0; base < n; base += 32 * kPullBatch) {
-        const uint32_t groups = (n - base + 127) / 128;
-        if (groups >= kPullBatch / 4)
-            pull_pass<kPullBatch, WK, kMask>(a, pg, s_hot, lo, base, n, pol, lane, skip, sink);
-        else if (groups == 1)
-            pull_pass<4, WK, kMask>(a, pg, s_hot, lo, base, n, pol, lane, skip, sink);
-        else if (groups == 2)
-            pull_pass<8, WK, kMask>(a, pg, s_hot, lo, base, n, pol, lane, skip, sink);
-        else
-            pull_pass<(kPullBatch >= 12 ? 12 : kPullBatch), WK, kMask>(a, pg, s_hot, lo, base, n, pol, lane, skip, sink);
-    }
-}
-
-#ifndef HYT_PULL_THREADS
-#define HYT_PULL_THREADS 1024
-#endif
-constexpr int kPullThreads = HYT_PULL_THREADS;  // one CTA per SM, like the PageRank kernel
+constexpr int kPullThreads = 1024;  // one CTA per SM, like the PageRank kernel
 
 // Row skipping.  Let F be this round's frontier (every vertex whose label
 // dropped since its out-edges were last relaxed) and fmin its lowest label.
@@ -247,316 +187,107 @@ __device__ __forceinline__ uint32_t skip_bound(const SSArgs &a, bool &on) {
     return on ? extend<WK>(fmin, a.min_w) : 0u;
 }
 
-// Sets bits [lo, hi) of a warp's edge mask (shared-memory words).
-__device__ __forceinline__ void mask_range(uint32_t *mw, uint32_t lo, uint32_t hi) {
-    for (uint32_t x = lo; x < hi;) {
-        const uint32_t b = x & 31, cnt = min(32u - b, hi - x);
-        atomicOr(mw + (x >> 5), (cnt == 32 ? 0xFFFFFFFFu : ((1u << cnt) - 1u)) << b);
-        x += cnt;
-    }
-}
-
+// a: the solve's arguments as kernel parameters (the constant bank: no
+// registers held across the tasks).  Labels are read live, not from a
+// snapshot: rows lowered early in a sweep feed the rows after them (a
+// snapshot of the hottest labels in shared memory cost a round).
 template <int WK>
-__global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const SSArgs *__restrict__ args, PullGraph pg) {
-    extern __shared__ __align__(16) uint32_t s_dyn_u[];
-    const SSArgs a = *args;
+__global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid_constant__ SSArgs a,
+                                                                    const __grid_constant__ PullGraph pg) {
+    extern __shared__ __align__(16) uint32_t s_hot[];  // vertex ids of the hot slots (tagged sources in the CSC)
     if (*(volatile uint32_t *)&a.hdr->done || !pull_round(a)) return;
     const RoundView rv = round_view(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // vertex ids of the hot slots (tagged sources in the CSC)
-    uint32_t *s_hot = s_dyn_u;
     for (uint32_t i = threadIdx.x; i < pg.num_hot; i += blockDim.x) s_hot[i] = pg.hot_vertex[i];
     __syncthreads();
-    uint32_t *sv = s_dyn_u + pg.num_hot + warp * (2 * pg.tile_cost + 8);
     const uint64_t pol = dev::policy_evict_last();
-    const uint64_t total = pg.num_chunks + pg.num_tiles;
+    const auto label = [&](uint32_t u) { return dev::ld_keep_u32(a.dist + u, pol); };
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPullThreads / 32);
     const uint32_t *pf_w = (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w;
     bool skip_on;
     const uint32_t skip_at = skip_bound<WK>(a, skip_on);
-    unsigned long long relaxed = 0;  // in-edges this lane's warp relaxed (lane 0 counts tiles and chunks)
-    for (uint64_t task = uint64_t(blockIdx.x) * (kPullThreads / 32) + warp; task < total; task += nwarps) {
-        // the next task's descriptor now; its edge lines are warmed in L2
-        // once this task's gathers are issued
+    unsigned long long relaxed = 0;  // in-edges relaxed (chunks counted by lane 0, tile rows by their lanes)
+    Gain gain;
+    uint64_t task = uint64_t(blockIdx.x) * (kPullThreads / 32) + warp;
+    // each task's descriptor is read while the task before it runs
+    uint4 d = task < pg.num_tasks ? pg.tasks[task] : make_uint4(0, 0, 0, 0);
+    for (; task < pg.num_tasks; task += nwarps) {
         const uint64_t next = task + nwarps;
-        const uint4 nd = next < total ? pg.tasks[next] : make_uint4(0, 0, 0, 0);
-        if (task < pg.num_chunks) {
+        const uint4 nd = next < pg.num_tasks ? pg.tasks[next] : make_uint4(0, 0, 0, 0);
+        const uint64_t e0 = task_first_edge(d);
+        const ssp::InEdges E{pg.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w + e0, s_hot};
+        if (task_is_chunk(d)) {
             // slice of a long row: warp minimum, then one relaxation
-            const uint2 t = pg.chunk_tasks[task];
-            const LongRow L = pg.long_rows[t.x];
-            const uint64_t rb = pg.in_off[L.row], re = pg.in_off[L.row + 1];
-            const uint64_t lo = rb + uint64_t(t.y) * kLongChunk;
-            const uint64_t hi = (lo + kLongChunk < re) ? lo + kLongChunk : re;
-            if (skip_on && __shfl_sync(0xffffffffu, __ldcg(a.dist + L.row), 0) <= skip_at) continue;
-            if (lane == 0) relaxed += hi - lo;
-            uint32_t best = a.inf;
-            pull_span<WK, false>(a, pg, s_hot, lo, hi, pol, lane, nullptr,
-                                 [&](uint32_t, uint32_t c) { best = min(best, c); });
+            const uint32_t r = pg.long_rows[d.z].row, n = task_edges(d);
             prefetch_task(nd, pg.in_src, pf_w, lane);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane == 0 && pull_relax(a, rv, L.row, best)) append(rv.qnext, rv.qnext_size, L.row);
+            if (!(skip_on && __shfl_sync(0xffffffffu, __ldcg(a.dist + r), 0) <= skip_at)) {
+                const uint32_t best = ssp::span_min<WK>(E, 0, n, a.inf, label, lane);
+                if (lane == 0) {
+                    relaxed += n;
+                    if (best < a.inf) {
+                        bool joined = false;
+                        if (pull_relax(a, rv, r, best, joined)) gain.low = min(gain.low, best);
+                        if (joined) {
+                            gain.edges += a.out_deg[r];
+                            append(rv.qnext, rv.qnext_size, r);
+                        }
+                    }
+                }
+            }
         } else {
-            // merge-path tile of short rows: candidates staged per edge
-            const uint64_t k = task - pg.num_chunks;
-            const uint32_t r0 = pg.tile_start[k], r1 = pg.tile_start[k + 1];
-            if (r0 == r1) continue;
-            const uint64_t last_b = pg.in_off[r1 - 1], last_e = pg.in_off[r1];
-            const uint32_t rl = (last_e - last_b >= pg.tile_cost) ? r1 - 1 : r1;  // long last row is chunked
-            const uint64_t e0 = pg.in_off[r0];
-            const uint64_t e1 = (rl == r1) ? last_e : last_b;
-            // the first 32 rows' bounds (relative to e0) and labels, loaded
-            // before the gathers so that they arrive with them
-            uint32_t lo_p = 0, hi_p = 0, seen_p = 0;
-            if (r0 + lane < rl) {
-                lo_p = static_cast<uint32_t>(pg.in_off[r0 + lane] - e0);
-                hi_p = static_cast<uint32_t>(pg.in_off[r0 + lane + 1] - e0);
-                seen_p = __ldcg(a.dist + r0 + lane);
-            }
-            if (lane == 0) relaxed += e1 - e0;
-            // rows that cannot improve: their edges' bits in a mask kept at
-            // the end of the warp's slice, past the tile's candidates (no
-            // shared memory beyond the slice: more would shrink L1)
-            const uint32_t *skip = nullptr;
-            const uint32_t words = static_cast<uint32_t>((e1 - e0 + 31) >> 5);
-            if (skip_on && (e1 - e0) + words <= 2 * pg.tile_cost + 8) {
-                uint32_t *mw = sv + (2 * pg.tile_cost + 8) - words;
-                for (uint32_t x = lane; x < words; x += 32) mw[x] = 0u;
-                __syncwarp();
-                uint32_t any = 0;
-                for (uint32_t rb = r0; rb < rl; rb += 32) {
-                    const uint32_t r = rb + lane;
-                    uint32_t lo = lo_p, hi = hi_p, seen = seen_p;
-                    if (rb != r0 && r < rl) {
-                        lo = static_cast<uint32_t>(pg.in_off[r] - e0);
-                        hi = static_cast<uint32_t>(pg.in_off[r + 1] - e0);
-                        seen = __ldcg(a.dist + r);
-                    }
-                    const bool sk = r < rl && seen <= skip_at;
-                    any |= __ballot_sync(0xffffffffu, sk);
-                    if (sk) {
-                        relaxed -= hi - lo;
-                        mask_range(mw, lo, hi);
-                    }
+            // merge-path tile of short rows, 32 at a time, one per lane: the
+            // next batch's bounds and labels load before this one's gathers
+            const uint32_t rl = d.w;
+            uint32_t lo = 0, hi = 0, seen = 0;
+            auto load_row = [&](uint32_t r, uint32_t &l, uint32_t &h, uint32_t &sn) {
+                l = h = sn = 0;
+                if (r < rl) {
+                    l = static_cast<uint32_t>(pg.in_off[r] - e0);
+                    h = static_cast<uint32_t>(pg.in_off[r + 1] - e0);
+                    sn = __ldcg(a.dist + r);
                 }
-                __syncwarp();
-                if (any) skip = mw;
-            }
-            if (skip)
-                pull_span<WK, true>(a, pg, s_hot, e0, e1, pol, lane, skip, [&](uint32_t i, uint32_t c) { sv[i] = c; });
-            else
-                pull_span<WK, false>(a, pg, s_hot, e0, e1, pol, lane, nullptr,
-                                     [&](uint32_t i, uint32_t c) { sv[i] = c; });
+            };
+            load_row(d.z + lane, lo, hi, seen);
             prefetch_task(nd, pg.in_src, pf_w, lane);
-            __syncwarp();
-            for (uint32_t rb = r0; rb < rl; rb += 32) {
+            for (uint32_t rb = d.z; rb < rl; rb += 32) {
+                uint32_t lo_n, hi_n, seen_n;
+                load_row(rb + 32 + lane, lo_n, hi_n, seen_n);
                 const uint32_t r = rb + lane;
-                const bool active = r < rl;
-                uint32_t lo = lo_p, hi = hi_p, seen = seen_p;
-                if (rb != r0) {
-                    lo = active ? static_cast<uint32_t>(pg.in_off[r] - e0) : 0u;
-                    hi = active ? static_cast<uint32_t>(pg.in_off[r + 1] - e0) : 0u;
-                    seen = active ? __ldcg(a.dist + r) : 0u;
-                }
-                bool joined = false;
-                const bool live = active && !(skip && seen <= skip_at);  // skipped rows were not gathered
-                if (live && hi - lo < 64) {
-                    uint32_t best = a.inf;
-                    for (uint32_t x = lo; x < hi; ++x) best = min(best, sv[x]);
-                    joined = pull_store(a, rv, r, best, seen);
-                }
-                uint32_t big = __ballot_sync(0xffffffffu, live && (hi - lo >= 64));
-                while (big) {
-                    const int src = __ffs(big) - 1;
-                    big &= big - 1;
-                    const uint32_t bb = __shfl_sync(0xffffffffu, lo, src);
-                    const uint32_t ee = __shfl_sync(0xffffffffu, hi, src);
-                    const uint32_t sn = __shfl_sync(0xffffffffu, seen, src);
-                    uint32_t best = a.inf;
-                    for (uint32_t x = bb + lane; x < ee; x += 32) best = min(best, sv[x]);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-                    const bool j = (lane == 0) && pull_store(a, rv, rb + src, best, sn);
-                    if (__shfl_sync(0xffffffffu, j ? 1u : 0u, 0) && lane == src) joined = true;
+                if (skip_on && seen <= skip_at) hi = lo;  // no in-edge can lower it: neither read nor gathered
+                relaxed += hi - lo;
+                const uint32_t best = ssp::rows_min<WK>(E, lo, hi, a.inf, label, lane);
+                const bool joined = r < rl && pull_store(a, rv, r, best, seen);
+                if (joined) {
+                    gain.low = min(gain.low, best);
+                    gain.edges += a.out_deg[r];
                 }
                 const uint32_t vals[1] = {r};
                 warp_append<1>(rv.qnext, rv.qnext_size, vals, joined ? 1u : 0u, lane);
+                lo = lo_n;
+                hi = hi_n;
+                seen = seen_n;
             }
-            __syncwarp();
         }
+        d = nd;
     }
+    flush_gain(a, gain, lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) relaxed += __shfl_xor_sync(0xffffffffu, relaxed, o);
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.hdr->pull_rounds, 1u);
 }
 
-// ---- staged pull sweeps (CSC in HBM; pipeline in stage.cuh) ----------------
-
-// Candidate labels d[u] + w of staged edges [lo, hi) (ids at slot[x - a0]):
-// lane l takes edges lo + 32k + l; weights stream straight from HBM while
-// the label gathers are in flight.  sink(i, candidate) receives edge lo + i.
-template <int WK, class Sink>
-__device__ __forceinline__ void pull_staged(const SSArgs &a, const PullGraph &pg, const uint32_t *s_hot,
-                                            const uint32_t *slot, uint64_t a0, uint64_t lo, uint64_t hi, uint64_t pol,
-                                            int lane, Sink &&sink) {
-    constexpr int kB = stage::kUnitEdges / 32;
-    const uint32_t n = static_cast<uint32_t>(hi - lo);
-    const uint32_t *ids = slot + (lo - a0);
-    uint32_t w[kB], du[kB];
-#pragma unroll
-    for (int k = 0; k < kB; ++k) {
-        const uint32_t i = 32 * k + lane;
-        w[k] = (i < n) ? edge_weight<WK>(pg.in_w, lo + i) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < kB; ++k) {
-        const uint32_t i = 32 * k + lane;
-        uint32_t id = (i < n) ? ids[i] : 0u;
-        if (id & kHotTag) id = s_hot[id & ~kHotTag];  // hot slot -> vertex id
-        du[k] = dev::ld_keep_u32(a.dist + id, pol);
-    }
-#pragma unroll
-    for (int k = 0; k < kB; ++k) {
-        const uint32_t i = 32 * k + lane;
-        if (i < n) sink(i, du[k] == a.inf ? a.inf : extend<WK>(du[k], w[k]));
-    }
-}
-
-// pull_relax with the row's label read ahead of time: a stale (higher)
-// label only lets through an atomicMin that then finds no improvement.
-__device__ __forceinline__ bool pull_relax_seen(const SSArgs &a, const RoundView &rv, uint32_t r, uint32_t c,
-                                                uint32_t seen) {
-    if (c >= seen) return false;
-    const uint32_t old = atomicMin(a.dist + r, c);
-    if (c >= old) return false;
-    return atomicExch(a.stamp + r, rv.next_stamp) != rv.next_stamp;
-}
-
-template <int WK>
-__global__ void __launch_bounds__(stage::kStageThreads, 1) sssp_pull_staged_kernel(const SSArgs *__restrict__ args,
-                                                                                   PullGraph pg) {
-    extern __shared__ __align__(128) unsigned char s_stage[];
-    const SSArgs a = *args;
-    if (*(volatile uint32_t *)&a.hdr->done || !pull_round(a)) return;
-    const RoundView rv = round_view(a);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const stage::WarpStage ws = stage::warp_stage(s_stage, warp, lane);
-    uint32_t *s_hot = reinterpret_cast<uint32_t *>(s_stage + stage::kStageBytes);  // vertex ids of the hot slots
-    for (uint32_t i = threadIdx.x; i < pg.num_hot; i += blockDim.x) s_hot[i] = pg.hot_vertex[i];
-    __syncthreads();
-    const uint64_t pol = dev::policy_evict_last();
-    const uint64_t total = pg.num_chunks + pg.num_tiles;
-    const uint64_t nwarps = uint64_t(gridDim.x) * stage::kStageWarps;
-    uint32_t best = a.inf;  // running minimum of the current chunk
-    const bool ok = stage::stage_pipeline(
-        pg.tasks, pg.in_src, uint64_t(blockIdx.x) * stage::kStageWarps + warp, nwarps, total, ws,
-        lane, [&](uint4 d, uint64_t, uint32_t j, uint32_t nu, uint32_t *slot, uint64_t a0) {
-            if (task_is_chunk(d)) {
-                // slice of a long row: warp minimum, then one relaxation
-                const stage::Unit u = stage::unit_of(d, j);
-                if (j == 0) best = a.inf;
-                pull_staged<WK>(a, pg, s_hot, slot, a0, u.lo, u.hi, pol, lane,
-                                [&](uint32_t, uint32_t c) { best = min(best, c); });
-                if (j + 1 < nu) return;
-                uint32_t m = best;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-                if (lane == 0) {
-                    const uint32_t row = pg.long_rows[d.z].row;
-                    if (pull_relax(a, rv, row, m)) append(rv.qnext, rv.qnext_size, row);
-                }
-                return;
-            }
-            // merge-path tile of short rows: candidates replace the ids in
-            // the slot, then each row takes its minimum
-            const uint32_t r0 = d.z, rl = d.w;
-            const uint64_t e0 = task_first_edge(d), e1 = e0 + task_edges(d);
-            const uint32_t r = r0 + lane;
-            const bool act0 = r < rl;
-            const uint64_t lo0 = act0 ? pg.in_off[r] : 0, hi0 = act0 ? pg.in_off[r + 1] : 0;  // in flight
-            const uint32_t seen0 = act0 ? __ldcg(a.dist + r) : 0u;
-            pull_staged<WK>(a, pg, s_hot, slot, a0, e0, e1, pol, lane,
-                            [&](uint32_t i, uint32_t c) { slot[e0 - a0 + i] = c; });
-            __syncwarp();
-            for (uint32_t rb = r0; rb < rl; rb += 32) {
-                const uint32_t rr = rb + lane;
-                const bool active = rr < rl;
-                const bool first = rb == r0;
-                const uint64_t lo = first ? lo0 : (active ? pg.in_off[rr] : 0);
-                const uint64_t hi = first ? hi0 : (active ? pg.in_off[rr + 1] : 0);
-                bool joined = false;
-                if (active && hi - lo < 64) {
-                    uint32_t m = a.inf;
-                    for (uint64_t x = lo; x < hi; ++x) m = min(m, slot[x - a0]);
-                    joined = first ? pull_relax_seen(a, rv, rr, m, seen0) : pull_relax(a, rv, rr, m);
-                }
-                uint32_t big = __ballot_sync(0xffffffffu, active && (hi - lo >= 64));
-                while (big) {
-                    const int src = __ffs(big) - 1;
-                    big &= big - 1;
-                    const uint64_t bb = __shfl_sync(0xffffffffu, lo, src);
-                    const uint64_t ee = __shfl_sync(0xffffffffu, hi, src);
-                    uint32_t m = a.inf;
-                    for (uint64_t x = bb + lane; x < ee; x += 32) m = min(m, slot[x - a0]);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-                    const bool jn = (lane == 0) && pull_relax(a, rv, rb + src, m);
-                    if (__shfl_sync(0xffffffffu, jn ? 1u : 0u, 0) && lane == src) joined = true;
-                }
-                const uint32_t vals[1] = {rr};
-                warp_append<1>(rv.qnext, rv.qnext_size, vals, joined ? 1u : 0u, lane);
-            }
-        });
-    if (!ok) {
-        atomicExch(&a.hdr->error, 1u);
-        atomicExch(&a.hdr->done, 1u);
-        if (a.use_cond) cudaGraphSetConditional(a.cond, 0);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&a.hdr->relaxations, static_cast<unsigned long long>(a.num_edges));
-        atomicAdd(&a.hdr->pull_rounds, 1u);
-    }
-}
-
-// End of a round of a pull-capable solve, in one grid launch: the whole
-// grid sums the out-edges of the next frontier (the next round's push /
-// pull decision) and, with row skipping, finds its lowest label; then the
-// last block to finish runs the round-end logic.
-__global__ void __launch_bounds__(kSSThreads) sssp_round_close_kernel(const SSArgs *__restrict__ args) {
+// End of a round of a pull-capable solve (one thread): the round's kernels
+// have gathered the next frontier's out-edges (the next round's push / pull
+// decision) and its lowest label while they filled it; a pass over the
+// frontier for these took up to 0.1 ms a round on R-MAT scale 24.
+__global__ void sssp_round_close_kernel(const SSArgs *__restrict__ args) {
     const SSArgs a = *args;
     SSHeader *h = a.hdr;
-    if (*(volatile uint32_t *)&h->done) return;
-    const uint32_t r = *(volatile uint32_t *)&h->round;
-    const uint32_t qn = *(volatile uint32_t *)&h->qsize[(r + 1) & 1];
-    const uint32_t *q = ((r + 1) & 1) ? a.queue[1] : a.queue[0];
-    unsigned long long sum = 0;
-    uint32_t low = 0xFFFFFFFFu;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < qn; i += gridDim.x * blockDim.x) {
-        const uint32_t v = q[i];
-        sum += a.row_off[v + 1] - a.row_off[v];
-        if (a.skip_rows) low = min(low, __ldcg(a.dist + v));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&h->frontier_edges_next, sum);
-    if (a.skip_rows) {
-        low = __reduce_min_sync(0xffffffffu, low);
-        if ((threadIdx.x & 31) == 0 && low != 0xFFFFFFFFu) atomicMax(&h->fmin_inv, ~low);
-    }
-    __shared__ uint32_t s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&h->close_ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
-    }
-    __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
-    __threadfence();
-    const unsigned long long fe = atomicAdd(&h->frontier_edges_next, 0ull);
+    if (h->done) return;
+    const unsigned long long fe = h->frontier_edges_next;
     h->frontier_edges_next = 0;
-    h->close_ticket = 0;
-    h->fmin = ~atomicAdd(&h->fmin_inv, 0u);  // all ones when the next frontier is empty
+    h->fmin = ~h->fmin_inv;  // all ones when the next frontier is empty
     h->fmin_inv = 0;
     const bool finish = round_end(h);
     h->frontier_edges = fe;
@@ -736,29 +467,17 @@ uint32_t sssp_pull_div() {
 }
 
 template <int WK>
-int pull_grid(bool staged, unsigned smem) {
-    static bool attr = false;
-    if (!attr) {
+int pull_grid() {
+    static int grid = 0;
+    if (grid == 0) {
+        int per_sm = 0;
         HYT_CUDA(cudaFuncSetAttribute(sssp_pull_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaFuncSetAttribute(sssp_pull_staged_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPRSmemMax)));
-        attr = true;
+        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK>, kPullThreads,
+                                                               kPRSmemMax));
+        grid = sm_count() * std::max(per_sm, 1);
     }
-    int per_sm = 0;
-    if (staged)
-        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_staged_kernel<WK>,
-                                                               stage::kStageThreads, smem));
-    else
-        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK>, kPullThreads, smem));
-    return sm_count() * std::max(per_sm, 1);
-}
-
-// Staged pull sweeps when asked for (HYT_STAGED=1) and the graph's tiles
-// fit a staging slot.
-bool pull_use_staged(const GraphImpl &g) {
-    return stage::staged_requested() && g.tile_cost <= kStageTileMax && g.pull_tasks.get() &&
-           stage::staged_shared_bytes(g.num_hot) <= kPRSmemMax;
+    return grid;
 }
 
 template <int WK>
@@ -790,7 +509,8 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     SSArgs *d_args = reinterpret_cast<SSArgs *>(g.sssp_state.get());
     SSHeader *hdr = reinterpret_cast<SSHeader *>(g.sssp_state.get() + 256);
 
-    SSArgs a{};
+    SSArgs a;
+    std::memset(&a, 0, sizeof(a));  // compared bytewise below
     a.row_off = g.row_offsets.get();
     a.cols = g.cols.get();
     a.weights = g.weights.get();
@@ -811,34 +531,29 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     const bool pull_ok = (g.flags & HYT_GRAPH_PULL) && (WK == HYT_WEIGHTS_NONE || g.in_weights.get()) &&
                          delta == kNoDelta && g.E > 0;
     a.pull_div = pull_ok ? sssp_pull_div() : 0u;
-    PullGraph pg{};
+    PullGraph pg;
+    std::memset(&pg, 0, sizeof(pg));
     if (a.pull_div) {
         pg.in_off = g.in_offsets.get();
         pg.in_src = g.in_sources.get();
         pg.in_w = g.in_weights.get();
-        pg.tile_start = g.tile_start.get();
         pg.long_rows = g.long_rows.get();
-        pg.chunk_tasks = g.chunk_tasks.get();
         pg.hot_vertex = g.hot_vertex.get();
         pg.tasks = g.pull_tasks.get();
-        pg.num_tiles = g.num_tiles;
+        pg.num_tasks = g.num_chunks + g.num_tiles;
         pg.num_chunks = g.num_chunks;
-        pg.tile_cost = g.tile_cost;
         pg.num_hot = g.num_hot;
+        a.out_deg = g.out_degree.get();
     }
-    const bool staged = a.pull_div && pull_use_staged(g);
-    // row skipping (register-path sweeps): the smallest edge weight bounds
-    // what any in-edge adds
-    if (a.pull_div && !staged && sssp_pull_skip()) {
+    // row skipping: the smallest edge weight bounds what any in-edge adds
+    if (a.pull_div && sssp_pull_skip()) {
         a.skip_rows = 1;
         a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_min_in_weight(g, WK == HYT_WEIGHTS_F32, s);
     }
-    const unsigned pull_smem =
-        staged ? static_cast<unsigned>(stage::staged_shared_bytes(g.num_hot))
-               : static_cast<unsigned>((g.num_hot + kPullThreads / 32 * (2 * size_t(g.tile_cost) + 8)) * 4);
-    const int pgrid = a.pull_div ? pull_grid<WK>(staged, pull_smem) : 0;
-    const void *pull_fn = staged ? reinterpret_cast<const void *>(sssp_pull_staged_kernel<WK>)
-                                 : reinterpret_cast<const void *>(sssp_pull_kernel<WK>);
+    const unsigned pull_smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
+    const int pgrid = a.pull_div ? pull_grid<WK>() : 0;
+    SSArgs pa = a;  // the sweep's parameter copy: nothing that changes between solves
+    pa.source = 0;
 
     SSHeader h0{};
     h0.qsize[0] = 1;
@@ -849,12 +564,17 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
 
     const bool use_graph = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = expand_grid<WK>();
+    const void *expand_fn = a.pull_div ? reinterpret_cast<const void *>(sssp_expand_kernel<WK, false, true>)
+                                       : reinterpret_cast<const void *>(sssp_expand_kernel<WK>);
+    const void *hub_fn = a.pull_div ? reinterpret_cast<const void *>(sssp_hub_kernel<WK, false, true>)
+                                    : reinterpret_cast<const void *>(sssp_hub_kernel<WK>);
     // The round loop's shape; an instantiated loop of the same shape (kept
     // with the graph object) is launched again instead of being rebuilt.
     struct LoopKey {
         int wk, grid, pgrid;
-        uint32_t far_pile, pull_div, staged, pull_smem;
+        uint32_t far_pile, pull_div, pull_smem;
         const void *args;
+        SSArgs pa;
         PullGraph pg;
     } key;
     std::memset(&key, 0, sizeof(key));
@@ -863,9 +583,9 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     key.pgrid = pgrid;
     key.far_pile = far_pile;
     key.pull_div = a.pull_div;
-    key.staged = staged;
     key.pull_smem = pull_smem;
     key.args = d_args;
+    key.pa = pa;
     key.pg = pg;
     LoopGraph &loop = g.sssp_loop;
     const bool reuse = use_graph && loop.matches(&key, sizeof(key));
@@ -915,14 +635,14 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
                 HYT_CUDA(cudaGraphAddKernelNode(&node, body, prev ? &prev : nullptr, prev ? 1 : 0, &kp));
                 prev = node;
             };
-            void *pargs[] = {&d_args, &pg};
+            void *pargs[] = {&pa, &pg};
             // one bucket (no threshold): the far pile stays empty, nothing to split
             if (far_pile) add(reinterpret_cast<void *>(sssp_split_kernel), dim3(grid), dim3(kSSThreads), 0, kargs);
-            add(reinterpret_cast<void *>(sssp_expand_kernel<WK>), dim3(grid), dim3(kSSThreads), 0, kargs);
-            add(reinterpret_cast<void *>(sssp_hub_kernel<WK>), dim3(grid), dim3(kSSThreads), 0, kargs);
+            add(expand_fn, dim3(grid), dim3(kSSThreads), 0, kargs);
+            add(hub_fn, dim3(grid), dim3(kSSThreads), 0, kargs);
             if (a.pull_div) {
-                add(pull_fn, dim3(pgrid), dim3(staged ? stage::kStageThreads : kPullThreads), pull_smem, pargs);
-                add(reinterpret_cast<void *>(sssp_round_close_kernel), dim3(grid), dim3(kSSThreads), 0, kargs);
+                add(reinterpret_cast<void *>(sssp_pull_kernel<WK>), dim3(pgrid), dim3(kPullThreads), pull_smem, pargs);
+                add(reinterpret_cast<void *>(sssp_round_close_kernel), dim3(1), dim3(1), 0, kargs);
             } else {
                 add(reinterpret_cast<void *>(sssp_round_end_kernel), dim3(1), dim3(1), 0, kargs);
             }
@@ -935,16 +655,15 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         for (uint32_t r = 0; r < max_rounds; ++r) {
             if (flags & HYT_RUN_PROFILE) kt.start(s);
             if (far_pile) sssp_split_kernel<<<grid, kSSThreads, 0, s>>>(d_args);
-            sssp_expand_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
-            sssp_hub_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
             if (a.pull_div) {
-                if (staged)
-                    sssp_pull_staged_kernel<WK><<<pgrid, stage::kStageThreads, pull_smem, s>>>(d_args, pg);
-                else
-                    sssp_pull_kernel<WK><<<pgrid, kPullThreads, pull_smem, s>>>(d_args, pg);
+                sssp_expand_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
+                sssp_hub_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
+                sssp_pull_kernel<WK><<<pgrid, kPullThreads, pull_smem, s>>>(pa, pg);
+                sssp_round_close_kernel<<<1, 1, 0, s>>>(d_args);
+            } else {
+                sssp_expand_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
+                sssp_hub_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
             }
-            if (a.pull_div)
-                sssp_round_close_kernel<<<grid, kSSThreads, 0, s>>>(d_args);  // frontier-edge count + round end
             if (flags & HYT_RUN_PROFILE) kt.stop(s);
             if (!a.pull_div) sssp_round_end_kernel<<<1, 1, 0, s>>>(d_args);
             HYT_CUDA(cudaGetLastError());

@@ -77,6 +77,7 @@ struct SSArgs {
     uint32_t part_shift;  // partition of vertex v = v >> part_shift
     uint32_t pull_div;    // > 0: a round whose frontier has more than E / pull_div out-edges is a pull sweep
     uint64_t num_edges;
+    const uint32_t *out_deg;  // out-degrees (pull-capable solves: the next frontier's out-edges)
     uint32_t skip_rows;   // 1: pull sweeps skip rows whose label no in-edge can lower (needs fmin)
     uint32_t min_w;       // smallest edge weight (bit pattern; 1 when unweighted)
 };
@@ -165,15 +166,34 @@ __device__ __forceinline__ void warp_append(uint32_t *list, uint32_t *size, cons
         if ((mask >> k) & 1u) list[base + __popc(mask & ((1u << k) - 1u))] = vals[k];
 }
 
+// What a pull-capable solve needs to know of the next frontier, gathered by
+// the kernels that fill it: its out-edges and its lowest label.
+struct Gain {
+    unsigned long long edges = 0;
+    uint32_t low = 0xFFFFFFFFu;
+};
+
+// Adds a warp's share to the header; all 32 lanes.
+__device__ __forceinline__ void flush_gain(const SSArgs &a, Gain &g, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) g.edges += __shfl_xor_sync(0xffffffffu, g.edges, o);
+    g.low = __reduce_min_sync(0xffffffffu, g.low);
+    if (lane == 0) {
+        if (g.edges) atomicAdd(&a.hdr->frontier_edges_next, g.edges);
+        if (g.low != 0xFFFFFFFFu) atomicMax(&a.hdr->fmin_inv, ~g.low);
+    }
+}
+
 // Relaxes K candidate edges per lane with all atomics of a phase in flight
 // together: atomicMin on every improving label, then the stamp exchange of
 // every success, then one warp-aggregated append per list.  nd[k] >= du[k]
 // (including padding lanes, whose nd is the infinity label) is a no-op.
+// kTrack: the next frontier's out-edges and lowest label go to `gain`.
 // Must be called by all 32 lanes.
-template <int K>
+template <int K, bool kTrack = false>
 __device__ __forceinline__ void relax_batch(const SSArgs &a, const RoundView &rv, const uint32_t (&u)[K],
                                             const uint32_t (&nd)[K], const uint32_t (&du)[K], int lane,
-                                            unsigned long long &improved) {
+                                            unsigned long long &improved, Gain *gain = nullptr) {
     uint32_t old[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) old[k] = (nd[k] < du[k]) ? atomicMin(a.dist + u[k], nd[k]) : 0u;
@@ -197,6 +217,13 @@ __device__ __forceinline__ void relax_batch(const SSArgs &a, const RoundView &rv
             }
         }
     }
+    if constexpr (kTrack) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (nd[k] < old[k]) gain->low = min(gain->low, nd[k]);
+            if ((nmask >> k) & 1u) gain->edges += a.out_deg[u[k]];
+        }
+    }
     warp_append<K>(rv.qnext, rv.qnext_size, u, nmask, lane);
     warp_append<K>(rv.far, rv.far_size, u, fmask, lane);
 }
@@ -211,10 +238,10 @@ __device__ __forceinline__ void relax_batch(const SSArgs &a, const RoundView &rv
 // kB: 32-edge batches in flight.  The in-HBM solver's expansion takes 16;
 // the batch engine's and the out-of-HBM expansion keep kEdgeBatch (with 16
 // their kernels spill registers).
-template <int WK, bool HYB, int kB = kEdgeBatch, class HubSink>
+template <int WK, bool HYB, int kB = kEdgeBatch, bool kTrack = false, class HubSink>
 __device__ __forceinline__ void expand_warp(const SSArgs &a, const RoundView &rv, uint32_t i0, int lane,
                                             uint32_t hub_degree, unsigned long long &relaxed,
-                                            unsigned long long &improved, HubSink &&hub) {
+                                            unsigned long long &improved, HubSink &&hub, Gain *gain = nullptr) {
     const uint32_t i = i0 + lane;
     uint32_t deg = 0, d = a.inf;
     uint64_t off = 0;
@@ -278,16 +305,16 @@ __device__ __forceinline__ void expand_warp(const SSArgs &a, const RoundView &rv
         }
 #pragma unroll
         for (int k = 0; k < kB; ++k) du[k] = __ldcg(a.dist + u[k]);
-        relax_batch<kB>(a, rv, u, nd, du, lane, improved);
+        relax_batch<kB, kTrack>(a, rv, u, nd, du, lane, improved, gain);
     }
 }
 
 // One kHubChunk-edge slice (chunk c) of frontier row v, edges read from
 // hc / hw (global-edge-indexed).  Must be called by all 32 lanes.
-template <int WK>
+template <int WK, bool kTrack = false>
 __device__ __forceinline__ void hub_chunk(const SSArgs &a, const RoundView &rv, const uint32_t *hc,
                                           const uint32_t *hw, uint32_t v, uint32_t c, int lane,
-                                          unsigned long long &improved) {
+                                          unsigned long long &improved, Gain *gain = nullptr) {
     const uint64_t rb = a.row_off[v], re = a.row_off[v + 1];
     const uint64_t b = rb + uint64_t(c) * kHubChunk;
     const uint32_t len = static_cast<uint32_t>(((b + kHubChunk < re) ? b + kHubChunk : re) - b);
@@ -306,7 +333,7 @@ __device__ __forceinline__ void hub_chunk(const SSArgs &a, const RoundView &rv, 
         }
 #pragma unroll
         for (int k = 0; k < kHubBatch; ++k) du[k] = __ldcg(a.dist + u[k]);
-        relax_batch<kHubBatch>(a, rv, u, nd, du, lane, improved);
+        relax_batch<kHubBatch, kTrack>(a, rv, u, nd, du, lane, improved, gain);
     }
 }
 
