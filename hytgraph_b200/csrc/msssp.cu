@@ -17,11 +17,16 @@
 //   pull sweep -- when the frontier's out-edges exceed E / 4, every row
 //                 takes, per lane, the minimum of d[u] + w over its
 //                 in-edges: one id and one 32-byte label row per in-edge
-//                 for all lanes, 4 label rows in flight per thread; ids
-//                 read in place on the default 512-unit tiles, or staged
-//                 by bulk copies (stage.cuh) on 256-unit tiles
-//                 (HYT_STAGED=1).  Tile rows are written with plain stores
-//                 (one writer per row during a sweep).
+//                 for all lanes, 1 to 32 edges of a row side by side, 4
+//                 label rows in flight per thread.  A row is skipped when no in-edge can
+//                 lower it in any lane: its label is at most (lowest label
+//                 of the frontier in that lane + smallest weight).  Tile
+//                 rows are written with plain stores (one writer per row
+//                 during a sweep).
+// A sweep used to walk short rows one lane per row and extend labels with
+// saturation: 8 sources on R-MAT scale 20 / 24 took 1.98 / 8.74 ms, now 1.69 /
+// 7.81 ms (768 threads: 1024 spill, 1.78 ms; 8 rows in flight in 512 threads
+// 1.72 ms; 2 rows 1.71 ms).
 // Per edge the memory traffic is about that of one single-source
 // relaxation, whatever the number of lanes; the rounds are those of the
 // deepest source.  Rounds run as a CUDA-graph conditional while-loop.
@@ -29,13 +34,11 @@
 #include <cstring>
 #include <vector>
 
-#include "bulk.cuh"
 #include "common.cuh"
 #include "graph.cuh"
 #include "scratch.cuh"
 #include "solvers.cuh"
 #include "sssp_core.cuh"
-#include "stage.cuh"
 
 namespace hyt {
 namespace {
@@ -46,18 +49,20 @@ using ssc::kHubDegree;
 
 constexpr int kML = 8;             // labels per vertex row (32 bytes)
 constexpr int kMSThreads = 256;    // push kernels
-constexpr int kMPThreads = stage::kStageThreads;   // pull sweep (one CTA per SM)
+constexpr int kMPThreads = 768;    // pull sweep (one CTA per SM; 85 registers a thread)
 
 struct MSHeader {
-    uint32_t round, done, converged, error;
+    uint32_t round, done, converged, pad0;
     uint32_t qsize[2];
     uint32_t hub_count;
     uint32_t max_rounds;
-    unsigned long long relaxations;     // push: frontier out-edges; pull: E per sweep
+    unsigned long long relaxations;     // push: frontier out-edges; pull: in-edges of the rows not skipped
     unsigned long long frontier_total;  // frontier vertices expanded
     unsigned long long frontier_edges;  // out-edges of this round's frontier
-    uint32_t pull_rounds, close_ticket;  // close_ticket: blocks of the round-close kernel finished
-    unsigned long long frontier_edges_next;  // out-edges of the next frontier, summed at round close
+    uint32_t pull_rounds, pad;
+    unsigned long long frontier_edges_next;  // out-edges of the next frontier, summed by the kernels that fill it
+    uint32_t fmin[kML];      // lowest label of this round's frontier, per lane
+    uint32_t fmin_inv[kML];  // ~(lowest label of the next frontier)
 };
 
 struct MSArgs {
@@ -74,38 +79,55 @@ struct MSArgs {
     uint32_t pull_div;
     uint64_t num_edges;
     uint32_t sources[kML];
-    // pull side (CSC, weights in CSC order, staged task list)
+    // pull side (CSC, weights in CSC order, task list)
     const uint64_t *in_off;
     const uint32_t *in_src;
     const uint32_t *in_w;
     const uint32_t *hot_vertex;
     const LongRow *long_rows;
     const uint4 *tasks;
+    const uint32_t *out_deg;
     uint64_t num_tasks;
     uint32_t num_hot;
+    uint32_t skip_rows;  // 1: sweeps skip rows whose labels no in-edge can lower
+    uint32_t min_w;      // smallest edge weight (bit pattern; 1 when unweighted)
 };
 
 struct Row8 {
     uint32_t d[kML];
 };
 
+// Arithmetic of a solve's labels.  kBounded: no shortest path of the graph
+// can reach a.inf ((V - 1) * largest weight < a.inf) and a.inf + any weight
+// does not wrap, so a label is extended by one add, and an unreached source's
+// candidate stays at or above a.inf and never lowers anything.  Otherwise
+// labels saturate (extend) and unreached sources are tested for.  With 8
+// labels per edge the difference is a third of a sweep's instructions.
+template <int WK, bool kBounded>
+__device__ __forceinline__ uint32_t candidate(uint32_t d, uint32_t w, uint32_t inf) {
+    if constexpr (WK == HYT_WEIGHTS_F32) {
+        return extend<WK>(d, w);  // infinity stays infinity
+    } else if constexpr (kBounded) {
+        return d + w;
+    } else {
+        return d == inf ? inf : extend<WK>(d, w);
+    }
+}
+
+// min(m, candidate(d, w)).
+template <int WK, bool kBounded>
+__device__ __forceinline__ uint32_t lower_by(uint32_t m, uint32_t d, uint32_t w, uint32_t inf) {
+    if constexpr (kBounded && WK != HYT_WEIGHTS_F32) {
+        return __viaddmin_u32(d, w, m);  // one instruction
+    } else {
+        return min(m, candidate<WK, kBounded>(d, w, inf));
+    }
+}
+
 __device__ __forceinline__ Row8 load_row(const uint32_t *dist, uint32_t v) {
     const uint4 *p = reinterpret_cast<const uint4 *>(dist + size_t(v) * kML);
     const uint4 a = __ldcg(p), b = __ldcg(p + 1);
     return Row8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
-}
-
-// Label row read through L2 with an evict-last policy (pull gathers).
-__device__ __forceinline__ Row8 load_row_keep(const uint32_t *dist, uint32_t v, uint64_t pol) {
-    const uint32_t *p = dist + size_t(v) * kML;
-    Row8 r;
-    asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(r.d[0]), "=r"(r.d[1]), "=r"(r.d[2]), "=r"(r.d[3])
-                 : "l"(p), "l"(pol));
-    asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(r.d[4]), "=r"(r.d[5]), "=r"(r.d[6]), "=r"(r.d[7])
-                 : "l"(p + 4), "l"(pol));
-    return r;
 }
 
 __device__ __forceinline__ bool pull_round(const MSArgs &a) {
@@ -132,19 +154,47 @@ __device__ __forceinline__ View view(const MSArgs &a) {
     return w;
 }
 
-// Relaxes edge (u -> v, weight w) in every lane with u's labels du; true
-// when some lane of v improved and v joins the next frontier now.
-template <int WK>
-__device__ __forceinline__ bool relax_row(const MSArgs &a, const View &w, const Row8 &du, uint32_t v, uint32_t wt) {
-    const Row8 dv = load_row(a.dist, v);
-    bool improved = false;
+// What the next round needs to know of its frontier, gathered while it is
+// filled: its out-edges and, in lane l < kML of the warp, the lowest label of
+// lane l.
+struct Gain {
+    unsigned long long edges = 0;
+    uint32_t low = 0xFFFFFFFFu;
+};
+
+// Notes the labels `now` of the lanes in `lower` (a bit mask, 0 in threads
+// that lowered none); all 32 lanes.
+__device__ __forceinline__ void note_lower(Gain &g, const Row8 &now, uint32_t lower, int lane) {
+    uint32_t any = __reduce_or_sync(0xffffffffu, lower);
 #pragma unroll
     for (int l = 0; l < kML; ++l) {
-        if (l >= static_cast<int>(a.k) || du.d[l] == a.inf) continue;
-        const uint32_t c = extend<WK>(du.d[l], wt);
-        if (c < dv.d[l]) improved |= c < atomicMin(a.dist + size_t(v) * kML + l, c);
+        if (!((any >> l) & 1u)) continue;
+        const uint32_t t = __reduce_min_sync(0xffffffffu, ((lower >> l) & 1u) ? now.d[l] : 0xFFFFFFFFu);
+        if (lane == l) g.low = min(g.low, t);
     }
-    return improved && atomicExch(a.stamp + v, w.next_stamp) != w.next_stamp;
+}
+
+__device__ __forceinline__ void flush_gain(const MSArgs &a, Gain &g, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) g.edges += __shfl_xor_sync(0xffffffffu, g.edges, o);
+    if (lane == 0 && g.edges) atomicAdd(&a.hdr->frontier_edges_next, g.edges);
+    if (lane < kML && g.low != 0xFFFFFFFFu) atomicMax(&a.hdr->fmin_inv[lane], ~g.low);
+}
+
+// Relaxes edge (u -> v, weight w) in every lane with u's labels du; true
+// when some lane of v improved and v joins the next frontier now.  c gets the
+// candidates, `lower` the lanes that improved.
+template <int WK, bool kB>
+__device__ __forceinline__ bool relax_row(const MSArgs &a, const View &w, const Row8 &du, uint32_t v, uint32_t wt,
+                                          Row8 &c, uint32_t &lower) {
+    const Row8 dv = load_row(a.dist, v);
+#pragma unroll
+    for (int l = 0; l < kML; ++l) {
+        if (l >= static_cast<int>(a.k)) continue;
+        c.d[l] = candidate<WK, kB>(du.d[l], wt, a.inf);
+        if (c.d[l] < dv.d[l] && c.d[l] < atomicMin(a.dist + size_t(v) * kML + l, c.d[l])) lower |= 1u << l;
+    }
+    return lower && atomicExch(a.stamp + v, w.next_stamp) != w.next_stamp;
 }
 
 __global__ void ms_init_kernel(const MSArgs *__restrict__ args) {
@@ -179,7 +229,7 @@ __global__ void ms_sources_kernel(const MSArgs *__restrict__ args) {
 // kHubDegree are walked as one combined edge list (each lane finds its
 // edge's owner by a shuffle binary search and receives the owner's label
 // row by shuffles), longer rows become hub tasks.
-template <int WK>
+template <int WK, bool kB>
 __global__ void __launch_bounds__(kMSThreads) ms_expand_kernel(const MSArgs *__restrict__ args) {
     const MSArgs a = *args;
     if (*(volatile uint32_t *)&a.hdr->done || pull_round(a)) return;
@@ -188,6 +238,7 @@ __global__ void __launch_bounds__(kMSThreads) ms_expand_kernel(const MSArgs *__r
     const uint32_t gwarp = (blockIdx.x * kMSThreads + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * kMSThreads) >> 5;
     unsigned long long relaxed = 0;
+    Gain gain;
     for (uint32_t base0 = gwarp * 32; base0 < w.qn; base0 += nwarps * 32) {
         const uint32_t i = base0 + lane;
         uint32_t deg = 0, u = 0;
@@ -231,23 +282,29 @@ __global__ void __launch_bounds__(kMSThreads) ms_expand_kernel(const MSArgs *__r
 #pragma unroll
             for (int l = 0; l < kML; ++l) ou.d[l] = __shfl_sync(0xffffffffu, du.d[l], lo);
             bool join = false;
-            uint32_t v = 0;
+            uint32_t v = 0, lower = 0;
+            Row8 c{};
             if (j < total) {
                 const uint64_t e = o_off + (j - (o_incl - o_deg));
                 v = dev::ld_stream(a.cols + e);
-                join = relax_row<WK>(a, w, ou, v, ssc::edge_weight<WK>(a.weights, e));
+                join = relax_row<WK, kB>(a, w, ou, v, ssc::edge_weight<WK>(a.weights, e), c, lower);
+            }
+            if (a.pull_div) {
+                note_lower(gain, c, lower, lane);
+                if (join) gain.edges += a.out_deg[v];
             }
             const uint32_t vals[1] = {v};
             ssc::warp_append<1>(w.qnext, w.qnext_size, vals, join ? 1u : 0u, lane);
         }
     }
+    if (a.pull_div) flush_gain(a, gain, lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) relaxed += __shfl_xor_sync(0xffffffffu, relaxed, o);
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
 }
 
 // One warp per kHubChunk-edge slice of a long frontier row.
-template <int WK>
+template <int WK, bool kB>
 __global__ void __launch_bounds__(kMSThreads) ms_hub_kernel(const MSArgs *__restrict__ args) {
     const MSArgs a = *args;
     if (*(volatile uint32_t *)&a.hdr->done || pull_round(a)) return;
@@ -256,6 +313,7 @@ __global__ void __launch_bounds__(kMSThreads) ms_hub_kernel(const MSArgs *__rest
     const int lane = threadIdx.x & 31;
     const uint32_t gwarp = (blockIdx.x * kMSThreads + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * kMSThreads) >> 5;
+    Gain gain;
     for (uint32_t t = gwarp; t < n; t += nwarps) {
         const uint2 h = a.hubs[t];
         const uint64_t rb = a.row_off[h.x], re = a.row_off[h.x + 1];
@@ -264,180 +322,242 @@ __global__ void __launch_bounds__(kMSThreads) ms_hub_kernel(const MSArgs *__rest
         const Row8 du = load_row(a.dist, h.x);
         for (uint32_t x = 0; x < len; x += 32) {
             bool join = false;
-            uint32_t v = 0;
+            uint32_t v = 0, lower = 0;
+            Row8 c{};
             if (x + lane < len) {
                 const uint64_t e = b + x + lane;
                 v = dev::ld_stream(a.cols + e);
-                join = relax_row<WK>(a, w, du, v, ssc::edge_weight<WK>(a.weights, e));
+                join = relax_row<WK, kB>(a, w, du, v, ssc::edge_weight<WK>(a.weights, e), c, lower);
+            }
+            if (a.pull_div) {
+                note_lower(gain, c, lower, lane);
+                if (join) gain.edges += a.out_deg[v];
             }
             const uint32_t vals[1] = {v};
             ssc::warp_append<1>(w.qnext, w.qnext_size, vals, join ? 1u : 0u, lane);
         }
     }
+    if (a.pull_div) flush_gain(a, gain, lane);
 }
 
-// Tile row r: lowers its labels to m where that improves them, with plain
-// stores -- a tile row has exactly one writer during a sweep (the warp that
-// owns its tile) and no push runs beside a sweep; true when r joins the
-// next frontier.
-__device__ __forceinline__ bool pull_store_row(const MSArgs &a, const View &w, uint32_t r, const Row8 &m) {
-    const Row8 cur = load_row(a.dist, r);
-    Row8 nx;
-    bool improved = false;
+// ---- pull sweeps ------------------------------------------------------------
+//
+// Labels are read live (not snapshotted): rows lowered earlier in the same
+// sweep -- the hub rows, whose chunks come first -- feed the rows after them.
+// A minimum does not mind an edge taken twice, so threads without an edge of
+// their own repeat their row's last one (the same sector) in place of
+// predicated loads; a sweep is bound by instructions: 8 labels to extend per
+// edge.
+
+constexpr int kPullN = 4;                  // edges in flight per thread
+constexpr uint32_t kWideRow = 16 * kPullN;  // rows with this many in-edges are taken by the whole warp
+
+// In-edges of one task, addressed relative to its first edge.
+struct InEdges {
+    const uint32_t *src, *w, *s_hot;
+    const uint32_t *dist;
+    uint32_t inf;
+};
+
+// Minimum of the candidates of edges b, b + step, ..., capped at edge `last`
+// (kPullN of them, all loaded before the first is used) into m.
+template <int WK, bool kB>
+__device__ __forceinline__ void edges_min(const InEdges &E, uint32_t b, uint32_t last, uint32_t step, Row8 &m) {
+    uint32_t u[kPullN], wt[kPullN];
 #pragma unroll
-    for (int l = 0; l < kML; ++l) {
-        const bool lower = l < static_cast<int>(a.k) && m.d[l] < cur.d[l];
-        nx.d[l] = lower ? m.d[l] : cur.d[l];
-        improved |= lower;
+    for (int j = 0; j < kPullN; ++j) u[j] = dev::ld_stream(E.src + min(b + j * step, last));
+#pragma unroll
+    for (int j = 0; j < kPullN; ++j) wt[j] = ssc::edge_weight<WK>(E.w, min(b + j * step, last));
+#pragma unroll
+    for (int j = 0; j < kPullN; ++j)
+        if (u[j] & kHotTag) u[j] = E.s_hot[u[j] & ~kHotTag];
+    Row8 du[kPullN];
+#pragma unroll
+    for (int j = 0; j < kPullN; ++j) {
+        // the whole 32-byte row in one load: one L1 access per edge (two
+        // 16-byte loads took the sector twice)
+        asm volatile("ld.global.L2::evict_last.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(du[j].d[0]), "=r"(du[j].d[1]), "=r"(du[j].d[2]), "=r"(du[j].d[3]), "=r"(du[j].d[4]),
+                       "=r"(du[j].d[5]), "=r"(du[j].d[6]), "=r"(du[j].d[7])
+                     : "l"(E.dist + size_t(u[j]) * kML));
     }
-    if (!improved) return false;
-    uint4 *p = reinterpret_cast<uint4 *>(a.dist + size_t(r) * kML);
-    p[0] = make_uint4(nx.d[0], nx.d[1], nx.d[2], nx.d[3]);
-    p[1] = make_uint4(nx.d[4], nx.d[5], nx.d[6], nx.d[7]);
-    a.stamp[r] = w.next_stamp;
-    return true;
+#pragma unroll
+    for (int j = 0; j < kPullN; ++j)
+#pragma unroll
+        for (int l = 0; l < kML; ++l) m.d[l] = lower_by<WK, kB>(m.d[l], du[j].d[l], wt[j], E.inf);
+}
+
+// Lowest candidates over edges [b, e), b < e, by the whole warp; every lane
+// returns them.
+template <int WK, bool kB>
+__device__ __forceinline__ Row8 span_min(const InEdges &E, uint32_t b, uint32_t e, int lane) {
+    Row8 m;
+#pragma unroll
+    for (int l = 0; l < kML; ++l) m.d[l] = E.inf;
+    for (uint32_t at = b; at < e; at += 32 * kPullN) edges_min<WK, kB>(E, at + lane, e - 1, 32, m);
+#pragma unroll
+    for (int l = 0; l < kML; ++l) m.d[l] = __reduce_min_sync(0xffffffffu, m.d[l]);
+    return m;
+}
+
+// Lowest candidates of the warp's 32 rows (lane l: edges [lo, hi)), `slots`
+// edges of a row side by side, 32 / slots rows a step; rows have at most
+// slots * kPullN in-edges.  Rows without edges get an arbitrary result.
+template <int WK, bool kB>
+__device__ __forceinline__ Row8 group_min(const InEdges &E, uint32_t lo, uint32_t hi, int slots, int lane) {
+    const int rows = 32 / slots;
+    const uint32_t live = __ballot_sync(0xffffffffu, hi > lo);
+    Row8 mine;
+#pragma unroll
+    for (int l = 0; l < kML; ++l) mine.d[l] = E.inf;
+    for (int first = 0; first < 32; first += rows) {
+        if (!((live >> first) & (rows == 32 ? 0xFFFFFFFFu : (1u << rows) - 1u))) continue;
+        const int owner = first + lane / slots;
+        const uint32_t b = __shfl_sync(0xffffffffu, lo, owner);
+        const uint32_t e = __shfl_sync(0xffffffffu, hi, owner);
+        Row8 m;
+#pragma unroll
+        for (int l = 0; l < kML; ++l) m.d[l] = E.inf;
+        edges_min<WK, kB>(E, b + lane % slots, e > b ? e - 1 : 0u, slots, m);
+        for (int o = 1; o < slots; o <<= 1)
+#pragma unroll
+            for (int l = 0; l < kML; ++l) m.d[l] = min(m.d[l], __shfl_xor_sync(0xffffffffu, m.d[l], o));
+        const int from = ((lane - first) & (rows - 1)) * slots;
+        const bool own = lane >= first && lane < first + rows;
+#pragma unroll
+        for (int l = 0; l < kML; ++l) {
+            const uint32_t t = __shfl_sync(0xffffffffu, m.d[l], from);
+            if (own) mine.d[l] = t;
+        }
+    }
+    return mine;
 }
 
 // Lowers row r's labels to m (lanes that improve); true when r joins the
 // next frontier now.  Long rows: every chunk of the row may lower it.
-__device__ __forceinline__ bool pull_lower(const MSArgs &a, const View &w, uint32_t r, const Row8 &m) {
+__device__ __forceinline__ bool pull_lower(const MSArgs &a, const View &w, uint32_t r, const Row8 &m, uint32_t &lower) {
     const Row8 cur = load_row(a.dist, r);
-    bool improved = false;
 #pragma unroll
     for (int l = 0; l < kML; ++l)
-        if (l < static_cast<int>(a.k) && m.d[l] < cur.d[l])
-            improved |= m.d[l] < atomicMin(a.dist + size_t(r) * kML + l, m.d[l]);
-    return improved && atomicExch(a.stamp + r, w.next_stamp) != w.next_stamp;
+        if (l < static_cast<int>(a.k) && m.d[l] < cur.d[l] && m.d[l] < atomicMin(a.dist + size_t(r) * kML + l, m.d[l]))
+            lower |= 1u << l;
+    return lower && atomicExch(a.stamp + r, w.next_stamp) != w.next_stamp;
 }
 
-// Per-lane minimum of d[u] + w over in-edges [lo, hi) into m (ids at
-// slot[x - a0]: staged, or the CSC itself); each thread of the caller walks
-// its own edges lo, lo + step, ..., kPullU of them loaded before any is
-// relaxed so that their label-row gathers overlap.  Labels are read live
-// (not snapshotted): rows lowered earlier in the same sweep -- the hub rows,
-// whose chunks come first -- feed the rows after them.
-constexpr int kPullU = 4;
-
-template <int WK>
-__device__ __forceinline__ void pull_edges(const MSArgs &a, const uint32_t *s_hot, const uint32_t *slot, uint64_t a0,
-                                           uint64_t lo, uint64_t hi, uint64_t step, uint64_t pol, Row8 &m) {
-    for (uint64_t x0 = lo; x0 < hi; x0 += step * kPullU) {
-        uint32_t u[kPullU], wt[kPullU];
+// True when no in-edge can lower row labels `cur` in any lane this round.
+__device__ __forceinline__ bool row_settled(const MSArgs &a, const uint32_t *s_skip, const Row8 &cur) {
+    bool settled = true;
 #pragma unroll
-        for (int j = 0; j < kPullU; ++j) {
-            const uint64_t x = x0 + j * step;
-            u[j] = x < hi ? slot[x - a0] : 0u;
-            wt[j] = x < hi ? ssc::edge_weight<WK>(a.in_w, x) : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < kPullU; ++j)
-            if (u[j] & kHotTag) u[j] = s_hot[u[j] & ~kHotTag];
-        Row8 du[kPullU];
-#pragma unroll
-        for (int j = 0; j < kPullU; ++j) {
-            if (x0 + j * step < hi) {
-                du[j] = load_row_keep(a.dist, u[j], pol);
-            } else {
-#pragma unroll
-                for (int l = 0; l < kML; ++l) du[j].d[l] = a.inf;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kPullU; ++j)
-#pragma unroll
-            for (int l = 0; l < kML; ++l)
-                if (du[j].d[l] != a.inf) m.d[l] = min(m.d[l], extend<WK>(du[j].d[l], wt[j]));
-    }
+    for (int l = 0; l < kML; ++l)
+        if (l < static_cast<int>(a.k)) settled &= cur.d[l] <= s_skip[l];
+    return settled;
 }
 
-// kStaged: ids staged into shared memory by bulk copies (tiles fit a
-// staging slot); otherwise read from global memory in place.
-template <int WK, bool kStaged>
+template <int WK, bool kB>
 __global__ void __launch_bounds__(kMPThreads, 1) ms_pull_kernel(const MSArgs *__restrict__ args) {
-    extern __shared__ __align__(128) unsigned char s_stage[];
+    extern __shared__ __align__(16) uint32_t s_hot[];  // vertex ids of the hot slots
+    __shared__ uint32_t s_skip[kML];
     const MSArgs a = *args;
     if (*(volatile uint32_t *)&a.hdr->done || !pull_round(a)) return;
     const View w = view(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    stage::WarpStage ws{};
-    if constexpr (kStaged) ws = stage::warp_stage(s_stage, warp, lane);
-    uint32_t *s_hot = reinterpret_cast<uint32_t *>(s_stage + (kStaged ? stage::kStageBytes : 0));
     for (uint32_t i = threadIdx.x; i < a.num_hot; i += blockDim.x) s_hot[i] = a.hot_vertex[i];
+    if (threadIdx.x < kML) {
+        // an in-edge lowers lane l only from a source whose label of that
+        // lane dropped last round; a lane without any cannot improve
+        const uint32_t f = *(volatile const uint32_t *)&a.hdr->fmin[threadIdx.x];
+        s_skip[threadIdx.x] = f < a.inf ? extend<WK>(f, a.min_w) : 0xFFFFFFFFu;
+    }
     __syncthreads();
-    const uint64_t pol = dev::policy_evict_last();
     const uint64_t nwarps = uint64_t(gridDim.x) * (kMPThreads / 32);
-    const uint64_t first = uint64_t(blockIdx.x) * (kMPThreads / 32) + warp;
-    Row8 acc;  // per-lane minima of the current chunk
-    auto task = [&](uint4 d, uint64_t, uint32_t j, uint32_t nu, const uint32_t *slot, uint64_t a0) {
-            if (task_is_chunk(d)) {
-                const stage::Unit u = stage::unit_of(d, j);
-                if (j == 0)
-#pragma unroll
-                    for (int l = 0; l < kML; ++l) acc.d[l] = a.inf;
-                pull_edges<WK>(a, s_hot, slot, a0, u.lo + lane, u.hi, 32, pol, acc);
-                if (j + 1 < nu) return;
-                Row8 m = acc;
-#pragma unroll
-                for (int l = 0; l < kML; ++l)
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) m.d[l] = min(m.d[l], __shfl_xor_sync(0xffffffffu, m.d[l], o));
+    const uint32_t *pf_w = (WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w;
+    InEdges E{nullptr, nullptr, s_hot, a.dist, a.inf};
+    unsigned long long relaxed = 0;  // in-edges relaxed (chunks counted by lane 0, tile rows by their lanes)
+    Gain gain;
+    uint64_t task = uint64_t(blockIdx.x) * (kMPThreads / 32) + warp;
+    uint4 d = task < a.num_tasks ? a.tasks[task] : make_uint4(0, 0, 0, 0);
+    for (; task < a.num_tasks; task += nwarps) {
+        const uint64_t next = task + nwarps;
+        const uint4 nd = next < a.num_tasks ? a.tasks[next] : make_uint4(0, 0, 0, 0);
+        const uint64_t e0 = task_first_edge(d);
+        E.src = a.in_src + e0;
+        E.w = (WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w + e0;
+        prefetch_task(nd, a.in_src, pf_w, lane);
+        if (task_is_chunk(d)) {
+            const uint32_t r = a.long_rows[d.z].row, n = task_edges(d);
+            uint32_t settled = 0;
+            if (lane == 0 && a.skip_rows) settled = row_settled(a, s_skip, load_row(a.dist, r));
+            if (!__shfl_sync(0xffffffffu, settled, 0)) {
+                const Row8 m = span_min<WK, kB>(E, 0, n, lane);
+                uint32_t lower = 0;
                 if (lane == 0) {
-                    const uint32_t row = a.long_rows[d.z].row;
-                    if (pull_lower(a, w, row, m)) ssc::append(w.qnext, w.qnext_size, row);
+                    relaxed += n;
+                    if (pull_lower(a, w, r, m, lower)) {
+                        gain.edges += a.out_deg[r];
+                        ssc::append(w.qnext, w.qnext_size, r);
+                    }
                 }
-                return;
+                note_lower(gain, m, lower, lane);
             }
-            // tile: rows [r0, rl); short rows one lane each, rows of >= 64
-            // in-edges by the whole warp
-            const uint32_t r0 = d.z, rl = d.w;
-            for (uint32_t rb = r0; rb < rl; rb += 32) {
-                const uint32_t rr = rb + lane;
-                const bool active = rr < rl;
-                const uint64_t lo = active ? a.in_off[rr] : 0, hi = active ? a.in_off[rr + 1] : 0;
-                bool joined = false;
-                if (active && hi - lo < 64) {
-                    Row8 m;
-#pragma unroll
-                    for (int l = 0; l < kML; ++l) m.d[l] = a.inf;
-                    pull_edges<WK>(a, s_hot, slot, a0, lo, hi, 1, pol, m);
-                    joined = pull_store_row(a, w, rr, m);
+        } else {
+            for (uint32_t rb = d.z; rb < d.w; rb += 32) {
+                const uint32_t r = rb + lane;
+                uint32_t lo = 0, hi = 0;
+                Row8 cur{};
+                if (r < d.w) {
+                    lo = static_cast<uint32_t>(a.in_off[r] - e0);
+                    hi = static_cast<uint32_t>(a.in_off[r + 1] - e0);
+                    if (hi > lo) {
+                        cur = load_row(a.dist, r);
+                        if (a.skip_rows && row_settled(a, s_skip, cur)) hi = lo;
+                    }
                 }
-                uint32_t big = __ballot_sync(0xffffffffu, active && (hi - lo >= 64));
-                while (big) {
-                    const int src = __ffs(big) - 1;
-                    big &= big - 1;
-                    const uint64_t bb = __shfl_sync(0xffffffffu, lo, src);
-                    const uint64_t ee = __shfl_sync(0xffffffffu, hi, src);
-                    Row8 m;
+                relaxed += hi - lo;
+                const bool wide = hi - lo >= kWideRow;
+                const uint32_t hs = wide ? lo : hi;  // group steps see a wide row as empty
+                const uint32_t most = __reduce_max_sync(0xffffffffu, hs - lo);
+                const uint32_t big = __ballot_sync(0xffffffffu, wide);
+                if (!most && !big) continue;
+                Row8 m;
 #pragma unroll
-                    for (int l = 0; l < kML; ++l) m.d[l] = a.inf;
-                    pull_edges<WK>(a, s_hot, slot, a0, bb + lane, ee, 32, pol, m);
+                for (int l = 0; l < kML; ++l) m.d[l] = a.inf;
+                // the fewest slots a row that hold its edges in one round of loads
+                if (most) m = group_min<WK, kB>(E, lo, hs, most > 32 ? 16 : most > 16 ? 8 : most > 8 ? 4 : most > 4 ? 2 : 1, lane);
+                for (uint32_t b = big; b; b &= b - 1) {
+                    const int o = __ffs(b) - 1;
+                    const Row8 t = span_min<WK, kB>(E, __shfl_sync(0xffffffffu, lo, o), __shfl_sync(0xffffffffu, hi, o), lane);
+                    if (lane == o) m = t;
+                }
+                // a tile row has exactly one writer during a sweep (the warp
+                // that owns its tile) and no push runs beside a sweep: plain stores
+                uint32_t lower = 0;
+                if (hi > lo) {
 #pragma unroll
                     for (int l = 0; l < kML; ++l)
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1)
-                            m.d[l] = min(m.d[l], __shfl_xor_sync(0xffffffffu, m.d[l], o));
-                    const bool jn = (lane == 0) && pull_store_row(a, w, rb + src, m);
-                    if (__shfl_sync(0xffffffffu, jn ? 1u : 0u, 0) && lane == src) joined = true;
+                        if (l < static_cast<int>(a.k) && m.d[l] < cur.d[l]) {
+                            cur.d[l] = m.d[l];
+                            lower |= 1u << l;
+                        }
+                    if (lower) {
+                        uint4 *p = reinterpret_cast<uint4 *>(a.dist + size_t(r) * kML);
+                        p[0] = make_uint4(cur.d[0], cur.d[1], cur.d[2], cur.d[3]);
+                        p[1] = make_uint4(cur.d[4], cur.d[5], cur.d[6], cur.d[7]);
+                        a.stamp[r] = w.next_stamp;
+                        gain.edges += a.out_deg[r];
+                    }
                 }
-                const uint32_t vals[1] = {rr};
-                ssc::warp_append<1>(w.qnext, w.qnext_size, vals, joined ? 1u : 0u, lane);
+                note_lower(gain, cur, lower, lane);
+                const uint32_t vals[1] = {r};
+                ssc::warp_append<1>(w.qnext, w.qnext_size, vals, lower ? 1u : 0u, lane);
             }
-        };
-    bool ok = true;
-    if constexpr (kStaged)
-        ok = stage::stage_pipeline(a.tasks, a.in_src, first, nwarps, a.num_tasks, ws, lane, task);
-    else
-        stage::direct_tasks(a.tasks, a.in_src, first, nwarps, a.num_tasks, task);
-    if (!ok) {
-        atomicExch(&a.hdr->error, 1u);
-        atomicExch(&a.hdr->done, 1u);
-        if (a.use_cond) cudaGraphSetConditional(a.cond, 0);
+        }
+        d = nd;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&a.hdr->relaxations, static_cast<unsigned long long>(a.num_edges));
-        atomicAdd(&a.hdr->pull_rounds, 1u);
-    }
+    flush_gain(a, gain, lane);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) relaxed += __shfl_xor_sync(0xffffffffu, relaxed, o);
+    if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.hdr->pull_rounds, 1u);
 }
 
 // Round-end bookkeeping (one thread): true when the solve is finished.
@@ -466,64 +586,49 @@ __global__ void ms_round_end_kernel(const MSArgs *__restrict__ args) {
     ms_end_round(a, h);
 }
 
-// End of a round of a pull-capable solve, in one grid launch: the whole
-// grid sums the out-edges of the next frontier (the next round's push /
-// pull decision), then the last block to finish ends the round.
-__global__ void __launch_bounds__(kMSThreads) ms_round_close_kernel(const MSArgs *__restrict__ args) {
+// End of a round of a pull-capable solve (one thread): the round's kernels
+// have summed the next frontier's out-edges (the next round's push / pull
+// decision) and found its lowest labels.
+__global__ void ms_round_close_kernel(const MSArgs *__restrict__ args) {
     const MSArgs a = *args;
     MSHeader *h = a.hdr;
-    if (*(volatile uint32_t *)&h->done) return;
-    const uint32_t r = *(volatile uint32_t *)&h->round;
-    const uint32_t qn = *(volatile uint32_t *)&h->qsize[(r + 1) & 1];
-    const uint32_t *q = ((r + 1) & 1) ? a.queue[1] : a.queue[0];
-    unsigned long long sum = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < qn; i += gridDim.x * blockDim.x) {
-        const uint32_t v = q[i];
-        sum += a.row_off[v + 1] - a.row_off[v];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&h->frontier_edges_next, sum);
-    __shared__ uint32_t s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(&h->close_ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
-    }
-    __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
-    __threadfence();
-    const unsigned long long fe = atomicAdd(&h->frontier_edges_next, 0ull);
+    if (h->done) return;
+    const unsigned long long fe = h->frontier_edges_next;
     h->frontier_edges_next = 0;
-    h->close_ticket = 0;
+#pragma unroll
+    for (int l = 0; l < kML; ++l) {
+        h->fmin[l] = ~h->fmin_inv[l];  // all ones when no label of the lane dropped
+        h->fmin_inv[l] = 0;
+    }
     ms_end_round(a, h);
     h->frontier_edges = fe;
 }
 
-// out[l][c] = dist[inv[c]][l] (caller order c; inv NULL: identity).
+// out[l][c] = dist[inv[c]][l] (caller order c; inv NULL: identity); labels of
+// unreached vertices (inf or above) become `unreached`.
 __global__ void ms_emit_kernel(const uint32_t *__restrict__ dist, const uint32_t *__restrict__ inv, uint64_t V,
-                               uint32_t k, uint32_t *__restrict__ out) {
+                               uint32_t k, uint32_t inf, uint32_t unreached, uint32_t *__restrict__ out) {
     for (uint64_t c = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; c < V; c += uint64_t(gridDim.x) * blockDim.x) {
         const uint32_t v = inv ? inv[c] : static_cast<uint32_t>(c);
         const Row8 r = load_row(dist, v);
-        for (uint32_t l = 0; l < k; ++l) out[l * V + c] = r.d[l];
+        for (uint32_t l = 0; l < k; ++l) out[l * V + c] = r.d[l] < inf ? r.d[l] : unreached;
     }
 }
 
-template <int WK>
+template <int WK, bool kB>
 int ms_push_grid() {
     static int g = 0;
     if (g == 0) {
         int per_sm = 0;
-        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_expand_kernel<WK>, kMSThreads, 0));
+        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ms_expand_kernel<WK, kB>, kMSThreads, 0));
         g = sm_count() * std::max(per_sm, 1);
     }
     return g;
 }
 
-template <int WK>
+template <int WK, bool kB>
 void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_rounds, uint32_t flags, cudaStream_t s,
-              uint32_t *out, hyt_run_stats *stats) {
+              uint32_t max_w, uint32_t *out, hyt_run_stats *stats) {
     const uint64_t V = g.V;
     if (g.ms_dist.count < V * kML) g.ms_dist.allocate(V * kML);
     if (g.stamp.count < 2 * V) g.stamp.allocate(2 * V);
@@ -534,8 +639,8 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
     const size_t sb = 512 + sizeof(MSHeader);
     if (g.ms_state.count < sb) g.ms_state.allocate(sb);
     MSArgs *d_args = reinterpret_cast<MSArgs *>(g.ms_state.get());
-    MSHeader *hdr = reinterpret_cast<MSHeader *>(g.ms_state.get() + 256);
-    static_assert(sizeof(MSArgs) <= 256, "MSArgs must fit its 256-byte slot");
+    MSHeader *hdr = reinterpret_cast<MSHeader *>(g.ms_state.get() + 512);
+    static_assert(sizeof(MSArgs) <= 512, "MSArgs must fit its 512-byte slot");
 
     MSArgs a{};
     a.row_off = g.row_offsets.get();
@@ -549,11 +654,10 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
     a.hdr = hdr;
     a.V = static_cast<uint32_t>(V);
     a.k = k;
-    a.inf = (WK == HYT_WEIGHTS_F32) ? 0x7F800000u : HYT_DIST_INF_U32;
+    const uint32_t unreached = (WK == HYT_WEIGHTS_F32) ? 0x7F800000u : HYT_DIST_INF_U32;
+    a.inf = kB ? HYT_DIST_INF_U32 - max_w : unreached;
     a.num_edges = g.E;
     for (uint32_t l = 0; l < k; ++l) a.sources[l] = graph_vertex(g, sources[l], s);
-    // staged pull when the graph's tiles fit a staging slot, else ids read in place
-    const bool staged = g.tile_cost <= kStageTileMax && stage::staged_shared_bytes(g.num_hot) <= kPRSmemMax;
     const bool pull_ok = (g.flags & HYT_GRAPH_PULL) && (WK == HYT_WEIGHTS_NONE || g.in_weights.get()) && g.E > 0 &&
                          g.pull_tasks.get() && size_t(g.num_hot) * 4 <= kPRSmemMax;
     a.pull_div = pull_ok ? 4u : 0u;
@@ -567,19 +671,19 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
         a.num_tasks = g.num_chunks + g.num_tiles;
         a.num_hot = g.num_hot;
     }
-    const unsigned pull_smem =
-        static_cast<unsigned>(staged ? stage::staged_shared_bytes(g.num_hot) : size_t(g.num_hot) * 4);
-    const void *pull_fn = staged ? reinterpret_cast<const void *>(ms_pull_kernel<WK, true>)
-                                 : reinterpret_cast<const void *>(ms_pull_kernel<WK, false>);
+    if (pull_ok) {
+        a.out_deg = g.out_degree.get();
+        a.skip_rows = sssp_pull_skip() ? 1u : 0u;
+        if (a.skip_rows) a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_weight_range(g, WK == HYT_WEIGHTS_F32, s).low;
+    }
+    const unsigned pull_smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
     static bool attr = false;
     if (!attr) {
-        HYT_CUDA(cudaFuncSetAttribute(ms_pull_kernel<WK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaFuncSetAttribute(ms_pull_kernel<WK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HYT_CUDA(cudaFuncSetAttribute(ms_pull_kernel<WK, kB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
         attr = true;
     }
-    const int grid = ms_push_grid<WK>();
+    const int grid = ms_push_grid<WK, kB>();
     const int pgrid = sm_count();
 
     MSHeader h0{};
@@ -621,11 +725,11 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
             HYT_CUDA(cudaGraphAddKernelNode(&node, body, prev ? &prev : nullptr, prev ? 1 : 0, &kp));
             prev = node;
         };
-        add(reinterpret_cast<void *>(ms_expand_kernel<WK>), dim3(grid), dim3(kMSThreads), 0);
-        add(reinterpret_cast<void *>(ms_hub_kernel<WK>), dim3(grid), dim3(kMSThreads), 0);
+        add(reinterpret_cast<void *>(ms_expand_kernel<WK, kB>), dim3(grid), dim3(kMSThreads), 0);
+        add(reinterpret_cast<void *>(ms_hub_kernel<WK, kB>), dim3(grid), dim3(kMSThreads), 0);
         if (a.pull_div) {
-            add(pull_fn, dim3(pgrid), dim3(kMPThreads), pull_smem);
-            add(reinterpret_cast<void *>(ms_round_close_kernel), dim3(grid), dim3(kMSThreads), 0);
+            add(reinterpret_cast<void *>(ms_pull_kernel<WK, kB>), dim3(pgrid), dim3(kMPThreads), pull_smem);
+            add(reinterpret_cast<void *>(ms_round_close_kernel), dim3(1), dim3(1), 0);
         } else {
             add(reinterpret_cast<void *>(ms_round_end_kernel), dim3(1), dim3(1), 0);
         }
@@ -633,16 +737,14 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
         HYT_CUDA(cudaGraphLaunch(exec, s));
     } else {
         for (uint32_t r = 0; r < max_rounds; ++r) {
-            ms_expand_kernel<WK><<<grid, kMSThreads, 0, s>>>(d_args);
-            ms_hub_kernel<WK><<<grid, kMSThreads, 0, s>>>(d_args);
+            ms_expand_kernel<WK, kB><<<grid, kMSThreads, 0, s>>>(d_args);
+            ms_hub_kernel<WK, kB><<<grid, kMSThreads, 0, s>>>(d_args);
             if (a.pull_div) {
-                void *pargs[] = {&d_args};
-                HYT_CUDA(cudaLaunchKernel(pull_fn, dim3(pgrid), dim3(kMPThreads), pargs, pull_smem, s));
-            }
-            if (a.pull_div)
-                ms_round_close_kernel<<<grid, kMSThreads, 0, s>>>(d_args);
-            else
+                ms_pull_kernel<WK, kB><<<pgrid, kMPThreads, pull_smem, s>>>(d_args);
+                ms_round_close_kernel<<<1, 1, 0, s>>>(d_args);
+            } else {
                 ms_round_end_kernel<<<1, 1, 0, s>>>(d_args);
+            }
             HYT_CUDA(cudaGetLastError());
             launches += a.pull_div ? 4 : 3;
             uint32_t done = 0;
@@ -658,14 +760,13 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (use_graph) launches += (a.pull_div ? 4 : 3) * h.round;
-    if (h.error) fail(HYT_E_TIMEOUT, "hyt_sssp_multi: a bounded wait for a staged copy ran out");
     if (out) {
         if (is_device_pointer(out)) {
-            ms_emit_kernel<<<grid_for(V, 256), 256, 0, s>>>(g.ms_dist.get(), g.inv.get(), V, k, out);
+            ms_emit_kernel<<<grid_for(V, 256), 256, 0, s>>>(g.ms_dist.get(), g.inv.get(), V, k, a.inf, unreached, out);
             HYT_CUDA(cudaGetLastError());
         } else {
             Scratch<uint32_t> tmp(V * k, s);
-            ms_emit_kernel<<<grid_for(V, 256), 256, 0, s>>>(g.ms_dist.get(), g.inv.get(), V, k, tmp.get());
+            ms_emit_kernel<<<grid_for(V, 256), 256, 0, s>>>(g.ms_dist.get(), g.inv.get(), V, k, a.inf, unreached, tmp.get());
             HYT_CUDA(cudaGetLastError());
             copy_from_device(out, tmp.get(), V * k * sizeof(uint32_t), s);
         }
@@ -697,10 +798,25 @@ void sssp_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_
     if (!g.weights_ok) fail(HYT_E_INVALID, "SSSP requires finite non-negative edge weights");
     const uint64_t cap = std::min<uint64_t>(4 * g.V + 1024, 0x7FFFFFFFull);
     const uint32_t rounds = max_rounds ? max_rounds : static_cast<uint32_t>(cap);
+    // bounded labels: a path has at most V - 1 edges (candidate)
+    const uint32_t max_w = g.weight_kind == HYT_WEIGHTS_NONE ? 1u
+                           : g.weight_kind == HYT_WEIGHTS_U32 && g.in_weights.get() ? graph_weight_range(g, false, s).high
+                                                                                    : 0xFFFFFFFFu;
+    const bool bounded = max_w < 0x80000000u && (g.V - 1) * uint64_t(max_w) < HYT_DIST_INF_U32 - max_w;
     switch (g.weight_kind) {
-        case HYT_WEIGHTS_NONE: ms_solve<HYT_WEIGHTS_NONE>(g, sources, k, rounds, flags, s, out, stats); break;
-        case HYT_WEIGHTS_U32: ms_solve<HYT_WEIGHTS_U32>(g, sources, k, rounds, flags, s, out, stats); break;
-        case HYT_WEIGHTS_F32: ms_solve<HYT_WEIGHTS_F32>(g, sources, k, rounds, flags, s, out, stats); break;
+        case HYT_WEIGHTS_NONE:
+            if (bounded)
+                ms_solve<HYT_WEIGHTS_NONE, true>(g, sources, k, rounds, flags, s, max_w, out, stats);
+            else
+                ms_solve<HYT_WEIGHTS_NONE, false>(g, sources, k, rounds, flags, s, max_w, out, stats);
+            break;
+        case HYT_WEIGHTS_U32:
+            if (bounded)
+                ms_solve<HYT_WEIGHTS_U32, true>(g, sources, k, rounds, flags, s, max_w, out, stats);
+            else
+                ms_solve<HYT_WEIGHTS_U32, false>(g, sources, k, rounds, flags, s, max_w, out, stats);
+            break;
+        case HYT_WEIGHTS_F32: ms_solve<HYT_WEIGHTS_F32, false>(g, sources, k, rounds, flags, s, max_w, out, stats); break;
         default: fail(HYT_E_INTERNAL, "unknown weight kind");
     }
 }

@@ -416,6 +416,25 @@ __global__ void __launch_bounds__(kSSThreads) sssp_expand_packed_kernel(const SS
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
 }
 
+// Smallest and largest of n weights (bit patterns of u32 or non-negative f32
+// weights; -0.0 counts as 0) into out[0] and ~out[1], which start at all ones.
+__global__ void weight_range_kernel(const uint32_t *__restrict__ w, uint64_t n, uint32_t f32, uint32_t *out) {
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t x = f32 ? (__ldcs(w + i) & 0x7FFFFFFFu) : __ldcs(w + i);
+        lo = min(lo, x);
+        hi = max(hi, x);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(out, lo);
+        atomicMin(out + 1, ~hi);
+    }
+}
+
+}  // namespace
+
 // Row skipping in pull sweeps (env HYT_SSSP_PULL_SKIP, 0 = off; default on).
 bool sssp_pull_skip() {
     static bool on = [] {
@@ -425,35 +444,24 @@ bool sssp_pull_skip() {
     return on;
 }
 
-// Smallest of n weights (bit patterns of u32 or non-negative f32 weights;
-// -0.0 counts as 0) into *out, which starts at all ones.
-__global__ void min_weight_kernel(const uint32_t *__restrict__ w, uint64_t n, uint32_t f32, uint32_t *out) {
-    uint32_t m = 0xFFFFFFFFu;
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t x = __ldcs(w + i);
-        m = min(m, f32 ? (x & 0x7FFFFFFFu) : x);
+WeightRange graph_weight_range(GraphImpl &g, bool f32, cudaStream_t s) {
+    if (!g.weight_range_ready) {
+        Scratch<uint32_t> m(2, s);
+        HYT_CUDA(cudaMemsetAsync(m.get(), 0xFF, 2 * sizeof(uint32_t), s));
+        weight_range_kernel<<<grid_for(g.E, 256, 148 * 8), 256, 0, s>>>(g.in_weights.get(), g.E, f32 ? 1u : 0u,
+                                                                         m.get());
+        HYT_CUDA(cudaGetLastError());
+        uint32_t local[2] = {0, 0};
+        uint32_t *h = g.host_scratch.ptr ? reinterpret_cast<uint32_t *>(g.host_scratch.ptr) : local;
+        HYT_CUDA(cudaMemcpyAsync(h, m.get(), 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        HYT_CUDA(cudaStreamSynchronize(s));
+        g.weight_range = WeightRange{h[0], ~h[1]};
+        g.weight_range_ready = true;
     }
-    m = __reduce_min_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMin(out, m);
+    return g.weight_range;
 }
 
-// The graph's smallest CSC weight, found once per graph.
-uint32_t graph_min_in_weight(GraphImpl &g, bool f32, cudaStream_t s) {
-    if (!g.min_in_weight_ready) {
-        Scratch<uint32_t> m(1, s);
-        HYT_CUDA(cudaMemsetAsync(m.get(), 0xFF, sizeof(uint32_t), s));
-        min_weight_kernel<<<grid_for(g.E, 256, 148 * 8), 256, 0, s>>>(g.in_weights.get(), g.E, f32 ? 1u : 0u,
-                                                                       m.get());
-        HYT_CUDA(cudaGetLastError());
-        uint32_t local = 0;
-        uint32_t *h = g.host_scratch.ptr ? reinterpret_cast<uint32_t *>(g.host_scratch.ptr) : &local;
-        HYT_CUDA(cudaMemcpyAsync(h, m.get(), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        HYT_CUDA(cudaStreamSynchronize(s));
-        g.min_in_weight = *h;
-        g.min_in_weight_ready = true;
-    }
-    return g.min_in_weight;
-}
+namespace {
 
 // Pull sweeps when the frontier's out-edges exceed E / div (env
 // HYT_SSSP_PULL_DIV, 0 = never; default 4: a sweep reads every in-edge once,
@@ -548,7 +556,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     // row skipping: the smallest edge weight bounds what any in-edge adds
     if (a.pull_div && sssp_pull_skip()) {
         a.skip_rows = 1;
-        a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_min_in_weight(g, WK == HYT_WEIGHTS_F32, s);
+        a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_weight_range(g, WK == HYT_WEIGHTS_F32, s).low;
     }
     const unsigned pull_smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
     const int pgrid = a.pull_div ? pull_grid<WK>() : 0;

@@ -75,3 +75,18 @@ def test_sssp_row_degrees(hyt, oracle, gpu, order, weights):
                 want = np.where(np.isfinite(ref), ref, 0).astype(np.uint64)
                 want = np.where(np.isfinite(ref), want, 0xFFFFFFFF).astype(np.uint32)
                 assert np.array_equal(d, want)
+
+
+@pytest.mark.parametrize("weights", ["none", "u32", "f32", "u32_large"])
+def test_sssp_multi_row_degrees(hyt, gpu, weights):
+    """Every lane of a packed solve equals the single solve, also where labels
+    may saturate (u32_large) and where they cannot."""
+    g = _graph(hyt, "mixed")
+    w = {"none": None, "u32": g.weights, "f32": (g.weights * np.float32(0.37)).astype(np.float32),
+         "u32_large": (g.weights.astype(np.uint64) * 40000001).astype(np.uint32)}[weights]
+    with hyt.Graph(hyt.CSR(g.row_offsets, g.column_indices, w)) as dg:
+        sources = [0, 5, g.num_vertices - 1, 17, 30000, 5, 39000]
+        d, st = dg.sssp_multi(sources)
+        assert st["converged"] == 1
+        for lane, s in enumerate(sources):
+            assert np.array_equal(d[lane], dg.sssp(s)[0]), s
