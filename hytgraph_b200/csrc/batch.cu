@@ -676,7 +676,6 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
         a.max_iter = it;
         a.source = graph_vertex(g, q.source, stream_);
         a.personalized = 1;
-        a.use_cond = 0;
         h.pr[s] = a;
         h.px[s] = x;
         sl.kind = kPPR;

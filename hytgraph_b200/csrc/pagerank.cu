@@ -36,7 +36,7 @@
 // and the FP64 residual and dangling mass are summed in a fixed slot order
 // (PRSlots), independent of the grid size and of warp arrival order: each
 // task stores its slot, then pr_reduce_kernel sums the slots and evaluates
-// the stop rule, ending the CUDA-graph conditional while-loop when done.
+// the stop rule.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -44,6 +44,7 @@
 
 #include "common.cuh"
 #include "graph.cuh"
+#include "grid_sync.cuh"
 #include "hybrid.cuh"
 #include "pagerank_core.cuh"
 #include "solvers.cuh"
@@ -92,27 +93,17 @@ struct PRRange {
     const uint4 *tasks;  // the graph's task descriptors (whole-graph launches; NULL: no prefetch)
 };
 
-// a: the solve's arguments as kernel parameters (the constant bank: no
-// registers held across the tasks); its scalars may be of an earlier solve,
-// those of this one are in *args.
-__global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs *__restrict__ args,
-                                                                   const __grid_constant__ PRArgs a,
-                                                                   const __grid_constant__ PRRange rg) {
-    extern __shared__ __align__(16) float s_dyn[];
-
-    const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
-    if (*(volatile uint32_t *)&a.hdr->done) return;
-
-    const PRBuffers b = buffers(a, it);
-    const PRState ps = make_state(*args, a.dangling[it]);
+// The tasks of one iteration, over the whole grid.  a: the solve's arguments
+// as kernel parameters (the constant bank: no registers held across the
+// tasks).
+__device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, const PRState &ps, const PRBuffers &b,
+                                          double2 *slots, float *s_hot) {
     const uint64_t n_chunks = rg.chunk_end - rg.chunk_begin;
     const uint64_t total_tasks = n_chunks + (rg.tile_end - rg.tile_begin);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *s_hot = s_dyn;
     load_hot(a, b, s_hot);
     __syncthreads();
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPRThreads / 32);
-
     uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp;
     // whole-graph launches read each task's descriptor while the task before
     // it runs (one 16-byte load in place of a chain of table reads)
@@ -125,23 +116,131 @@ __global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs 
         if (task < n_chunks) {
             const TaskSpan t = rg.tasks ? task_span(d) : chunk_span(a, rg.chunk_begin + task);
             const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
-            if (row != ~0u) slot_store(a, long_slot(row), dev::warp_sum(res), dev::warp_sum(dang), lane);
+            if (row != ~0u) slot_store(slots, long_slot(row), dev::warp_sum(res), dev::warp_sum(dang), lane);
         } else {
             const uint64_t k = rg.tile_begin + (task - n_chunks);
             const TaskSpan t = rg.tasks ? task_span(d) : tile_span(a, k);
             tile_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
-            slot_store(a, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
+            slot_store(slots, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
         }
         d = nd;
     }
 }
 
+// One iteration (or a part of one: out-of-HBM partitions); the scalars of
+// this solve are in *args.
+__global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs *__restrict__ args,
+                                                                   const __grid_constant__ PRArgs a,
+                                                                   const __grid_constant__ PRRange rg) {
+    extern __shared__ __align__(16) float s_dyn[];
+    const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
+    if (*(volatile uint32_t *)&a.hdr->done) return;
+    run_tasks(a, rg, make_state(*args, a.dangling[it]), buffers(a, it), a.red.slot, s_dyn);
+}
+
+// (residual, dangling) of slot group g: thread t of 256 takes slots t, t +
+// 256, ..., then a fixed tree.  Called by 256 consecutive threads (8 warps, of
+// which warp `w`); s_part holds 8 entries of theirs; the result is in lane 0
+// of their first warp after the caller's barrier and fold_group.
+constexpr int kReduceThreads = 256;
+
+__device__ __forceinline__ double2 group_part(const PRSlots &R, const double2 *slots, uint32_t g, uint32_t t) {
+    const uint32_t b = g * kSlotGroup, n = min(kSlotGroup, R.num_slots - b);
+    double r = 0.0, d = 0.0;
+    for (uint32_t i = t; i < n; i += kReduceThreads) {
+        const double2 x = __ldcg(slots + b + i);
+        r += x.x;
+        d += x.y;
+    }
+    return make_double2(dev::warp_sum(r), dev::warp_sum(d));
+}
+
+__device__ __forceinline__ double2 fold_group(const double2 *s_part, int lane) {
+    const double2 v = lane < kReduceThreads / 32 ? s_part[lane] : make_double2(0.0, 0.0);
+    return make_double2(dev::warp_sum(v.x), dev::warp_sum(v.y));
+}
+
+// The whole solve in one cooperative launch: iterations separated by grid
+// barriers in place of two kernel launches and a conditional-graph step each
+// (on 65 K edges those cost more than the work; the graph was also built and
+// instantiated for every solve): 523 -> 235 us a call on 4099 vertices and 65 K
+// edges, 19.7 -> 19.4 ms on R-MAT scale 24.  Every CTA takes the stop decision by itself
+// from the same sums.  Up to kOwnGroups slot groups are summed by every CTA
+// (one barrier an iteration); more are shared out, with a second barrier.
+// Slots alternate between two halves, so an iteration's slots are not
+// overwritten before every CTA has passed the next barrier.  The sums'
+// association is that of pr_reduce_kernel.
+constexpr uint32_t kOwnGroups = kPRThreads / kReduceThreads;
+
+__global__ void __launch_bounds__(kPRThreads, 1) pr_solve_kernel(const __grid_constant__ PRArgs a,
+                                                                 const __grid_constant__ PRRange rg) {
+    extern __shared__ __align__(16) float s_dyn[];
+    __shared__ double2 s_part[kPRThreads / 32];
+    __shared__ double2 s_group[kOwnGroups];
+    __shared__ double2 s_total;
+    const PRSlots &R = a.red;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t sub = threadIdx.x / kReduceThreads, t = threadIdx.x % kReduceThreads;
+    constexpr int kSubWarps = kReduceThreads / 32;
+    uint32_t barriers = 0;
+    double dangling = a.dangling[0];
+    bool ok = true;
+    for (uint32_t it = 0; ok; ++it) {
+        double2 *slots = R.slot + ((it & 1) ? R.num_slots : 0);
+        run_tasks(a, rg, make_state(a, dangling), buffers(a, it), slots, s_dyn);
+        ok = dev::grid_sync(R.blocks_done, barriers);
+        if (!ok) break;
+        const bool own = R.num_groups <= kOwnGroups;
+        const uint32_t first = own ? sub : blockIdx.x * kOwnGroups + sub;
+        const uint32_t step = own ? kOwnGroups : gridDim.x * kOwnGroups;
+        const uint32_t rounds = (R.num_groups + step - 1) / step;
+        for (uint32_t k = 0; k < rounds; ++k) {
+            const uint32_t g = first + k * step;
+            double2 p = make_double2(0.0, 0.0);
+            if (g < R.num_groups) p = group_part(R, slots, g, t);
+            if (lane == 0) s_part[warp] = p;
+            __syncthreads();
+            if (warp % kSubWarps == 0 && g < R.num_groups) {
+                const double2 v = fold_group(s_part + sub * kSubWarps, lane);
+                if (lane == 0) {
+                    if (own)
+                        s_group[sub] = v;
+                    else
+                        R.group_sum[g] = v;
+                }
+            }
+            __syncthreads();
+        }
+        if (!own) {
+            ok = dev::grid_sync(R.blocks_done, barriers);
+            if (!ok) break;
+        }
+        if (warp == 0) {
+            double r = 0.0, d = 0.0;
+            for (uint32_t g = lane; g < R.num_groups; g += 32) {
+                const double2 x = own ? s_group[g] : __ldcg(R.group_sum + g);
+                r += x.x;
+                d += x.y;
+            }
+            r = dev::warp_sum(r);
+            d = dev::warp_sum(d);
+            if (lane == 0) s_total = make_double2(r, d);
+        }
+        __syncthreads();
+        const double2 total = s_total;
+        dangling = total.y;
+        const bool done = total.x <= static_cast<double>(a.tolerance) || it + 1 >= a.max_iter;
+        if (blockIdx.x == 0 && threadIdx.x == 0) close_iteration(a, it, total.x, total.y);
+        if (done) return;
+        __syncthreads();  // s_total and the hot table are rewritten
+    }
+    if (threadIdx.x == 0) atomicExch(&a.hdr->error, 1u);
+}
+
 // Closes an iteration: block b sums slot groups b, b + grid, ... (thread t
 // takes slots t, t + 256, ... of the group, then a fixed block tree); the
 // last block to finish sums the group sums in group order, then applies
-// the stop rule (ending the CUDA-graph loop when the solve is done).
-constexpr int kReduceThreads = 256;
-
+// the stop rule.
 __global__ void __launch_bounds__(kReduceThreads) pr_reduce_kernel(const PRArgs *__restrict__ args) {
     __shared__ double s_red[32];
     __shared__ uint32_t s_last;
@@ -186,11 +285,10 @@ __global__ void __launch_bounds__(kReduceThreads) pr_reduce_kernel(const PRArgs 
 constexpr uint32_t kInitChunk = 4096;
 constexpr int kInitThreads = 256;
 
-__global__ void __launch_bounds__(kInitThreads) pr_init_kernel(const PRArgs *__restrict__ args, double *part,
+__global__ void __launch_bounds__(kInitThreads) pr_init_kernel(const __grid_constant__ PRArgs a, double *part,
                                                                uint32_t *count) {
     __shared__ double s_red[32];
     __shared__ uint32_t s_last;
-    const PRArgs a = *args;
     const uint32_t V = a.V;
     const uint32_t nchunks = (V + kInitChunk - 1) / kInitChunk;
     const float r0_uniform = __fdiv_rn(1.0f, static_cast<float>(V));
@@ -228,6 +326,8 @@ int pr_occupancy_grid() {
         int per_sm = 0;
         HYT_CUDA(cudaFuncSetAttribute(pr_iterate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
+        HYT_CUDA(cudaFuncSetAttribute(pr_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kPRSmemMax - 4096)));
         HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_iterate_kernel, kPRThreads, kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
         if (const char *e = std::getenv("HYT_PR_GRID")) {
@@ -273,7 +373,7 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
     const size_t args_bytes = (sizeof(PRArgs) + 255) & ~size_t(255);
     const size_t head = sizeof(PRHeader) + size_t(max_iter) * sizeof(double) + size_t(max_iter + 1) * sizeof(double) +
                         size_t(init_chunks) * sizeof(double) + 2 * sizeof(uint32_t);
-    const size_t sb = args_bytes + up16(head) + size_t(num_groups + num_slots) * sizeof(double2) + 64;
+    const size_t sb = args_bytes + up16(head) + size_t(num_groups + 2 * num_slots) * sizeof(double2) + 64;
     if (g.pr_state.count < sb) g.pr_state.allocate(sb);
 
     unsigned char *base = g.pr_state.get();
@@ -328,7 +428,6 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
     a.max_iter = max_iter;
     a.source = source;
     a.personalized = personalized ? 1u : 0u;
-    a.use_cond = 0;
     a.red = PRSlots{slots, group_sum, blocks_done, static_cast<uint32_t>(num_slots),
                     static_cast<uint32_t>(num_groups)};
     a.tasks = g.pull_tasks.get();
@@ -337,7 +436,7 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
 }
 
 static void pr_check_header(const PRHeader &h) {
-    if (h.error) fail(HYT_E_TIMEOUT, "PageRank: a bounded wait for a staged copy ran out");
+    if (h.error) fail(HYT_E_TIMEOUT, "PageRank: a bounded wait at a grid barrier ran out");
     if (h.iter == 0) fail(HYT_E_INTERNAL, "PageRank made no progress");
 }
 
@@ -348,7 +447,7 @@ static unsigned pr_reduce_grid(const PRArgs &a) {
 
 static void pr_init(const PRSolveState &st, uint64_t V, cudaStream_t s) {
     const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((V + kInitChunk - 1) / kInitChunk, 148ull * 8));
-    pr_init_kernel<<<blocks, kInitThreads, 0, s>>>(st.d_args, st.init_part, st.init_count);
+    pr_init_kernel<<<blocks, kInitThreads, 0, s>>>(st.a, st.init_part, st.init_count);
     HYT_CUDA(cudaGetLastError());
 }
 
@@ -360,17 +459,11 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
     PRArgs &a = st0.a;
     PRArgs *d_args = st0.d_args;
     PRHeader *hdr = st0.hdr;
-    const bool use_graph = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
+    // one persistent launch, or (profiling, launch-by-launch runs) a host loop
+    const bool persistent = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = pr_occupancy_grid();
     const unsigned smem = static_cast<unsigned>(pr_hot_bytes(g.num_hot));
     PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get()};
-    void *kargs[] = {&d_args, &a, &full};
-    const unsigned rgrid = pr_reduce_grid(a);
-    auto launch = [&] {
-        pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(d_args, a, full);
-        pr_reduce_kernel<<<rgrid, kReduceThreads, 0, s>>>(d_args);
-        HYT_CUDA(cudaGetLastError());
-    };
 
     EventTimer total;
     total.start(s);
@@ -379,49 +472,27 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
 
     uint32_t launches = 0, hot_launches = 0;
     double kernel_ms = 0.0;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if (use_graph) {
-        HYT_CUDA(cudaGraphCreate(&graph, 0));
-        cudaGraphConditionalHandle cond;
-        HYT_CUDA(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
-        a.cond = cond;
-        a.use_cond = 1;
-    }
-    HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(PRArgs), cudaMemcpyHostToDevice, s));
     pr_init(st0, V, s);
     ++launches;
 
-    if (use_graph) {
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = a.cond;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cnode;
-        HYT_CUDA(cudaGraphAddNode(&cnode, graph, nullptr, 0, &cp));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        cudaKernelNodeParams kp = {};
-        kp.func = reinterpret_cast<void *>(pr_iterate_kernel);
-        kp.gridDim = dim3(grid);
-        kp.blockDim = dim3(kPRThreads);
-        kp.sharedMemBytes = smem;
-        kp.kernelParams = kargs;
-        cudaGraphNode_t knode, rnode;
-        HYT_CUDA(cudaGraphAddKernelNode(&knode, body, nullptr, 0, &kp));
-        cudaKernelNodeParams rp = {};
-        rp.func = reinterpret_cast<void *>(pr_reduce_kernel);
-        rp.gridDim = dim3(rgrid);
-        rp.blockDim = dim3(kReduceThreads);
-        rp.kernelParams = kargs;
-        HYT_CUDA(cudaGraphAddKernelNode(&rnode, body, &knode, 1, &rp));
-        HYT_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-        HYT_CUDA(cudaGraphLaunch(exec, s));
+    if (persistent) {
+        // every CTA must be resident; no more of them than have tasks
+        const uint64_t tasks = g.num_chunks + g.num_tiles;
+        const unsigned ctas = static_cast<unsigned>(
+            std::min<uint64_t>({static_cast<uint64_t>(grid), static_cast<uint64_t>(sm_count()),
+                                std::max<uint64_t>(1, (tasks + kPRThreads / 32 - 1) / (kPRThreads / 32))}));
+        void *kargs[] = {&a, &full};
+        HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(pr_solve_kernel), dim3(ctas), dim3(kPRThreads),
+                                             kargs, smem, s));
+        ++launches;
     } else {
+        HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(PRArgs), cudaMemcpyHostToDevice, s));
         EventTimer kt;
         for (uint32_t i = 0; i < max_iter; ++i) {
             if (flags & HYT_RUN_PROFILE) kt.start(s);
-            launch();
+            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(d_args, a, full);
+            pr_reduce_kernel<<<pr_reduce_grid(a), kReduceThreads, 0, s>>>(d_args);
+            HYT_CUDA(cudaGetLastError());
             launches += 2;
             if (flags & HYT_RUN_PROFILE) {
                 kt.stop(s);
@@ -440,13 +511,12 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
             }
         }
     }
-    PRHeader h{};
-    HYT_CUDA(cudaMemcpyAsync(&h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s));
+    PRHeader local{};
+    PRHeader *hp = g.host_scratch.ptr ? reinterpret_cast<PRHeader *>(g.host_scratch.ptr) : &local;
+    HYT_CUDA(cudaMemcpyAsync(hp, hdr, sizeof(PRHeader), cudaMemcpyDeviceToHost, s));
     total.stop(s);
     const double total_ms = total.ms();
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    if (use_graph) launches += 2 * h.iter;
+    const PRHeader h = *hp;
     pr_check_header(h);
     if (ranks_out) graph_emit(g, ranks_out, g.rank[h.iter & 1].get(), s);
 

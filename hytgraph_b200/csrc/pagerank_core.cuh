@@ -26,7 +26,7 @@ struct PRHeader {
     uint32_t iter;       // iterations completed
     uint32_t done;
     uint32_t converged;
-    uint32_t error;      // 1: a bounded wait for a staged copy ran out
+    uint32_t error;      // 1: a bounded wait at a grid barrier ran out
     double last_residual;
 };
 
@@ -42,9 +42,9 @@ struct PRHeader {
 constexpr uint32_t kSlotGroup = 1024;
 
 struct PRSlots {
-    double2 *slot;          // [num_slots] (residual, dangling)
+    double2 *slot;          // [2 * num_slots] (residual, dangling); the persistent solver alternates halves
     double2 *group_sum;     // [num_groups]
-    uint32_t *blocks_done;  // [1] reduce blocks finished, over the whole solve
+    uint32_t *blocks_done;  // [1] reduce blocks finished, over the whole solve (persistent solver: barrier count)
     uint32_t num_slots, num_groups;
 };
 
@@ -75,8 +75,6 @@ struct PRArgs {
     uint32_t max_iter;
     uint32_t source;    // PPR
     uint32_t personalized;
-    cudaGraphConditionalHandle cond;
-    uint32_t use_cond;
     PRSlots red;        // fixed-order residual / dangling reduction (single-query solver)
     const uint4 *tasks; // pull task descriptors
 };
@@ -145,7 +143,9 @@ __device__ __forceinline__ Sources make_sources(const PRArgs &a, const float *cc
     return Sources{ccur, hot, kHotTag | a.num_hot, dev::policy_evict_last()};
 }
 
-// Loads one source's contribution: its bits end in `g | id`.  The two loads
+// Loads one source's contribution: its bits end in `g | id`.  Not through the
+// read-only path: the persistent solver rewrites the vector between
+// iterations.  The two loads
 // are predicated on the tag and write registers of their own (the hot one
 // its id's), so that neither waits for the other and no branch splits a run
 // of gathers.
@@ -156,7 +156,7 @@ __device__ __forceinline__ void load_contribution(uint32_t &id, uint32_t &g, con
         const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(S.hot)) + (id << 2);  // drops the tag
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, 0;\n\t"
-            "@!p ld.global.nc.L2::cache_hint.b32 %0, [%2], %3;\n\t"
+            "@!p ld.global.L2::cache_hint.b32 %0, [%2], %3;\n\t"
             "@!p mov.b32 %1, 0;\n\t"
             "@p ld.shared.b32 %1, [%4];\n\t}"
             : "+r"(g), "+r"(id)
@@ -164,9 +164,9 @@ __device__ __forceinline__ void load_contribution(uint32_t &id, uint32_t &g, con
     } else {
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, 0;\n\t"
-            "@!p ld.global.nc.L2::cache_hint.b32 %0, [%2], %3;\n\t"
+            "@!p ld.global.L2::cache_hint.b32 %0, [%2], %3;\n\t"
             "@!p mov.b32 %1, 0;\n\t"
-            "@p ld.global.nc.b32 %1, [%4];\n\t}"
+            "@p ld.global.b32 %1, [%4];\n\t}"
             : "+r"(g), "+r"(id)
             : "l"(S.ccur + id), "l"(S.pol), "l"(S.hot + (id & ~kHotTag)));
     }
@@ -229,7 +229,6 @@ __device__ __forceinline__ void end_iteration(const PRArgs &a, uint32_t it) {
     if (conv || n_it >= a.max_iter) {
         a.hdr->done = 1;
         a.hdr->converged = conv ? 1u : 0u;
-        if (a.use_cond) cudaGraphSetConditional(a.cond, 0);
     }
 }
 
@@ -246,13 +245,12 @@ __device__ __forceinline__ void close_iteration(const PRArgs &a, uint32_t it, do
     if (conv || n_it >= a.max_iter) {
         a.hdr->done = 1;
         a.hdr->converged = conv ? 1u : 0u;
-        if (a.use_cond) cudaGraphSetConditional(a.cond, 0);
     }
 }
 
 // Records task slot `slot`'s (res, dang); lane 0 stores, no wait.
-__device__ __forceinline__ void slot_store(const PRArgs &a, uint32_t slot, double res, double dang, int lane) {
-    if (lane == 0) a.red.slot[slot] = make_double2(res, dang);
+__device__ __forceinline__ void slot_store(double2 *slots, uint32_t slot, double res, double dang, int lane) {
+    if (lane == 0) slots[slot] = make_double2(res, dang);
 }
 
 // Solver scalars of an iteration whose dangling mass (sum of x over
