@@ -434,6 +434,18 @@ void build_pull_tiles(GraphImpl &g, cudaStream_t s) {
     HYT_CUDA(cudaStreamSynchronize(s));
 }
 
+// Tile size: large tiles cost less per edge (fewer task starts, and rows of up
+// to 1023 in-edges stay out of the chunk path), small ones leave more warps
+// something to do.  The line lies where 1024-unit tiles still give every warp
+// of the GPU three: PageRank in 1024- / 512-unit tiles takes 17.3 / 18.5 ms at
+// 16.7 M vertices and 263 M edges, 1.10 / 1.27 ms at 1 M and 16 M, but 0.57 /
+// 0.53 ms at 262 K and 4 M (SSSP: 2.94 / 3.07, 0.75 / 0.83, 0.61 / 0.58 ms).
+// Smaller tiles gained 10 % on a PageRank of 65 K edges and cost a batch of
+// queries on such graphs 20 to 50 %.
+static uint32_t tile_cost_for(uint64_t V, uint64_t E) {
+    return (V + E) / kTileCostDefault >= 3ull * 148 * (kPRThreads / 32) ? kTileCostDefault : kTileCostSmall;
+}
+
 void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
     const uint64_t V = csr.num_vertices, E = csr.num_edges;
     if (V == 0) fail(HYT_E_INVALID, "graph requires at least one vertex");
@@ -446,17 +458,16 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         fail(HYT_E_INVALID, "weights is NULL for a weighted graph");
     if (flags == 0) flags = HYT_GRAPH_ALL;
     // PageRank decomposition knobs (same work, different tiling): tile cost
-    // in {64..512} and hot-source cache size, bounded by shared memory.  The
-    // staged kernels (HYT_STAGED=1) need tiles that fit one staging slot.
-    g.tile_cost = stage::staged_requested() ? kStageTileMax : kTileCostDefault;
+    // in {64..1024} and hot-source cache size.  The staged kernels
+    // (HYT_STAGED=1) need tiles that fit one staging slot.
+    g.tile_cost = stage::staged_requested() ? kStageTileMax : tile_cost_for(V, E);
     if (const char *t = std::getenv("HYT_PR_TILE")) {
         const unsigned long v = std::strtoul(t, nullptr, 10);
-        if (v >= 64 && v <= kTileCostMax) g.tile_cost = static_cast<uint32_t>(v);
+        if (v >= kTileCostMin && v <= kTileCostDefault) g.tile_cost = static_cast<uint32_t>(v);
     }
-    uint32_t hot_request = kHotSourcesDefault;
+    uint32_t hot_request = V >= kHotLargeVertices ? kHotSourcesLarge : kHotSourcesDefault;
     if (const char *t = std::getenv("HYT_PR_HOT")) hot_request = static_cast<uint32_t>(std::strtoul(t, nullptr, 10));
     hot_request = std::min(hot_request, kHotSourcesMax);
-    while (hot_request && pr_shared_bytes(hot_request, g.tile_cost) > kPRSmemMax) hot_request /= 2;
     if ((flags & HYT_GRAPH_PULL) && V > (kHotTag >> 0) - 1)
         fail(HYT_E_UNSUPPORTED, "pull graphs hold fewer than 2^31 vertices (bit 31 tags cached sources)");
 

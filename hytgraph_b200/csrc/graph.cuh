@@ -24,13 +24,16 @@ namespace hyt {
 // so its rows hold fewer than tile_cost edges except for its last row.  A
 // last row with in-degree >= tile_cost is a "long row": it is excluded from
 // the tile and split into kLongChunk-edge chunks.  One warp processes one
-// task (tile or chunk), so a tile's staged SSSP candidates fit in a per-warp
-// shared-memory slice of 2 * tile_cost floats.
-constexpr uint32_t kTileCostDefault = 512;   // merge-path units per tile (tunable: HYT_PR_TILE)
-constexpr uint32_t kTileCostMax = 512;       // register-path tiles; bulk-staged tasks need <= kStageTileMax
-constexpr uint32_t kStageTileMax = 256;      // a tile's edges (< 2 * tile_cost) fit one staging slot
+// task (tile or chunk).
+constexpr uint32_t kTileCostMin = 64;
+constexpr uint32_t kTileCostSmall = 512;     // ... on small ones
+constexpr uint32_t kTileCostDefault = 1024;  // merge-path units per tile on large graphs (tunable: HYT_PR_TILE)
+constexpr uint32_t kStageTileMax = 256;      // bulk-staged kernels: a tile's edges (< 2 * tile_cost) fit one slot
 constexpr uint32_t kLongChunk = 4096;
 constexpr uint32_t kHotSourcesDefault = 8192;   // shared-memory source cache (tunable: HYT_PR_HOT)
+constexpr uint32_t kHotSourcesLarge = 24576;    // ... of graphs of kHotLargeVertices or more
+constexpr uint64_t kHotLargeVertices = uint64_t(1) << 22;  // PageRank 8192 -> 24576 entries: 18.45 -> 17.75 ms at 2^24 vertices,
+                                                           // 4.58 -> 4.52 at 2^22; 1.43 -> 1.53 at 2^20 (loading them costs more)
 constexpr uint32_t kHotSourcesMax = 32768;
 constexpr uint32_t kPRSmemMax = 226 * 1024;     // dynamic shared memory per CTA (227 KB opt-in - static)
 constexpr uint32_t kHotTag = 0x80000000u;       // in_sources tag: source is hot slot (low bits)
@@ -180,12 +183,6 @@ struct GraphImpl {
 // cache and its zero slot.
 constexpr int kPRThreads = 1024;
 inline size_t pr_hot_bytes(uint32_t num_hot) { return (size_t(num_hot) + 1) * sizeof(float); }
-// SSSP sweeps of the same shape: hot slots + one staging slice (2 * tile_cost
-// + 8 words) per warp.
-inline size_t pr_shared_bytes(uint32_t num_hot, uint32_t tile_cost) {
-    return (size_t(num_hot) + size_t(kPRThreads / 32) * (2 * size_t(tile_cost) + 8)) * sizeof(float);
-}
-
 // Builds the device graph from a CSR (host or device pointers).
 void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags);
 

@@ -800,7 +800,7 @@ HybridImpl *hybrid_create(const hyt_csr *csr, const hyt_csc *csc, const hyt_hybr
         g.in_offsets.allocate(V + 1);
         HYT_CUDA(cudaMemcpyAsync(g.in_offsets.get(), h->h_in_off, (V + 1) * 8, cudaMemcpyHostToDevice, g.stream));
         HYT_CUDA(cudaStreamSynchronize(g.stream));
-        g.tile_cost = kTileCostDefault;
+        g.tile_cost = kTileCostSmall;
         g.num_hot = 0;  // host sources are untagged
         build_pull_tiles(g, g.stream);
         build_pull_pieces(*h, slot / 4);
