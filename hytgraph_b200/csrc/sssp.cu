@@ -36,10 +36,11 @@
 // lowest label summed by the kernels that fill it, a solve of R-MAT scale 24
 // went from 4.76 to 4.33 ms.  A sweep skips the rows whose label
 // is at most (lowest frontier label + smallest weight): no in-edge can
-// lower them, so their in-edges are neither read nor gathered.  All round state lives on the
-// device; inside a CUDA graph the rounds run as a conditional while-loop
-// (expand, hub chunks, pull sweep, round close), instantiated once per
-// graph and launched again by later solves.
+// lower them, so their in-edges are neither read nor gathered.  All round
+// state lives on the device; with one bucket the whole solve is one
+// cooperative launch (sssp_solve_kernel), with a finite bucket width the
+// rounds run as a conditional CUDA graph (split, expand, hub chunks, round
+// end), instantiated once per graph and launched again by later solves.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -52,6 +53,7 @@
 
 #include "common.cuh"
 #include "graph.cuh"
+#include "grid_sync.cuh"
 #include "host_checks.hpp"
 #include "scratch.cuh"
 #include "hybrid.cuh"
@@ -181,33 +183,26 @@ constexpr int kPullThreads = 1024;  // one CTA per SM, like the PageRank kernel
 // frontier, so the argument holds again next round; distances are
 // unchanged.
 template <int WK>
-__device__ __forceinline__ uint32_t skip_bound(const SSArgs &a, bool &on) {
-    const uint32_t fmin = *(volatile const uint32_t *)&a.hdr->fmin;
+__device__ __forceinline__ uint32_t skip_bound(const SSArgs &a, uint32_t fmin, bool &on) {
     on = a.skip_rows && fmin < a.inf;
     return on ? extend<WK>(fmin, a.min_w) : 0u;
 }
 
-// a: the solve's arguments as kernel parameters (the constant bank: no
-// registers held across the tasks).  Labels are read live, not from a
-// snapshot: rows lowered early in a sweep feed the rows after them (a
-// snapshot of the hottest labels in shared memory cost a round).
+// One sweep over the whole grid.  fmin: the frontier's lowest label; relaxed
+// and gain are added to (chunks counted by lane 0, tile rows by their lanes).
+// Labels are read live, not from a snapshot: rows lowered early in a sweep
+// feed the rows after them (a snapshot of the hottest labels in shared memory
+// cost a round).
 template <int WK>
-__global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid_constant__ SSArgs a,
-                                                                    const __grid_constant__ PullGraph pg) {
-    extern __shared__ __align__(16) uint32_t s_hot[];  // vertex ids of the hot slots (tagged sources in the CSC)
-    if (*(volatile uint32_t *)&a.hdr->done || !pull_round(a)) return;
-    const RoundView rv = round_view(a);
+__device__ __forceinline__ void pull_sweep(const SSArgs &a, const PullGraph &pg, const RoundView &rv, uint32_t fmin,
+                                           const uint32_t *s_hot, unsigned long long &relaxed, Gain &gain) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t i = threadIdx.x; i < pg.num_hot; i += blockDim.x) s_hot[i] = pg.hot_vertex[i];
-    __syncthreads();
     const uint64_t pol = dev::policy_evict_last();
     const auto label = [&](uint32_t u) { return dev::ld_keep_u32(a.dist + u, pol); };
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPullThreads / 32);
     const uint32_t *pf_w = (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w;
     bool skip_on;
-    const uint32_t skip_at = skip_bound<WK>(a, skip_on);
-    unsigned long long relaxed = 0;  // in-edges relaxed (chunks counted by lane 0, tile rows by their lanes)
-    Gain gain;
+    const uint32_t skip_at = skip_bound<WK>(a, fmin, skip_on);
     uint64_t task = uint64_t(blockIdx.x) * (kPullThreads / 32) + warp;
     // each task's descriptor is read while the task before it runs
     uint4 d = task < pg.num_tasks ? pg.tasks[task] : make_uint4(0, 0, 0, 0);
@@ -270,11 +265,134 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid
         }
         d = nd;
     }
-    flush_gain(a, gain, lane);
+}
+
+// Vertex ids of the hot slots into shared memory.
+__device__ __forceinline__ void load_hot_ids(const PullGraph &pg, uint32_t *s_hot) {
+    for (uint32_t i = threadIdx.x; i < pg.num_hot; i += blockDim.x) s_hot[i] = pg.hot_vertex[i];
+    __syncthreads();
+}
+
+__device__ __forceinline__ void flush_relaxed(const SSArgs &a, unsigned long long relaxed, int lane) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) relaxed += __shfl_xor_sync(0xffffffffu, relaxed, o);
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
+}
+
+// A sweep as a launch of its own (profiling and launch-by-launch runs).  a:
+// the solve's arguments as kernel parameters (the constant bank: no registers
+// held across the tasks).
+template <int WK>
+__global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid_constant__ SSArgs a,
+                                                                    const __grid_constant__ PullGraph pg) {
+    extern __shared__ __align__(16) uint32_t s_hot[];  // vertex ids of the hot slots (tagged sources in the CSC)
+    if (*(volatile uint32_t *)&a.hdr->done || !pull_round(a)) return;
+    load_hot_ids(pg, s_hot);
+    unsigned long long relaxed = 0;
+    Gain gain;
+    pull_sweep<WK>(a, pg, round_view(a), *(volatile const uint32_t *)&a.hdr->fmin, s_hot, relaxed, gain);
+    flush_gain(a, gain, threadIdx.x & 31);
+    flush_relaxed(a, relaxed, threadIdx.x & 31);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.hdr->pull_rounds, 1u);
+}
+
+// ---- a whole solve in one cooperative launch -------------------------------
+
+// Totals of one round's frontier.  Three of them take turns: round r reads
+// its own, fills the next round's and clears the one after (which every CTA
+// left behind at the last barrier).
+struct FrontierTotals {
+    uint32_t qsize, hub_count, fmin_inv, pad;
+    unsigned long long edges;
+};
+struct SolveState {
+    FrontierTotals round[3];
+    uint32_t barrier, pad;
+};
+
+constexpr int kSolveBatch = 8;  // 32-edge batches in flight of a push round's warp: 4 lose 5 % on 2^24 vertices, 16 spill and lose 10 %
+
+// Rounds separated by grid barriers (one after a sweep; one between expansion
+// and hub chunks and one after) in place of four launches and a conditional-
+// graph step each, most of which found nothing to do: a solve of 65 K edges
+// has 16 rounds (605 -> 318 us a call; 500 K vertices, 8 M edges: 935 -> 694
+// us).  One bucket only; the loop of launches serves finite bucket
+// widths.
+template <int WK>
+__global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __grid_constant__ SSArgs a,
+                                                                     const __grid_constant__ PullGraph pg,
+                                                                     SolveState *st, uint32_t max_rounds) {
+    extern __shared__ __align__(16) uint32_t s_hot[];
+    const int lane = threadIdx.x & 31;
+    const uint32_t gwarp = (blockIdx.x * kPullThreads + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * kPullThreads) >> 5;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    uint32_t barriers = 0;
+    load_hot_ids(pg, s_hot);
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x) {
+        const bool s = v == a.source;
+        a.dist[v] = s ? 0u : a.inf;
+        a.stamp[v] = s ? 0u : 0xFFFFFFFFu;
+    }
+    if (lead) {
+        a.queue[0][0] = a.source;
+        st->round[0].qsize = 1;
+        st->round[0].fmin_inv = ~0u;
+        st->round[0].edges = a.row_off[a.source + 1] - a.row_off[a.source];
+    }
+    bool ok = dev::grid_sync(&st->barrier, barriers);
+    unsigned long long relaxed = 0, frontier_total = 0;
+    uint32_t sweeps = 0;
+    for (uint32_t r = 0; ok; ++r) {
+        FrontierTotals *cur = &st->round[r % 3], *nxt = &st->round[(r + 1) % 3];
+        RoundView rv{};
+        rv.r = r;
+        rv.qn = __ldcg(&cur->qsize);
+        if (rv.qn == 0 || r >= max_rounds) {
+            if (lead) {
+                a.hdr->round = r;
+                a.hdr->converged = rv.qn == 0 ? 1u : 0u;
+                a.hdr->frontier_total = frontier_total;
+                a.hdr->pull_rounds = sweeps;
+                a.hdr->done = 1;
+            }
+            flush_relaxed(a, relaxed, lane);
+            return;
+        }
+        if (lead) st->round[(r + 2) % 3] = FrontierTotals{0, 0, 0, 0, 0};
+        rv.threshold = 0xFFFFFFFFu;  // one bucket
+        rv.next_stamp = r + 1;
+        rv.q = a.queue[r & 1];
+        rv.qnext = a.queue[(r + 1) & 1];
+        rv.qnext_size = &nxt->qsize;
+        rv.far = a.far[0];
+        rv.far_size = &a.hdr->fsize[0];
+        rv.far_stamp = 1;
+        frontier_total += rv.qn;
+        Gain gain;
+        if (a.pull_div && __ldcg(&cur->edges) * a.pull_div > a.num_edges) {
+            pull_sweep<WK>(a, pg, rv, ~__ldcg(&cur->fmin_inv), s_hot, relaxed, gain);
+            ++sweeps;
+        } else {
+            unsigned long long improved = 0;
+            auto hub = [&](uint32_t v, uint32_t nch) {
+                const uint32_t base = atomicAdd(&cur->hub_count, nch);
+                for (uint32_t c = 0; c < nch; ++c) a.hubs[base + c] = make_uint2(v, c);
+            };
+            for (uint32_t w = gwarp; uint64_t(w) * 32 < rv.qn; w += nwarps)
+                expand_warp<WK, false, kSolveBatch, true>(a, rv, w * 32, lane, kHubDegree, relaxed, improved, hub, &gain);
+            ok = dev::grid_sync(&st->barrier, barriers);
+            if (!ok) break;
+            const uint32_t n = __ldcg(&cur->hub_count);
+            for (uint32_t t = gwarp; t < n; t += nwarps) {
+                const uint2 h = a.hubs[t];
+                hub_chunk<WK, true, kSolveBatch>(a, rv, a.cols, a.weights, h.x, h.y, lane, improved, &gain);
+            }
+        }
+        flush_gain(&nxt->edges, &nxt->fmin_inv, gain, lane);
+        ok = dev::grid_sync(&st->barrier, barriers);
+    }
+    if (threadIdx.x == 0) atomicExch(&a.hdr->error, 1u);
 }
 
 // End of a round of a pull-capable solve (one thread): the round's kernels
@@ -481,6 +599,8 @@ int pull_grid() {
         int per_sm = 0;
         HYT_CUDA(cudaFuncSetAttribute(sssp_pull_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
+        HYT_CUDA(cudaFuncSetAttribute(sssp_solve_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kPRSmemMax)));
         HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK>, kPullThreads,
                                                                kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
@@ -512,13 +632,14 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     // each frontier vertex appears once per round: <= V rows, E/kHubChunk + V chunks
     const uint64_t hub_cap = V + g.E / kHubChunk + 2;
     if (g.hub_tasks.count < hub_cap) g.hub_tasks.allocate(hub_cap);
-    const size_t sb = 512 + sizeof(SSHeader);
+    static_assert(sizeof(SSArgs) <= 256 && sizeof(SSHeader) <= 256, "state block layout");
+    const size_t sb = 512 + sizeof(SolveState);
     if (g.sssp_state.count < sb) g.sssp_state.allocate(sb);
     SSArgs *d_args = reinterpret_cast<SSArgs *>(g.sssp_state.get());
     SSHeader *hdr = reinterpret_cast<SSHeader *>(g.sssp_state.get() + 256);
+    SolveState *solve_state = reinterpret_cast<SolveState *>(g.sssp_state.get() + 512);
 
-    SSArgs a;
-    std::memset(&a, 0, sizeof(a));  // compared bytewise below
+    SSArgs a{};
     a.row_off = g.row_offsets.get();
     a.cols = g.cols.get();
     a.weights = g.weights.get();
@@ -539,8 +660,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     const bool pull_ok = (g.flags & HYT_GRAPH_PULL) && (WK == HYT_WEIGHTS_NONE || g.in_weights.get()) &&
                          delta == kNoDelta && g.E > 0;
     a.pull_div = pull_ok ? sssp_pull_div() : 0u;
-    PullGraph pg;
-    std::memset(&pg, 0, sizeof(pg));
+    PullGraph pg{};
     if (a.pull_div) {
         pg.in_off = g.in_offsets.get();
         pg.in_src = g.in_sources.get();
@@ -551,17 +671,15 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         pg.num_tasks = g.num_chunks + g.num_tiles;
         pg.num_chunks = g.num_chunks;
         pg.num_hot = g.num_hot;
-        a.out_deg = g.out_degree.get();
     }
+    a.out_deg = g.out_degree.get();
     // row skipping: the smallest edge weight bounds what any in-edge adds
     if (a.pull_div && sssp_pull_skip()) {
         a.skip_rows = 1;
         a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_weight_range(g, WK == HYT_WEIGHTS_F32, s).low;
     }
-    const unsigned pull_smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
-    const int pgrid = a.pull_div ? pull_grid<WK>() : 0;
-    SSArgs pa = a;  // the sweep's parameter copy: nothing that changes between solves
-    pa.source = 0;
+    const unsigned pull_smem = static_cast<unsigned>(pg.num_hot * sizeof(uint32_t));
+    const int pgrid = pull_grid<WK>();
 
     SSHeader h0{};
     h0.qsize[0] = 1;
@@ -570,55 +688,57 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
     h0.threshold = (WK == HYT_WEIGHTS_F32 || delta == kNoDelta) ? 0xFFFFFFFFu : delta;
     const bool far_pile = h0.threshold != 0xFFFFFFFFu;  // labels above the threshold wait in the far pile
 
-    const bool use_graph = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
+    const bool in_graph = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
+    const bool persistent = in_graph && !far_pile;
     const int grid = expand_grid<WK>();
-    const void *expand_fn = a.pull_div ? reinterpret_cast<const void *>(sssp_expand_kernel<WK, false, true>)
-                                       : reinterpret_cast<const void *>(sssp_expand_kernel<WK>);
-    const void *hub_fn = a.pull_div ? reinterpret_cast<const void *>(sssp_hub_kernel<WK, false, true>)
-                                    : reinterpret_cast<const void *>(sssp_hub_kernel<WK>);
-    // The round loop's shape; an instantiated loop of the same shape (kept
-    // with the graph object) is launched again instead of being rebuilt.
+    // With a far pile the rounds are a conditional CUDA graph; an
+    // instantiated loop of the same shape (kept with the graph object) is
+    // launched again instead of being rebuilt.
     struct LoopKey {
-        int wk, grid, pgrid;
-        uint32_t far_pile, pull_div, pull_smem;
+        int wk, grid;
         const void *args;
-        SSArgs pa;
-        PullGraph pg;
     } key;
     std::memset(&key, 0, sizeof(key));
     key.wk = WK;
     key.grid = grid;
-    key.pgrid = pgrid;
-    key.far_pile = far_pile;
-    key.pull_div = a.pull_div;
-    key.pull_smem = pull_smem;
     key.args = d_args;
-    key.pa = pa;
-    key.pg = pg;
     LoopGraph &loop = g.sssp_loop;
-    const bool reuse = use_graph && loop.matches(&key, sizeof(key));
-    if (use_graph && !reuse) {
-        loop.reset();
-        HYT_CUDA(cudaGraphCreate(&loop.graph, 0));
-        HYT_CUDA(cudaGraphConditionalHandleCreate(&loop.cond, loop.graph, 1, cudaGraphCondAssignDefault));
-    }
-    if (use_graph) {
+    const bool reuse = in_graph && far_pile && loop.matches(&key, sizeof(key));
+    if (in_graph && far_pile) {
+        if (!reuse) {
+            loop.reset();
+            HYT_CUDA(cudaGraphCreate(&loop.graph, 0));
+            HYT_CUDA(cudaGraphConditionalHandleCreate(&loop.cond, loop.graph, 1, cudaGraphCondAssignDefault));
+        }
         a.cond = loop.cond;
         a.use_cond = 1;
     }
 
     EventTimer total;
     total.start(s);
-    HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(a), cudaMemcpyHostToDevice, s));
-    HYT_CUDA(cudaMemcpyAsync(hdr, &h0, sizeof(h0), cudaMemcpyHostToDevice, s));
-    sssp_init_kernel<<<grid_for(V, 256, 148 * 8), 256, 0, s>>>(d_args);
-    HYT_CUDA(cudaGetLastError());
     uint32_t launches = 1, hot = 0;
     double kernel_ms = 0.0;
     // split (finite bucket width), expand, hub, pull sweep + round close or round end
     const uint32_t per_round = (far_pile ? 1u : 0u) + 3u + (a.pull_div ? 1u : 0u);
 
-    if (use_graph) {
+    if (persistent) {
+        HYT_CUDA(cudaMemsetAsync(hdr, 0, sizeof(SSHeader), s));
+        HYT_CUDA(cudaMemsetAsync(solve_state, 0, sizeof(SolveState), s));
+        // every CTA must be resident; no more of them than a sweep or a full
+        // frontier has work for
+        const uint64_t work = std::max<uint64_t>(pg.num_tasks, (V + 127) / 128);
+        const unsigned ctas = static_cast<unsigned>(
+            std::min<uint64_t>(pgrid, std::max<uint64_t>(1, (work + kPullThreads / 32 - 1) / (kPullThreads / 32))));
+        void *kargs[] = {&a, &pg, &solve_state, &max_rounds};
+        HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(sssp_solve_kernel<WK>), dim3(ctas),
+                                             dim3(kPullThreads), kargs, pull_smem, s));
+    } else {
+        HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(a), cudaMemcpyHostToDevice, s));
+        HYT_CUDA(cudaMemcpyAsync(hdr, &h0, sizeof(h0), cudaMemcpyHostToDevice, s));
+        sssp_init_kernel<<<grid_for(V, 256, 148 * 8), 256, 0, s>>>(d_args);
+        HYT_CUDA(cudaGetLastError());
+    }
+    if (in_graph && far_pile) {
         if (!reuse) {
             cudaGraphNodeParams cp = {};
             cp.type = cudaGraphNodeTypeConditional;
@@ -629,36 +749,25 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
             HYT_CUDA(cudaGraphAddNode(&cnode, loop.graph, nullptr, 0, &cp));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             void *kargs[] = {&d_args};
-            cudaKernelNodeParams kp = {};
-            kp.kernelParams = kargs;
-            kp.blockDim = dim3(kSSThreads);
-            kp.gridDim = dim3(grid);
             cudaGraphNode_t prev = nullptr, node;
-            auto add = [&](const void *f, dim3 gd, dim3 bd, unsigned smem, void **params) {
+            auto add = [&](const void *f, dim3 gd, dim3 bd) {
+                cudaKernelNodeParams kp = {};
                 kp.func = const_cast<void *>(f);
                 kp.gridDim = gd;
                 kp.blockDim = bd;
-                kp.sharedMemBytes = smem;
-                kp.kernelParams = params;
+                kp.kernelParams = kargs;
                 HYT_CUDA(cudaGraphAddKernelNode(&node, body, prev ? &prev : nullptr, prev ? 1 : 0, &kp));
                 prev = node;
             };
-            void *pargs[] = {&pa, &pg};
-            // one bucket (no threshold): the far pile stays empty, nothing to split
-            if (far_pile) add(reinterpret_cast<void *>(sssp_split_kernel), dim3(grid), dim3(kSSThreads), 0, kargs);
-            add(expand_fn, dim3(grid), dim3(kSSThreads), 0, kargs);
-            add(hub_fn, dim3(grid), dim3(kSSThreads), 0, kargs);
-            if (a.pull_div) {
-                add(reinterpret_cast<void *>(sssp_pull_kernel<WK>), dim3(pgrid), dim3(kPullThreads), pull_smem, pargs);
-                add(reinterpret_cast<void *>(sssp_round_close_kernel), dim3(1), dim3(1), 0, kargs);
-            } else {
-                add(reinterpret_cast<void *>(sssp_round_end_kernel), dim3(1), dim3(1), 0, kargs);
-            }
+            add(reinterpret_cast<void *>(sssp_split_kernel), dim3(grid), dim3(kSSThreads));
+            add(reinterpret_cast<void *>(sssp_expand_kernel<WK>), dim3(grid), dim3(kSSThreads));
+            add(reinterpret_cast<void *>(sssp_hub_kernel<WK>), dim3(grid), dim3(kSSThreads));
+            add(reinterpret_cast<void *>(sssp_round_end_kernel), dim3(1), dim3(1));
             HYT_CUDA(cudaGraphInstantiate(&loop.exec, loop.graph, 0));
             loop.set_key(&key, sizeof(key));
         }
         HYT_CUDA(cudaGraphLaunch(loop.exec, s));
-    } else {
+    } else if (!persistent) {
         EventTimer kt;
         for (uint32_t r = 0; r < max_rounds; ++r) {
             if (flags & HYT_RUN_PROFILE) kt.start(s);
@@ -666,7 +775,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
             if (a.pull_div) {
                 sssp_expand_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
                 sssp_hub_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
-                sssp_pull_kernel<WK><<<pgrid, kPullThreads, pull_smem, s>>>(pa, pg);
+                sssp_pull_kernel<WK><<<pgrid, kPullThreads, pull_smem, s>>>(a, pg);
                 sssp_round_close_kernel<<<1, 1, 0, s>>>(d_args);
             } else {
                 sssp_expand_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
@@ -684,12 +793,15 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
             if (done) break;
         }
     }
-    SSHeader h{};
-    HYT_CUDA(cudaMemcpyAsync(&h, hdr, sizeof(h), cudaMemcpyDeviceToHost, s));
+    SSHeader local{};
+    SSHeader *hp = g.host_scratch.ptr ? reinterpret_cast<SSHeader *>(g.host_scratch.ptr) : &local;
+    static_assert(sizeof(SSHeader) <= 64 * sizeof(uint64_t), "the header fits the pinned readback area");
+    HYT_CUDA(cudaMemcpyAsync(hp, hdr, sizeof(SSHeader), cudaMemcpyDeviceToHost, s));
     total.stop(s);
     const double total_ms = total.ms();
-    if (use_graph) launches += per_round * h.round;
-    if (h.error) fail(HYT_E_TIMEOUT, "SSSP: a bounded wait for a staged copy ran out");
+    const SSHeader h = *hp;
+    if (in_graph && far_pile) launches += per_round * h.round;
+    if (h.error) fail(HYT_E_TIMEOUT, "SSSP: a bounded wait at a grid barrier ran out");
     if (dist_out) graph_emit(g, dist_out, g.dist.get(), s);
     if (stats) {
         stats->iterations = h.round;

@@ -49,7 +49,7 @@ struct SSHeader {
     unsigned long long frontier_total;  // frontier vertices expanded
     unsigned long long frontier_edges;  // out-edges of this round's frontier (pull-capable solves)
     uint32_t pull_rounds;               // rounds run as pull sweeps
-    uint32_t error;                     // 1: a bounded wait for a staged copy ran out
+    uint32_t error;                     // 1: a bounded wait at a grid barrier ran out
     unsigned long long frontier_edges_next;  // out-edges of the next frontier, summed at round close
     uint32_t close_ticket;                   // blocks of the round-close kernel finished
     uint32_t fmin;      // lowest label in this round's frontier (pull-capable solves with row skipping)
@@ -173,15 +173,19 @@ struct Gain {
     uint32_t low = 0xFFFFFFFFu;
 };
 
-// Adds a warp's share to the header; all 32 lanes.
-__device__ __forceinline__ void flush_gain(const SSArgs &a, Gain &g, int lane) {
+// Adds a warp's share to the next frontier's totals; all 32 lanes.
+__device__ __forceinline__ void flush_gain(unsigned long long *edges, uint32_t *fmin_inv, Gain &g, int lane) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) g.edges += __shfl_xor_sync(0xffffffffu, g.edges, o);
     g.low = __reduce_min_sync(0xffffffffu, g.low);
     if (lane == 0) {
-        if (g.edges) atomicAdd(&a.hdr->frontier_edges_next, g.edges);
-        if (g.low != 0xFFFFFFFFu) atomicMax(&a.hdr->fmin_inv, ~g.low);
+        if (g.edges) atomicAdd(edges, g.edges);
+        if (g.low != 0xFFFFFFFFu) atomicMax(fmin_inv, ~g.low);
     }
+}
+
+__device__ __forceinline__ void flush_gain(const SSArgs &a, Gain &g, int lane) {
+    flush_gain(&a.hdr->frontier_edges_next, &a.hdr->fmin_inv, g, lane);
 }
 
 // Relaxes K candidate edges per lane with all atomics of a phase in flight
@@ -311,7 +315,7 @@ __device__ __forceinline__ void expand_warp(const SSArgs &a, const RoundView &rv
 
 // One kHubChunk-edge slice (chunk c) of frontier row v, edges read from
 // hc / hw (global-edge-indexed).  Must be called by all 32 lanes.
-template <int WK, bool kTrack = false>
+template <int WK, bool kTrack = false, int kB = kHubBatch>
 __device__ __forceinline__ void hub_chunk(const SSArgs &a, const RoundView &rv, const uint32_t *hc,
                                           const uint32_t *hw, uint32_t v, uint32_t c, int lane,
                                           unsigned long long &improved, Gain *gain = nullptr) {
@@ -319,10 +323,10 @@ __device__ __forceinline__ void hub_chunk(const SSArgs &a, const RoundView &rv, 
     const uint64_t b = rb + uint64_t(c) * kHubChunk;
     const uint32_t len = static_cast<uint32_t>(((b + kHubChunk < re) ? b + kHubChunk : re) - b);
     const uint32_t d = __ldcg(a.dist + v);
-    for (uint32_t base = 0; base < len; base += 32 * kHubBatch) {
-        uint32_t u[kHubBatch], nd[kHubBatch], du[kHubBatch];
+    for (uint32_t base = 0; base < len; base += 32 * kB) {
+        uint32_t u[kB], nd[kB], du[kB];
 #pragma unroll
-        for (int k = 0; k < kHubBatch; ++k) {
+        for (int k = 0; k < kB; ++k) {
             const uint32_t j = base + 32 * k + lane;
             u[k] = 0;
             nd[k] = a.inf;
@@ -332,8 +336,8 @@ __device__ __forceinline__ void hub_chunk(const SSArgs &a, const RoundView &rv, 
             }
         }
 #pragma unroll
-        for (int k = 0; k < kHubBatch; ++k) du[k] = __ldcg(a.dist + u[k]);
-        relax_batch<kHubBatch, kTrack>(a, rv, u, nd, du, lane, improved, gain);
+        for (int k = 0; k < kB; ++k) du[k] = __ldcg(a.dist + u[k]);
+        relax_batch<kB, kTrack>(a, rv, u, nd, du, lane, improved, gain);
     }
 }
 

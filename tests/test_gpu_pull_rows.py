@@ -59,9 +59,10 @@ def test_sssp_row_degrees(hyt, oracle, gpu, order, weights):
     w = {"none": None, "u32": g.weights, "f32": (g.weights * np.float32(0.37)).astype(np.float32),
          "u32_large": (g.weights.astype(np.uint64) * 40000001).astype(np.uint32)}[weights]
     csr = hyt.CSR(g.row_offsets, g.column_indices, w)
-    with hyt.Graph(csr) as dg:
+    with hyt.Graph(csr) as dg, hyt.Graph(csr, flags=hyt.capi.HYT_GRAPH_PUSH) as push_only:
         for s in (0, 5, g.num_vertices - 1):
             d, st = dg.sssp(s)
+            assert np.array_equal(d, push_only.sssp(s)[0])
             n, _ = dg.sssp(s, flags=hyt.capi.HYT_RUN_NO_GRAPH)
             assert st["converged"] == 1 and np.array_equal(d, n)
             if weights == "u32_large":  # beyond what floats hold exactly: the push-only path
