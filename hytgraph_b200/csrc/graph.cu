@@ -34,24 +34,39 @@ __global__ void validate_offsets_kernel(const uint64_t *off, uint64_t V, uint64_
     }
 }
 
+// range[0] = smallest weight, range[1] = ~largest (bit patterns of u32 or f32
+// weights, sign of -0.0 cleared; both start at all ones).
 __global__ void validate_edges_kernel(const uint32_t *cols, const uint32_t *w, uint32_t wkind, uint64_t V,
-                                      uint64_t E, uint32_t *err, unsigned long long *weight_sum) {
+                                      uint64_t E, uint32_t *err, unsigned long long *weight_sum, uint32_t *range) {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    uint32_t bad = 0;
+    uint32_t bad = 0, lo = 0xFFFFFFFFu, hi = 0;
     unsigned long long wsum = 0;
     for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < E; e += stride) {
         if (cols[e] >= V) bad |= kBadColumn;
+        if (wkind == HYT_WEIGHTS_NONE) continue;
+        uint32_t x = w[e];
         if (wkind == HYT_WEIGHTS_F32) {
-            const float x = __uint_as_float(w[e]);
-            if (!(x >= 0.0f) || isinf(x)) bad |= kBadWeight;  // NaN fails x >= 0
-        } else if (wkind == HYT_WEIGHTS_U32) {
-            wsum += w[e];
+            const float f = __uint_as_float(x);
+            if (!(f >= 0.0f) || isinf(f)) bad |= kBadWeight;  // NaN fails f >= 0
+            x &= 0x7FFFFFFFu;
+        } else {
+            wsum += x;
         }
+        lo = min(lo, x);
+        hi = max(hi, x);
     }
     if (bad) atomicOr(err, bad);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-    if ((threadIdx.x & 31) == 0 && wsum) atomicAdd(weight_sum, wsum);
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        if (wsum) atomicAdd(weight_sum, wsum);
+        if (wkind != HYT_WEIGHTS_NONE) {
+            atomicMin(range, lo);
+            atomicMin(range + 1, ~hi);
+        }
+    }
 }
 
 __global__ void out_degree_kernel(const uint64_t *off, uint64_t V, uint32_t *deg, unsigned long long *dangling) {
@@ -184,13 +199,15 @@ __global__ void pack_pairs_kernel(const uint32_t *__restrict__ hi, const uint32_
         out[i] = (uint64_t(hi[i]) << 32) | lo[i];
 }
 
-// hi[i] = in[i] >> 32, lo[i] = in[i] & 0xFFFFFFFF.
-__global__ void unpack_pairs_kernel(const uint64_t *__restrict__ in, uint64_t n, uint32_t *__restrict__ hi,
-                                    uint32_t *__restrict__ lo) {
+// hi[i] = in[i] >> 32, lo[i] = in[i] & 0xFFFFFFFF; with bits > 0, lo[i] =
+// hi[i] | in[i] << bits (both halves in one word).
+__global__ void unpack_pairs_kernel(const uint64_t *__restrict__ in, uint64_t n, uint32_t bits,
+                                    uint32_t *__restrict__ hi, uint32_t *__restrict__ lo) {
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
         const uint64_t v = in[i];
-        hi[i] = static_cast<uint32_t>(v >> 32);
-        lo[i] = static_cast<uint32_t>(v);
+        const uint32_t h = static_cast<uint32_t>(v >> 32), l = static_cast<uint32_t>(v);
+        hi[i] = h;
+        lo[i] = bits ? (h | (l << bits)) : l;
     }
 }
 
@@ -434,6 +451,17 @@ void build_pull_tiles(GraphImpl &g, cudaStream_t s) {
     HYT_CUDA(cudaStreamSynchronize(s));
 }
 
+// Bits of a source id in packed (id, weight) words, 0 when the two do not fit
+// 32 bits together or a shortest path could reach the infinity label of
+// unpacked sums (at most V - 1 edges: labels then need saturating adds).
+static uint32_t pack_bits_for(const GraphImpl &g) {
+    if (g.weight_kind != HYT_WEIGHTS_U32) return 0;
+    const uint32_t high = g.weight_range.high;
+    const int id_bits = bits_for(g.V - 1), w_bits = bits_for(high);
+    if (id_bits + w_bits > 32 || id_bits > 31) return 0;
+    return (g.V - 1) * uint64_t(high) < HYT_DIST_INF_U32 - uint64_t(high) ? static_cast<uint32_t>(id_bits) : 0u;
+}
+
 // Tile size: large tiles cost less per edge (fewer task starts, and rows of up
 // to 1023 in-edges stay out of the chunk path), small ones leave more warps
 // something to do.  The line lies where 1024-unit tiles still give every warp
@@ -505,12 +533,16 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
     if (h_err & kBadTerminal) fail(HYT_E_INVALID, "terminal row offset must equal the number of edges");
     if (E) {
         Scratch<unsigned long long> wsum(1, s);
+        Scratch<uint32_t> range(2, s);
         HYT_CUDA(cudaMemsetAsync(wsum.get(), 0, sizeof(unsigned long long), s));
+        HYT_CUDA(cudaMemsetAsync(range.get(), 0xFF, 2 * sizeof(uint32_t), s));
         validate_edges_kernel<<<grid_for(E, 256), 256, 0, s>>>(g.cols.get(), keep_weights ? g.weights.get() : nullptr,
                                                                 keep_weights ? csr.weight_kind : 0u, V, E, err.get(),
-                                                                wsum.get());
+                                                                wsum.get(), range.get());
         HYT_CUDA(cudaGetLastError());
         unsigned long long h_wsum = 0;
+        uint32_t h_range[2] = {0, 0};
+        HYT_CUDA(cudaMemcpyAsync(h_range, range.get(), sizeof(h_range), cudaMemcpyDeviceToHost, s));
         HYT_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(h_err), cudaMemcpyDeviceToHost, s));
         HYT_CUDA(cudaMemcpyAsync(&h_wsum, wsum.get(), sizeof(h_wsum), cudaMemcpyDeviceToHost, s));
         HYT_CUDA(cudaStreamSynchronize(s));
@@ -518,6 +550,7 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         // Negative / non-finite float weights are legal for PageRank; SSSP
         // rejects them when it is called (reference: sssp.cpp:117-124).
         g.weights_ok = (h_err & kBadWeight) == 0;
+        if (keep_weights) g.weight_range = WeightRange{h_range[0], ~h_range[1]};
         if (keep_weights && csr.weight_kind == HYT_WEIGHTS_U32) {
             const double mean = static_cast<double>(h_wsum) / static_cast<double>(E);
             g.default_delta = static_cast<uint32_t>(std::min(4.0e9, std::max(1.0, 2.0 * mean)));
@@ -554,7 +587,8 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
                 }
                 prims::sort_pairs_u32_u64(keys.get(), sw.get(), E, bits_for(V - 1), s);
                 g.in_weights.allocate(E);
-                unpack_pairs_kernel<<<grid_for(E, 256), 256, 0, s>>>(sw.get(), E, g.in_sources.get(),
+                g.in_pack_bits = pack_bits_for(g);
+                unpack_pairs_kernel<<<grid_for(E, 256), 256, 0, s>>>(sw.get(), E, g.in_pack_bits, g.in_sources.get(),
                                                                       g.in_weights.get());
                 HYT_CUDA(cudaGetLastError());
                 HYT_CUDA(cudaStreamSynchronize(s));

@@ -134,7 +134,11 @@ struct GraphImpl {
     // pull side
     GraphArray<uint64_t> in_offsets;
     GraphArray<uint32_t> in_sources;
-    GraphArray<uint32_t> in_weights;   // [E] weights in CSC order (PUSH|PULL weighted graphs; SSSP pull rounds)
+    // [E] weights in CSC order (PUSH|PULL weighted graphs; SSSP pull rounds).
+    // in_pack_bits > 0: (source id | weight << in_pack_bits) in one word, with
+    // which a sweep loads one stream in place of two and looks up no hot slot.
+    GraphArray<uint32_t> in_weights;
+    uint32_t in_pack_bits = 0;
     GraphArray<uint32_t> tile_start;   // [num_tiles + 1]
     GraphArray<LongRow> long_rows;     // [num_long]
     GraphArray<uint2> chunk_tasks;     // [num_chunks] = (long row index, chunk)
@@ -169,8 +173,7 @@ struct GraphImpl {
     GraphArray<uint32_t> ppr_wide;         // packed PPR: rows of 32+ in-edges below the long-row threshold
     uint64_t ppr_wide_n = 0;
     bool ppr_wide_ready = false;
-    WeightRange weight_range;              // of the CSC weights
-    bool weight_range_ready = false;
+    WeightRange weight_range;              // of the weights kept
     GraphArray<uint32_t> ms_dist;          // multi-source labels [V][8]
     GraphArray<unsigned char> ms_state;
     PinnedArray<uint64_t> host_scratch;  // small pinned readback area

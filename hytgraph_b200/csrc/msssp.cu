@@ -91,6 +91,7 @@ struct MSArgs {
     uint32_t num_hot;
     uint32_t skip_rows;  // 1: sweeps skip rows whose labels no in-edge can lower
     uint32_t min_w;      // smallest edge weight (bit pattern; 1 when unweighted)
+    uint32_t bits;       // packed words in in_w: bits of the source id
 };
 
 struct Row8 {
@@ -354,9 +355,9 @@ constexpr uint32_t kWideRow = 16 * kPullN;  // rows with this many in-edges are 
 
 // In-edges of one task, addressed relative to its first edge.
 struct InEdges {
-    const uint32_t *src, *w, *s_hot;
+    const uint32_t *src, *w, *s_hot;  // ids and weights, or w: packed words (no hot slots)
     const uint32_t *dist;
-    uint32_t inf;
+    uint32_t inf, bits;
 };
 
 // Minimum of the candidates of edges b, b + step, ..., capped at edge `last`
@@ -364,13 +365,23 @@ struct InEdges {
 template <int WK, bool kB>
 __device__ __forceinline__ void edges_min(const InEdges &E, uint32_t b, uint32_t last, uint32_t step, Row8 &m) {
     uint32_t u[kPullN], wt[kPullN];
+    if constexpr (kB && WK == HYT_WEIGHTS_U32) {
+        const uint32_t mask = (1u << E.bits) - 1u;
 #pragma unroll
-    for (int j = 0; j < kPullN; ++j) u[j] = dev::ld_stream(E.src + min(b + j * step, last));
+        for (int j = 0; j < kPullN; ++j) {
+            const uint32_t x = dev::ld_stream(E.w + min(b + j * step, last));
+            u[j] = x & mask;
+            wt[j] = x >> E.bits;
+        }
+    } else {
 #pragma unroll
-    for (int j = 0; j < kPullN; ++j) wt[j] = ssc::edge_weight<WK>(E.w, min(b + j * step, last));
+        for (int j = 0; j < kPullN; ++j) u[j] = dev::ld_stream(E.src + min(b + j * step, last));
 #pragma unroll
-    for (int j = 0; j < kPullN; ++j)
-        if (u[j] & kHotTag) u[j] = E.s_hot[u[j] & ~kHotTag];
+        for (int j = 0; j < kPullN; ++j) wt[j] = ssc::edge_weight<WK>(E.w, min(b + j * step, last));
+#pragma unroll
+        for (int j = 0; j < kPullN; ++j)
+            if (u[j] & kHotTag) u[j] = E.s_hot[u[j] & ~kHotTag];
+    }
     Row8 du[kPullN];
 #pragma unroll
     for (int j = 0; j < kPullN; ++j) {
@@ -470,8 +481,10 @@ __global__ void __launch_bounds__(kMPThreads, 1) ms_pull_kernel(const MSArgs *__
     }
     __syncthreads();
     const uint64_t nwarps = uint64_t(gridDim.x) * (kMPThreads / 32);
-    const uint32_t *pf_w = (WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w;
-    InEdges E{nullptr, nullptr, s_hot, a.dist, a.inf};
+    constexpr bool kPacked = kB && WK == HYT_WEIGHTS_U32;
+    const uint32_t *pf_a = kPacked ? a.in_w : a.in_src;
+    const uint32_t *pf_w = (kPacked || WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w;
+    InEdges E{nullptr, nullptr, s_hot, a.dist, a.inf, a.bits};
     unsigned long long relaxed = 0;  // in-edges relaxed (chunks counted by lane 0, tile rows by their lanes)
     Gain gain;
     uint64_t task = uint64_t(blockIdx.x) * (kMPThreads / 32) + warp;
@@ -482,7 +495,7 @@ __global__ void __launch_bounds__(kMPThreads, 1) ms_pull_kernel(const MSArgs *__
         const uint64_t e0 = task_first_edge(d);
         E.src = a.in_src + e0;
         E.w = (WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w + e0;
-        prefetch_task(nd, a.in_src, pf_w, lane);
+        prefetch_task(nd, pf_a, pf_w, lane);
         if (task_is_chunk(d)) {
             const uint32_t r = a.long_rows[d.z].row, n = task_edges(d);
             uint32_t settled = 0;
@@ -669,14 +682,15 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
         a.long_rows = g.long_rows.get();
         a.tasks = g.pull_tasks.get();
         a.num_tasks = g.num_chunks + g.num_tiles;
-        a.num_hot = g.num_hot;
+        a.bits = g.in_pack_bits;
+        a.num_hot = a.bits ? 0u : g.num_hot;
     }
     if (pull_ok) {
         a.out_deg = g.out_degree.get();
         a.skip_rows = sssp_pull_skip() ? 1u : 0u;
-        if (a.skip_rows) a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_weight_range(g, WK == HYT_WEIGHTS_F32, s).low;
+        if (a.skip_rows) a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : g.weight_range.low;
     }
-    const unsigned pull_smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
+    const unsigned pull_smem = static_cast<unsigned>(a.num_hot * sizeof(uint32_t));
     static bool attr = false;
     if (!attr) {
         HYT_CUDA(cudaFuncSetAttribute(ms_pull_kernel<WK, kB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -798,11 +812,10 @@ void sssp_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_
     if (!g.weights_ok) fail(HYT_E_INVALID, "SSSP requires finite non-negative edge weights");
     const uint64_t cap = std::min<uint64_t>(4 * g.V + 1024, 0x7FFFFFFFull);
     const uint32_t rounds = max_rounds ? max_rounds : static_cast<uint32_t>(cap);
-    // bounded labels: a path has at most V - 1 edges (candidate)
-    const uint32_t max_w = g.weight_kind == HYT_WEIGHTS_NONE ? 1u
-                           : g.weight_kind == HYT_WEIGHTS_U32 && g.in_weights.get() ? graph_weight_range(g, false, s).high
-                                                                                    : 0xFFFFFFFFu;
-    const bool bounded = max_w < 0x80000000u && (g.V - 1) * uint64_t(max_w) < HYT_DIST_INF_U32 - max_w;
+    // bounded labels: packed words say so for u32 weights; unweighted paths
+    // have at most V - 1 edges
+    const uint32_t max_w = g.weight_kind == HYT_WEIGHTS_NONE ? 1u : g.weight_range.high;
+    const bool bounded = g.weight_kind == HYT_WEIGHTS_NONE ? g.V < HYT_DIST_INF_U32 : g.in_pack_bits > 0;
     switch (g.weight_kind) {
         case HYT_WEIGHTS_NONE:
             if (bounded)

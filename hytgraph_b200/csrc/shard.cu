@@ -177,6 +177,7 @@ struct SSPull {
     uint64_t chunk_begin, chunk_end, tile_begin, tile_end;
     uint64_t edges;  // in-edges of the sweep's rows
     uint32_t num_hot;
+    uint32_t bits, inf;  // packed words: bits of the source id, infinity label of the sweep
 };
 
 // Same answer in every kernel of a round and on every shard (the count is
@@ -314,7 +315,7 @@ __device__ __forceinline__ void shard_pull_relax(const SSShard &a, uint32_t r, u
 // its in-edges of d[u] + w (the single-GPU sweep's task decomposition and row
 // minima, sssp_pull.cuh; the chunks of a long row meet in an atomic min).
 // Nothing in a push round.
-template <int WK>
+template <int WK, bool kPacked>
 __global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(const __grid_constant__ SSShard a,
                                                                         const __grid_constant__ SSPull p) {
     extern __shared__ __align__(16) uint32_t s_hot[];
@@ -323,8 +324,12 @@ __global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(const __
     for (uint32_t i = threadIdx.x; i < p.num_hot; i += blockDim.x) s_hot[i] = p.hot_vertex[i];
     __syncthreads();
     const uint64_t pol = dev::policy_evict_last();
+    // packed words: unreached labels are lowered to an infinity that leaves
+    // room for one more weight, and candidates from it never reach a row below
+    const uint32_t inf = kPacked ? p.inf : a.inf;
     const auto label = [&](uint32_t u) {
-        return dev::ld_keep_u32(reinterpret_cast<const uint32_t *>(a.keys) + u, pol) ^ kKeyBias;
+        const uint32_t d = dev::ld_keep_u32(reinterpret_cast<const uint32_t *>(a.keys) + u, pol) ^ kKeyBias;
+        return kPacked ? min(d, inf) : d;
     };
     const uint64_t n_chunks = p.chunk_end - p.chunk_begin;
     const uint64_t total = n_chunks + (p.tile_end - p.tile_begin);
@@ -332,10 +337,10 @@ __global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(const __
     for (uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp; task < total; task += nwarps) {
         const uint4 d = p.tasks[task < n_chunks ? p.chunk_begin + task : p.num_chunks + p.tile_begin + (task - n_chunks)];
         const uint64_t e0 = task_first_edge(d);
-        const ssp::InEdges E{p.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : p.in_w + e0, s_hot};
+        const ssp::InEdges E{p.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : p.in_w + e0, s_hot, p.bits, inf};
         if (task < n_chunks) {
-            const uint32_t best = ssp::span_min<WK>(E, 0, task_edges(d), a.inf, label, lane);
-            if (lane == 0) shard_pull_relax(a, p.long_rows[d.z].row, best);
+            const uint32_t best = ssp::span_min<WK, kPacked>(E, 0, task_edges(d), label, lane);
+            if (lane == 0 && best < inf) shard_pull_relax(a, p.long_rows[d.z].row, best);
             continue;
         }
         for (uint32_t rb = d.z; rb < d.w; rb += 32) {
@@ -345,8 +350,8 @@ __global__ void __launch_bounds__(kPRThreads, 1) shard_sssp_pull_kernel(const __
                 lo = static_cast<uint32_t>(p.in_off[r] - e0);
                 hi = static_cast<uint32_t>(p.in_off[r + 1] - e0);
             }
-            const uint32_t best = ssp::rows_min<WK>(E, lo, hi, a.inf, label, lane);
-            if (r < d.w) shard_pull_relax(a, r, best);
+            const uint32_t best = ssp::rows_min<WK, kPacked>(E, lo, hi, label, lane);
+            if (r < d.w && best < inf) shard_pull_relax(a, r, best);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.edges) atomicAdd(&a.ctr[2], static_cast<unsigned long long>(p.edges));
@@ -392,7 +397,9 @@ SSPull pull_view(const ShardImpl &sh) {
     p.tile_begin = sh.tile_begin;
     p.tile_end = sh.tile_end;
     p.edges = sh.pull_edges;
-    p.num_hot = g.num_hot;
+    p.num_hot = g.in_pack_bits ? 0u : g.num_hot;
+    p.bits = g.in_pack_bits;
+    p.inf = HYT_DIST_INF_U32 - g.weight_range.high;
     return p;
 }
 
@@ -654,10 +661,16 @@ void launch_relax(const ShardImpl &sh, const SSShard &a, cudaStream_t s) {
     const SSPull p = pull_view(sh);
     const uint64_t tasks = (p.chunk_end - p.chunk_begin) + (p.tile_end - p.tile_begin);
     if (tasks == 0) return;
-    static const int full = pull_grid_for(reinterpret_cast<const void *>(shard_sssp_pull_kernel<WK>));
+    const bool packed = WK == HYT_WEIGHTS_U32 && p.bits;
+    static const int full[2] = {
+        pull_grid_for(reinterpret_cast<const void *>(shard_sssp_pull_kernel<WK, false>)),
+        pull_grid_for(reinterpret_cast<const void *>(shard_sssp_pull_kernel<WK, WK == HYT_WEIGHTS_U32>))};
     const uint64_t want = (tasks + kPRThreads / 32 - 1) / (kPRThreads / 32);
-    const int grid = static_cast<int>(std::min<uint64_t>(full, want));
-    shard_sssp_pull_kernel<WK><<<grid, kPRThreads, p.num_hot * sizeof(uint32_t), s>>>(a, p);
+    const int grid = static_cast<int>(std::min<uint64_t>(full[packed], want));
+    if (packed)
+        shard_sssp_pull_kernel<WK, WK == HYT_WEIGHTS_U32><<<grid, kPRThreads, 0, s>>>(a, p);
+    else
+        shard_sssp_pull_kernel<WK, false><<<grid, kPRThreads, p.num_hot * sizeof(uint32_t), s>>>(a, p);
     HYT_CUDA(cudaGetLastError());
 }
 

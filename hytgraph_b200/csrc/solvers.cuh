@@ -12,8 +12,6 @@ void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart,
 void sssp_run(GraphImpl &g, const hyt_sssp_params &p, uint32_t *dist_out, hyt_run_stats *stats);
 // Row skipping in pull sweeps (HYT_SSSP_PULL_SKIP).
 bool sssp_pull_skip();
-// Smallest and largest CSC weight (bit patterns), found once per graph.
-WeightRange graph_weight_range(GraphImpl &g, bool f32, cudaStream_t s);
 void sssp_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_rounds, uint32_t flags,
                 cudaStream_t s, uint32_t *out, hyt_run_stats *stats);
 void sssp_noalloc(const hyt_csr &csr, uint32_t source, uint32_t *dist_out, void *stream, hyt_run_stats *stats);

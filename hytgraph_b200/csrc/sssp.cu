@@ -142,12 +142,14 @@ __global__ void __launch_bounds__(kSSThreads) sssp_hub_kernel(const SSArgs *__re
 struct PullGraph {
     const uint64_t *in_off;
     const uint32_t *in_src;   // hot sources tagged kHotTag | slot
-    const uint32_t *in_w;     // weights in CSC order (NULL when unweighted)
+    const uint32_t *in_w;     // weights in CSC order (NULL when unweighted), or packed words
     const LongRow *long_rows;
     const uint32_t *hot_vertex;
     const uint4 *tasks;       // pull task descriptors: chunks of long rows, then tiles
     uint64_t num_tasks, num_chunks;
+    uint64_t dealt;           // tasks dealt to the warps in turn; the rest go to whoever is free
     uint32_t num_hot;
+    uint32_t bits;            // packed words: bits of the source id
 };
 
 
@@ -193,30 +195,41 @@ __device__ __forceinline__ uint32_t skip_bound(const SSArgs &a, uint32_t fmin, b
 // Labels are read live, not from a snapshot: rows lowered early in a sweep
 // feed the rows after them (a snapshot of the hottest labels in shared memory
 // cost a round).
-template <int WK>
+// Tasks cost uneven amounts (rows skipped, mixed degrees), so only the first
+// pg.dealt are dealt in turn; the others are taken one by one from `cursor`
+// (on R-MAT in input order a quarter of the warps' time went idle at the end
+// of a sweep).
+template <int WK, bool kPacked>
 __device__ __forceinline__ void pull_sweep(const SSArgs &a, const PullGraph &pg, const RoundView &rv, uint32_t fmin,
-                                           const uint32_t *s_hot, unsigned long long &relaxed, Gain &gain) {
+                                           const uint32_t *s_hot, uint32_t *cursor, unsigned long long &relaxed,
+                                           Gain &gain) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t pol = dev::policy_evict_last();
     const auto label = [&](uint32_t u) { return dev::ld_keep_u32(a.dist + u, pol); };
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPullThreads / 32);
-    const uint32_t *pf_w = (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w;
+    const uint32_t *pf_a = kPacked ? pg.in_w : pg.in_src;
+    const uint32_t *pf_w = (kPacked || WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w;
     bool skip_on;
     const uint32_t skip_at = skip_bound<WK>(a, fmin, skip_on);
+    const uint64_t dealt = max(pg.dealt, min(pg.num_tasks, nwarps));  // every warp's first task is dealt
     uint64_t task = uint64_t(blockIdx.x) * (kPullThreads / 32) + warp;
-    // each task's descriptor is read while the task before it runs
+    // each dealt task's descriptor is read while the task before it runs
     uint4 d = task < pg.num_tasks ? pg.tasks[task] : make_uint4(0, 0, 0, 0);
-    for (; task < pg.num_tasks; task += nwarps) {
-        const uint64_t next = task + nwarps;
-        const uint4 nd = next < pg.num_tasks ? pg.tasks[next] : make_uint4(0, 0, 0, 0);
+    while (task < pg.num_tasks) {
+        // the next task: dealt, or asked for now and looked at when this one is done
+        uint64_t next = task + nwarps;
+        uint32_t ticket = 0;
+        const bool ask = next >= dealt;
+        if (ask && lane == 0) ticket = atomicAdd(cursor, 1u);
+        uint4 nd = ask ? make_uint4(0, 0, 0, 0) : pg.tasks[next];
         const uint64_t e0 = task_first_edge(d);
-        const ssp::InEdges E{pg.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w + e0, s_hot};
+        const ssp::InEdges E{pg.in_src + e0, (WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w + e0, s_hot, pg.bits, a.inf};
         if (task_is_chunk(d)) {
             // slice of a long row: warp minimum, then one relaxation
             const uint32_t r = pg.long_rows[d.z].row, n = task_edges(d);
-            prefetch_task(nd, pg.in_src, pf_w, lane);
+            if (!ask) prefetch_task(nd, pf_a, pf_w, lane);
             if (!(skip_on && __shfl_sync(0xffffffffu, __ldcg(a.dist + r), 0) <= skip_at)) {
-                const uint32_t best = ssp::span_min<WK>(E, 0, n, a.inf, label, lane);
+                const uint32_t best = ssp::span_min<WK, kPacked>(E, 0, n, label, lane);
                 if (lane == 0) {
                     relaxed += n;
                     if (best < a.inf) {
@@ -243,14 +256,14 @@ __device__ __forceinline__ void pull_sweep(const SSArgs &a, const PullGraph &pg,
                 }
             };
             load_row(d.z + lane, lo, hi, seen);
-            prefetch_task(nd, pg.in_src, pf_w, lane);
+            if (!ask) prefetch_task(nd, pf_a, pf_w, lane);
             for (uint32_t rb = d.z; rb < rl; rb += 32) {
                 uint32_t lo_n, hi_n, seen_n;
                 load_row(rb + 32 + lane, lo_n, hi_n, seen_n);
                 const uint32_t r = rb + lane;
                 if (skip_on && seen <= skip_at) hi = lo;  // no in-edge can lower it: neither read nor gathered
                 relaxed += hi - lo;
-                const uint32_t best = ssp::rows_min<WK>(E, lo, hi, a.inf, label, lane);
+                const uint32_t best = ssp::rows_min<WK, kPacked>(E, lo, hi, label, lane);
                 const bool joined = r < rl && pull_store(a, rv, r, best, seen);
                 if (joined) {
                     gain.low = min(gain.low, best);
@@ -263,6 +276,11 @@ __device__ __forceinline__ void pull_sweep(const SSArgs &a, const PullGraph &pg,
                 seen = seen_n;
             }
         }
+        if (ask) {
+            next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
+            if (next < pg.num_tasks) nd = pg.tasks[next];
+        }
+        task = next;
         d = nd;
     }
 }
@@ -282,7 +300,7 @@ __device__ __forceinline__ void flush_relaxed(const SSArgs &a, unsigned long lon
 // A sweep as a launch of its own (profiling and launch-by-launch runs).  a:
 // the solve's arguments as kernel parameters (the constant bank: no registers
 // held across the tasks).
-template <int WK>
+template <int WK, bool kPacked>
 __global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid_constant__ SSArgs a,
                                                                     const __grid_constant__ PullGraph pg) {
     extern __shared__ __align__(16) uint32_t s_hot[];  // vertex ids of the hot slots (tagged sources in the CSC)
@@ -290,7 +308,8 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid
     load_hot_ids(pg, s_hot);
     unsigned long long relaxed = 0;
     Gain gain;
-    pull_sweep<WK>(a, pg, round_view(a), *(volatile const uint32_t *)&a.hdr->fmin, s_hot, relaxed, gain);
+    pull_sweep<WK, kPacked>(a, pg, round_view(a), *(volatile const uint32_t *)&a.hdr->fmin, s_hot,
+                            &a.hdr->task_cursor, relaxed, gain);
     flush_gain(a, gain, threadIdx.x & 31);
     flush_relaxed(a, relaxed, threadIdx.x & 31);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.hdr->pull_rounds, 1u);
@@ -302,7 +321,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_pull_kernel(const __grid
 // its own, fills the next round's and clears the one after (which every CTA
 // left behind at the last barrier).
 struct FrontierTotals {
-    uint32_t qsize, hub_count, fmin_inv, pad;
+    uint32_t qsize, hub_count, fmin_inv, task_cursor;
     unsigned long long edges;
 };
 struct SolveState {
@@ -318,7 +337,7 @@ constexpr int kSolveBatch = 8;  // 32-edge batches in flight of a push round's w
 // has 16 rounds (605 -> 318 us a call; 500 K vertices, 8 M edges: 935 -> 694
 // us).  One bucket only; the loop of launches serves finite bucket
 // widths.
-template <int WK>
+template <int WK, bool kPacked>
 __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __grid_constant__ SSArgs a,
                                                                      const __grid_constant__ PullGraph pg,
                                                                      SolveState *st, uint32_t max_rounds) {
@@ -349,6 +368,9 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __gri
         rv.r = r;
         rv.qn = __ldcg(&cur->qsize);
         if (rv.qn == 0 || r >= max_rounds) {
+            if constexpr (kPacked)  // the solve's own infinity becomes the caller's
+                for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.V; v += gridDim.x * blockDim.x)
+                    if (__ldcg(a.dist + v) >= a.inf) a.dist[v] = HYT_DIST_INF_U32;
             if (lead) {
                 a.hdr->round = r;
                 a.hdr->converged = rv.qn == 0 ? 1u : 0u;
@@ -371,7 +393,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __gri
         frontier_total += rv.qn;
         Gain gain;
         if (a.pull_div && __ldcg(&cur->edges) * a.pull_div > a.num_edges) {
-            pull_sweep<WK>(a, pg, rv, ~__ldcg(&cur->fmin_inv), s_hot, relaxed, gain);
+            pull_sweep<WK, kPacked>(a, pg, rv, ~__ldcg(&cur->fmin_inv), s_hot, &cur->task_cursor, relaxed, gain);
             ++sweeps;
         } else {
             unsigned long long improved = 0;
@@ -407,9 +429,16 @@ __global__ void sssp_round_close_kernel(const SSArgs *__restrict__ args) {
     h->frontier_edges_next = 0;
     h->fmin = ~h->fmin_inv;  // all ones when the next frontier is empty
     h->fmin_inv = 0;
+    h->task_cursor = 0;
     const bool finish = round_end(h);
     h->frontier_edges = fe;
     if (finish && a.use_cond) cudaGraphSetConditional(a.cond, 0);
+}
+
+// Unreached labels (inf or above) as the caller's infinity.
+__global__ void sssp_unreached_kernel(uint32_t *dist, uint32_t V, uint32_t inf) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+        if (dist[v] >= inf) dist[v] = HYT_DIST_INF_U32;
 }
 
 __global__ void sssp_round_end_kernel(const SSArgs *__restrict__ args) {
@@ -534,23 +563,6 @@ __global__ void __launch_bounds__(kSSThreads) sssp_expand_packed_kernel(const SS
     if (lane == 0 && relaxed) atomicAdd(&a.hdr->relaxations, relaxed);
 }
 
-// Smallest and largest of n weights (bit patterns of u32 or non-negative f32
-// weights; -0.0 counts as 0) into out[0] and ~out[1], which start at all ones.
-__global__ void weight_range_kernel(const uint32_t *__restrict__ w, uint64_t n, uint32_t f32, uint32_t *out) {
-    uint32_t lo = 0xFFFFFFFFu, hi = 0;
-    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t x = f32 ? (__ldcs(w + i) & 0x7FFFFFFFu) : __ldcs(w + i);
-        lo = min(lo, x);
-        hi = max(hi, x);
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(out, lo);
-        atomicMin(out + 1, ~hi);
-    }
-}
-
 }  // namespace
 
 // Row skipping in pull sweeps (env HYT_SSSP_PULL_SKIP, 0 = off; default on).
@@ -560,23 +572,6 @@ bool sssp_pull_skip() {
         return !(e && e[0] == '0');
     }();
     return on;
-}
-
-WeightRange graph_weight_range(GraphImpl &g, bool f32, cudaStream_t s) {
-    if (!g.weight_range_ready) {
-        Scratch<uint32_t> m(2, s);
-        HYT_CUDA(cudaMemsetAsync(m.get(), 0xFF, 2 * sizeof(uint32_t), s));
-        weight_range_kernel<<<grid_for(g.E, 256, 148 * 8), 256, 0, s>>>(g.in_weights.get(), g.E, f32 ? 1u : 0u,
-                                                                         m.get());
-        HYT_CUDA(cudaGetLastError());
-        uint32_t local[2] = {0, 0};
-        uint32_t *h = g.host_scratch.ptr ? reinterpret_cast<uint32_t *>(g.host_scratch.ptr) : local;
-        HYT_CUDA(cudaMemcpyAsync(h, m.get(), 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        HYT_CUDA(cudaStreamSynchronize(s));
-        g.weight_range = WeightRange{h[0], ~h[1]};
-        g.weight_range_ready = true;
-    }
-    return g.weight_range;
 }
 
 namespace {
@@ -592,16 +587,16 @@ uint32_t sssp_pull_div() {
     return div;
 }
 
-template <int WK>
+template <int WK, bool kPacked>
 int pull_grid() {
     static int grid = 0;
     if (grid == 0) {
         int per_sm = 0;
-        HYT_CUDA(cudaFuncSetAttribute(sssp_pull_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HYT_CUDA(cudaFuncSetAttribute(sssp_pull_kernel<WK, kPacked>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaFuncSetAttribute(sssp_solve_kernel<WK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HYT_CUDA(cudaFuncSetAttribute(sssp_solve_kernel<WK, kPacked>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK>, kPullThreads,
+        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK, kPacked>, kPullThreads,
                                                                kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
     }
@@ -619,7 +614,9 @@ int expand_grid() {
     return g;
 }
 
-template <int WK>
+// kPacked: the graph keeps packed words, so its labels cannot wrap; sweeps use
+// an infinity that leaves room for one more weight.
+template <int WK, bool kPacked>
 void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_rounds, uint32_t flags, cudaStream_t s,
                 uint32_t *dist_out, hyt_run_stats *stats) {
     const uint64_t V = g.V;
@@ -670,16 +667,19 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         pg.tasks = g.pull_tasks.get();
         pg.num_tasks = g.num_chunks + g.num_tiles;
         pg.num_chunks = g.num_chunks;
-        pg.num_hot = g.num_hot;
+        pg.dealt = pg.num_tasks - pg.num_tasks / 4;
+        pg.num_hot = kPacked ? 0u : g.num_hot;
+        pg.bits = g.in_pack_bits;
+        if (kPacked) a.inf = HYT_DIST_INF_U32 - g.weight_range.high;
     }
     a.out_deg = g.out_degree.get();
     // row skipping: the smallest edge weight bounds what any in-edge adds
     if (a.pull_div && sssp_pull_skip()) {
         a.skip_rows = 1;
-        a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : graph_weight_range(g, WK == HYT_WEIGHTS_F32, s).low;
+        a.min_w = (WK == HYT_WEIGHTS_NONE) ? 1u : g.weight_range.low;
     }
     const unsigned pull_smem = static_cast<unsigned>(pg.num_hot * sizeof(uint32_t));
-    const int pgrid = pull_grid<WK>();
+    const int pgrid = pull_grid<WK, kPacked>();
 
     SSHeader h0{};
     h0.qsize[0] = 1;
@@ -730,7 +730,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         const unsigned ctas = static_cast<unsigned>(
             std::min<uint64_t>(pgrid, std::max<uint64_t>(1, (work + kPullThreads / 32 - 1) / (kPullThreads / 32))));
         void *kargs[] = {&a, &pg, &solve_state, &max_rounds};
-        HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(sssp_solve_kernel<WK>), dim3(ctas),
+        HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(sssp_solve_kernel<WK, kPacked>), dim3(ctas),
                                              dim3(kPullThreads), kargs, pull_smem, s));
     } else {
         HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(a), cudaMemcpyHostToDevice, s));
@@ -775,7 +775,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
             if (a.pull_div) {
                 sssp_expand_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
                 sssp_hub_kernel<WK, false, true><<<grid, kSSThreads, 0, s>>>(d_args);
-                sssp_pull_kernel<WK><<<pgrid, kPullThreads, pull_smem, s>>>(a, pg);
+                sssp_pull_kernel<WK, kPacked><<<pgrid, kPullThreads, pull_smem, s>>>(a, pg);
                 sssp_round_close_kernel<<<1, 1, 0, s>>>(d_args);
             } else {
                 sssp_expand_kernel<WK><<<grid, kSSThreads, 0, s>>>(d_args);
@@ -792,6 +792,10 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
             if (flags & HYT_RUN_PROFILE) kernel_ms += kt.ms();
             if (done) break;
         }
+    }
+    if (kPacked && !persistent && a.inf != HYT_DIST_INF_U32) {
+        sssp_unreached_kernel<<<grid_for(V, 256, 148 * 8), 256, 0, s>>>(a.dist, a.V, a.inf);
+        HYT_CUDA(cudaGetLastError());
     }
     SSHeader local{};
     SSHeader *hp = g.host_scratch.ptr ? reinterpret_cast<SSHeader *>(g.host_scratch.ptr) : &local;
@@ -843,9 +847,15 @@ void sssp_run(GraphImpl &g, const hyt_sssp_params &p, uint32_t *dist_out, hyt_ru
     const uint32_t delta = p.delta ? p.delta : sssp_default_delta(g);
     const uint32_t src = graph_vertex(g, p.source, s);
     switch (g.weight_kind) {
-        case HYT_WEIGHTS_NONE: sssp_solve<HYT_WEIGHTS_NONE>(g, src, delta, max_rounds, p.flags, s, dist_out, stats); break;
-        case HYT_WEIGHTS_U32: sssp_solve<HYT_WEIGHTS_U32>(g, src, delta, max_rounds, p.flags, s, dist_out, stats); break;
-        case HYT_WEIGHTS_F32: sssp_solve<HYT_WEIGHTS_F32>(g, src, kNoDelta, max_rounds, p.flags, s, dist_out, stats); break;
+        case HYT_WEIGHTS_NONE: sssp_solve<HYT_WEIGHTS_NONE, false>(g, src, delta, max_rounds, p.flags, s, dist_out, stats); break;
+        case HYT_WEIGHTS_U32:
+            // sweeps run with one bucket only; other solves do not read the CSC
+            if (g.in_pack_bits && delta == kNoDelta)
+                sssp_solve<HYT_WEIGHTS_U32, true>(g, src, delta, max_rounds, p.flags, s, dist_out, stats);
+            else
+                sssp_solve<HYT_WEIGHTS_U32, false>(g, src, delta, max_rounds, p.flags, s, dist_out, stats);
+            break;
+        case HYT_WEIGHTS_F32: sssp_solve<HYT_WEIGHTS_F32, false>(g, src, kNoDelta, max_rounds, p.flags, s, dist_out, stats); break;
         default: fail(HYT_E_INTERNAL, "unknown weight kind");
     }
 }
