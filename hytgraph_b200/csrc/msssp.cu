@@ -59,7 +59,7 @@ struct MSHeader {
     unsigned long long relaxations;     // push: frontier out-edges; pull: in-edges of the rows not skipped
     unsigned long long frontier_total;  // frontier vertices expanded
     unsigned long long frontier_edges;  // out-edges of this round's frontier
-    uint32_t pull_rounds, pad;
+    uint32_t pull_rounds, task_cursor;  // task_cursor: pull tasks handed out beyond the dealt ones
     unsigned long long frontier_edges_next;  // out-edges of the next frontier, summed by the kernels that fill it
     uint32_t fmin[kML];      // lowest label of this round's frontier, per lane
     uint32_t fmin_inv[kML];  // ~(lowest label of the next frontier)
@@ -87,7 +87,7 @@ struct MSArgs {
     const LongRow *long_rows;
     const uint4 *tasks;
     const uint32_t *out_deg;
-    uint64_t num_tasks;
+    uint64_t num_tasks, dealt;  // dealt: dealt_tasks
     uint32_t num_hot;
     uint32_t skip_rows;  // 1: sweeps skip rows whose labels no in-edge can lower
     uint32_t min_w;      // smallest edge weight (bit pattern; 1 when unweighted)
@@ -487,15 +487,19 @@ __global__ void __launch_bounds__(kMPThreads, 1) ms_pull_kernel(const MSArgs *__
     InEdges E{nullptr, nullptr, s_hot, a.dist, a.inf, a.bits};
     unsigned long long relaxed = 0;  // in-edges relaxed (chunks counted by lane 0, tile rows by their lanes)
     Gain gain;
+    const uint64_t dealt = max(a.dealt, min(a.num_tasks, nwarps));
     uint64_t task = uint64_t(blockIdx.x) * (kMPThreads / 32) + warp;
     uint4 d = task < a.num_tasks ? a.tasks[task] : make_uint4(0, 0, 0, 0);
-    for (; task < a.num_tasks; task += nwarps) {
-        const uint64_t next = task + nwarps;
-        const uint4 nd = next < a.num_tasks ? a.tasks[next] : make_uint4(0, 0, 0, 0);
+    while (task < a.num_tasks) {
+        uint64_t next = task + nwarps;
+        uint32_t ticket = 0;
+        const bool ask = next >= dealt;
+        if (ask && lane == 0) ticket = atomicAdd(&a.hdr->task_cursor, 1u);
+        uint4 nd = ask ? make_uint4(0, 0, 0, 0) : a.tasks[next];
         const uint64_t e0 = task_first_edge(d);
         E.src = a.in_src + e0;
         E.w = (WK == HYT_WEIGHTS_NONE) ? nullptr : a.in_w + e0;
-        prefetch_task(nd, pf_a, pf_w, lane);
+        if (!ask) prefetch_task(nd, pf_a, pf_w, lane);
         if (task_is_chunk(d)) {
             const uint32_t r = a.long_rows[d.z].row, n = task_edges(d);
             uint32_t settled = 0;
@@ -564,6 +568,11 @@ __global__ void __launch_bounds__(kMPThreads, 1) ms_pull_kernel(const MSArgs *__
                 ssc::warp_append<1>(w.qnext, w.qnext_size, vals, lower ? 1u : 0u, lane);
             }
         }
+        if (ask) {
+            next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
+            if (next < a.num_tasks) nd = a.tasks[next];
+        }
+        task = next;
         d = nd;
     }
     flush_gain(a, gain, lane);
@@ -608,6 +617,7 @@ __global__ void ms_round_close_kernel(const MSArgs *__restrict__ args) {
     if (h->done) return;
     const unsigned long long fe = h->frontier_edges_next;
     h->frontier_edges_next = 0;
+    h->task_cursor = 0;
 #pragma unroll
     for (int l = 0; l < kML; ++l) {
         h->fmin[l] = ~h->fmin_inv[l];  // all ones when no label of the lane dropped
@@ -682,6 +692,7 @@ void ms_solve(GraphImpl &g, const uint32_t *sources, uint32_t k, uint32_t max_ro
         a.long_rows = g.long_rows.get();
         a.tasks = g.pull_tasks.get();
         a.num_tasks = g.num_chunks + g.num_tiles;
+        a.dealt = dealt_tasks(g);
         a.bits = g.in_pack_bits;
         a.num_hot = a.bits ? 0u : g.num_hot;
     }

@@ -91,13 +91,16 @@ struct PRRange {
     const uint32_t *in_src;
     uint64_t chunk_begin, chunk_end, tile_begin, tile_end;
     const uint4 *tasks;  // the graph's task descriptors (whole-graph launches; NULL: no prefetch)
+    uint64_t dealt;      // dealt_tasks (whole-graph solves)
 };
 
 // The tasks of one iteration, over the whole grid.  a: the solve's arguments
 // as kernel parameters (the constant bank: no registers held across the
 // tasks).
+// cursor (whole-graph launches): the first rg.dealt tasks are dealt to the
+// warps in turn, the others taken one by one.
 __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, const PRState &ps, const PRBuffers &b,
-                                          double2 *slots, float *s_hot) {
+                                          double2 *slots, float *s_hot, uint32_t *cursor) {
     const uint64_t n_chunks = rg.chunk_end - rg.chunk_begin;
     const uint64_t total_tasks = n_chunks + (rg.tile_end - rg.tile_begin);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -105,14 +108,18 @@ __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, co
     __syncthreads();
     const uint64_t nwarps = uint64_t(gridDim.x) * (kPRThreads / 32);
     uint64_t task = uint64_t(blockIdx.x) * (kPRThreads / 32) + warp;
-    // whole-graph launches read each task's descriptor while the task before
-    // it runs (one 16-byte load in place of a chain of table reads)
+    const uint64_t dealt = cursor ? max(rg.dealt, min(total_tasks, nwarps)) : total_tasks;
+    // whole-graph launches read a dealt task's descriptor while the task
+    // before it runs (one 16-byte load in place of a chain of table reads)
     uint4 d = (rg.tasks && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
-    for (; task < total_tasks; task += nwarps) {
+    while (task < total_tasks) {
         double res = 0.0, dang = 0.0;
-        const uint64_t next = task + nwarps;
-        const uint4 nd = (rg.tasks && next < total_tasks) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
-        const uint4 *pf = rg.tasks ? &nd : nullptr;
+        uint64_t next = task + nwarps;
+        uint32_t ticket = 0;
+        const bool ask = cursor && next >= dealt;
+        if (ask && lane == 0) ticket = atomicAdd(cursor, 1u);
+        uint4 nd = (rg.tasks && next < dealt) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
+        const uint4 *pf = (rg.tasks && !ask) ? &nd : nullptr;
         if (task < n_chunks) {
             const TaskSpan t = rg.tasks ? task_span(d) : chunk_span(a, rg.chunk_begin + task);
             const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
@@ -123,6 +130,11 @@ __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, co
             tile_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
             slot_store(slots, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
         }
+        if (ask) {
+            next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
+            if (rg.tasks && next < total_tasks) nd = rg.tasks[next];
+        }
+        task = next;
         d = nd;
     }
 }
@@ -135,7 +147,7 @@ __global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs 
     extern __shared__ __align__(16) float s_dyn[];
     const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
     if (*(volatile uint32_t *)&a.hdr->done) return;
-    run_tasks(a, rg, make_state(*args, a.dangling[it]), buffers(a, it), a.red.slot, s_dyn);
+    run_tasks(a, rg, make_state(*args, a.dangling[it]), buffers(a, it), a.red.slot, s_dyn, nullptr);
 }
 
 // (residual, dangling) of slot group g: thread t of 256 takes slots t, t +
@@ -187,7 +199,9 @@ __global__ void __launch_bounds__(kPRThreads, 1) pr_solve_kernel(const __grid_co
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
         double2 *slots = R.slot + ((it & 1) ? R.num_slots : 0);
-        run_tasks(a, rg, make_state(a, dangling), buffers(a, it), slots, s_dyn);
+        // three cursors take turns: this one was cleared two iterations ago
+        if (blockIdx.x == 0 && threadIdx.x == 0) R.blocks_done[1 + (it + 2) % 3] = 0;
+        run_tasks(a, rg, make_state(a, dangling), buffers(a, it), slots, s_dyn, R.blocks_done + 1 + it % 3);
         ok = dev::grid_sync(R.blocks_done, barriers);
         if (!ok) break;
         const bool own = R.num_groups <= kOwnGroups;
@@ -352,7 +366,8 @@ struct PRSolveState {
 };
 
 // pr_state layout: args | header | residual[max_iter] | dangling[max_iter+1]
-// | init partials | init counter | reduce-blocks counter | (16-byte aligned)
+// | init partials | init counter | reduce-blocks counter, 3 task cursors |
+// (16-byte aligned)
 // group sums | slots.  Everything from the header through the counters is
 // cleared at the start of a solve.
 static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source, float damping, float tolerance,
@@ -372,7 +387,7 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
     auto up16 = [](size_t x) { return (x + 15) & ~size_t(15); };  // double2 needs 16-byte alignment
     const size_t args_bytes = (sizeof(PRArgs) + 255) & ~size_t(255);
     const size_t head = sizeof(PRHeader) + size_t(max_iter) * sizeof(double) + size_t(max_iter + 1) * sizeof(double) +
-                        size_t(init_chunks) * sizeof(double) + 2 * sizeof(uint32_t);
+                        size_t(init_chunks) * sizeof(double) + 5 * sizeof(uint32_t);
     const size_t sb = args_bytes + up16(head) + size_t(num_groups + 2 * num_slots) * sizeof(double2) + 64;
     if (g.pr_state.count < sb) g.pr_state.allocate(sb);
 
@@ -390,7 +405,7 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
     uint32_t *init_count = reinterpret_cast<uint32_t *>(p);
     p += sizeof(uint32_t);
     uint32_t *blocks_done = reinterpret_cast<uint32_t *>(p);
-    p += 4;
+    p += 4 * sizeof(uint32_t);
     const size_t zero_bytes = static_cast<size_t>(p - reinterpret_cast<unsigned char *>(hdr));
     p = base + args_bytes + up16(head);
     double2 *group_sum = reinterpret_cast<double2 *>(p);
@@ -463,7 +478,7 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
     const bool persistent = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = pr_occupancy_grid();
     const unsigned smem = static_cast<unsigned>(pr_hot_bytes(g.num_hot));
-    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get()};
+    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get(), dealt_tasks(g)};
 
     EventTimer total;
     total.start(s);

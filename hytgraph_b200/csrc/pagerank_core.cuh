@@ -44,7 +44,8 @@ constexpr uint32_t kSlotGroup = 1024;
 struct PRSlots {
     double2 *slot;          // [2 * num_slots] (residual, dangling); the persistent solver alternates halves
     double2 *group_sum;     // [num_groups]
-    uint32_t *blocks_done;  // [1] reduce blocks finished, over the whole solve (persistent solver: barrier count)
+    uint32_t *blocks_done;  // [4] reduce blocks finished, over the whole solve (persistent solver: barrier
+                            // count), then the persistent solver's three task cursors
     uint32_t num_slots, num_groups;
 };
 

@@ -667,7 +667,7 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         pg.tasks = g.pull_tasks.get();
         pg.num_tasks = g.num_chunks + g.num_tiles;
         pg.num_chunks = g.num_chunks;
-        pg.dealt = pg.num_tasks - pg.num_tasks / 4;
+        pg.dealt = pg.num_tasks - pg.num_tasks / 4;  // skipped rows make tasks uneven in any vertex order
         pg.num_hot = kPacked ? 0u : g.num_hot;
         pg.bits = g.in_pack_bits;
         if (kPacked) a.inf = HYT_DIST_INF_U32 - g.weight_range.high;
