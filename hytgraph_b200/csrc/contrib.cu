@@ -6,18 +6,18 @@
 // (src/algorithms/pagerank.cpp:165-241, src/algorithms/sssp.cpp:236-290):
 //   PageRank: |next(v) - current(v)| of one synchronous pull step,
 //     next(v) = (1 - d)/n + d * dangling / n + d * sum_{u->v} current(u)/deg(u);
-//     here the sums run in FP64 (one warp per row, a fixed-order warp
-//     tree; dangling mass by per-block partials summed in a fixed order), so
-//     the values are deterministic and agree with the reference's FP32 to
-//     within its rounding;
+//     here the sums run in FP64 (each row in a fixed association over 1 to 8
+//     lanes or a warp; dangling mass by per-block partials summed in a fixed
+//     order), so the values are deterministic and agree with the reference's
+//     FP32 to within its rounding;
 //   SSSP: current - candidate when both are finite and the improvement
 //     exceeds the tolerance, 1 when an unreachable vertex becomes
 //     reachable, else 0 — the same FP32 operations, bit for bit.
 // The schedule follows ContributionScheduler::schedule
 // (src/scheduling/contribution_scheduler.cpp:23-121): items by descending
 // contribution, ties by lower item index (deterministic tie-break; or input
-// order otherwise), computed as two stable radix sorts (item index, then
-// contribution), with the plan metrics (reordered, zero, redundant,
+// order otherwise), computed as stable radix sorts (item index where the items
+// do not ascend already, then contribution), with the plan metrics (reordered, zero, redundant,
 // log2(n) overhead).
 #include <cmath>
 #include <cstring>
@@ -58,17 +58,60 @@ __global__ void source_shares_kernel(const uint32_t *__restrict__ deg, const flo
     }
 }
 
-__device__ __forceinline__ double row_sum(const uint32_t *__restrict__ in_src, const uint32_t *__restrict__ hot_vertex,
-                                          const double *__restrict__ x, uint64_t b, uint64_t e, int lane) {
-    double acc = 0.0;
-    for (uint64_t i = b + lane; i < e; i += 32) {
-        uint32_t u = in_src[i];
-        if (u & kHotTag) u = hot_vertex[u & ~kHotTag];
-        acc += x[u];
-    }
+// In-edges of one task, addressed relative to its first edge.
+struct InEdges {
+    const uint32_t *src;    // source ids, hot ones tagged kHotTag | slot
+    const uint32_t *s_hot;  // vertex ids of the hot slots
+    const double *x;
+};
+
+// Sum of x over the edges b, b + kStep, ... below e, at most kN of them, all
+// loaded before the first is added.
+template <int kN, int kStep>
+__device__ __forceinline__ double edges_sum(const InEdges &E, uint32_t b, uint32_t e, double acc) {
+    uint32_t u[kN];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int j = 0; j < kN; ++j) u[j] = (b + j * kStep < e) ? dev::ld_stream(E.src + b + j * kStep) : 0u;
+#pragma unroll
+    for (int j = 0; j < kN; ++j)
+        if (u[j] & kHotTag) u[j] = E.s_hot[u[j] & ~kHotTag];
+    double v[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j) v[j] = (b + j * kStep < e) ? __ldg(E.x + u[j]) : 0.0;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) acc += v[j];
     return acc;
+}
+
+// Sum over edges [b, e) by the whole warp; every lane returns it.
+__device__ __forceinline__ double span_sum(const InEdges &E, uint32_t b, uint32_t e, int lane) {
+    double acc = 0.0;
+    for (uint32_t at = b; at < e; at += 256) {
+        if (e - at <= 128)
+            acc = edges_sum<4, 32>(E, at + lane, e, acc);
+        else
+            acc = edges_sum<8, 32>(E, at + lane, e, acc);
+    }
+    return dev::warp_sum(acc);
+}
+
+// Sums of the warp's 32 rows (lane l: edges [lo, hi)), kG lanes per row and
+// 32 / kG rows a step; rows have at most kG * kN in-edges.
+template <int kG, int kN>
+__device__ __forceinline__ double group_sum(const InEdges &E, uint32_t lo, uint32_t hi, int lane) {
+    constexpr int kRows = 32 / kG;
+    double mine = 0.0;
+    for (int step = 0; step < kG; ++step) {
+        const int owner = step * kRows + lane / kG;
+        const uint32_t b = __shfl_sync(0xffffffffu, lo, owner) + (lane % kG);
+        const uint32_t e = __shfl_sync(0xffffffffu, hi, owner);
+        double acc = edges_sum<kN, kG>(E, b, e, 0.0);
+#pragma unroll
+        for (int o = 1; o < kG; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        const double t = __shfl_sync(0xffffffffu, acc, (lane % kRows) * kG);
+        if (lane / kRows == step) mine = t;
+    }
+    return mine;
 }
 
 // (1 - d)/n + d * dangling / n from the per-block dangling partials, summed
@@ -83,42 +126,78 @@ __device__ __forceinline__ double base_share(const double *__restrict__ partial,
     return (1.0 - d) / double(V) + d * dm / double(V);
 }
 
-// One warp per row below the long-row threshold (a fixed-order warp tree).
-__global__ void pagerank_contrib_kernel(const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in_src,
-                                        const uint32_t *__restrict__ hot_vertex, const double *__restrict__ x,
-                                        const float *__restrict__ rank, uint64_t V, uint64_t long_from, double damping,
-                                        const double *__restrict__ partial, int parts, double *__restrict__ out) {
+// The graph's pull tasks (graph.cuh): a chunk of a long row gives its partial
+// sum, a tile its rows' contributions, 32 rows at a time.  Three quarters of
+// the tasks are dealt to the warps in turn, the others taken from `cursor`.
+// Bound by the gathers, one L2 sector per in-edge: on R-MAT scale 22 (64 M
+// edges) one warp per row and one per chunk took 1100 us, the tasks take 333 us.
+constexpr int kContribThreads = 1024;
+
+__global__ void __launch_bounds__(kContribThreads, 1) pagerank_contrib_kernel(
+    const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in_src, const uint32_t *__restrict__ hot_vertex,
+    uint32_t num_hot, const uint4 *__restrict__ tasks, uint64_t num_tasks, const LongRow *__restrict__ long_rows,
+    const double *__restrict__ x, const float *__restrict__ rank, uint64_t V, double damping,
+    const double *__restrict__ partial, int parts, uint32_t *cursor, double *__restrict__ chunk_sum,
+    double *__restrict__ out) {
+    extern __shared__ __align__(16) uint32_t s_hot[];
     __shared__ double s_share;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t i = threadIdx.x; i < num_hot; i += blockDim.x) s_hot[i] = hot_vertex[i];
     if (threadIdx.x < 32) {
         const double sh = base_share(partial, parts, V, damping, threadIdx.x);
         if (threadIdx.x == 0) s_share = sh;
     }
     __syncthreads();
     const double share = s_share;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
-    for (uint64_t v = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; v < V; v += warps) {
-        const uint64_t b = in_off[v], e = in_off[v + 1];
-        if (e - b >= long_from) continue;  // summed by the chunk kernels
-        const double acc = row_sum(in_src, hot_vertex, x, b, e, lane);
-        if (lane == 0) out[v] = fabs(share + damping * acc - double(rank[v]));
-    }
-}
-
-// One warp per chunk of a long row: its partial sum.
-__global__ void contrib_chunks_kernel(const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in_src,
-                                      const uint32_t *__restrict__ hot_vertex, const double *__restrict__ x,
-                                      const LongRow *__restrict__ long_rows, const uint2 *__restrict__ tasks,
-                                      uint64_t num_tasks, double *__restrict__ chunk_sum) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
-    for (uint64_t t = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; t < num_tasks; t += warps) {
-        const uint2 task = tasks[t];
-        const LongRow lr = long_rows[task.x];
-        const uint64_t b = in_off[lr.row] + uint64_t(task.y) * kLongChunk;
-        const uint64_t e = min(b + kLongChunk, in_off[lr.row + 1]);
-        const double acc = row_sum(in_src, hot_vertex, x, b, e, lane);
-        if (lane == 0) chunk_sum[lr.first_chunk + task.y] = acc;
+    const uint64_t nwarps = uint64_t(gridDim.x) * (kContribThreads / 32);
+    const uint64_t dealt = max(num_tasks - num_tasks / 4, min(num_tasks, nwarps));
+    uint64_t task = uint64_t(blockIdx.x) * (kContribThreads / 32) + warp;
+    while (task < num_tasks) {
+        uint64_t next = task + nwarps;
+        uint32_t ticket = 0;
+        const bool ask = next >= dealt;
+        if (ask && lane == 0) ticket = atomicAdd(cursor, 1u);
+        const uint4 d = tasks[task];
+        if (!ask) prefetch_task(tasks[next], in_src, nullptr, lane);
+        const uint64_t e0 = task_first_edge(d);
+        const InEdges E{in_src + e0, s_hot, x};
+        if (task_is_chunk(d)) {
+            const double acc = span_sum(E, 0, task_edges(d), lane);
+            if (lane == 0) chunk_sum[long_rows[d.z].first_chunk + d.w] = acc;
+        } else {
+            for (uint32_t rb = d.z; rb < d.w; rb += 32) {
+                const uint32_t r = rb + lane;
+                uint32_t lo = 0, hi = 0;
+                double old = 0.0;
+                if (r < d.w) {
+                    lo = static_cast<uint32_t>(in_off[r] - e0);
+                    hi = static_cast<uint32_t>(in_off[r + 1] - e0);
+                    old = rank[r];
+                }
+                const bool wide = hi - lo >= 64;
+                const uint32_t hs = wide ? lo : hi;  // group steps see a wide row as empty
+                const uint32_t most = __reduce_max_sync(0xffffffffu, hs - lo);
+                double acc = 0.0;
+                if (most > 32)
+                    acc = group_sum<8, 8>(E, lo, hs, lane);
+                else if (most > 16)
+                    acc = group_sum<4, 8>(E, lo, hs, lane);
+                else if (most > 8)
+                    acc = group_sum<2, 8>(E, lo, hs, lane);
+                else if (most > 4)
+                    acc = group_sum<1, 8>(E, lo, hs, lane);
+                else if (most)
+                    acc = group_sum<1, 4>(E, lo, hs, lane);
+                for (uint32_t big = __ballot_sync(0xffffffffu, wide); big; big &= big - 1) {
+                    const int o = __ffs(big) - 1;
+                    const double t = span_sum(E, __shfl_sync(0xffffffffu, lo, o), __shfl_sync(0xffffffffu, hi, o), lane);
+                    if (lane == o) acc = t;
+                }
+                if (r < d.w) out[r] = fabs(share + damping * acc - old);
+            }
+        }
+        if (ask) next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
+        task = next;
     }
 }
 
@@ -166,35 +245,67 @@ __device__ __forceinline__ uint64_t double_key(double c) {
     return (b >> 63) ? ~b : (b | (uint64_t(1) << 63));
 }
 
-__global__ void schedule_prep_kernel(const double *__restrict__ c, uint64_t n, double eps, uint64_t *__restrict__ pos,
-                                     unsigned long long *__restrict__ counts) {
-    unsigned long long zero = 0, nonfinite = 0;
+// What the host decides the sorts by.
+struct ScheduleFacts {
+    unsigned long long zero, nonfinite, moved, duplicates;  // metrics
+    unsigned long long keys_or, keys_nand;                  // bits set in some key; bits clear in some key
+    unsigned long long max_item;
+    uint32_t descents;  // 1: some item does not exceed the one before it
+    uint32_t pad;
+};
+
+// Keys and positions in input order, the zero and non-finite counts, which
+// key bits differ, and whether the items ascend strictly.
+__global__ void schedule_prep_kernel(const uint64_t *__restrict__ item, const double *__restrict__ c, uint64_t n,
+                                     double eps, uint64_t *__restrict__ key, uint32_t *__restrict__ pos,
+                                     ScheduleFacts *__restrict__ f) {
+    unsigned long long zero = 0, nonfinite = 0, ones = 0, zeros = 0, top = 0;
+    uint32_t descents = 0;
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-        pos[i] = i;
         const double x = c[i];
+        const uint64_t k = double_key(x), it = item[i];
+        key[i] = k;
+        pos[i] = static_cast<uint32_t>(i);
         if (!isfinite(x)) ++nonfinite;
         if (fabs(x) <= eps) ++zero;
+        ones |= k;
+        zeros |= ~k;
+        top = max(top, static_cast<unsigned long long>(it));
+        if (i && it <= item[i - 1]) descents = 1;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         zero += __shfl_xor_sync(0xffffffffu, zero, o);
         nonfinite += __shfl_xor_sync(0xffffffffu, nonfinite, o);
+        ones |= __shfl_xor_sync(0xffffffffu, ones, o);
+        zeros |= __shfl_xor_sync(0xffffffffu, zeros, o);
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
     }
+    descents = __reduce_or_sync(0xffffffffu, descents);
     if ((threadIdx.x & 31) == 0) {
-        if (zero) atomicAdd(counts, zero);
-        if (nonfinite) atomicAdd(counts + 1, nonfinite);
+        if (zero) atomicAdd(&f->zero, zero);
+        if (nonfinite) atomicAdd(&f->nonfinite, nonfinite);
+        atomicOr(&f->keys_or, ones);
+        atomicOr(&f->keys_nand, zeros);
+        atomicMax(&f->max_item, top);
+        if (descents) atomicOr(&f->descents, 1u);
     }
 }
 
-__global__ void contribution_keys_kernel(const double *__restrict__ c, const uint64_t *__restrict__ pos, uint64_t n,
+__global__ void contribution_keys_kernel(const double *__restrict__ c, const uint32_t *__restrict__ pos, uint64_t n,
                                          uint64_t *__restrict__ key) {
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
         key[i] = double_key(c[pos[i]]);
 }
 
-// ordered[p] = item[order[p]]; counts[2] += moved positions.
-__global__ void schedule_emit_kernel(const uint64_t *__restrict__ item, const uint64_t *__restrict__ order, uint64_t n,
-                                     uint64_t *__restrict__ ordered, unsigned long long *__restrict__ counts) {
+__global__ void positions_kernel(uint32_t *pos, uint64_t n) {
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
+        pos[i] = static_cast<uint32_t>(i);
+}
+
+// ordered[p] = item[order[p]]; counts moved positions.
+__global__ void schedule_emit_kernel(const uint64_t *__restrict__ item, const uint32_t *__restrict__ order, uint64_t n,
+                                     uint64_t *__restrict__ ordered, ScheduleFacts *__restrict__ f) {
     unsigned long long moved = 0;
     for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < n; p += uint64_t(gridDim.x) * blockDim.x) {
         const uint64_t o = order[p];
@@ -203,39 +314,39 @@ __global__ void schedule_emit_kernel(const uint64_t *__restrict__ item, const ui
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) moved += __shfl_xor_sync(0xffffffffu, moved, o);
-    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(counts + 2, moved);
+    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&f->moved, moved);
 }
 
-// counts[3] += adjacent equal item indices in the sorted copy.
-__global__ void duplicates_kernel(const uint64_t *__restrict__ sorted, uint64_t n, unsigned long long *counts) {
+// Counts adjacent equal item indices in the sorted copy.
+__global__ void duplicates_kernel(const uint64_t *__restrict__ sorted, uint64_t n, ScheduleFacts *f) {
     unsigned long long dup = 0;
     for (uint64_t i = 1 + blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
         dup += sorted[i] == sorted[i - 1];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dup += __shfl_xor_sync(0xffffffffu, dup, o);
-    if ((threadIdx.x & 31) == 0 && dup) atomicAdd(counts + 3, dup);
+    if ((threadIdx.x & 31) == 0 && dup) atomicAdd(&f->duplicates, dup);
 }
 
 unsigned grid_sm(unsigned per_sm) { return static_cast<unsigned>(sm_count()) * per_sm; }
 
-// Stable radix sort of (key, value) pairs on key bits [0, bits).
+// Stable radix sort of (key, value) pairs on key bits [first, bits).
 template <class K, class V>
 void sort_pairs(K *&keys, K *keys_alt, V *&vals, V *vals_alt, uint64_t n, bool descending, cudaStream_t s,
-                int bits = int(sizeof(K) * 8)) {
-    if (n < 2) return;
+                int first, int bits) {
+    if (n < 2 || first >= bits) return;
     cub::DoubleBuffer<K> kb(keys, keys_alt);
     cub::DoubleBuffer<V> vb(vals, vals_alt);
     size_t tb = 0;
     if (descending) {
-        HYT_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, kb, vb, static_cast<int64_t>(n), 0, bits, s));
+        HYT_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, kb, vb, static_cast<int64_t>(n), first, bits, s));
     } else {
-        HYT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, static_cast<int64_t>(n), 0, bits, s));
+        HYT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, static_cast<int64_t>(n), first, bits, s));
     }
     Scratch<uint8_t> tmp(tb, s);
     if (descending) {
-        HYT_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.get(), tb, kb, vb, static_cast<int64_t>(n), 0, bits, s));
+        HYT_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.get(), tb, kb, vb, static_cast<int64_t>(n), first, bits, s));
     } else {
-        HYT_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tb, kb, vb, static_cast<int64_t>(n), 0, bits, s));
+        HYT_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tb, kb, vb, static_cast<int64_t>(n), first, bits, s));
     }
     keys = kb.Current();
     vals = vb.Current();
@@ -264,18 +375,19 @@ void pagerank_contributions(GraphImpl &g, const float *ranks, float damping, dou
     Scratch<double> partial(kPartBlocks, s), x(V, s);
     const uint64_t chunks = g.num_long ? g.num_chunks : 0;
     Scratch<double> chunk_sum(chunks ? chunks : 1, s);
-    // a row is long (chunked) when its in-degree >= tile_cost
-    const uint64_t long_from = g.num_long ? g.tile_cost : ~uint64_t(0);
+    Scratch<uint32_t> cursor(1, s);
+    const unsigned smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
+    HYT_CUDA(cudaFuncSetAttribute(pagerank_contrib_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kPRSmemMax)));
     EventTimer t;
     t.start(s);
+    HYT_CUDA(cudaMemsetAsync(cursor.get(), 0, sizeof(uint32_t), s));
     source_shares_kernel<<<kPartBlocks, 256, 0, s>>>(g.out_degree.get(), r, V, x.get(), partial.get());
-    pagerank_contrib_kernel<<<grid_sm(8), 256, 0, s>>>(g.in_offsets.get(), g.in_sources.get(), g.hot_vertex.get(),
-                                                       x.get(), r, V, long_from, double(damping), partial.get(),
-                                                       kPartBlocks, o);
+    pagerank_contrib_kernel<<<grid_sm(1), kContribThreads, smem, s>>>(
+        g.in_offsets.get(), g.in_sources.get(), g.hot_vertex.get(), g.num_hot, g.pull_tasks.get(),
+        g.num_chunks + g.num_tiles, g.long_rows.get(), x.get(), r, V, double(damping), partial.get(), kPartBlocks,
+        cursor.get(), chunk_sum.get(), o);
     if (chunks) {
-        contrib_chunks_kernel<<<grid_sm(8), 256, 0, s>>>(g.in_offsets.get(), g.in_sources.get(), g.hot_vertex.get(),
-                                                         x.get(), g.long_rows.get(), g.chunk_tasks.get(), chunks,
-                                                         chunk_sum.get());
         contrib_long_rows_kernel<<<grid_for(g.num_long * 32, 256), 256, 0, s>>>(
             g.long_rows.get(), g.num_long, chunk_sum.get(), r, V, double(damping), partial.get(), kPartBlocks, o);
     }
@@ -323,62 +435,56 @@ void contribution_schedule(const uint64_t *item, const double *contribution, uin
     std::unique_ptr<Scratch<double>> chold;
     const uint64_t *it = device_view(item, n, ih, s);
     const double *c = device_view(contribution, n, chold, s);
-    Scratch<uint64_t> pos(n, s), pos_alt(n, s), key(n, s), key_alt(n, s), out_d(n, s);
-    Scratch<unsigned long long> counts(4, s);
-    HYT_CUDA(cudaMemsetAsync(counts.get(), 0, 32, s));
-    schedule_prep_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(c, n, eps, pos.get(), counts.get());
-    HYT_CUDA(cudaGetLastError());
-    // item sorts run on the bits the largest item index needs
-    int item_bits = 1;
-    {
-        Scratch<uint64_t> mx(1, s);
-        size_t tb = 0;
-        HYT_CUDA(cub::DeviceReduce::Max(nullptr, tb, it, mx.get(), static_cast<int64_t>(n), s));
-        Scratch<uint8_t> tmp(tb, s);
-        HYT_CUDA(cub::DeviceReduce::Max(tmp.get(), tb, it, mx.get(), static_cast<int64_t>(n), s));
-        uint64_t h = 0;
-        HYT_CUDA(cudaMemcpyAsync(&h, mx.get(), 8, cudaMemcpyDeviceToHost, s));
-        HYT_CUDA(cudaStreamSynchronize(s));
-        item_bits = h ? 64 - __builtin_clzll(h) : 1;
-    }
-    // redundant work: equal neighbours among the sorted item indices
-    HYT_CUDA(cudaMemcpyAsync(key.get(), it, n * 8, cudaMemcpyDeviceToDevice, s));
-    uint64_t *vp = pos.get();
-    {
-        uint64_t *k = key.get();
-        uint64_t *k_alt = key_alt.get();
-        size_t tb = 0;
-        cub::DoubleBuffer<uint64_t> kb(k, k_alt);
-        HYT_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, static_cast<int64_t>(n), 0, item_bits, s));
-        Scratch<uint8_t> tmp(tb, s);
-        HYT_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(), tb, kb, static_cast<int64_t>(n), 0, item_bits, s));
-        duplicates_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(kb.Current(), n, counts.get());
-        HYT_CUDA(cudaGetLastError());
-    }
-    // the order: positions by item index (stable), then by descending
-    // contribution (stable), or by contribution alone
-    if (deterministic) {
-        HYT_CUDA(cudaMemcpyAsync(key.get(), it, n * 8, cudaMemcpyDeviceToDevice, s));
-        uint64_t *kp = key.get();
-        sort_pairs(kp, key_alt.get(), vp, pos_alt.get(), n, false, s, item_bits);
-    }
-    uint64_t *ck = key.get(), *ck_alt = key_alt.get();
-    uint64_t *vp_alt = vp == pos.get() ? pos_alt.get() : pos.get();
-    contribution_keys_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(c, vp, n, ck);
-    HYT_CUDA(cudaGetLastError());
-    sort_pairs(ck, ck_alt, vp, vp_alt, n, true, s);
+    if (n > 0xFFFFFFFFull) fail(HYT_E_OOM, "contribution schedules hold fewer than 2^32 items");
     const bool ordered_dev = is_device_pointer(ordered);
+    Scratch<uint32_t> pos(n, s), pos_alt(n, s);
+    Scratch<uint64_t> key(n, s), key_alt(n, s), out_d(ordered_dev ? 1 : n, s);
+    Scratch<ScheduleFacts> facts(1, s);
+    HYT_CUDA(cudaMemsetAsync(facts.get(), 0, sizeof(ScheduleFacts), s));
+    schedule_prep_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(it, c, n, eps, key.get(), pos.get(), facts.get());
+    HYT_CUDA(cudaGetLastError());
+    ScheduleFacts h{};
+    HYT_CUDA(cudaMemcpyAsync(&h, facts.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    HYT_CUDA(cudaStreamSynchronize(s));
+    if (h.nonfinite) fail(HYT_E_INVALID, "contribution priority must be finite");
+    uint32_t *vp = pos.get(), *vp_alt = pos_alt.get();
+    uint64_t *ck = key.get(), *ck_alt = key_alt.get();
+    // Items that ascend strictly (the vertices of a graph, say) are in item
+    // order already and hold no duplicates; others are sorted for both, on
+    // the bits the largest item needs.
+    if (h.descents) {
+        const int item_bits = h.max_item ? 64 - __builtin_clzll(h.max_item) : 1;
+        Scratch<uint64_t> ik(n, s), ik_alt(n, s);
+        uint64_t *ip = ik.get();
+        HYT_CUDA(cudaMemcpyAsync(ip, it, n * 8, cudaMemcpyDeviceToDevice, s));
+        sort_pairs(ip, ik_alt.get(), vp, vp_alt, n, false, s, 0, item_bits);
+        duplicates_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(ip, n, facts.get());
+        HYT_CUDA(cudaGetLastError());
+        if (deterministic) {
+            vp_alt = vp == pos.get() ? pos_alt.get() : pos.get();
+            contribution_keys_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(c, vp, n, ck);
+            HYT_CUDA(cudaGetLastError());
+        } else {  // ties stay in input order
+            vp = pos.get();
+            vp_alt = pos_alt.get();
+            positions_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(vp, n);
+            HYT_CUDA(cudaGetLastError());
+        }
+    }
+    // by descending contribution, over the key bits that differ at all
+    // (contributions that are differences of floats leave the low 29 alone)
+    const unsigned long long differ = h.keys_or & h.keys_nand;
+    if (differ)
+        sort_pairs(ck, ck_alt, vp, vp_alt, n, true, s, __builtin_ctzll(differ), 64 - __builtin_clzll(differ));
     uint64_t *od = ordered_dev ? ordered : out_d.get();
-    schedule_emit_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(it, vp, n, od, counts.get());
+    schedule_emit_kernel<<<grid_for(n, 256, 148u * 8u), 256, 0, s>>>(it, vp, n, od, facts.get());
     HYT_CUDA(cudaGetLastError());
     if (!ordered_dev) HYT_CUDA(cudaMemcpyAsync(ordered, od, n * 8, cudaMemcpyDeviceToHost, s));
-    unsigned long long h[4] = {};
-    HYT_CUDA(cudaMemcpyAsync(h, counts.get(), 32, cudaMemcpyDeviceToHost, s));
+    HYT_CUDA(cudaMemcpyAsync(&h, facts.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     HYT_CUDA(cudaStreamSynchronize(s));
-    if (h[1]) fail(HYT_E_INVALID, "contribution priority must be finite");
-    m->zero_contribution_count = h[0];
-    m->reordered_item_count = h[2];
-    m->redundant_work_count = h[3];
+    m->zero_contribution_count = h.zero;
+    m->reordered_item_count = h.moved;
+    m->redundant_work_count = h.duplicates;
     m->scheduling_overhead = std::log2(static_cast<double>(n));
 }
 
