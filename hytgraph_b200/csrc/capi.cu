@@ -10,6 +10,7 @@
 #include "scratch.cuh"
 #include "graph.cuh"
 #include "solvers.cuh"
+#include "staging.cuh"
 
 namespace hyt {
 namespace {
@@ -64,6 +65,7 @@ PointerPlace pointer_place(const void *p, int current_device, int *pointer_devic
 void copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (!bytes) return;
     const cudaMemcpyKind kind = is_device_pointer(src) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    if (kind == cudaMemcpyHostToDevice && staged_copy(dst, src, bytes, true, s)) return;
     HYT_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, s));
     HYT_CUDA(cudaStreamSynchronize(s));
 }
@@ -71,6 +73,7 @@ void copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
 void copy_from_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (!bytes) return;
     const cudaMemcpyKind kind = is_device_pointer(dst) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    if (kind == cudaMemcpyDeviceToHost && staged_copy(dst, src, bytes, false, s)) return;
     HYT_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, s));
     HYT_CUDA(cudaStreamSynchronize(s));
 }
@@ -142,6 +145,8 @@ int hyt_copy(void *dst, const void *src, uint64_t bytes, void *stream) {
         if (!dst || !src) fail(HYT_E_INVALID, "hyt_copy: NULL pointer");
         require_device();
         cudaStream_t s = static_cast<cudaStream_t>(stream);
+        const bool to_device = is_device_pointer(dst), from_device = is_device_pointer(src);
+        if (to_device != from_device && staged_copy(dst, src, bytes, to_device, s)) return;
         HYT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s));
         HYT_CUDA(cudaStreamSynchronize(s));
     });
@@ -417,6 +422,7 @@ int hyt_trim_device_memory(int device) {
         HYT_CUDA(cudaDeviceSynchronize());
         HYT_CUDA(cudaMemPoolTrimTo(graph_pool(device), 0));
         HYT_CUDA(cudaMemPoolTrimTo(scratch_pool(), 0));
+        staging_release(device);
         HYT_CUDA(cudaSetDevice(cur));
     });
 }

@@ -17,6 +17,7 @@
 #include "scratch.cuh"
 #include "solvers.cuh"
 #include "stage.cuh"
+#include "staging.cuh"
 
 namespace hyt {
 namespace {
@@ -245,11 +246,12 @@ void graph_create(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         copy_to_device(d_cols.get(), csr.column_indices, E * 4, g.stream);
         dev.column_indices = d_cols.get();
     }
-    // the weights are first needed by the reorder: their upload runs on the
-    // graph's stream while the hub sort (its own stream) ranks the vertices
+    // the weights are first needed by the reorder: pinned ones are uploaded on
+    // the graph's stream while the hub sort (its own stream) ranks the vertices
     if (weighted && csr.weights && !is_device_pointer(csr.weights)) {
         d_w.allocate(E);
-        HYT_CUDA(cudaMemcpyAsync(d_w.get(), csr.weights, E * 4, cudaMemcpyHostToDevice, g.stream));
+        if (!staged_copy(d_w.get(), csr.weights, E * 4, true, g.stream))
+            HYT_CUDA(cudaMemcpyAsync(d_w.get(), csr.weights, E * 4, cudaMemcpyHostToDevice, g.stream));
         dev.weights = d_w.get();
     }
     GraphArray<uint32_t> perm(V);

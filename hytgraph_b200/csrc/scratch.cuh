@@ -8,6 +8,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "staging.cuh"
 
 namespace hyt {
 
@@ -61,7 +62,8 @@ template <class T>
 const T *device_view(const T *p, uint64_t n, std::unique_ptr<Scratch<T>> &hold, cudaStream_t s) {
     if (!p || n == 0 || is_device_pointer(p)) return p;
     hold = std::make_unique<Scratch<T>>(n, s);
-    HYT_CUDA(cudaMemcpyAsync(hold->get(), p, n * sizeof(T), cudaMemcpyHostToDevice, s));
+    if (!staged_copy(hold->get(), p, n * sizeof(T), true, s))
+        HYT_CUDA(cudaMemcpyAsync(hold->get(), p, n * sizeof(T), cudaMemcpyHostToDevice, s));
     return hold->get();
 }
 
