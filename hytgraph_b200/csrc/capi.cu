@@ -34,6 +34,20 @@ cudaMemPool_t graph_pool(int device) {
     HYT_CUDA(cudaMemPoolCreate(&pool, &props));
     uint64_t keep = kGraphPoolKeep;
     HYT_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    // reachable from the peers that could reach a plain allocation (device
+    // CSRs handed to callers live here)
+    int n = 0;
+    HYT_CUDA(cudaGetDeviceCount(&n));
+    for (int peer = 0; peer < n; ++peer) {
+        int can = 0;
+        if (peer == device || cudaDeviceCanAccessPeer(&can, peer, device) != cudaSuccess || !can) continue;
+        cudaMemAccessDesc d{};
+        d.location.type = cudaMemLocationTypeDevice;
+        d.location.id = peer;
+        d.flags = cudaMemAccessFlagsProtReadWrite;
+        (void)cudaMemPoolSetAccess(pool, &d, 1);
+    }
+    (void)cudaGetLastError();
     pools[device] = pool;
     return pool;
 }

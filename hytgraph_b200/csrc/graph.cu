@@ -37,7 +37,7 @@ __global__ void validate_offsets_kernel(const uint64_t *off, uint64_t V, uint64_
 
 // range[0] = smallest weight, range[1] = ~largest (bit patterns of u32 or f32
 // weights, sign of -0.0 cleared; both start at all ones).
-__global__ void validate_edges_kernel(const uint32_t *cols, const uint32_t *w, uint32_t wkind, uint64_t V,
+__global__ void __launch_bounds__(256) validate_edges_kernel(const uint32_t *cols, const uint32_t *w, uint32_t wkind, uint64_t V,
                                       uint64_t E, uint32_t *err, unsigned long long *weight_sum, uint32_t *range) {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     uint32_t bad = 0, lo = 0xFFFFFFFFu, hi = 0;
@@ -57,16 +57,29 @@ __global__ void validate_edges_kernel(const uint32_t *cols, const uint32_t *w, u
         hi = max(hi, x);
     }
     if (bad) atomicOr(err, bad);
+    // one atomic per block and value: thousands of warps queueing at one
+    // address took longer than the pass itself
+    __shared__ unsigned long long s_sum[8];
+    __shared__ uint32_t s_lo[8], s_hi[8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     if ((threadIdx.x & 31) == 0) {
-        if (wsum) atomicAdd(weight_sum, wsum);
-        if (wkind != HYT_WEIGHTS_NONE) {
-            atomicMin(range, lo);
-            atomicMin(range + 1, ~hi);
+        s_sum[threadIdx.x >> 5] = wsum;
+        s_lo[threadIdx.x >> 5] = lo;
+        s_hi[threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && wkind != HYT_WEIGHTS_NONE) {
+        for (int k = 1; k < 8; ++k) {
+            wsum += s_sum[k];
+            lo = min(lo, s_lo[k]);
+            hi = max(hi, s_hi[k]);
         }
+        if (wsum) atomicAdd(weight_sum, wsum);
+        atomicMin(range, lo);
+        atomicMin(range + 1, ~hi);
     }
 }
 
@@ -78,7 +91,9 @@ __global__ void out_degree_kernel(const uint64_t *off, uint64_t V, uint32_t *deg
         deg[v] = d;
         nd += (d == 0);
     }
-    if (nd) atomicAdd(dangling, (unsigned long long)nd);
+    // one atomic per warp: one per thread (331 us) queued up at the counter
+    nd = __reduce_add_sync(0xffffffffu, nd);
+    if ((threadIdx.x & 31) == 0 && nd) atomicAdd(dangling, (unsigned long long)nd);
 }
 
 // Writes the source vertex of every CSR edge.  A CTA owns 256 consecutive
@@ -538,7 +553,7 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         Scratch<uint32_t> range(2, s);
         HYT_CUDA(cudaMemsetAsync(wsum.get(), 0, sizeof(unsigned long long), s));
         HYT_CUDA(cudaMemsetAsync(range.get(), 0xFF, 2 * sizeof(uint32_t), s));
-        validate_edges_kernel<<<grid_for(E, 256), 256, 0, s>>>(g.cols.get(), keep_weights ? g.weights.get() : nullptr,
+        validate_edges_kernel<<<grid_for(E, 256, 148 * 8), 256, 0, s>>>(g.cols.get(), keep_weights ? g.weights.get() : nullptr,
                                                                 keep_weights ? csr.weight_kind : 0u, V, E, err.get(),
                                                                 wsum.get(), range.get());
         HYT_CUDA(cudaGetLastError());
@@ -560,7 +575,7 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
     }
 
     g.out_degree.allocate(V);
-    out_degree_kernel<<<grid_for(V, 256), 256, 0, s>>>(g.row_offsets.get(), V, g.out_degree.get(), counter.get());
+    out_degree_kernel<<<grid_for(V, 256, 148 * 8), 256, 0, s>>>(g.row_offsets.get(), V, g.out_degree.get(), counter.get());
     HYT_CUDA(cudaGetLastError());
     unsigned long long h_dangling = 0;
     HYT_CUDA(cudaMemcpyAsync(&h_dangling, counter.get(), sizeof(h_dangling), cudaMemcpyDeviceToHost, s));

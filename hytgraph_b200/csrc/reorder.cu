@@ -12,9 +12,9 @@
 // the x86-64 extended format (64-bit significand), which the kernel
 // reproduces with an exact integer long division rounded to 64 bits and then
 // to 53 bits, both to nearest-even.  The ranking sorts those doubles' bit
-// patterns (non-negative doubles order like their bits) with a stable
-// descending radix sort over ids in ascending order, which is the
-// reference's comparator.
+// patterns (non-negative doubles order like their bits), or the degree
+// products where these rank alike, with a stable descending radix sort over
+// ids in ascending order, which is the reference's comparator.
 //
 // Reordering follows CSRGraph::reorder_vertices
 // (src/graph/csr_graph.cpp:171-283): vertex_order[new] = old; new row
@@ -64,22 +64,56 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t x) {
     return x;
 }
 
-// One pass over the CSR: in-degrees by atomics, out-degrees, the largest
-// out-degree, and the structure checks of the reference's
-// CSRGraph::validate (offsets start at 0, never decrease, end at E; every
-// destination is a vertex).
-__global__ void degree_pass_kernel(const uint64_t *__restrict__ off, const uint32_t *__restrict__ cols, uint64_t V,
-                                   uint64_t E, uint32_t *__restrict__ indeg, uint64_t *__restrict__ outdeg,
-                                   unsigned long long *__restrict__ maxes, uint32_t *__restrict__ bad) {
+// One pass over the CSR: in-degrees, out-degrees, the largest out-degree, and
+// the structure checks of the reference's CSRGraph::validate (offsets start
+// at 0, never decrease, end at E; every destination is a vertex).
+//
+// Plain global atomics were bound by the hub destinations, whose additions
+// queue up at one address each (671 us on R-MAT scale 22, 58 M edges).  Every
+// CTA therefore counts in a small direct-mapped table in shared memory first:
+// the first destination to come by a slot keeps it -- most likely the most
+// frequent of those that share it -- and the others go to global memory: 536
+// us.
+constexpr int kDegreeThreads = 1024;
+constexpr uint32_t kDegreeSlots = 8192;
+constexpr int kDegreeUnroll = 4;
+
+__global__ void __launch_bounds__(kDegreeThreads, 2) degree_pass_kernel(
+    const uint64_t *__restrict__ off, const uint32_t *__restrict__ cols, uint64_t V, uint64_t E,
+    uint32_t *__restrict__ indeg, uint64_t *__restrict__ outdeg, unsigned long long *__restrict__ maxes,
+    uint32_t *__restrict__ bad) {
+    extern __shared__ uint32_t s_tab[];
+    uint32_t *s_key = s_tab, *s_cnt = s_tab + kDegreeSlots;
+    constexpr uint32_t kFree = 0xFFFFFFFFu;  // no destination: ids are below V < 2^32
+    for (uint32_t i = threadIdx.x; i < kDegreeSlots; i += kDegreeThreads) {
+        s_key[i] = kFree;
+        s_cnt[i] = 0;
+    }
+    __syncthreads();
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     const uint64_t tid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
     uint32_t b = 0;
-    for (uint64_t e = tid; e < E; e += stride) {
-        const uint32_t c = ld_stream(cols + e);
-        if (c < V) {
-            atomicAdd(indeg + c, 1u);
-        } else {
-            b |= kBadColumn;
+    for (uint64_t e = tid; e < E; e += kDegreeUnroll * stride) {
+        uint32_t c[kDegreeUnroll];
+#pragma unroll
+        for (int j = 0; j < kDegreeUnroll; ++j) c[j] = e + j * stride < E ? ld_stream(cols + e + j * stride) : kFree;
+#pragma unroll
+        for (int j = 0; j < kDegreeUnroll; ++j) {
+            if (e + j * stride >= E) continue;
+            if (c[j] >= V) {
+                b |= kBadColumn;
+                continue;
+            }
+            const uint32_t slot = (c[j] * 2654435761u) >> 19;  // top 13 bits
+            uint32_t k = *reinterpret_cast<volatile uint32_t *>(s_key + slot);
+            if (k == kFree) {
+                k = atomicCAS(s_key + slot, kFree, c[j]);
+                if (k == kFree) k = c[j];
+            }
+            if (k == c[j])
+                atomicAdd(s_cnt + slot, 1u);
+            else
+                atomicAdd(indeg + c[j], 1u);
         }
     }
     uint64_t mo = 0;
@@ -101,6 +135,9 @@ __global__ void degree_pass_kernel(const uint64_t *__restrict__ off, const uint3
     mo = warp_max_u64(mo);
     if ((threadIdx.x & 31) == 0 && mo) atomicMax(maxes, static_cast<unsigned long long>(mo));
     if (b) atomicOr(bad, b);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kDegreeSlots; i += kDegreeThreads)
+        if (s_cnt[i]) atomicAdd(indeg + s_key[i], s_cnt[i]);
 }
 
 __global__ void max_in_degree_kernel(const uint32_t *__restrict__ indeg, uint64_t V, unsigned long long *maxes) {
@@ -156,23 +193,54 @@ __device__ double extended_quotient(uint64_t n, uint64_t d) {
     return __longlong_as_double(static_cast<long long>(bits));
 }
 
-// Scores and ranking keys (the score's bits), ids in ascending order.  The
+// extended_quotient for 0 < n <= d < 2^52, from one IEEE division.  Rounding
+// to 64 and then to 53 bits differs from rounding to 53 at once only where the
+// 64-bit value is a 53-bit tie, so where the exact remainder shows the
+// quotient within 2^-9 of half a unit from the double (or the double is a
+// power of two, whose neighbours are unevenly spaced), the long division
+// decides.
+__device__ __forceinline__ double short_quotient(uint64_t n, uint64_t d) {
+    const double x = static_cast<double>(n), y = static_cast<double>(d);
+    const double q = __ddiv_rn(x, y);
+    const double r = fabs(__fma_rn(-q, y, x));  // exact
+    const uint64_t bits = static_cast<uint64_t>(__double_as_longlong(q));
+    const double half = __longlong_as_double(static_cast<long long>(((bits >> 52) - 53) << 52)) * y;
+    const bool sure = fabs(r - half) > half * 0x1p-9 && (bits << 12) != 0;
+    return sure || r == 0.0 ? q : extended_quotient(n, d);
+}
+
+// Scores, ranking keys and which vertices have a score above 0.  The
 // denominator Do_max * Di_max is read from device memory (maxes[0..1]).
+// Products below 2^52 rank exactly as their quotients do (two that differ are
+// more than one unit in the last place apart after the division, so rounding
+// keeps them apart), and have fewer bits to sort; above, the key is the
+// score's bit pattern.
+__device__ __forceinline__ bool rank_by_product(uint64_t denom) { return denom < (uint64_t(1) << 52); }
+
 __global__ void hub_scores_kernel(const uint64_t *__restrict__ outdeg, const uint32_t *__restrict__ indeg, uint64_t V,
                                   const unsigned long long *__restrict__ maxes, double *__restrict__ scores,
-                                  uint64_t *__restrict__ key, uint32_t *__restrict__ id, uint32_t *__restrict__ bad) {
+                                  uint64_t *__restrict__ key, uint8_t *__restrict__ scored, uint32_t *__restrict__ bad) {
     const uint64_t max_out = maxes[0], max_in = maxes[1];
     const bool overflow = max_in && max_out > ~uint64_t(0) / max_in;
     if (overflow && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(bad, kBadOverflow);
     const uint64_t denom = max_out * max_in;
+    const bool product = !overflow && rank_by_product(denom);
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < V; v += stride) {
         const uint64_t num = outdeg[v] * uint64_t(indeg[v]);
-        const double sc = (num && !overflow) ? extended_quotient(num, denom) : 0.0;
+        double sc = 0.0;
+        if (num && !overflow && (scores || !product)) sc = product ? short_quotient(num, denom) : extended_quotient(num, denom);
         if (scores) scores[v] = sc;
-        key[v] = static_cast<uint64_t>(__double_as_longlong(sc));
-        id[v] = static_cast<uint32_t>(v);
+        key[v] = product ? num : static_cast<uint64_t>(__double_as_longlong(sc));
+        scored[v] = num && !overflow;
     }
+}
+
+// keys[i] = key[ids[i]]
+__global__ void gather_keys_kernel(const uint64_t *__restrict__ key, const uint32_t *__restrict__ ids, uint64_t n,
+                                   uint64_t *__restrict__ keys) {
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += stride) keys[i] = key[ids[i]];
 }
 
 __global__ void mark_kernel(const uint32_t *ids, uint64_t n, uint8_t *flag) {
@@ -245,25 +313,29 @@ __global__ void tile_rows_kernel(const uint64_t *__restrict__ noff, uint64_t V, 
 // New edge e of new row r copies old edge off[order[r]] + (e - noff[r]),
 // destination renamed through inv, weight carried.  Tiles of 2048
 // consecutive output edges; rows tile_row[t] .. tile_row[t + 1] cover the
-// tile.  Their new and old starts are staged in shared memory, and each
-// edge's row comes from a load-balanced search: every row start inside the
-// tile marks its position, and an inclusive max-scan over the 2048
-// positions hands each edge the last row starting at or before it (empty
-// rows share a start with the next row and lose to its larger index).  A
-// tile spanning more than 2048 rows (long runs of empty rows) searches the
-// global offsets per edge instead.  Consecutive lanes take consecutive
+// tile.  Each row's distance from new to old edge numbers is staged in shared
+// memory, and each edge's row comes from a load-balanced search: every
+// non-empty row marks its start inside the tile, and an inclusive max-scan
+// over the 2048 positions hands each edge the last row starting at or before
+// it.  A tile spanning more than 2048 rows (long runs of empty rows) searches
+// the global offsets per edge instead.  Consecutive lanes take consecutive
 // edges, so id / weight reads and writes are coalesced within a row; each
 // thread keeps its 8 edges' loads in flight together (ids and weights, then
 // the renaming gathers).
+//
+// The renaming gathers bound it, at the rate that the L1 beside shared memory
+// allows (1.02 sectors per clock and SM with all of it, 0.28 beside 200 KB): 40
+// KB of shared memory per CTA, five to an SM, held it to 771 us on R-MAT scale
+// 22 (58 M edges); 20 KB take 484 us.
 __global__ void __launch_bounds__(kPermThreads) permute_edges_kernel(
     const uint64_t *__restrict__ off, const uint32_t *__restrict__ cols, const uint32_t *__restrict__ w,
     const uint64_t *__restrict__ noff, const uint64_t *__restrict__ tile_row, const uint32_t *__restrict__ order,
     const uint32_t *__restrict__ inv, uint64_t V, uint64_t E, uint32_t *__restrict__ ncols,
     uint32_t *__restrict__ nw, uint32_t *__restrict__ bad) {
-    __shared__ uint64_t s_noff[kTileRows + 1];
-    __shared__ uint64_t s_base[kTileRows];
-    __shared__ __align__(16) uint32_t s_row[kTileEdges];
+    __shared__ int64_t s_shift[kTileRows];  // old minus new edge number of row k's edges
+    __shared__ __align__(16) uint16_t s_row[kTileEdges];
     __shared__ uint32_t s_warp[kPermThreads / 32];
+    static_assert(kTileRows <= 65536 && kPermEdges == 8, "a thread scans 8 16-bit marks");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t b = 0;
     const uint64_t pol = policy_evict_last();
@@ -274,24 +346,19 @@ __global__ void __launch_bounds__(kPermThreads) permute_edges_kernel(
         const uint64_t rows = tile_row[t + 1] - r0 + 1;  // r0 + rows <= V
         const bool staged = rows <= kTileRows;
         if (staged) {
-#pragma unroll
-            for (int j = 0; j < kPermEdges; ++j) s_row[j * kPermThreads + threadIdx.x] = 0;
-            for (uint64_t k = threadIdx.x; k <= rows; k += kPermThreads) {
-                s_noff[k] = noff[r0 + k];
-                if (k < rows) s_base[k] = off[order[r0 + k]];
-            }
+            reinterpret_cast<uint4 *>(s_row)[threadIdx.x] = make_uint4(0, 0, 0, 0);
             __syncthreads();
-            // rows k >= 1 start after e0 (row r0 holds e0); mark the ones
-            // starting inside the tile
-            for (uint32_t k = 1 + threadIdx.x; k < rows; k += kPermThreads) {
-                const uint64_t pos = s_noff[k] - e0;
-                if (pos < kTileEdges) atomicMax(s_row + pos, k);
+            // row r0 holds e0; rows k >= 1 start after it
+            for (uint32_t k = threadIdx.x; k < rows; k += kPermThreads) {
+                const uint64_t at = noff[r0 + k], end = noff[r0 + k + 1];
+                s_shift[k] = static_cast<int64_t>(off[order[r0 + k]]) - static_cast<int64_t>(at);
+                if (k && end > at && at - e0 < kTileEdges) s_row[at - e0] = static_cast<uint16_t>(k);
             }
             __syncthreads();
             // inclusive max-scan; thread i owns positions [8i, 8i + 8)
-            const uint4 lo4 = reinterpret_cast<const uint4 *>(s_row)[2 * threadIdx.x];
-            const uint4 hi4 = reinterpret_cast<const uint4 *>(s_row)[2 * threadIdx.x + 1];
-            uint32_t v[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+            const uint4 q = reinterpret_cast<const uint4 *>(s_row)[threadIdx.x];
+            uint32_t v[8] = {q.x & 0xFFFFu, q.x >> 16, q.y & 0xFFFFu, q.y >> 16,
+                             q.z & 0xFFFFu, q.z >> 16, q.w & 0xFFFFu, q.w >> 16};
 #pragma unroll
             for (int j = 1; j < 8; ++j) v[j] = max(v[j], v[j - 1]);
             uint32_t run = v[7];
@@ -304,11 +371,11 @@ __global__ void __launch_bounds__(kPermThreads) permute_edges_kernel(
             uint32_t before = __shfl_up_sync(0xffffffffu, run, 1);
             if (lane == 0) before = 0;
             __syncthreads();
-            for (int q = 0; q < warp; ++q) before = max(before, s_warp[q]);
+            for (int x = 0; x < warp; ++x) before = max(before, s_warp[x]);
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[j] = max(v[j], before);
-            reinterpret_cast<uint4 *>(s_row)[2 * threadIdx.x] = make_uint4(v[0], v[1], v[2], v[3]);
-            reinterpret_cast<uint4 *>(s_row)[2 * threadIdx.x + 1] = make_uint4(v[4], v[5], v[6], v[7]);
+            reinterpret_cast<uint4 *>(s_row)[threadIdx.x] = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16),
+                                                                       v[4] | (v[5] << 16), v[6] | (v[7] << 16));
             __syncthreads();
         }
         uint64_t src[kPermEdges];
@@ -318,8 +385,7 @@ __global__ void __launch_bounds__(kPermThreads) permute_edges_kernel(
             src[i] = 0;
             if (e < e1) {
                 if (staged) {
-                    const uint32_t k = s_row[i * kPermThreads + threadIdx.x];
-                    src[i] = s_base[k] + (e - s_noff[k]);
+                    src[i] = static_cast<uint64_t>(static_cast<int64_t>(e) + s_shift[s_row[i * kPermThreads + threadIdx.x]]);
                 } else {
                     const uint64_t r = row_of(noff, V, e);
                     src[i] = off[order[r]] + (e - noff[r]);
@@ -434,13 +500,21 @@ void hub_sort(const hyt_csr &csr, double fraction, uint32_t *order_out, double *
     const uint64_t *off = device_view(csr.row_offsets, V + 1, off_h, s);
     const uint32_t *cols = device_view(csr.column_indices, E, cols_h, s);
     Scratch<uint32_t> indeg(V, s), bad(1, s), ids(V, s), ids_alt(V, s);
-    Scratch<uint64_t> outdeg(V, s), key(V, s), key_alt(V, s), rest(1, s);
+    Scratch<uint64_t> outdeg(V, s), key(V, s), key_srt(V, s), key_alt(V, s), rest(1, s);
+    Scratch<uint8_t> is_other(V, s);
     Scratch<unsigned long long> maxes(2, s);
     HYT_CUDA(cudaMemsetAsync(indeg.get(), 0, V * 4, s));
     HYT_CUDA(cudaMemsetAsync(bad.get(), 0, 4, s));
     HYT_CUDA(cudaMemsetAsync(maxes.get(), 0, 16, s));
     main_k.start(s);
-    degree_pass_kernel<<<grid_sm(8), 256, 0, s>>>(off, cols, V, E, indeg.get(), outdeg.get(), maxes.get(), bad.get());
+    constexpr int kTable = 2 * kDegreeSlots * sizeof(uint32_t);
+    HYT_CUDA(cudaFuncSetAttribute(degree_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTable));
+    // no more CTAs than have a few edges per table slot (each clears and
+    // flushes its table)
+    const unsigned ctas = static_cast<unsigned>(
+        std::min<uint64_t>(grid_sm(2), std::max<uint64_t>(1, std::max(E, V) / (2 * kDegreeThreads))));
+    degree_pass_kernel<<<ctas, kDegreeThreads, kTable, s>>>(off, cols, V, E, indeg.get(), outdeg.get(), maxes.get(),
+                                                            bad.get());
     main_k.stop(s);
     max_in_degree_kernel<<<grid_for(V, 256, 148u * 8u), 256, 0, s>>>(indeg.get(), V, maxes.get());
     const bool scores_dev = scores_out && is_device_pointer(scores_out);
@@ -448,33 +522,49 @@ void hub_sort(const hyt_csr &csr, double fraction, uint32_t *order_out, double *
     if (scores_out && !scores_dev) sc = std::make_unique<Scratch<double>>(V, s);
     double *scores_d = scores_dev ? scores_out : (sc ? sc->get() : nullptr);
     hub_scores_kernel<<<grid_sm(8), 256, 0, s>>>(outdeg.get(), indeg.get(), V, maxes.get(), scores_d, key.get(),
-                                                 ids.get(), bad.get());
+                                                 is_other.get(), bad.get());
     HYT_CUDA(cudaGetLastError());
     if (scores_out && !scores_dev) HYT_CUDA(cudaMemcpyAsync(scores_out, scores_d, V * 8, cudaMemcpyDeviceToHost, s));
-    // scores lie in [0, 1]: their bit patterns fit in 62 bits
-    uint64_t *keys = key.get();
+    // Only vertices with a score are ranked: the others tie at 0 and keep
+    // their id order, which is where the stable sort would leave them too.
+    select_index(is_other.get(), ids.get(), V, rest.get(), s);
+    uint64_t scored = 0;
+    unsigned long long h_max[2] = {0, 0};
+    HYT_CUDA(cudaMemcpyAsync(&scored, rest.get(), 8, cudaMemcpyDeviceToHost, s));
+    HYT_CUDA(cudaMemcpyAsync(h_max, maxes.get(), 16, cudaMemcpyDeviceToHost, s));
+    const uint32_t h = read_flags(bad.get(), s);
+    fail_on_csr_flags(h);
+    if (h & kBadOverflow) fail(HYT_E_INVALID, "degree product exceeds 2^64");
+    const uint64_t denom = uint64_t(h_max[0]) * h_max[1];
+    // products: the bits of the largest; scores in [0, 1]: 62 bits
+    const int bits = denom < (uint64_t(1) << 52) ? (denom ? 64 - __builtin_clzll(denom) : 1) : 62;
+    uint64_t *keys = key_srt.get();
     uint32_t *ranked = ids.get();
-    sort_desc(keys, key_alt.get(), ranked, ids_alt.get(), V, 62, s);
+    if (scored) {
+        gather_keys_kernel<<<grid_for(scored, 256, 148u * 8u), 256, 0, s>>>(key.get(), ranked, scored, keys);
+        HYT_CUDA(cudaGetLastError());
+        sort_desc(keys, key_alt.get(), ranked, ids_alt.get(), scored, bits, s);
+    }
     const uint64_t hubs = hub_count_for(V, fraction);
-    // order = hubs (ranked) then the other vertices in id order
-    Scratch<uint8_t> is_other(V, s);
+    const uint64_t top = std::min(hubs, scored);
+    // order = hubs (ranked; where the ranked run out, vertices of score 0 by
+    // id), then the other vertices in id order: after the ranked hubs, all
+    // the others in id order either way -- unless ranked ones are left over
     HYT_CUDA(cudaMemsetAsync(is_other.get(), 1, V, s));
-    if (hubs) mark_kernel<<<grid_for(hubs, 256), 256, 0, s>>>(ranked, hubs, is_other.get());
+    if (top) mark_kernel<<<grid_for(top, 256), 256, 0, s>>>(ranked, top, is_other.get());
     HYT_CUDA(cudaGetLastError());
     const bool order_dev = is_device_pointer(order_out);
     std::unique_ptr<Scratch<uint32_t>> ord;
     if (!order_dev) ord = std::make_unique<Scratch<uint32_t>>(V, s);
     uint32_t *order_d = order_dev ? order_out : ord->get();
-    if (hubs) HYT_CUDA(cudaMemcpyAsync(order_d, ranked, hubs * 4, cudaMemcpyDeviceToDevice, s));
-    select_index(is_other.get(), order_d + hubs, V, rest.get(), s);
+    if (top) HYT_CUDA(cudaMemcpyAsync(order_d, ranked, top * 4, cudaMemcpyDeviceToDevice, s));
+    select_index(is_other.get(), order_d + top, V, rest.get(), s);
     if (!order_dev) HYT_CUDA(cudaMemcpyAsync(order_out, order_d, V * 4, cudaMemcpyDeviceToHost, s));
     whole.stop(s);
     uint64_t h_rest = 0;
     HYT_CUDA(cudaMemcpyAsync(&h_rest, rest.get(), 8, cudaMemcpyDeviceToHost, s));
-    const uint32_t h = read_flags(bad.get(), s);
-    fail_on_csr_flags(h);
-    if (h & kBadOverflow) fail(HYT_E_INVALID, "degree product exceeds 2^64");
-    if (h_rest + hubs != V) fail(HYT_E_INTERNAL, "hub ordering lost vertices");
+    HYT_CUDA(cudaStreamSynchronize(s));
+    if (h_rest + top != V) fail(HYT_E_INTERNAL, "hub ordering lost vertices");
     if (hub_count) *hub_count = hubs;
     if (stats) {
         stats->device_ms = whole.ms();
@@ -525,13 +615,11 @@ void csr_reorder(const hyt_csr &csr, const uint32_t *vertex_order, bool on_devic
     fail_on_csr_flags(h);
     auto alloc = [&](size_t bytes) -> void * {
         void *p = nullptr;
-        if (on_device && pooled) {
+        if (on_device) {  // pool memory: freed by cudaFree or cudaFreeAsync alike
             int dev = 0;
             HYT_CUDA(cudaGetDevice(&dev));
             HYT_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, graph_pool(dev), cudaStreamLegacy));
             HYT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-        } else if (on_device) {
-            HYT_CUDA(cudaMalloc(&p, bytes ? bytes : 16));
         } else {
             p = std::malloc(bytes ? bytes : 16);
             if (!p) fail(HYT_E_OOM, "host allocation failed");
