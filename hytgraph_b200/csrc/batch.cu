@@ -652,6 +652,7 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
         a.hot_vertex = g.hot_vertex.get();
         a.num_hot = g.num_hot;
         a.tile_cost = g.tile_cost;
+        a.chunk_edges = g.chunk_edges;
         for (int i = 0; i < 2; ++i) a.rank[i] = reinterpret_cast<float *>(take(V * 4 + 16));
         for (int i = 0; i < 2; ++i) a.contrib[i] = reinterpret_cast<float *>(take(V * 4 + 16));
         a.partial = reinterpret_cast<float2 *>(take(g.num_chunks * 8 + 16));

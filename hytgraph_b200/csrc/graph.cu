@@ -377,7 +377,7 @@ size_t GraphImpl::device_bytes() const {
 // Descriptor of pull task i (graph.cuh): chunks [0, num_chunks), then tiles.
 __global__ void pull_task_kernel(const uint64_t *in_off, const uint32_t *tile_start, const LongRow *long_rows,
                                  const uint2 *chunk_tasks, uint64_t num_chunks, uint64_t num_tiles, uint32_t tile_cost,
-                                 uint4 *out) {
+                                 uint32_t chunk_edges, uint4 *out) {
     const uint64_t n = num_chunks + num_tiles, stride = uint64_t(gridDim.x) * blockDim.x;
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += stride) {
         uint64_t e0 = 0, len = 0;
@@ -386,8 +386,8 @@ __global__ void pull_task_kernel(const uint64_t *in_off, const uint32_t *tile_st
             const uint2 t = chunk_tasks[i];
             const LongRow L = long_rows[t.x];
             const uint64_t rb = in_off[L.row], re = in_off[L.row + 1];
-            e0 = rb + uint64_t(t.y) * kLongChunk;
-            len = ((e0 + kLongChunk < re) ? e0 + kLongChunk : re) - e0;
+            e0 = rb + uint64_t(t.y) * chunk_edges;
+            len = ((e0 + chunk_edges < re) ? e0 + chunk_edges : re) - e0;
             a = t.x;
             b = t.y;
             chunk = 1;
@@ -443,7 +443,7 @@ void build_pull_tiles(GraphImpl &g, cudaStream_t s) {
         HYT_CUDA(cudaStreamSynchronize(s));
         uint32_t next = 0;
         for (uint64_t i = 0; i < g.num_long; ++i) {
-            const uint32_t nc = (degs[i] + kLongChunk - 1) / kLongChunk;
+            const uint32_t nc = (degs[i] + g.chunk_edges - 1) / g.chunk_edges;
             lr[i] = LongRow{ids[i], next, nc, 0};
             for (uint32_t c = 0; c < nc; ++c) tasks.push_back(make_uint2(static_cast<uint32_t>(i), c));
             next += nc;
@@ -463,7 +463,7 @@ void build_pull_tiles(GraphImpl &g, cudaStream_t s) {
     g.pull_tasks.allocate(ntasks);
     pull_task_kernel<<<grid_for(ntasks, 256), 256, 0, s>>>(g.in_offsets.get(), g.tile_start.get(), g.long_rows.get(),
                                                             g.chunk_tasks.get(), g.num_chunks, g.num_tiles, g.tile_cost,
-                                                            g.pull_tasks.get());
+                                                            g.chunk_edges, g.pull_tasks.get());
     HYT_CUDA(cudaGetLastError());
     HYT_CUDA(cudaStreamSynchronize(s));
 }
@@ -510,6 +510,7 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         const unsigned long v = std::strtoul(t, nullptr, 10);
         if (v >= kTileCostMin && v <= kTileCostDefault) g.tile_cost = static_cast<uint32_t>(v);
     }
+    g.chunk_edges = long_chunk_edges(V + E);
     uint32_t hot_request = V >= kHotLargeVertices ? kHotSourcesLarge : kHotSourcesDefault;
     if (const char *t = std::getenv("HYT_PR_HOT")) hot_request = static_cast<uint32_t>(std::strtoul(t, nullptr, 10));
     hot_request = std::min(hot_request, kHotSourcesMax);

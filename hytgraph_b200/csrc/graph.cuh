@@ -23,13 +23,25 @@ namespace hyt {
 // merge path (1 unit per row + 1 per in-edge): a tile spans tile_cost units,
 // so its rows hold fewer than tile_cost edges except for its last row.  A
 // last row with in-degree >= tile_cost is a "long row": it is excluded from
-// the tile and split into kLongChunk-edge chunks.  One warp processes one
-// task (tile or chunk).
+// the tile and split into chunks.  One warp processes one task (tile or
+// chunk).
 constexpr uint32_t kTileCostMin = 64;
 constexpr uint32_t kTileCostSmall = 512;     // ... on small ones
 constexpr uint32_t kTileCostDefault = 1024;  // merge-path units per tile on large graphs (tunable: HYT_PR_TILE)
 constexpr uint32_t kStageTileMax = 256;      // bulk-staged kernels: a tile's edges (< 2 * tile_cost) fit one slot
+// Edges per chunk of a long row.  A warp takes a chunk 256 edges at a time, so a
+// chunk is also the longest serial chain of a pass: 4096 edges cost 25 us, which
+// small graphs and out-of-HBM pieces have no other work to hide, while on large
+// graphs every chunk more is a hand-over more.  Measured with 1024 / 2048 / 4096
+// edges: PageRank on 131 K vertices, 2 M edges 468 / 500 / 598 us; on 1 M, 17 M
+// 1254 / 1121 / 1122 us; eight packed PPRs on 2 M, 34 M 5.13 / 5.17 / 5.39 ms;
+// PageRank on 16 M, 263 M 17.9 / 17.2 / 16.9 ms.
+constexpr uint32_t kLongChunkSmall = 1024;
 constexpr uint32_t kLongChunk = 4096;
+inline uint32_t long_chunk_edges(uint64_t rows_and_edges) {
+    if (rows_and_edges < uint64_t(1) << 23) return kLongChunkSmall;
+    return rows_and_edges < uint64_t(1) << 26 ? 2048u : kLongChunk;
+}
 constexpr uint32_t kHotSourcesDefault = 8192;   // shared-memory source cache (tunable: HYT_PR_HOT)
 constexpr uint32_t kHotSourcesLarge = 24576;    // ... of graphs of kHotLargeVertices or more
 constexpr uint64_t kHotLargeVertices = uint64_t(1) << 22;  // PageRank 8192 -> 24576 entries: 18.45 -> 17.75 ms at 2^24 vertices,
@@ -145,6 +157,7 @@ struct GraphImpl {
     GraphArray<uint4> pull_tasks;      // [num_chunks + num_tiles] descriptors (task_first_edge, ...)
     uint64_t num_tiles = 0, num_long = 0, num_chunks = 0;
     uint32_t tile_cost = kTileCostDefault;  // a row is long when its in-degree >= tile_cost
+    uint32_t chunk_edges = kLongChunk;      // edges per chunk of a long row
     // Hot sources: the num_hot vertices of largest out-degree.  Their
     // occurrences in in_sources carry kHotTag | slot, and each PageRank CTA
     // keeps their contributions in shared memory for the iteration.

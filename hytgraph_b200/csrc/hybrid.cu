@@ -641,6 +641,17 @@ public:
         }
     }
 
+    bool joined(size_t i) const override {
+        if (i + 1 >= h_.pull_pieces.size()) return false;
+        const size_t p = h_.pull_pieces[i].part, q = h_.pull_pieces[i + 1].part;
+        if (engines_[p] != engines_[q]) return false;
+        switch (engines_[p]) {
+            case kResident: return h_.pull_res_pos[p] - h_.pull_e0[p] == h_.pull_res_pos[q] - h_.pull_e0[q];
+            case kFilter: return group_of_[i] == group_of_[i + 1];
+            default: return true;
+        }
+    }
+
     void release(size_t i, cudaStream_t s) override {
         const size_t gi = group_of_[i];
         if (gi == kNone || i + 1 != groups_[gi].last) return;
@@ -801,6 +812,7 @@ HybridImpl *hybrid_create(const hyt_csr *csr, const hyt_csc *csc, const hyt_hybr
         HYT_CUDA(cudaMemcpyAsync(g.in_offsets.get(), h->h_in_off, (V + 1) * 8, cudaMemcpyHostToDevice, g.stream));
         HYT_CUDA(cudaStreamSynchronize(g.stream));
         g.tile_cost = kTileCostSmall;
+        g.chunk_edges = kLongChunkSmall;
         g.num_hot = 0;  // host sources are untagged
         build_pull_tiles(g, g.stream);
         build_pull_pieces(*h, slot / 4);

@@ -38,6 +38,9 @@ public:
     virtual const uint32_t *acquire(size_t p, cudaStream_t compute) = 0;
     // Work reading partition p has been enqueued on `compute`.
     virtual void release(size_t p, cudaStream_t compute) = 0;
+    // True when pieces p and p + 1 are readable together: acquired one after
+    // the other they share a base pointer, so one launch may work on both.
+    virtual bool joined(size_t p) const = 0;
 };
 
 // PageRank / personalized PageRank over a graph whose CSC sources come from

@@ -12,9 +12,8 @@
 //
 // One persistent kernel per iteration (1024 threads, one CTA per SM).  The
 // work list is the graph's pull tasks, assigned to warps round-robin
-// (warp w takes tasks w, w + W, ...; every task costs at most kLongChunk
-// edges, so no shared counter is needed):
-//   chunk tasks  -- kLongChunk-edge slices of rows with in-degree >=
+// (warp w takes tasks w, w + W, ..., the last ones on demand):
+//   chunk tasks  -- 1024- or 4096-edge slices of rows with in-degree >=
 //                   tile_cost; each warp writes a compensated partial, the
 //                   last arriving warp of a row merges the partials in chunk
 //                   order;
@@ -425,6 +424,7 @@ static PRSolveState pr_prepare(GraphImpl &g, bool personalized, uint32_t source,
     a.hot_vertex = g.hot_vertex.get();
     a.num_hot = g.num_hot;
     a.tile_cost = g.tile_cost;
+    a.chunk_edges = g.chunk_edges;
     for (int i = 0; i < 2; ++i) {
         a.rank[i] = g.rank[i].get();
         a.contrib[i] = g.contrib[i].get();
@@ -589,16 +589,33 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
     PRHeader h{};
     for (uint32_t it = 0; it < max_iter; ++it) {
         src.begin_iteration(s);
-        for (size_t p = 0; p < src.parts(); ++p) {
-            const PullPart pp = src.part(p);
-            if (pp.chunk_begin == pp.chunk_end && pp.tile_begin == pp.tile_end) continue;
-            const uint32_t *base = src.acquire(p, s);
-            const PRRange rg{base, pp.chunk_begin, pp.chunk_end, pp.tile_begin, pp.tile_end};
-            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
-            HYT_CUDA(cudaGetLastError());
-            src.release(p, s);
-            ++launches;
-            ++hot;
+        for (size_t p = 0; p < src.parts();) {
+            // Pieces readable together, with consecutive tasks, share a launch: a
+            // launch's time is that of its slowest task, not its size.  16 M
+            // edges in 64 partitions, 32 MB on the device: 71 launches an
+            // iteration -> 40, 16 iterations 31.9 -> 22.8 ms (shorter chunks
+            // of long rows included).
+            PullPart run = src.part(p);
+            size_t last = p;
+            while (src.joined(last)) {
+                const PullPart nx = src.part(last + 1);
+                if (nx.chunk_begin != run.chunk_end || nx.tile_begin != run.tile_end) break;
+                run.chunk_end = nx.chunk_end;
+                run.tile_end = nx.tile_end;
+                ++last;
+            }
+            const bool any = run.chunk_begin != run.chunk_end || run.tile_begin != run.tile_end;
+            const uint32_t *base = nullptr;
+            for (size_t q = p; q <= last; ++q) base = src.acquire(q, s);
+            if (any) {
+                const PRRange rg{base, run.chunk_begin, run.chunk_end, run.tile_begin, run.tile_end};
+                pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
+                HYT_CUDA(cudaGetLastError());
+                ++launches;
+                ++hot;
+            }
+            for (size_t q = p; q <= last; ++q) src.release(q, s);
+            p = last + 1;
         }
         pr_reduce_kernel<<<pr_reduce_grid(a), kReduceThreads, 0, s>>>(st0.d_args);
         HYT_CUDA(cudaGetLastError());

@@ -59,7 +59,7 @@ struct PRArgs {
     const uint2 *chunk_tasks;
     const uint32_t *hot_vertex;  // [num_hot] vertices cached in shared memory
     uint32_t num_hot;
-    uint32_t tile_cost;
+    uint32_t tile_cost, chunk_edges;
     float *rank[2];
     float *contrib[2];
     float2 *partial;
@@ -296,8 +296,8 @@ __device__ __forceinline__ TaskSpan task_span(uint4 d) {
 __device__ __forceinline__ TaskSpan chunk_span(const PRArgs &a, uint64_t ci) {
     const uint2 t = a.chunk_tasks[ci];
     const uint32_t row = a.long_rows[t.x].row;
-    const uint64_t lo = a.in_off[row] + uint64_t(t.y) * kLongChunk, re = a.in_off[row + 1];
-    return TaskSpan{lo, static_cast<uint32_t>((lo + kLongChunk < re ? lo + kLongChunk : re) - lo), t.x, t.y};
+    const uint64_t lo = a.in_off[row] + uint64_t(t.y) * a.chunk_edges, re = a.in_off[row + 1];
+    return TaskSpan{lo, static_cast<uint32_t>((lo + a.chunk_edges < re ? lo + a.chunk_edges : re) - lo), t.x, t.y};
 }
 
 __device__ __forceinline__ TaskSpan tile_span(const PRArgs &a, uint64_t k) {
@@ -309,7 +309,7 @@ __device__ __forceinline__ TaskSpan tile_span(const PRArgs &a, uint64_t k) {
     return TaskSpan{e0, static_cast<uint32_t>((chunked ? last_b : last_e) - e0), r0, chunked ? r1 - 1 : r1};
 }
 
-// Chunk task: a kLongChunk-edge slice of a long row.  The warp stores its
+// Chunk task: a chunk_edges-edge slice of a long row.  The warp stores its
 // compensated partial; the last arriving warp of the row merges every partial
 // in chunk order (lane j takes chunks j, j+32, ...) and finalizes the row.
 // Returns the row's long-row index when this warp finalized it (lane 0 holds

@@ -316,16 +316,17 @@ __global__ void ppr8_wide_flags_kernel(const uint64_t *__restrict__ in_off, uint
 // per-lane partial sums, stored at (chunk * pieces + piece).
 __global__ void ppr8_chunks_kernel(const uint64_t *__restrict__ in_off, Ids ids, const float *__restrict__ c,
                                    const LongRow *__restrict__ long_rows, const uint2 *__restrict__ tasks,
-                                   uint64_t num_tasks, uint32_t pieces, double *__restrict__ chunk_sum) {
+                                   uint64_t num_tasks, uint32_t chunk_edges, uint32_t pieces,
+                                   double *__restrict__ chunk_sum) {
     const int t = threadIdx.x & 31;
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
-    const uint64_t piece_edges = (kLongChunk + pieces - 1) / pieces;
+    const uint64_t piece_edges = (chunk_edges + pieces - 1) / pieces;
     for (uint64_t k = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5; k < num_tasks * pieces; k += warps) {
         const uint64_t ci = k / pieces, pc = k % pieces;
         const uint2 task = tasks[ci];
         const LongRow lr = long_rows[task.x];
-        const uint64_t cb = in_off[lr.row] + uint64_t(task.y) * kLongChunk;
-        const uint64_t ce = min(cb + kLongChunk, in_off[lr.row + 1]);
+        const uint64_t cb = in_off[lr.row] + uint64_t(task.y) * chunk_edges;
+        const uint64_t ce = min(cb + chunk_edges, in_off[lr.row + 1]);
         const uint64_t b = min(cb + pc * piece_edges, ce), e = min(b + piece_edges, ce);
         double sum[4];
         row_quad_sum(ids, c, b, e, t, sum);
@@ -666,7 +667,8 @@ void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart,
                 HYT_CUDA(cudaStreamWaitEvent(side.stream[0], side.fork, 0));
                 ppr8_chunks_kernel<<<grid_sm(8), 256, 0, side.stream[0]>>>(g.in_offsets.get(), ids, c.get(),
                                                                            g.long_rows.get(), g.chunk_tasks.get(),
-                                                                           chunks, pieces, chunk_sum.get());
+                                                                           chunks, g.chunk_edges, pieces,
+                                                                           chunk_sum.get());
                 ppr8_long_rows_kernel<<<long_grid, 256, 0, side.stream[0]>>>(g.long_rows.get(), g.num_long, pieces,
                                                                              chunk_sum.get(), x, p, dm.get(), nx,
                                                                              lpart.get());

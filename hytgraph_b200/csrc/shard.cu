@@ -605,6 +605,7 @@ void shard_pagerank_step(ShardImpl &sh, const hyt_shard_pagerank &p, uint32_t it
     a.hot_vertex = g.hot_vertex.get();
     a.num_hot = g.num_hot;
     a.tile_cost = g.tile_cost;
+    a.chunk_edges = g.chunk_edges;
     a.partial = reinterpret_cast<float2 *>(sh.partial.get());
     a.ticket = sh.ticket.get();
     a.num_tiles = g.num_tiles;
