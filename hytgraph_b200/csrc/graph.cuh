@@ -27,6 +27,7 @@ namespace hyt {
 // chunk).
 constexpr uint32_t kTileCostMin = 64;
 constexpr uint32_t kTileCostSmall = 512;     // ... on small ones
+constexpr uint32_t kTileCostHybrid = 128;    // ... of launches over one staged piece
 constexpr uint32_t kTileCostDefault = 1024;  // merge-path units per tile on large graphs (tunable: HYT_PR_TILE)
 constexpr uint32_t kStageTileMax = 256;      // bulk-staged kernels: a tile's edges (< 2 * tile_cost) fit one slot
 // Edges per chunk of a long row.  A warp takes a chunk 256 edges at a time, so a

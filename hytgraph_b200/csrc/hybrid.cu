@@ -811,8 +811,14 @@ HybridImpl *hybrid_create(const hyt_csr *csr, const hyt_csc *csc, const hyt_hybr
         g.in_offsets.allocate(V + 1);
         HYT_CUDA(cudaMemcpyAsync(g.in_offsets.get(), h->h_in_off, (V + 1) * 8, cudaMemcpyHostToDevice, g.stream));
         HYT_CUDA(cudaStreamSynchronize(g.stream));
-        g.tile_cost = kTileCostSmall;
-        g.chunk_edges = kLongChunkSmall;
+        // A launch covers one staged group, a few hundred thousand edges: its
+        // time is that of one task, so tasks are short while their descriptors
+        // stay small beside the rows (1 M vertices, 16 M edges, 1.5-MB groups,
+        // 16 iterations: tiles 512, chunks 1024 23.1 ms; 256, 1024 21.5 ms;
+        // 128, 512 20.4 ms; 128, 256 20.3 ms).
+        const bool small = V + E < uint64_t(1) << 26;
+        g.tile_cost = small ? kTileCostHybrid : kTileCostSmall;
+        g.chunk_edges = small ? 512 : kLongChunkSmall;
         g.num_hot = 0;  // host sources are untagged
         build_pull_tiles(g, g.stream);
         build_pull_pieces(*h, slot / 4);
