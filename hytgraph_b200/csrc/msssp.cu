@@ -49,7 +49,7 @@ using ssc::kHubDegree;
 
 constexpr int kML = 8;             // labels per vertex row (32 bytes)
 constexpr int kMSThreads = 256;    // push kernels
-constexpr int kMPThreads = 768;    // pull sweep (one CTA per SM; 85 registers a thread)
+constexpr int kMPThreads = 640;    // pull sweep (one CTA per SM; 102 registers a thread)
 
 struct MSHeader {
     uint32_t round, done, converged, pad0;
@@ -347,8 +347,15 @@ __global__ void __launch_bounds__(kMSThreads) ms_hub_kernel(const MSArgs *__rest
 // sweep -- the hub rows, whose chunks come first -- feed the rows after them.
 // A minimum does not mind an edge taken twice, so threads without an edge of
 // their own repeat their row's last one (the same sector) in place of
-// predicated loads; a sweep is bound by instructions: 8 labels to extend per
-// edge.
+// predicated loads.
+//
+// A sweep waits for L2: a step's ids, then its labels, with 20 to 24 warps an
+// SM to hide them (31 % of issue slots used, 0.3 of 1.0 sectors a clock).  So
+// the next step's ids are loaded while this step's labels are on their way,
+// at 640 threads for the registers that takes (768 spill, 512 hide less).  Eight
+// sources on 1 M vertices, 15 M edges 1.66 -> 1.57 ms (768 threads 1.66, 512
+// 1.62; 512 with 8 edges in flight 1.62); five on 2 M in input order 3.22 ->
+// 3.09 (3.14, 3.36; 3.61).
 
 constexpr int kPullN = 4;                  // edges in flight per thread
 constexpr uint32_t kWideRow = 16 * kPullN;  // rows with this many in-edges are taken by the whole warp
@@ -360,38 +367,52 @@ struct InEdges {
     uint32_t inf, bits;
 };
 
-// Minimum of the candidates of edges b, b + step, ..., capped at edge `last`
-// (kPullN of them, all loaded before the first is used) into m.
-template <int WK, bool kB>
-__device__ __forceinline__ void edges_min(const InEdges &E, uint32_t b, uint32_t last, uint32_t step, Row8 &m) {
+// kPullN edges' ids and weights as they were loaded (packed: `u` holds the
+// words, decoded when they are used).
+struct Edges {
     uint32_t u[kPullN], wt[kPullN];
-    if constexpr (kB && WK == HYT_WEIGHTS_U32) {
-        const uint32_t mask = (1u << E.bits) - 1u;
+};
+
+// Edges b, b + step, ..., capped at edge `last`.
+template <int WK, bool kB>
+__device__ __forceinline__ void load_edges(const InEdges &E, uint32_t b, uint32_t last, uint32_t step, Edges &x) {
+    constexpr bool kPacked = kB && WK == HYT_WEIGHTS_U32;
+    const uint32_t *ids = kPacked ? E.w : E.src;
 #pragma unroll
-        for (int j = 0; j < kPullN; ++j) {
-            const uint32_t x = dev::ld_stream(E.w + min(b + j * step, last));
-            u[j] = x & mask;
-            wt[j] = x >> E.bits;
-        }
-    } else {
+    for (int j = 0; j < kPullN; ++j) x.u[j] = dev::ld_stream(ids + min(b + j * step, last));
+    if constexpr (!kPacked) {
 #pragma unroll
-        for (int j = 0; j < kPullN; ++j) u[j] = dev::ld_stream(E.src + min(b + j * step, last));
-#pragma unroll
-        for (int j = 0; j < kPullN; ++j) wt[j] = ssc::edge_weight<WK>(E.w, min(b + j * step, last));
-#pragma unroll
-        for (int j = 0; j < kPullN; ++j)
-            if (u[j] & kHotTag) u[j] = E.s_hot[u[j] & ~kHotTag];
+        for (int j = 0; j < kPullN; ++j) x.wt[j] = ssc::edge_weight<WK>(E.w, min(b + j * step, last));
     }
+}
+
+// Minimum of the candidates of edges x (all their labels are loaded before the
+// first is used) into m; then() runs while the labels are on their way.
+template <int WK, bool kB, class F>
+__device__ __forceinline__ void edges_min(const InEdges &E, const Edges &x, Row8 &m, F then) {
+    constexpr bool kPacked = kB && WK == HYT_WEIGHTS_U32;
+    const uint32_t mask = (1u << E.bits) - 1u;
+    uint32_t wt[kPullN];
     Row8 du[kPullN];
 #pragma unroll
     for (int j = 0; j < kPullN; ++j) {
+        uint32_t u;
+        if constexpr (kPacked) {
+            u = x.u[j] & mask;
+            wt[j] = x.u[j] >> E.bits;
+        } else {
+            u = x.u[j];
+            wt[j] = x.wt[j];
+            if (u & kHotTag) u = E.s_hot[u & ~kHotTag];
+        }
         // the whole 32-byte row in one load: one L1 access per edge (two
         // 16-byte loads took the sector twice)
         asm volatile("ld.global.L2::evict_last.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=r"(du[j].d[0]), "=r"(du[j].d[1]), "=r"(du[j].d[2]), "=r"(du[j].d[3]), "=r"(du[j].d[4]),
                        "=r"(du[j].d[5]), "=r"(du[j].d[6]), "=r"(du[j].d[7])
-                     : "l"(E.dist + size_t(u[j]) * kML));
+                     : "l"(E.dist + size_t(u) * kML));
     }
+    then();
 #pragma unroll
     for (int j = 0; j < kPullN; ++j)
 #pragma unroll
@@ -405,7 +426,13 @@ __device__ __forceinline__ Row8 span_min(const InEdges &E, uint32_t b, uint32_t 
     Row8 m;
 #pragma unroll
     for (int l = 0; l < kML; ++l) m.d[l] = E.inf;
-    for (uint32_t at = b; at < e; at += 32 * kPullN) edges_min<WK, kB>(E, at + lane, e - 1, 32, m);
+    Edges x;
+    load_edges<WK, kB>(E, b + lane, e - 1, 32, x);
+    for (uint32_t at = b; at < e; at += 32 * kPullN) {
+        Edges nx;
+        edges_min<WK, kB>(E, x, m, [&] { load_edges<WK, kB>(E, at + 32 * kPullN + lane, e - 1, 32, nx); });
+        x = nx;
+    }
 #pragma unroll
     for (int l = 0; l < kML; ++l) m.d[l] = __reduce_min_sync(0xffffffffu, m.d[l]);
     return m;
@@ -413,23 +440,34 @@ __device__ __forceinline__ Row8 span_min(const InEdges &E, uint32_t b, uint32_t 
 
 // Lowest candidates of the warp's 32 rows (lane l: edges [lo, hi)), `slots`
 // edges of a row side by side, 32 / slots rows a step; rows have at most
-// slots * kPullN in-edges.  Rows without edges get an arbitrary result.
+// slots * kPullN in-edges.  Rows without edges get an arbitrary result.  The
+// next step's edges are loaded while this step's labels are on their way.
 template <int WK, bool kB>
 __device__ __forceinline__ Row8 group_min(const InEdges &E, uint32_t lo, uint32_t hi, int slots, int lane) {
     const int rows = 32 / slots;
-    const uint32_t live = __ballot_sync(0xffffffffu, hi > lo);
+    const uint32_t live = __ballot_sync(0xffffffffu, hi > lo);  // not 0
     Row8 mine;
 #pragma unroll
     for (int l = 0; l < kML; ++l) mine.d[l] = E.inf;
-    for (int first = 0; first < 32; first += rows) {
-        if (!((live >> first) & (rows == 32 ? 0xFFFFFFFFu : (1u << rows) - 1u))) continue;
+    // steps without a row that has edges are left out
+    const uint32_t step = rows == 32 ? 0xFFFFFFFFu : (1u << rows) - 1u;
+    auto load = [&](int first, Edges &x) {
         const int owner = first + lane / slots;
         const uint32_t b = __shfl_sync(0xffffffffu, lo, owner);
         const uint32_t e = __shfl_sync(0xffffffffu, hi, owner);
+        load_edges<WK, kB>(E, b + lane % slots, e > b ? e - 1 : 0u, slots, x);
+    };
+    int first = (__ffs(live) - 1) & ~(rows - 1);
+    Edges x;
+    load(first, x);
+    for (;;) {
+        const uint32_t rest = live & ~(step << first) & ~((1u << first) - 1u);
+        const int next = rest ? (__ffs(rest) - 1) & ~(rows - 1) : 32;
+        Edges nx;
         Row8 m;
 #pragma unroll
         for (int l = 0; l < kML; ++l) m.d[l] = E.inf;
-        edges_min<WK, kB>(E, b + lane % slots, e > b ? e - 1 : 0u, slots, m);
+        edges_min<WK, kB>(E, x, m, [&] { if (next < 32) load(next, nx); });
         for (int o = 1; o < slots; o <<= 1)
 #pragma unroll
             for (int l = 0; l < kML; ++l) m.d[l] = min(m.d[l], __shfl_xor_sync(0xffffffffu, m.d[l], o));
@@ -440,6 +478,9 @@ __device__ __forceinline__ Row8 group_min(const InEdges &E, uint32_t lo, uint32_
             const uint32_t t = __shfl_sync(0xffffffffu, m.d[l], from);
             if (own) mine.d[l] = t;
         }
+        if (next >= 32) break;
+        first = next;
+        x = nx;
     }
     return mine;
 }
