@@ -192,6 +192,7 @@ struct GraphImpl {
     GraphArray<unsigned char> ms_state;
     PinnedArray<uint64_t> host_scratch;  // small pinned readback area
     LoopGraph sssp_loop;                 // instantiated SSSP round loop (reused while its shape holds)
+    LoopGraph ms_loop;                   // ... of the multi-source solve
 
     size_t device_bytes() const;
 };
