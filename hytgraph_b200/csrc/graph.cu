@@ -503,8 +503,8 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
         fail(HYT_E_INVALID, "weights is NULL for a weighted graph");
     if (flags == 0) flags = HYT_GRAPH_ALL;
     // PageRank decomposition knobs (same work, different tiling): tile cost
-    // in {64..1024} and hot-source cache size.  The staged kernels
-    // (HYT_STAGED=1) need tiles that fit one staging slot.
+    // in {64..1024} and hot-source cache size.  The packed PPR's staged task
+    // pass (HYT_STAGED=1) needs tiles that fit one staging slot.
     g.tile_cost = stage::staged_requested() ? kStageTileMax : tile_cost_for(V, E);
     if (const char *t = std::getenv("HYT_PR_TILE")) {
         const unsigned long v = std::strtoul(t, nullptr, 10);

@@ -18,15 +18,15 @@
 //                 takes, per lane, the minimum of d[u] + w over its
 //                 in-edges: one id and one 32-byte label row per in-edge
 //                 for all lanes, 1 to 32 edges of a row side by side, 4
-//                 label rows in flight per thread.  A row is skipped when no in-edge can
-//                 lower it in any lane: its label is at most (lowest label
-//                 of the frontier in that lane + smallest weight).  Tile
-//                 rows are written with plain stores (one writer per row
-//                 during a sweep).
+//                 label rows in flight per thread.  A row is skipped when
+//                 no in-edge can lower it in any lane: its label is at most
+//                 (lowest label of the frontier in that lane + smallest
+//                 weight).  Tile rows are written with plain stores (one
+//                 writer per row during a sweep).
 // A sweep used to walk short rows one lane per row and extend labels with
 // saturation: 8 sources on R-MAT scale 20 / 24 took 1.98 / 8.74 ms, now 1.69 /
-// 7.81 ms (768 threads: 1024 spill, 1.78 ms; 8 rows in flight in 512 threads
-// 1.72 ms; 2 rows 1.71 ms).
+// 7.81 ms, before the changes noted at the sweep and at the loop's
+// instantiation.
 // Per edge the memory traffic is about that of one single-source
 // relaxation, whatever the number of lanes; the rounds are those of the
 // deepest source.  Rounds run as a CUDA-graph conditional while-loop.

@@ -10,17 +10,19 @@
 // are compensated (TwoSum/Kahan) in FP32; residual and dangling mass are
 // reduced in FP64.
 //
-// One persistent kernel per iteration (1024 threads, one CTA per SM).  The
+// The whole solve is one cooperative kernel (pr_solve_kernel: 1024 threads, one
+// CTA per SM, a grid barrier between the passes); out-of-HBM solves and solves
+// launched kernel by kernel run pr_iterate_kernel over a range of tasks.  The
 // work list is the graph's pull tasks, assigned to warps round-robin
 // (warp w takes tasks w, w + W, ..., the last ones on demand):
-//   chunk tasks  -- 1024- or 4096-edge slices of rows with in-degree >=
+//   chunk tasks  -- 1024- to 4096-edge slices of rows with in-degree >=
 //                   tile_cost; each warp writes a compensated partial, the
 //                   last arriving warp of a row merges the partials in chunk
 //                   order;
-//   tile tasks   -- merge-path tiles of consecutive shorter rows (512
-//                   units by default), 32 rows at a time: groups of 1 to 8
-//                   lanes, or the whole warp, gather a row's contributions
-//                   and sum them in registers (tile_task).
+//   tile tasks   -- merge-path tiles of consecutive shorter rows (512 or
+//                   1024 units), 32 rows at a time: groups of 1 to 8 lanes,
+//                   or the whole warp, gather a row's contributions and sum
+//                   them in registers (tile_task).
 //
 // What bounds it: random 4-byte gathers cost one 32-byte L2 sector each, and
 // an SM takes at most 1.02 sectors per clock (measured on a 64 MB table), but
@@ -34,8 +36,8 @@
 // Results are deterministic: every row sum has a fixed association order,
 // and the FP64 residual and dangling mass are summed in a fixed slot order
 // (PRSlots), independent of the grid size and of warp arrival order: each
-// task stores its slot, then pr_reduce_kernel sums the slots and evaluates
-// the stop rule.
+// task stores its slot, then the reduction sums the slots and evaluates the
+// stop rule.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

@@ -146,7 +146,7 @@ struct PullGraph {
     const LongRow *long_rows;
     const uint32_t *hot_vertex;
     const uint4 *tasks;       // pull task descriptors: chunks of long rows, then tiles
-    uint64_t num_tasks, num_chunks;
+    uint64_t num_tasks;
     uint64_t dealt;           // tasks dealt to the warps in turn; the rest go to whoever is free
     uint32_t num_hot;
     uint32_t bits;            // packed words: bits of the source id
@@ -666,7 +666,6 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         pg.hot_vertex = g.hot_vertex.get();
         pg.tasks = g.pull_tasks.get();
         pg.num_tasks = g.num_chunks + g.num_tiles;
-        pg.num_chunks = g.num_chunks;
         pg.dealt = pg.num_tasks - pg.num_tasks / 4;  // skipped rows make tasks uneven in any vertex order
         pg.num_hot = kPacked ? 0u : g.num_hot;
         pg.bits = g.in_pack_bits;

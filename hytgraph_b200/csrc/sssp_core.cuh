@@ -51,7 +51,6 @@ struct SSHeader {
     uint32_t pull_rounds;               // rounds run as pull sweeps
     uint32_t error;                     // 1: a bounded wait at a grid barrier ran out
     unsigned long long frontier_edges_next;  // out-edges of the next frontier, summed at round close
-    uint32_t close_ticket;                   // blocks of the round-close kernel finished
     uint32_t fmin;      // lowest label in this round's frontier (pull-capable solves with row skipping)
     uint32_t fmin_inv;  // ~(lowest label) of the next frontier, gathered by the kernels that fill it
     uint32_t task_cursor;  // pull tasks handed out beyond the dealt ones

@@ -1,20 +1,14 @@
-// Per-warp staging pipeline of the pull kernels (PageRank iterations and
-// SSSP pull sweeps over an in-HBM CSC).  A warp walks its pull tasks
-// (graph.cuh descriptors) as units -- a tile, or a kUnitEdges-edge piece of
-// a long-row chunk -- and stages each unit's source ids into shared memory
-// with one bulk copy (cp.async.bulk, completion on an mbarrier), one unit
-// ahead of the unit it is working on.  Ids then cost no registers and no
-// load latency on the warp's critical path; the warp's registers go to the
-// dependent gathers instead.
+// Per-warp staging pipeline of the packed PPR's task pass (ppr_multi.cu).  A
+// warp walks its pull tasks (graph.cuh descriptors) as units -- a tile, or a
+// kUnitEdges-edge piece of a long-row chunk -- and stages each unit's source
+// ids into shared memory with one bulk copy (cp.async.bulk, completion on an
+// mbarrier), one unit ahead of the unit it is working on.
 //
 // Sources are this GPU's own memory only (no multicast).
 //
-// The staged kernels are opt-in (HYT_STAGED=1, which also selects
-// kStageTileMax-unit tiles so that a tile fits one slot).  On R-MAT graphs
-// the register-path kernels with 512-unit tiles ran faster: the pull
-// kernels are bound by instruction issue over the dependent gathers, not by
-// the id stream, and half-size tiles leave half of each unit's gather
-// slots and row lanes idle.
+// Opt-in: tiles must fit a slot, so it runs on graphs built with tiles of at
+// most kStageTileMax units (HYT_STAGED=1, or HYT_PR_TILE).  PageRank and SSSP
+// sweeps sum from registers at every tile size.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,7 +37,7 @@ static_assert(kStageSlots >= 2, "at least double buffering");
 // A tile's edges: the rows starting inside a tile span < tile_cost merge
 // units, and its last short row adds < tile_cost more, so < 2 * tile_cost.
 static_assert(2 * kStageTileMax - 1 + 6 <= kSlotWords, "a tile's edges must fit one staging slot");
-static_assert(kLongChunk % kUnitEdges == 0, "chunks split into whole units");
+static_assert(kLongChunk % kUnitEdges == 0 && kLongChunkSmall % kUnitEdges == 0, "chunks split into whole units");
 
 // The unit a slot holds (written by lane 0 when its copy is issued).
 struct UnitMeta {
@@ -62,7 +56,7 @@ constexpr size_t kStageBytes = kStageHead + size_t(kStageWarps) * kStageSlots * 
 
 inline size_t staged_shared_bytes(uint32_t num_hot) { return kStageBytes + size_t(num_hot) * 4; }
 
-// HYT_STAGED=1: in-HBM PageRank and SSSP pull sweeps use the staged kernels.
+// HYT_STAGED=1: graphs are built with kStageTileMax-unit tiles.
 inline bool staged_requested() {
     static const bool on = [] {
         const char *e = std::getenv("HYT_STAGED");
@@ -179,19 +173,6 @@ __device__ __forceinline__ bool stage_pipeline(const uint4 *tasks, const uint32_
         }
     }
     return true;
-}
-
-// The same walk without staging, for graphs whose tiles exceed a slot:
-// consume(d, task, j, units, in_src, 0) for every unit of every task, the
-// consumer reading ids from global memory in place.
-template <class Consume>
-__device__ __forceinline__ void direct_tasks(const uint4 *tasks, const uint32_t *in_src, uint64_t first,
-                                             uint64_t stride, uint64_t total, Consume &&consume) {
-    for (uint64_t t = first; t < total; t += stride) {
-        const uint4 d = tasks[t];
-        const uint32_t nu = units_of(d);
-        for (uint32_t j = 0; j < nu; ++j) consume(d, t, j, nu, in_src, uint64_t(0));
-    }
 }
 
 #endif  // __CUDACC__
