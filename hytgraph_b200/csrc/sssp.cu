@@ -174,7 +174,14 @@ __device__ __forceinline__ bool pull_relax(const SSArgs &a, const RoundView &rv,
     return true;
 }
 
-constexpr int kPullThreads = 1024;  // one CTA per SM, like the PageRank kernel
+// One CTA per SM.  768 threads leave 80 registers: 1024 spill in the whole-solve
+// kernel and make every grid barrier wait for more warps.  Threads 1024 / 896 /
+// 768 / 640 / 512, one source: R-MAT 16 M vertices 2.34 / 2.35 / 2.34 / 2.42 /
+// 2.65 ms, 1 M 565 / 549 / 511 / 504 / 552 us, 2 M in input order 675 / 650 /
+// 650 / 688 / 714 us, 4099 vertices 323 / 322 / 300 / 272 / 267 us (one box
+// each side of 768).  Loading a step's ids ahead, as the multi-source sweep
+// does, was slower at every size (2.41 ms and up at 16 M).
+constexpr int kPullThreads = 768;
 
 // Row skipping.  Let F be this round's frontier (every vertex whose label
 // dropped since its out-edges were last relaxed) and fmin its lowest label.
