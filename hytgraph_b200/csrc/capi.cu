@@ -119,9 +119,10 @@ GraphImpl &impl(hyt_graph *g) {
 
 void use_device(const GraphImpl &g) { HYT_CUDA(cudaSetDevice(g.device)); }
 
-// HYT_LAUNCH=host selects host-driven launch loops instead of CUDA graphs
-// with conditional nodes (same kernels, same work; profilers such as ncu
-// cannot attribute kernels inside conditional graphs).
+// HYT_LAUNCH=host selects host-driven launch loops instead of whole-solve
+// kernels and CUDA graphs with conditional nodes (same device functions, same
+// work; profilers such as ncu cannot attribute kernels inside conditional
+// graphs, nor phases inside one kernel).
 uint32_t launch_flags(uint32_t flags) {
     static const bool host = [] {
         const char *v = std::getenv("HYT_LAUNCH");

@@ -145,7 +145,7 @@ int hyt_graph_get_info(const hyt_graph *graph, hyt_graph_info *out);
 
 enum hyt_run_flags {
     HYT_RUN_PROFILE = 1u,   /* time every hot-kernel launch with events */
-    HYT_RUN_NO_GRAPH = 2u   /* host-driven loop instead of a CUDA graph */
+    HYT_RUN_NO_GRAPH = 2u   /* host-driven loop instead of one on the device */
 };
 
 typedef struct hyt_pagerank_params {
