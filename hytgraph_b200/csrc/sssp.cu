@@ -182,6 +182,13 @@ __device__ __forceinline__ bool pull_relax(const SSArgs &a, const RoundView &rv,
 // each side of 768).  Loading a step's ids ahead, as the multi-source sweep
 // does, was slower at every size (2.41 ms and up at 16 M).
 constexpr int kPullThreads = 768;
+// A whole solve with fewer tasks than the GPU has warps runs with smaller CTAs, down
+// to 16 warps: its rounds are barriers, which wait for every warp, while fewer
+// warps mean more CTAs to meet.  At least 24 / 16 / 8 / 4 warps: 4099 vertices in
+// input order 312 / 300 / 298 / 325 us, in hub order 241 / 239 / 261 / 288 us,
+// 16001 in hub order 225 / 215 / 212 / 220 us; from 131 K vertices on all are the
+// same.
+constexpr uint64_t kMinWarps = 16;
 
 // Row skipping.  Let F be this round's frontier (every vertex whose label
 // dropped since its out-edges were last relaxed) and fmin its lowest label.
@@ -213,13 +220,13 @@ __device__ __forceinline__ void pull_sweep(const SSArgs &a, const PullGraph &pg,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t pol = dev::policy_evict_last();
     const auto label = [&](uint32_t u) { return dev::ld_keep_u32(a.dist + u, pol); };
-    const uint64_t nwarps = uint64_t(gridDim.x) * (kPullThreads / 32);
+    const uint64_t nwarps = uint64_t(gridDim.x) * (blockDim.x / 32);
     const uint32_t *pf_a = kPacked ? pg.in_w : pg.in_src;
     const uint32_t *pf_w = (kPacked || WK == HYT_WEIGHTS_NONE) ? nullptr : pg.in_w;
     bool skip_on;
     const uint32_t skip_at = skip_bound<WK>(a, fmin, skip_on);
     const uint64_t dealt = max(pg.dealt, min(pg.num_tasks, nwarps));  // every warp's first task is dealt
-    uint64_t task = uint64_t(blockIdx.x) * (kPullThreads / 32) + warp;
+    uint64_t task = uint64_t(blockIdx.x) * (blockDim.x / 32) + warp;
     // each dealt task's descriptor is read while the task before it runs
     uint4 d = task < pg.num_tasks ? pg.tasks[task] : make_uint4(0, 0, 0, 0);
     while (task < pg.num_tasks) {
@@ -350,8 +357,8 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __gri
                                                                      SolveState *st, uint32_t max_rounds) {
     extern __shared__ __align__(16) uint32_t s_hot[];
     const int lane = threadIdx.x & 31;
-    const uint32_t gwarp = (blockIdx.x * kPullThreads + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * kPullThreads) >> 5;
+    const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     uint32_t barriers = 0;
     load_hot_ids(pg, s_hot);
@@ -733,11 +740,12 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         // every CTA must be resident; no more of them than a sweep or a full
         // frontier has work for
         const uint64_t work = std::max<uint64_t>(pg.num_tasks, (V + 127) / 128);
+        const uint64_t warps = std::clamp<uint64_t>((work + pgrid - 1) / pgrid, kMinWarps, kPullThreads / 32);
         const unsigned ctas = static_cast<unsigned>(
-            std::min<uint64_t>(pgrid, std::max<uint64_t>(1, (work + kPullThreads / 32 - 1) / (kPullThreads / 32))));
+            std::min<uint64_t>(pgrid, std::max<uint64_t>(1, (work + warps - 1) / warps)));
         void *kargs[] = {&a, &pg, &solve_state, &max_rounds};
         HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(sssp_solve_kernel<WK, kPacked>), dim3(ctas),
-                                             dim3(kPullThreads), kargs, pull_smem, s));
+                                             dim3(static_cast<unsigned>(32 * warps)), kargs, pull_smem, s));
     } else {
         HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(a), cudaMemcpyHostToDevice, s));
         HYT_CUDA(cudaMemcpyAsync(hdr, &h0, sizeof(h0), cudaMemcpyHostToDevice, s));
