@@ -9,6 +9,7 @@
 #include "host_checks.hpp"
 #include "scratch.cuh"
 #include "graph.cuh"
+#include "outputs.cuh"
 #include "solvers.cuh"
 #include "staging.cuh"
 
@@ -34,20 +35,6 @@ cudaMemPool_t graph_pool(int device) {
     HYT_CUDA(cudaMemPoolCreate(&pool, &props));
     uint64_t keep = kGraphPoolKeep;
     HYT_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    // reachable from the peers that could reach a plain allocation (device
-    // CSRs handed to callers live here)
-    int n = 0;
-    HYT_CUDA(cudaGetDeviceCount(&n));
-    for (int peer = 0; peer < n; ++peer) {
-        int can = 0;
-        if (peer == device || cudaDeviceCanAccessPeer(&can, peer, device) != cudaSuccess || !can) continue;
-        cudaMemAccessDesc d{};
-        d.location.type = cudaMemLocationTypeDevice;
-        d.location.id = peer;
-        d.flags = cudaMemAccessFlagsProtReadWrite;
-        (void)cudaMemPoolSetAccess(pool, &d, 1);
-    }
-    (void)cudaGetLastError();
     pools[device] = pool;
     return pool;
 }
@@ -332,9 +319,9 @@ int hyt_csr_buffers_free(hyt_csr_buffers *b) {
     return guarded([&] {
         if (!b) return;
         if (b->on_device) {
-            if (b->row_offsets) cudaFree(b->row_offsets);
-            if (b->column_indices) cudaFree(b->column_indices);
-            if (b->weights) cudaFree(b->weights);
+            output_free(b->row_offsets, (b->num_vertices + 1) * 8);
+            output_free(b->column_indices, b->num_edges * 4);
+            output_free(b->weights, b->num_edges * 4);
         } else {
             std::free(b->row_offsets);
             std::free(b->column_indices);
@@ -438,6 +425,7 @@ int hyt_trim_device_memory(int device) {
         HYT_CUDA(cudaMemPoolTrimTo(graph_pool(device), 0));
         HYT_CUDA(cudaMemPoolTrimTo(scratch_pool(), 0));
         staging_release(device);
+        output_release(device);
         HYT_CUDA(cudaSetDevice(cur));
     });
 }

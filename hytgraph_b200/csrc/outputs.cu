@@ -1,0 +1,147 @@
+// Kept cudaMalloc blocks of caller-owned results; see outputs.cuh.
+#include <cuda.h>
+
+#include <algorithm>
+#include <mutex>
+#include <unordered_map>
+#include <vector>
+
+#include "common.cuh"
+#include "outputs.cuh"
+
+namespace hyt {
+namespace {
+
+struct Live {
+    int device;
+    size_t size, asked;  // of the block; by the caller it was handed to
+};
+struct Kept {
+    int device;
+    size_t size;
+    void *p;
+};
+struct Blocks {
+    std::mutex mu;
+    std::unordered_map<void *, Live> live;
+    std::vector<Kept> kept;  // oldest first
+};
+
+Blocks &blocks() {
+    static auto *b = new Blocks();  // never destroyed: the CUDA context may be gone before it
+    return *b;
+}
+
+// Waits for the work of every device in use (a peer may be reading too).
+bool wait_for_devices() {
+    static const auto state = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPoint("cuDevicePrimaryCtxGetState", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<CUresult (*)(CUdevice, unsigned *, int *)>(f);
+    }();
+    int n = 0, cur = 0;
+    if (cudaGetDevice(&cur) != cudaSuccess || cudaGetDeviceCount(&n) != cudaSuccess) return false;
+    bool ok = cudaDeviceSynchronize() == cudaSuccess;
+    for (int d = 0; d < n && ok; ++d) {
+        unsigned flags = 0;
+        int active = 0;
+        if (d == cur) continue;
+        if (!state || state(d, &flags, &active) != CUDA_SUCCESS) return false;
+        if (active) ok = cudaSetDevice(d) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+    }
+    if (n > 1) cudaSetDevice(cur);
+    return ok;
+}
+
+}  // namespace
+
+void *output_alloc(size_t bytes) {
+    Blocks &b = blocks();
+    int device = 0;
+    HYT_CUDA(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lk(b.mu);
+    // the smallest kept block that is large enough and wastes at most a quarter
+    auto best = b.kept.end();
+    for (auto k = b.kept.begin(); k != b.kept.end(); ++k)
+        if (k->device == device && k->size >= bytes && k->size - bytes <= bytes / 4 &&
+            (best == b.kept.end() || k->size < best->size))
+            best = k;
+    if (best != b.kept.end()) {
+        void *p = best->p;
+        b.live[p] = Live{device, best->size, bytes};
+        b.kept.erase(best);
+        return p;
+    }
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation && !b.kept.empty()) {  // what is kept may be what is missing
+        (void)cudaGetLastError();
+        for (const Kept &k : b.kept) cudaFree(k.p);
+        b.kept.clear();
+        e = cudaMalloc(&p, bytes ? bytes : 16);
+    }
+    cuda_check(e, "cudaMalloc of a result");
+    try {
+        b.live[p] = Live{device, bytes ? bytes : 16, bytes};
+    } catch (...) {
+        cudaFree(p);
+        throw;
+    }
+    return p;
+}
+
+void output_free(void *p, size_t bytes) noexcept {
+    if (!p) return;
+    Blocks &b = blocks();
+    Live l{};
+    {
+        std::lock_guard<std::mutex> lk(b.mu);
+        const auto it = b.live.find(p);
+        if (it != b.live.end()) {
+            // a block freed behind our back may have come back from cudaMalloc
+            // at another size: only one that matches is known to be ours
+            if (it->second.asked == bytes) l = it->second;
+            b.live.erase(it);
+        }
+    }
+    if (l.size == 0 || l.size > kOutputKeep || !wait_for_devices()) {
+        cudaFree(p);
+        return;
+    }
+    std::lock_guard<std::mutex> lk(b.mu);
+    try {
+        b.kept.push_back(Kept{l.device, l.size, p});
+    } catch (...) {
+        cudaFree(p);
+        return;
+    }
+    size_t held = 0;
+    for (const Kept &k : b.kept) held += k.device == l.device ? k.size : 0;
+    for (auto k = b.kept.begin(); held > kOutputKeep;) {
+        if (k->device != l.device) {
+            ++k;
+            continue;
+        }
+        held -= k->size;
+        cudaFree(k->p);
+        k = b.kept.erase(k);
+    }
+}
+
+void output_release(int device) noexcept {
+    Blocks &b = blocks();
+    std::lock_guard<std::mutex> lk(b.mu);
+    for (auto k = b.kept.begin(); k != b.kept.end();) {
+        if (k->device != device) {
+            ++k;
+            continue;
+        }
+        cudaFree(k->p);
+        k = b.kept.erase(k);
+    }
+}
+
+}  // namespace hyt

@@ -32,6 +32,7 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include "common.cuh"
+#include "outputs.cuh"
 #include "scratch.cuh"
 #include "solvers.cuh"
 
@@ -615,11 +616,13 @@ void csr_reorder(const hyt_csr &csr, const uint32_t *vertex_order, bool on_devic
     fail_on_csr_flags(h);
     auto alloc = [&](size_t bytes) -> void * {
         void *p = nullptr;
-        if (on_device) {  // pool memory: freed by cudaFree or cudaFreeAsync alike
+        if (on_device && pooled) {
             int dev = 0;
             HYT_CUDA(cudaGetDevice(&dev));
             HYT_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, graph_pool(dev), cudaStreamLegacy));
             HYT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        } else if (on_device) {
+            p = output_alloc(bytes);
         } else {
             p = std::malloc(bytes ? bytes : 16);
             if (!p) fail(HYT_E_OOM, "host allocation failed");
