@@ -124,8 +124,13 @@ bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaS
     } else if (attr.type != cudaMemoryTypeUnregistered) {
         return false;  // pinned (or device) memory copies at the link's speed by itself
     }
-    int device = 0;
+    int device = 0, of_stream = 0;
     HYT_CUDA(cudaGetDevice(&device));
+    if (cudaStreamGetDevice(s, &of_stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (of_stream != device) return false;  // the pool's events cannot be recorded on another device's stream
     Pool &p = pool_of(device);
     std::unique_lock<std::mutex> lk(p.mu, std::try_to_lock);
     if (!lk.owns_lock() || !p.open()) return false;

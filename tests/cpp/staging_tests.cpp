@@ -1,0 +1,114 @@
+// CPU tests of the pinned-chunk copies (hytgraph_b200/csrc/staging.cu) over a
+// runtime made up here: two devices whose "memory" is host memory, and streams
+// and events that know their device, as CUDA's do (an event recorded on a stream
+// of another device is an invalid handle).
+#include <cuda_runtime.h>
+
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "staging.cuh"
+
+namespace {
+struct Handle {
+    int device;
+    bool capturing = false;
+};
+thread_local int t_device = 0;
+int copies = 0, failures = 0;
+Handle g_legacy[2] = {{0}, {1}};
+
+Handle *of(cudaStream_t s) { return s ? reinterpret_cast<Handle *>(s) : &g_legacy[t_device]; }
+Handle *of(cudaEvent_t e) { return reinterpret_cast<Handle *>(e); }
+}  // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int *d) { return *d = t_device, cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { return t_device = d, cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorInvalidResourceHandle ? "invalid handle" : "error"; }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return *p = std::malloc(n), cudaSuccess; }
+cudaError_t cudaFreeHost(void *p) { return std::free(p), cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+    return *s = reinterpret_cast<cudaStream_t>(new Handle{t_device}), cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    return *e = reinterpret_cast<cudaEvent_t>(new Handle{t_device}), cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) { return delete of(s), cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { return delete of(e), cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    return of(e)->device == of(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamGetDevice(cudaStream_t s, int *d) { return *d = of(s)->device, cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind, cudaStream_t) {
+    __atomic_add_fetch(&copies, 1, __ATOMIC_SEQ_CST);
+    return std::memcpy(dst, src, n), cudaSuccess;
+}
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) {
+    std::memset(a, 0, sizeof(*a));
+    return a->type = cudaMemoryTypeUnregistered, cudaSuccess;
+}
+// no device code in this program
+void **__cudaRegisterFatBinary(void *) { return nullptr; }
+void __cudaRegisterFatBinaryEnd(void **) {}
+void __cudaUnregisterFatBinary(void **) {}
+char __cudaInitModule(void **) { return 0; }
+}
+
+namespace {
+// What a copy of n bytes on `s` did: true when it went through the chunks and
+// arrived; a copy that was left to the caller has touched nothing.
+bool through_chunks(size_t n, bool to_device, cudaStream_t s, const char *what) {
+    std::vector<unsigned char> src(n), dst(n, 0);
+    for (size_t i = 0; i < n; ++i) src[i] = static_cast<unsigned char>(i * 7 + (i >> 13));
+    copies = 0;
+    try {
+        const bool staged = hyt::staged_copy(dst.data(), src.data(), n, to_device, s);
+        if (staged ? dst != src : copies != 0) {
+            std::printf("FAILED %s: wrong bytes\n", what);
+            ++failures;
+        }
+        return staged;
+    } catch (const std::exception &e) {
+        std::printf("FAILED %s: %s\n", what, e.what());
+        ++failures;
+        return false;
+    }
+}
+void expect(bool got, bool want, const char *what) {
+    if (got == want) return;
+    std::printf("FAILED %s\n", what);
+    ++failures;
+}
+}  // namespace
+
+int main() {
+    constexpr size_t kLarge = (size_t(9) << 20) + 12345;
+    for (int current = 0; current < 2; ++current) {
+        cudaSetDevice(current);
+        cudaStream_t own = reinterpret_cast<cudaStream_t>(new Handle{current});
+        cudaStream_t other = reinterpret_cast<cudaStream_t>(new Handle{1 - current});
+        for (bool to_device : {true, false}) {
+            expect(through_chunks(kLarge, to_device, own, "own stream"), true, "own stream");
+            expect(through_chunks(kLarge, to_device, nullptr, "default stream"), true, "default stream");
+            expect(through_chunks(1000, to_device, own, "small copy"), false, "small copy");
+            // the runtime copies on a stream of any device: so must the caller, by itself
+            expect(through_chunks(kLarge, to_device, other, "another device's stream"), false,
+                   "another device's stream");
+            int d = -1;
+            cudaGetDevice(&d);
+            expect(d == current, true, "current device kept");
+        }
+    }
+    hyt::staging_release(0);
+    hyt::staging_release(1);
+    if (!failures) std::printf("staging tests passed\n");
+    return failures ? 1 : 0;
+}
