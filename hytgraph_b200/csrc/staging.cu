@@ -126,11 +126,13 @@ bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaS
     }
     int device = 0, of_stream = 0;
     HYT_CUDA(cudaGetDevice(&device));
-    if (cudaStreamGetDevice(s, &of_stream) != cudaSuccess) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamGetDevice(s, &of_stream) != cudaSuccess || cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
     if (of_stream != device) return false;  // the pool's events cannot be recorded on another device's stream
+    if (capture != cudaStreamCaptureStatusNone) return false;  // its streams would join the capture
     Pool &p = pool_of(device);
     std::unique_lock<std::mutex> lk(p.mu, std::try_to_lock);
     if (!lk.owns_lock() || !p.open()) return false;

@@ -17,7 +17,7 @@ namespace hyt {
 // after everything queued on s, and returns when they are there.  Returns
 // false, with nothing copied, when a plain copy is as good (under 4 MiB, pinned
 // host memory, another thread's copy holds the chunks) or the only one that can
-// follow s (a stream of another device).
+// follow s (a stream of another device, or one that is being captured).
 bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaStream_t s);
 
 // Gives back a device's chunks (at most 16 MiB pinned), streams and events.

@@ -1,7 +1,7 @@
 // CPU tests of the pinned-chunk copies (hytgraph_b200/csrc/staging.cu) over a
 // runtime made up here: two devices whose "memory" is host memory, and streams
 // and events that know their device, as CUDA's do (an event recorded on a stream
-// of another device is an invalid handle).
+// of another device is an invalid handle), and streams that a capture spreads to.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -40,14 +40,26 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { return delete of(s), cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return delete of(e), cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
-    return of(e)->device == of(s)->device ? cudaSuccess : cudaErrorInvalidResourceHandle;
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    return of(s)->capturing ? cudaErrorStreamCaptureUnsupported : cudaSuccess;
 }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    return of(e)->capturing ? cudaErrorCapturedEvent : cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    if (of(e)->device != of(s)->device) return cudaErrorInvalidResourceHandle;
+    return of(e)->capturing = of(s)->capturing, cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    if (of(e)->capturing) of(s)->capturing = true;  // joins the capture until that ends
+    return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *c) {
+    return *c = of(s)->capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone, cudaSuccess;
+}
 cudaError_t cudaStreamGetDevice(cudaStream_t s, int *d) { return *d = of(s)->device, cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind, cudaStream_t s) {
+    if (of(s)->capturing) return cudaSuccess;  // recorded, not run
     __atomic_add_fetch(&copies, 1, __ATOMIC_SEQ_CST);
     return std::memcpy(dst, src, n), cudaSuccess;
 }
@@ -102,6 +114,11 @@ int main() {
             // the runtime copies on a stream of any device: so must the caller, by itself
             expect(through_chunks(kLarge, to_device, other, "another device's stream"), false,
                    "another device's stream");
+            // neither may a capture spread to the streams that all callers share
+            Handle recording{current, true};
+            expect(through_chunks(kLarge, to_device, reinterpret_cast<cudaStream_t>(&recording), "capturing stream"),
+                   false, "capturing stream");
+            expect(through_chunks(kLarge, to_device, own, "after a capturing stream"), true, "after a capturing stream");
             int d = -1;
             cudaGetDevice(&d);
             expect(d == current, true, "current device kept");
