@@ -487,7 +487,7 @@ static uint32_t pack_bits_for(const GraphImpl &g) {
 // 0.53 ms at 262 K and 4 M (SSSP: 2.94 / 3.07, 0.75 / 0.83, 0.61 / 0.58 ms).
 // Smaller tiles gained 10 % on a PageRank of 65 K edges and cost a batch of
 // queries on such graphs 20 to 50 %.
-static uint32_t tile_cost_for(uint64_t V, uint64_t E) {
+uint32_t tile_cost_for(uint64_t V, uint64_t E) {
     return (V + E) / kTileCostDefault >= 3ull * 148 * (kPRThreads / 32) ? kTileCostDefault : kTileCostSmall;
 }
 

@@ -27,7 +27,6 @@ namespace hyt {
 // chunk).
 constexpr uint32_t kTileCostMin = 64;
 constexpr uint32_t kTileCostSmall = 512;     // ... on small ones
-constexpr uint32_t kTileCostHybrid = 128;    // ... of launches over one staged piece
 constexpr uint32_t kTileCostDefault = 1024;  // merge-path units per tile on large graphs (tunable: HYT_PR_TILE)
 constexpr uint32_t kStageTileMax = 256;      // bulk-staged kernels: a tile's edges (< 2 * tile_cost) fit one slot
 // Edges per chunk of a long row.  A warp takes a chunk 256 edges at a time, so a
@@ -213,6 +212,9 @@ inline uint64_t dealt_tasks(const GraphImpl &g) {
     const bool even = g.perm.get() && n < 16ull * 148 * (kPRThreads / 32);
     return even ? n : n - n / 4;
 }
+
+// Merge-path units per tile of a graph (graph.cu).
+uint32_t tile_cost_for(uint64_t V, uint64_t E);
 
 // Builds the device graph from a CSR (host or device pointers).
 void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags);

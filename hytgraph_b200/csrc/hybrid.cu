@@ -171,6 +171,7 @@ struct HybridImpl {
     // partition geometry: [e0, e1) of the CSR (push) and CSC (pull)
     std::vector<uint64_t> push_e0, push_e1, pull_e0, pull_e1;
     std::vector<Piece> push_pieces, pull_pieces;
+    GraphArray<uint2> whole_tiles;  // [pull tiles] rows of the tile that each part comes from
     std::vector<size_t> push_first, pull_first;  // first piece of each partition, [P + 1]
     std::vector<uint64_t> pull_zc_bytes;          // 128-byte lines of each partition's CSC
     std::vector<PartMetrics> pull_metrics;        // all vertices active
@@ -349,9 +350,17 @@ void build_push_pieces(HybridImpl &h, uint64_t cap) {
 }
 
 // Pull pieces: tiles are first split at partition boundaries (no tile
-// straddles two partitions); non-resident partitions are then cut between
-// tiles so that a piece holds at most `cap` in-edges.  A long row's chunk
-// tasks belong to the piece of the tile it ends.
+// straddles two partitions) and into parts of kPartRows rows; non-resident
+// partitions are then cut between parts so that a piece holds at most `cap`
+// in-edges.  A long row's chunk tasks belong to the piece of the part it ends.
+// A launch covers one staged group, a few hundred thousand edges, so its time is
+// that of one task: parts of 32 rows / 64 rows / whole tiles take PageRank on 1 M
+// vertices, 16 M edges with 32 MB on the device 22.8 / 23.5 / 26.9 ms, with 8 MB
+// 34.2 / 35.2 / 40.9, wholly resident 2.2 / 2.1 / 2.2.  Tiles of 128 units and
+// chunks of 512 edges took 20.7, 30.4 and 2.6 ms, but summed rows in another order
+// than the in-HBM solve.
+constexpr uint32_t kPartRows = 32;
+
 void build_pull_pieces(HybridImpl &h, uint64_t cap) {
     GraphImpl &g = h.g;
     cudaStream_t s = g.stream;
@@ -361,19 +370,31 @@ void build_pull_pieces(HybridImpl &h, uint64_t cap) {
     if (g.num_long)
         HYT_CUDA(cudaMemcpyAsync(lr.data(), g.long_rows.get(), lr.size() * sizeof(LongRow), cudaMemcpyDeviceToHost, s));
     HYT_CUDA(cudaStreamSynchronize(s));
+    const uint64_t *off = h.h_in_off;
     std::vector<uint32_t> bounds;
+    std::vector<uint2> whole;  // rows of the tile that each part comes from, without a long last row
     bounds.reserve(ts.size() + h.P + 1);
-    for (uint32_t v : ts) bounds.push_back(v);
-    for (size_t p = 0; p <= h.P; ++p)
-        bounds.push_back(static_cast<uint32_t>(std::min<uint64_t>(g.V, uint64_t(p) << h.part_shift)));
-    std::sort(bounds.begin(), bounds.end());
-    bounds.erase(std::unique(bounds.begin(), bounds.end()), bounds.end());
+    whole.reserve(ts.size() + h.P + 1);
+    for (size_t k = 0; k + 1 < ts.size(); ++k) {
+        const uint32_t r0 = ts[k], r1 = ts[k + 1];
+        if (r0 == r1) continue;
+        const uint32_t rl = off[r1] - off[r1 - 1] >= g.tile_cost ? r1 - 1 : r1;
+        for (uint64_t a = r0; a < r1;) {
+            bounds.push_back(static_cast<uint32_t>(a));
+            whole.push_back(make_uint2(r0, rl));
+            const uint64_t part_end = ((a >> h.part_shift) + 1) << h.part_shift;
+            const uint64_t rows_end = r0 + ((a - r0) / kPartRows + 1) * kPartRows;
+            a = std::min(part_end, rows_end);
+        }
+    }
+    bounds.push_back(static_cast<uint32_t>(g.V));
     g.num_tiles = bounds.size() - 1;
     g.tile_start.allocate(bounds.size());
+    h.whole_tiles.allocate(whole.size());
     HYT_CUDA(cudaMemcpyAsync(g.tile_start.get(), bounds.data(), bounds.size() * 4, cudaMemcpyHostToDevice, s));
+    HYT_CUDA(cudaMemcpyAsync(h.whole_tiles.get(), whole.data(), whole.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
     HYT_CUDA(cudaStreamSynchronize(s));
 
-    const uint64_t *off = h.h_in_off;
     h.pull_pieces.clear();
     h.pull_first.assign(h.P + 1, 0);
     uint64_t t = 0, c = 0, li = 0;
@@ -652,6 +673,8 @@ public:
         }
     }
 
+    const uint2 *whole_tiles() const override { return h_.whole_tiles.get(); }
+
     void release(size_t i, cudaStream_t s) override {
         const size_t gi = group_of_[i];
         if (gi == kNone || i + 1 != groups_[gi].last) return;
@@ -811,14 +834,9 @@ HybridImpl *hybrid_create(const hyt_csr *csr, const hyt_csc *csc, const hyt_hybr
         g.in_offsets.allocate(V + 1);
         HYT_CUDA(cudaMemcpyAsync(g.in_offsets.get(), h->h_in_off, (V + 1) * 8, cudaMemcpyHostToDevice, g.stream));
         HYT_CUDA(cudaStreamSynchronize(g.stream));
-        // A launch covers one staged group, a few hundred thousand edges: its
-        // time is that of one task, so tasks are short while their descriptors
-        // stay small beside the rows (1 M vertices, 16 M edges, 1.5-MB groups,
-        // 16 iterations: tiles 512, chunks 1024 23.1 ms; 256, 1024 21.5 ms;
-        // 128, 512 20.4 ms; 128, 256 20.3 ms).
-        const bool small = V + E < uint64_t(1) << 26;
-        g.tile_cost = small ? kTileCostHybrid : kTileCostSmall;
-        g.chunk_edges = small ? 512 : kLongChunkSmall;
+        // the tiles and chunks of an in-HBM graph: rows are summed alike
+        g.tile_cost = tile_cost_for(V, E);
+        g.chunk_edges = long_chunk_edges(V + E);
         g.num_hot = 0;  // host sources are untagged
         build_pull_tiles(g, g.stream);
         build_pull_pieces(*h, slot / 4);

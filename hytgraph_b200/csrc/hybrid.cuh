@@ -41,6 +41,8 @@ public:
     // True when pieces p and p + 1 are readable together: acquired one after
     // the other they share a base pointer, so one launch may work on both.
     virtual bool joined(size_t p) const = 0;
+    // Rows [x, y) of the whole tile that tile k is a part of (device array).
+    virtual const uint2 *whole_tiles() const = 0;
 };
 
 // PageRank / personalized PageRank over a graph whose CSC sources come from

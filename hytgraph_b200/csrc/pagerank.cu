@@ -91,8 +91,9 @@ __device__ __forceinline__ void load_hot(const PRArgs &a, const PRBuffers &b, fl
 struct PRRange {
     const uint32_t *in_src;
     uint64_t chunk_begin, chunk_end, tile_begin, tile_end;
-    const uint4 *tasks;  // the graph's task descriptors (whole-graph launches; NULL: no prefetch)
-    uint64_t dealt;      // dealt_tasks (whole-graph solves)
+    const uint4 *tasks;  // the graph's task descriptors (whole-graph launches)
+    uint64_t dealt;      // dealt_tasks (whole-graph launches)
+    const uint2 *whole;  // launches over pieces: rows of the tile that tile k is a part of
 };
 
 // The tasks of one iteration, over the whole grid.  a: the solve's arguments
@@ -100,6 +101,8 @@ struct PRRange {
 // tasks).
 // cursor (whole-graph launches): the first rg.dealt tasks are dealt to the
 // warps in turn, the others taken one by one.
+// kPieces: a launch over out-of-HBM pieces, whose tasks have no descriptors.
+template <bool kPieces>
 __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, const PRState &ps, const PRBuffers &b,
                                           double2 *slots, float *s_hot, uint32_t *cursor) {
     const uint64_t n_chunks = rg.chunk_end - rg.chunk_begin;
@@ -112,28 +115,29 @@ __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, co
     const uint64_t dealt = cursor ? max(rg.dealt, min(total_tasks, nwarps)) : total_tasks;
     // whole-graph launches read a dealt task's descriptor while the task
     // before it runs (one 16-byte load in place of a chain of table reads)
-    uint4 d = (rg.tasks && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
+    uint4 d = (!kPieces && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
     while (task < total_tasks) {
         double res = 0.0, dang = 0.0;
         uint64_t next = task + nwarps;
         uint32_t ticket = 0;
         const bool ask = cursor && next >= dealt;
         if (ask && lane == 0) ticket = atomicAdd(cursor, 1u);
-        uint4 nd = (rg.tasks && next < dealt) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
-        const uint4 *pf = (rg.tasks && !ask) ? &nd : nullptr;
+        uint4 nd = (!kPieces && next < dealt) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
+        const uint4 *pf = (!kPieces && !ask) ? &nd : nullptr;
         if (task < n_chunks) {
-            const TaskSpan t = rg.tasks ? task_span(d) : chunk_span(a, rg.chunk_begin + task);
+            const TaskSpan t = kPieces ? chunk_span(a, rg.chunk_begin + task) : task_span(d);
             const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
             if (row != ~0u) slot_store(slots, long_slot(row), dev::warp_sum(res), dev::warp_sum(dang), lane);
         } else {
             const uint64_t k = rg.tile_begin + (task - n_chunks);
-            const TaskSpan t = rg.tasks ? task_span(d) : tile_span(a, k);
-            tile_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
+            const TaskSpan t = kPieces ? tile_span(a, k) : task_span(d);
+            tile_task<true, kPieces>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf,
+                                     kPieces ? rg.whole[k] : make_uint2(0, 0));
             slot_store(slots, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
         }
         if (ask) {
             next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
-            if (rg.tasks && next < total_tasks) nd = rg.tasks[next];
+            if (!kPieces && next < total_tasks) nd = rg.tasks[next];
         }
         task = next;
         d = nd;
@@ -142,13 +146,14 @@ __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, co
 
 // One iteration (or a part of one: out-of-HBM partitions); the scalars of
 // this solve are in *args.
+template <bool kPieces>
 __global__ void __launch_bounds__(kPRThreads, 1) pr_iterate_kernel(const PRArgs *__restrict__ args,
                                                                    const __grid_constant__ PRArgs a,
                                                                    const __grid_constant__ PRRange rg) {
     extern __shared__ __align__(16) float s_dyn[];
     const uint32_t it = *(volatile uint32_t *)&a.hdr->iter;
     if (*(volatile uint32_t *)&a.hdr->done) return;
-    run_tasks(a, rg, make_state(*args, a.dangling[it]), buffers(a, it), a.red.slot, s_dyn, nullptr);
+    run_tasks<kPieces>(a, rg, make_state(*args, a.dangling[it]), buffers(a, it), a.red.slot, s_dyn, nullptr);
 }
 
 // (residual, dangling) of slot group g: thread t of 256 takes slots t, t +
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(kPRThreads, 1) pr_solve_kernel(const __grid_co
         double2 *slots = R.slot + ((it & 1) ? R.num_slots : 0);
         // three cursors take turns: this one was cleared two iterations ago
         if (blockIdx.x == 0 && threadIdx.x == 0) R.blocks_done[1 + (it + 2) % 3] = 0;
-        run_tasks(a, rg, make_state(a, dangling), buffers(a, it), slots, s_dyn, R.blocks_done + 1 + it % 3);
+        run_tasks<false>(a, rg, make_state(a, dangling), buffers(a, it), slots, s_dyn, R.blocks_done + 1 + it % 3);
         ok = dev::grid_sync(R.blocks_done, barriers);
         if (!ok) break;
         const bool own = R.num_groups <= kOwnGroups;
@@ -339,11 +344,11 @@ int pr_occupancy_grid() {
     static int grid = 0;
     if (grid == 0) {
         int per_sm = 0;
-        HYT_CUDA(cudaFuncSetAttribute(pr_iterate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HYT_CUDA(cudaFuncSetAttribute(pr_iterate_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
         HYT_CUDA(cudaFuncSetAttribute(pr_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax - 4096)));
-        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_iterate_kernel, kPRThreads, kPRSmemMax));
+        HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_iterate_kernel<false>, kPRThreads, kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
         if (const char *e = std::getenv("HYT_PR_GRID")) {
             const long v = std::strtol(e, nullptr, 10);
@@ -480,7 +485,7 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
     const bool persistent = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = pr_occupancy_grid();
     const unsigned smem = static_cast<unsigned>(pr_hot_bytes(g.num_hot));
-    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get(), dealt_tasks(g)};
+    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get(), dealt_tasks(g), nullptr};
 
     EventTimer total;
     total.start(s);
@@ -507,7 +512,7 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
         EventTimer kt;
         for (uint32_t i = 0; i < max_iter; ++i) {
             if (flags & HYT_RUN_PROFILE) kt.start(s);
-            pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(d_args, a, full);
+            pr_iterate_kernel<false><<<grid, kPRThreads, smem, s>>>(d_args, a, full);
             pr_reduce_kernel<<<pr_reduce_grid(a), kReduceThreads, 0, s>>>(d_args);
             HYT_CUDA(cudaGetLastError());
             launches += 2;
@@ -610,8 +615,9 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
             const uint32_t *base = nullptr;
             for (size_t q = p; q <= last; ++q) base = src.acquire(q, s);
             if (any) {
-                const PRRange rg{base, run.chunk_begin, run.chunk_end, run.tile_begin, run.tile_end};
-                pr_iterate_kernel<<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
+                const PRRange rg{base,    run.chunk_begin, run.chunk_end, run.tile_begin, run.tile_end,
+                                 nullptr, 0,               src.whole_tiles()};
+                pr_iterate_kernel<true><<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
                 HYT_CUDA(cudaGetLastError());
                 ++launches;
                 ++hot;

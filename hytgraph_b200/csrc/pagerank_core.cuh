@@ -400,34 +400,43 @@ __device__ __forceinline__ float group_rows(const uint32_t *src, uint32_t lo, ui
 // 24).  Must be called by all 32 lanes.
 // prefetch (optional): the warp's next pull task, whose edge lines are
 // warmed in L2 (warming its rows' offsets and ranks too gained nothing).
-template <bool kSmemHot>
+// kPart: the task is a part of a tile, cut where out-of-HBM pieces are.  Its
+// rows keep the batches, and so the lanes per row and the last bits, that they
+// have in the whole tile, rows [whole.x, whole.y): a row's sum depends on the
+// largest row beside it.
+template <bool kSmemHot, bool kPart = false>
 __device__ __forceinline__ void tile_task(const PRArgs &a, const PRState &ps, const PRBuffers &b,
                                           const uint32_t *in_src, const float *s_hot, const TaskSpan &t, int lane,
-                                          double &res, double &dang, const uint4 *prefetch = nullptr) {
+                                          double &res, double &dang, const uint4 *prefetch = nullptr,
+                                          uint2 whole = make_uint2(0, 0)) {
     const uint32_t r0 = t.a, rl = t.b;
     if (r0 == rl) return;
     const uint64_t e0 = t.e0;
     const uint32_t *src = in_src + e0;
     const Sources S = make_sources(a, b.ccur, s_hot);
     uint32_t lo = 0, hi = 0, od = 0;  // this lane's row: bounds relative to e0, out-degree, rank
+    uint32_t beside = 0;              // in-edges of a row of the tile's other parts
     float old = 0.0f;
-    auto load_row = [&](uint32_t r, uint32_t &l, uint32_t &h, uint32_t &d, float &o) {
-        l = h = d = 0;
+    auto load_row = [&](uint32_t r, uint32_t &l, uint32_t &h, uint32_t &d, float &o, uint32_t &bs) {
+        l = h = d = bs = 0;
         o = 0.0f;
-        if (r < rl) {
+        if ((!kPart || r >= r0) && r < rl) {
             l = static_cast<uint32_t>(a.in_off[r] - e0);
             h = static_cast<uint32_t>(a.in_off[r + 1] - e0);
             o = b.cur[r];
             d = a.out_deg[r];
+        } else if (kPart && r < whole.y) {
+            bs = static_cast<uint32_t>(a.in_off[r + 1] - a.in_off[r]);
         }
     };
-    load_row(r0 + lane, lo, hi, od, old);
+    const uint32_t rfirst = kPart ? whole.x + ((r0 - whole.x) & ~31u) : r0;
+    load_row(rfirst + lane, lo, hi, od, old, beside);
     if (prefetch) prefetch_task(*prefetch, in_src, nullptr, lane);
-    for (uint32_t rb = r0; rb < rl; rb += 32) {
-        uint32_t lo_n, hi_n, od_n;
+    for (uint32_t rb = rfirst; rb < rl; rb += 32) {
+        uint32_t lo_n, hi_n, od_n, beside_n;
         float old_n;
-        load_row(rb + 32 + lane, lo_n, hi_n, od_n, old_n);
-        const uint32_t deg = hi - lo;
+        load_row(rb + 32 + lane, lo_n, hi_n, od_n, old_n, beside_n);
+        const uint32_t deg = kPart ? hi - lo + beside : hi - lo;
         const bool wide = deg >= kWarpRowDegree;
         const uint32_t most = __reduce_max_sync(0xffffffffu, wide ? 0u : deg);
         const uint32_t hs = wide ? lo : hi;  // group steps see a wide row as empty
@@ -444,7 +453,7 @@ __device__ __forceinline__ void tile_task(const PRArgs &a, const PRState &ps, co
             sum = group_rows<1, 4, kSmemHot>(src, lo, hs, S, lane);
         else if (most)
             sum = group_rows<1, 2, kSmemHot>(src, lo, hs, S, lane);
-        uint32_t big = __ballot_sync(0xffffffffu, wide);
+        uint32_t big = __ballot_sync(0xffffffffu, wide && (!kPart || !beside));
         while (big) {
             const int w = __ffs(big) - 1;
             big &= big - 1;
@@ -455,11 +464,12 @@ __device__ __forceinline__ void tile_task(const PRArgs &a, const PRState &ps, co
             const float t = dev::warp_reduce(acc.total()).value();
             if (lane == w) sum = t;
         }
-        if (rb + lane < rl) finalize_row_with(ps, rb + lane, sum, old, od, b.nxt, b.cnxt, res, dang);
+        if ((!kPart || rb + lane >= r0) && rb + lane < rl) finalize_row_with(ps, rb + lane, sum, old, od, b.nxt, b.cnxt, res, dang);
         lo = lo_n;
         hi = hi_n;
         od = od_n;
         old = old_n;
+        beside = beside_n;
     }
 }
 
