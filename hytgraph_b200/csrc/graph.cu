@@ -514,6 +514,7 @@ void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {
     uint32_t hot_request = V >= kHotLargeVertices ? kHotSourcesLarge : kHotSourcesDefault;
     if (const char *t = std::getenv("HYT_PR_HOT")) hot_request = static_cast<uint32_t>(std::strtoul(t, nullptr, 10));
     hot_request = std::min(hot_request, kHotSourcesMax);
+    if (stage::staged_requested()) hot_request = std::min(hot_request, stage::kStageMaxHot);
     if ((flags & HYT_GRAPH_PULL) && V > (kHotTag >> 0) - 1)
         fail(HYT_E_UNSUPPORTED, "pull graphs hold fewer than 2^31 vertices (bit 31 tags cached sources)");
 

@@ -56,7 +56,13 @@ constexpr size_t kStageBytes = kStageHead + size_t(kStageWarps) * kStageSlots * 
 
 inline size_t staged_shared_bytes(uint32_t num_hot) { return kStageBytes + size_t(num_hot) * 4; }
 
-// HYT_STAGED=1: graphs are built with kStageTileMax-unit tiles.
+// Hot sources whose table fits beside the slots (4 KB left to the kernel's
+// static shared memory): 18656, fewer than large graphs have without HYT_STAGED.
+constexpr uint32_t kStageMaxHot = (kPRSmemMax - 4096 - kStageBytes) / 4;
+static_assert(kStageMaxHot >= kHotSourcesDefault, "the default table fits beside the slots");
+
+// HYT_STAGED=1: graphs are built with kStageTileMax-unit tiles and at most
+// kStageMaxHot hot sources.
 inline bool staged_requested() {
     static const bool on = [] {
         const char *e = std::getenv("HYT_STAGED");
