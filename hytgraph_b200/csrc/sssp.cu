@@ -343,7 +343,20 @@ struct SolveState {
     uint32_t barrier, pad;
 };
 
-constexpr int kSolveBatch = 8;  // 32-edge batches in flight of a push round's warp: 4 lose 5 % on 2^24 vertices, 16 spill and lose 10 %
+// 32-edge batches in flight of a push round's warp beside sweeps: 4 lose 5 % on
+// 2^24 vertices, 16 spill and lose 10 %.
+constexpr int kSolveBatch = 8;
+// Solves that only push (no CSC, or no sweeps wanted) do without the sweep's code
+// and the next frontier's out-degrees, a random read per improved vertex.  From
+// kWideFrontierEdges on their frontiers are large enough for 16 batches a warp.
+// Threads x batches 512 x 8 / 512 x 16 / 768 x 8 / the kernel with sweeps, one
+// source: R-MAT 1 M vertices, 16 M edges 0.88 / 0.95 / 0.90 / 0.93 ms in input
+// order, 0.99 / 1.10 / 1.01 / 1.05 in hub order; 16.7 M, 263 M 9.14 / 8.85 / 9.38 /
+// 9.98 and 8.86 / 8.33 / 8.93 / 9.48; a grid of 1024 x 1024 11.1 / 13.9 / 12.6 /
+// 15.1.
+constexpr int kPushThreads = 512;
+constexpr int kWideBatch = 16;
+constexpr uint64_t kWideFrontierEdges = uint64_t(1) << 27;
 
 // Rounds separated by grid barriers (one after a sweep; one between expansion
 // and hub chunks and one after) in place of four launches and a conditional-
@@ -351,10 +364,11 @@ constexpr int kSolveBatch = 8;  // 32-edge batches in flight of a push round's w
 // has 16 rounds (605 -> 318 us a call; 500 K vertices, 8 M edges: 935 -> 694
 // us).  One bucket only; the loop of launches serves finite bucket
 // widths.
-template <int WK, bool kPacked>
-__global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __grid_constant__ SSArgs a,
-                                                                     const __grid_constant__ PullGraph pg,
-                                                                     SolveState *st, uint32_t max_rounds) {
+// kPull: rounds may be sweeps.  kB: 32-edge batches in flight of a push round's warp.
+template <int WK, bool kPacked, bool kPull, int kB>
+__global__ void __launch_bounds__(kPull ? kPullThreads : kPushThreads, 1)
+    sssp_solve_kernel(const __grid_constant__ SSArgs a, const __grid_constant__ PullGraph pg, SolveState *st,
+                      uint32_t max_rounds) {
     extern __shared__ __align__(16) uint32_t s_hot[];
     const int lane = threadIdx.x & 31;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -406,8 +420,11 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __gri
         rv.far_stamp = 1;
         frontier_total += rv.qn;
         Gain gain;
-        if (a.pull_div && __ldcg(&cur->edges) * a.pull_div > a.num_edges) {
-            pull_sweep<WK, kPacked>(a, pg, rv, ~__ldcg(&cur->fmin_inv), s_hot, &cur->task_cursor, relaxed, gain);
+        bool sweep = false;
+        if constexpr (kPull) sweep = __ldcg(&cur->edges) * a.pull_div > a.num_edges;
+        if (sweep) {
+            if constexpr (kPull)
+                pull_sweep<WK, kPacked>(a, pg, rv, ~__ldcg(&cur->fmin_inv), s_hot, &cur->task_cursor, relaxed, gain);
             ++sweeps;
         } else {
             unsigned long long improved = 0;
@@ -416,16 +433,16 @@ __global__ void __launch_bounds__(kPullThreads, 1) sssp_solve_kernel(const __gri
                 for (uint32_t c = 0; c < nch; ++c) a.hubs[base + c] = make_uint2(v, c);
             };
             for (uint32_t w = gwarp; uint64_t(w) * 32 < rv.qn; w += nwarps)
-                expand_warp<WK, false, kSolveBatch, true>(a, rv, w * 32, lane, kHubDegree, relaxed, improved, hub, &gain);
+                expand_warp<WK, false, kB, kPull>(a, rv, w * 32, lane, kHubDegree, relaxed, improved, hub, &gain);
             ok = dev::grid_sync(&st->barrier, barriers);
             if (!ok) break;
             const uint32_t n = __ldcg(&cur->hub_count);
             for (uint32_t t = gwarp; t < n; t += nwarps) {
                 const uint2 h = a.hubs[t];
-                hub_chunk<WK, true, kSolveBatch>(a, rv, a.cols, a.weights, h.x, h.y, lane, improved, &gain);
+                hub_chunk<WK, kPull, kB>(a, rv, a.cols, a.weights, h.x, h.y, lane, improved, &gain);
             }
         }
-        flush_gain(&nxt->edges, &nxt->fmin_inv, gain, lane);
+        if constexpr (kPull) flush_gain(&nxt->edges, &nxt->fmin_inv, gain, lane);
         ok = dev::grid_sync(&st->barrier, barriers);
     }
     if (threadIdx.x == 0) atomicExch(&a.hdr->error, 1u);
@@ -608,8 +625,8 @@ int pull_grid() {
         int per_sm = 0;
         HYT_CUDA(cudaFuncSetAttribute(sssp_pull_kernel<WK, kPacked>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kPRSmemMax)));
-        HYT_CUDA(cudaFuncSetAttribute(sssp_solve_kernel<WK, kPacked>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kPRSmemMax)));
+        HYT_CUDA(cudaFuncSetAttribute(sssp_solve_kernel<WK, kPacked, true, kSolveBatch>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPRSmemMax)));
         HYT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_pull_kernel<WK, kPacked>, kPullThreads,
                                                                kPRSmemMax));
         grid = sm_count() * std::max(per_sm, 1);
@@ -740,12 +757,17 @@ void sssp_solve(GraphImpl &g, uint32_t source, uint32_t delta, uint32_t max_roun
         // every CTA must be resident; no more of them than a sweep or a full
         // frontier has work for
         const uint64_t work = std::max<uint64_t>(pg.num_tasks, (V + 127) / 128);
-        const uint64_t warps = std::clamp<uint64_t>((work + pgrid - 1) / pgrid, kMinWarps, kPullThreads / 32);
+        const void *solve = a.pull_div ? reinterpret_cast<void *>(sssp_solve_kernel<WK, kPacked, true, kSolveBatch>)
+                            : g.E < kWideFrontierEdges
+                                ? reinterpret_cast<void *>(sssp_solve_kernel<WK, false, false, kSolveBatch>)
+                                : reinterpret_cast<void *>(sssp_solve_kernel<WK, false, false, kWideBatch>);
+        const uint64_t warps = std::clamp<uint64_t>((work + pgrid - 1) / pgrid, kMinWarps,
+                                                    (a.pull_div ? kPullThreads : kPushThreads) / 32);
         const unsigned ctas = static_cast<unsigned>(
             std::min<uint64_t>(pgrid, std::max<uint64_t>(1, (work + warps - 1) / warps)));
         void *kargs[] = {&a, &pg, &solve_state, &max_rounds};
-        HYT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(sssp_solve_kernel<WK, kPacked>), dim3(ctas),
-                                             dim3(static_cast<unsigned>(32 * warps)), kargs, pull_smem, s));
+        HYT_CUDA(cudaLaunchCooperativeKernel(solve, dim3(ctas), dim3(static_cast<unsigned>(32 * warps)), kargs,
+                                             pull_smem, s));
     } else {
         HYT_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(a), cudaMemcpyHostToDevice, s));
         HYT_CUDA(cudaMemcpyAsync(hdr, &h0, sizeof(h0), cudaMemcpyHostToDevice, s));
