@@ -29,20 +29,24 @@ struct InEdges {
 
 // Lowest candidate label(u) + w over the edges b, b + kStep, ... below e, at
 // most kN of them, all loaded before the first is used (`best` when none is
-// lower); unreached sources give infinity or more.
+// lower); unreached sources give infinity or more.  A minimum does not mind an
+// edge taken twice, so threads without an edge of their own repeat the row's
+// last one (the same sector) in place of predicated loads: without packed words,
+// u32 weights on R-MAT scale 24 in input order take 3.58 ms in place of 4.12 and
+// f32 weights 5.95 in place of 6.06.  A row without edges gives an arbitrary
+// result.
 // kPacked: one word per edge, labels that cannot wrap (GraphImpl::
-// in_pack_bits): a candidate is one add-and-min, and as a minimum does not mind
-// an edge taken twice, threads without an edge of their own repeat the row's
-// last one (the same sector) in place of predicated loads.  A row without edges
-// gives an arbitrary result.  Half the instructions per edge of the general
-// form, which streams ids and weights apart, maps hot slots and saturates: one
-// source on R-MAT scale 24 takes 2.38 ms in place of 2.83 (hub order) and 2.63
-// in place of 4.12 (input order; both with uneven tasks handed out one by one).
+// in_pack_bits): a candidate is one add-and-min.  Half the instructions per edge
+// of the general form, which streams ids and weights apart, maps hot slots and
+// saturates: one source on R-MAT scale 24 took 2.38 ms in place of 2.83 (hub
+// order) and 2.63 in place of 4.12 (input order; both with uneven tasks handed
+// out one by one).
 template <int kN, int kStep, int WK, bool kPacked, class Label>
 __device__ __forceinline__ uint32_t edges_min(const InEdges &E, uint32_t b, uint32_t e, Label &&label, uint32_t best) {
+    const uint32_t last = e > 0 ? e - 1 : 0u;
+    uint32_t x[kN], du[kN];
     if constexpr (kPacked) {
-        const uint32_t last = e > 0 ? e - 1 : 0u, mask = (1u << E.bits) - 1u;
-        uint32_t x[kN], du[kN];
+        const uint32_t mask = (1u << E.bits) - 1u;
 #pragma unroll
         for (int j = 0; j < kN; ++j) x[j] = dev::ld_stream(E.w + min(b + j * kStep, last));
 #pragma unroll
@@ -50,18 +54,22 @@ __device__ __forceinline__ uint32_t edges_min(const InEdges &E, uint32_t b, uint
 #pragma unroll
         for (int j = 0; j < kN; ++j) best = __viaddmin_u32(du[j], x[j] >> E.bits, best);
     } else {
-        uint32_t id[kN], w[kN], du[kN];
+        uint32_t w[kN];
 #pragma unroll
-        for (int j = 0; j < kN; ++j) id[j] = (b + j * kStep < e) ? dev::ld_stream(E.src + b + j * kStep) : 0u;
+        for (int j = 0; j < kN; ++j) x[j] = dev::ld_stream(E.src + min(b + j * kStep, last));
 #pragma unroll
         for (int j = 0; j < kN; ++j)
-            if (id[j] & kHotTag) id[j] = E.s_hot[id[j] & ~kHotTag];
+            if (x[j] & kHotTag) x[j] = E.s_hot[x[j] & ~kHotTag];
 #pragma unroll
-        for (int j = 0; j < kN; ++j) du[j] = (b + j * kStep < e) ? label(id[j]) : E.inf;
+        for (int j = 0; j < kN; ++j) du[j] = label(x[j]);
 #pragma unroll
-        for (int j = 0; j < kN; ++j) w[j] = (b + j * kStep < e) ? ssc::edge_weight<WK>(E.w, b + j * kStep) : 0u;
+        for (int j = 0; j < kN; ++j) w[j] = ssc::edge_weight<WK>(E.w, min(b + j * kStep, last));
 #pragma unroll
-        for (int j = 0; j < kN; ++j) best = min(best, du[j] == E.inf ? E.inf : ssc::extend<WK>(du[j], w[j]));
+        for (int j = 0; j < kN; ++j) {
+            const uint32_t c = ssc::extend<WK>(du[j], w[j]);
+            // a float infinity stays one by itself
+            best = min(best, WK != HYT_WEIGHTS_F32 && du[j] == E.inf ? E.inf : c);
+        }
     }
     return best;
 }
