@@ -261,11 +261,6 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
     return pol;
 }
-__device__ __forceinline__ float ld_keep(const float *p, uint64_t pol) {
-    float v;
-    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
-    return v;
-}
 
 // Coherent 32-bit load with an L2 cache-eviction policy (for data other
 // threads may update during the kernel).

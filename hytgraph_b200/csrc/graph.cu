@@ -488,7 +488,7 @@ static uint32_t pack_bits_for(const GraphImpl &g) {
 // Smaller tiles gained 10 % on a PageRank of 65 K edges and cost a batch of
 // queries on such graphs 20 to 50 %.
 uint32_t tile_cost_for(uint64_t V, uint64_t E) {
-    return (V + E) / kTileCostDefault >= 3ull * 148 * (kPRThreads / 32) ? kTileCostDefault : kTileCostSmall;
+    return (V + E) / kTileCostDefault >= 3ull * sm_count() * (kPRThreads / 32) ? kTileCostDefault : kTileCostSmall;
 }
 
 void graph_build(GraphImpl &g, const hyt_csr &csr, uint32_t flags) {

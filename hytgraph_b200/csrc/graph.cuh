@@ -175,7 +175,6 @@ struct GraphImpl {
     GraphArray<float> partial;        // long-row chunk partial sums (s, c)
     GraphArray<uint32_t> ticket;      // long-row arrival counters
     GraphArray<unsigned char> pr_state;
-    uint32_t pr_state_iters = 0;
 
     GraphArray<uint32_t> dist;
     GraphArray<uint32_t> stamp;
@@ -209,7 +208,7 @@ inline size_t pr_hot_bytes(uint32_t num_hot) { return (size_t(num_hot) + 1) * si
 // 1.09 -> 1.22 ms at 1 M, where a warp has 4 tasks in all.
 inline uint64_t dealt_tasks(const GraphImpl &g) {
     const uint64_t n = g.num_chunks + g.num_tiles;
-    const bool even = g.perm.get() && n < 16ull * 148 * (kPRThreads / 32);
+    const bool even = g.perm.get() && n < 16ull * sm_count() * (kPRThreads / 32);
     return even ? n : n - n / 4;
 }
 

@@ -49,7 +49,8 @@ struct PRSlots {
     uint32_t num_slots, num_groups;
 };
 
-// Device-resident arguments (a cached CUDA graph reads them every launch).
+// Arguments of a solve: kernel parameters, or an array in device memory (the
+// launch-by-launch kernels' copy, the batch engine's slots).
 struct PRArgs {
     const uint64_t *in_off;
     const uint32_t *in_src;

@@ -12,10 +12,9 @@
 // four of a vertex's queries with one 16-byte load per in-edge: short rows
 // 16 per warp (two threads per row), longer rows by the whole warp in 16
 // edge slots; sums are FP64, folded with shuffles in a fixed order, and
-// rows at or above the graph's long-row threshold use its 4096-edge chunk
-// tasks, summed per row in chunk order.  The thread layout does not depend
-// on how many lanes are in use,
-// so a query's result is the same bit for bit alone or packed with others.
+// rows at or above the graph's long-row threshold use its chunk tasks
+// (chunk_edges edges each), summed per row in chunk order.  The thread layout
+// does not depend on how many lanes are in use, so a query's result is the same bit for bit alone or packed with others.
 // A lane whose step met its tolerance stops (its values are carried
 // unchanged) while the others continue.
 #include <algorithm>

@@ -23,7 +23,7 @@
 // a time, finding each edge's owner with a 5-step shuffle binary search.
 // Rows of >= kHubDegree edges become kHubChunk-edge warp tasks for a second
 // grid-wide kernel, so no warp owns more than ~2K edges of a round.  Each
-// lane keeps 16 edges in flight through loads and atomics (relax_batch).  A
+// lane keeps 8 or 16 edges in flight through loads and atomics (relax_batch).  A
 // vertex joins a frontier once per round (round stamp) and the far pile once
 // per phase (phase stamp), appended with one warp-aggregated atomic.
 //

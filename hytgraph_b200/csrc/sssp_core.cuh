@@ -238,7 +238,8 @@ __device__ __forceinline__ void relax_batch(const SSArgs &a, const RoundView &rv
 // are handed to hub(v, chunks) as kHubChunk-edge tasks.  HYB: the edges of
 // a vertex's partition are reached through a.loc (out-of-HBM solves).
 // Must be called by all 32 lanes.
-// kB: 32-edge batches in flight.  The in-HBM solver's expansion takes 16;
+// kB: 32-edge batches in flight.  The in-HBM solver's expansion takes 16 launched
+// by itself and 8 or 16 in a whole solve (sssp_solve_kernel);
 // the batch engine's and the out-of-HBM expansion keep kEdgeBatch (with 16
 // their kernels spill registers).
 template <int WK, bool HYB, int kB = kEdgeBatch, bool kTrack = false, class HubSink>
