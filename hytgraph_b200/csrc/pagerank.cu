@@ -91,9 +91,11 @@ __device__ __forceinline__ void load_hot(const PRArgs &a, const PRBuffers &b, fl
 struct PRRange {
     const uint32_t *in_src;
     uint64_t chunk_begin, chunk_end, tile_begin, tile_end;
-    const uint4 *tasks;  // the graph's task descriptors (whole-graph launches)
-    uint64_t dealt;      // dealt_tasks (whole-graph launches)
-    const uint2 *whole;  // launches over pieces: rows of the tile that tile k is a part of
+    const uint4 *tasks;  // the graph's task descriptors (whole-graph launches; NULL: no prefetch)
+    union {
+        uint64_t dealt;      // dealt_tasks (whole-graph launches)
+        const uint2 *whole;  // launches over pieces: rows of the tile that tile k is a part of
+    };
 };
 
 // The tasks of one iteration, over the whole grid.  a: the solve's arguments
@@ -101,7 +103,8 @@ struct PRRange {
 // tasks).
 // cursor (whole-graph launches): the first rg.dealt tasks are dealt to the
 // warps in turn, the others taken one by one.
-// kPieces: a launch over out-of-HBM pieces, whose tasks have no descriptors.
+// kPieces: a launch over out-of-HBM pieces, whose tasks have no descriptors and
+// whose tiles are parts of tiles.
 template <bool kPieces>
 __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, const PRState &ps, const PRBuffers &b,
                                           double2 *slots, float *s_hot, uint32_t *cursor) {
@@ -115,29 +118,29 @@ __device__ __forceinline__ void run_tasks(const PRArgs &a, const PRRange &rg, co
     const uint64_t dealt = cursor ? max(rg.dealt, min(total_tasks, nwarps)) : total_tasks;
     // whole-graph launches read a dealt task's descriptor while the task
     // before it runs (one 16-byte load in place of a chain of table reads)
-    uint4 d = (!kPieces && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
+    uint4 d = (rg.tasks && task < total_tasks) ? rg.tasks[task] : make_uint4(0, 0, 0, 0);
     while (task < total_tasks) {
         double res = 0.0, dang = 0.0;
         uint64_t next = task + nwarps;
         uint32_t ticket = 0;
         const bool ask = cursor && next >= dealt;
         if (ask && lane == 0) ticket = atomicAdd(cursor, 1u);
-        uint4 nd = (!kPieces && next < dealt) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
-        const uint4 *pf = (!kPieces && !ask) ? &nd : nullptr;
+        uint4 nd = (rg.tasks && next < dealt) ? rg.tasks[next] : make_uint4(0, 0, 0, 0);
+        const uint4 *pf = (rg.tasks && !ask) ? &nd : nullptr;
         if (task < n_chunks) {
-            const TaskSpan t = kPieces ? chunk_span(a, rg.chunk_begin + task) : task_span(d);
+            const TaskSpan t = rg.tasks ? task_span(d) : chunk_span(a, rg.chunk_begin + task);
             const uint32_t row = chunk_task<true>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf);
             if (row != ~0u) slot_store(slots, long_slot(row), dev::warp_sum(res), dev::warp_sum(dang), lane);
         } else {
             const uint64_t k = rg.tile_begin + (task - n_chunks);
-            const TaskSpan t = kPieces ? tile_span(a, k) : task_span(d);
+            const TaskSpan t = rg.tasks ? task_span(d) : tile_span(a, k);
             tile_task<true, kPieces>(a, ps, b, rg.in_src, s_hot, t, lane, res, dang, pf,
                                      kPieces ? rg.whole[k] : make_uint2(0, 0));
             slot_store(slots, tile_slot(a, k), dev::warp_sum(res), dev::warp_sum(dang), lane);
         }
         if (ask) {
             next = dealt + __shfl_sync(0xffffffffu, ticket, 0);
-            if (!kPieces && next < total_tasks) nd = rg.tasks[next];
+            if (rg.tasks && next < total_tasks) nd = rg.tasks[next];
         }
         task = next;
         d = nd;
@@ -485,7 +488,7 @@ static void pr_solve(GraphImpl &g, bool personalized, uint32_t source, float dam
     const bool persistent = !(flags & HYT_RUN_NO_GRAPH) && !(flags & HYT_RUN_PROFILE);
     const int grid = pr_occupancy_grid();
     const unsigned smem = static_cast<unsigned>(pr_hot_bytes(g.num_hot));
-    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get(), dealt_tasks(g), nullptr};
+    PRRange full{g.in_sources.get(), 0, g.num_chunks, 0, g.num_tiles, g.pull_tasks.get(), {dealt_tasks(g)}};
 
     EventTimer total;
     total.start(s);
@@ -615,8 +618,8 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
             const uint32_t *base = nullptr;
             for (size_t q = p; q <= last; ++q) base = src.acquire(q, s);
             if (any) {
-                const PRRange rg{base,    run.chunk_begin, run.chunk_end, run.tile_begin, run.tile_end,
-                                 nullptr, 0,               src.whole_tiles()};
+                PRRange rg{base, run.chunk_begin, run.chunk_end, run.tile_begin, run.tile_end, nullptr, {0}};
+                rg.whole = src.whole_tiles();
                 pr_iterate_kernel<true><<<grid, kPRThreads, smem, s>>>(st0.d_args, a, rg);
                 HYT_CUDA(cudaGetLastError());
                 ++launches;

@@ -111,7 +111,7 @@ typedef struct hyt_graph_options {
 
 /* In-HBM graph arrays and the one-shot transforms' scratch come from
  * per-device memory pools that keep freed memory mapped (graph arrays: up to
- * 16 GiB; scratch: up to 2 GiB), so repeated graph creation does not map
+ * 16 GiB; scratch: up to 8 GiB), so repeated graph creation does not map
  * fresh memory each time; freed device outputs of hyt_csr_reorder are kept for
  * the next call too (up to 1 GiB).  This returns that cached memory of
  * `device` to the driver (after waiting for the device). */
