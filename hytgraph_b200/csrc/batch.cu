@@ -600,7 +600,7 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
     }
     const GraphImpl &g = *graphs_[q.graph];
     void *mem = nullptr;
-    HYT_CUDA(cudaMallocFromPoolAsync(&mem, need, pool_, stream_));
+    HYT_ALLOC(cudaMallocFromPoolAsync(&mem, need, pool_, stream_));
     HYT_CUDA(cudaMemsetAsync(mem, 0, need, stream_));
     unsigned char *p = static_cast<unsigned char *>(mem);
     auto take = [&](uint64_t bytes) {

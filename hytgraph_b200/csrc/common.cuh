@@ -40,6 +40,19 @@ inline void cuda_check(cudaError_t e, const char *what) {
 }
 #define HYT_CUDA(call) ::hyt::cuda_check((call), #call)
 
+// When an allocation ended with `e` = out of memory: returns the device memory
+// that is kept for later results to the driver (outputs.cuh); true when that was
+// any, so that the allocation is worth another try.
+bool reclaim_device_memory(cudaError_t e);
+
+// An allocation of device memory.
+#define HYT_ALLOC(call)                                                  \
+    do {                                                                 \
+        cudaError_t hyt_e = (call);                                      \
+        if (::hyt::reclaim_device_memory(hyt_e)) hyt_e = (call);         \
+        ::hyt::cuda_check(hyt_e, #call);                                 \
+    } while (0)
+
 // Runs `body` and converts exceptions to a status code + thread-local message.
 template <class F>
 int guarded(F &&body) {
@@ -84,7 +97,7 @@ struct DeviceArray {
         // 16 bytes of tail padding so vectorised / bulk loads of the last
         // elements never touch memory outside the allocation.
         void *p = nullptr;
-        HYT_CUDA(cudaMalloc(&p, n * sizeof(T) + 16));
+        HYT_ALLOC(cudaMalloc(&p, n * sizeof(T) + 16));
         ptr = static_cast<T *>(p);
         count = n;
     }
@@ -137,7 +150,7 @@ struct GraphArray {
         HYT_CUDA(cudaGetDevice(&dev));
         void *p = nullptr;
         // 16 bytes of tail padding, as DeviceArray
-        HYT_CUDA(cudaMallocFromPoolAsync(&p, n * sizeof(T) + 16, graph_pool(dev), cudaStreamLegacy));
+        HYT_ALLOC(cudaMallocFromPoolAsync(&p, n * sizeof(T) + 16, graph_pool(dev), cudaStreamLegacy));
         HYT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         ptr = static_cast<T *>(p);
         count = n;

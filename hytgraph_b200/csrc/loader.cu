@@ -436,7 +436,7 @@ struct Output {
     void *alloc(size_t bytes) {
         void *p = nullptr;
         if (o->on_device) {
-            HYT_CUDA(cudaMalloc(&p, bytes ? bytes : 16));
+            HYT_ALLOC(cudaMalloc(&p, bytes ? bytes : 16));
         } else {
             p = std::malloc(bytes ? bytes : 16);
             if (!p) fail(HYT_E_OOM, "host allocation failed");

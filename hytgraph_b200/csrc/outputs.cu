@@ -62,7 +62,7 @@ void *output_alloc(size_t bytes) {
     Blocks &b = blocks();
     int device = 0;
     HYT_CUDA(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lk(b.mu);
+    std::unique_lock<std::mutex> lk(b.mu);
     // the smallest kept block that is large enough and wastes at most a quarter
     auto best = b.kept.end();
     for (auto k = b.kept.begin(); k != b.kept.end(); ++k)
@@ -76,14 +76,9 @@ void *output_alloc(size_t bytes) {
         return p;
     }
     void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-    if (e == cudaErrorMemoryAllocation && !b.kept.empty()) {  // what is kept may be what is missing
-        (void)cudaGetLastError();
-        for (const Kept &k : b.kept) cudaFree(k.p);
-        b.kept.clear();
-        e = cudaMalloc(&p, bytes ? bytes : 16);
-    }
-    cuda_check(e, "cudaMalloc of a result");
+    lk.unlock();
+    HYT_ALLOC(cudaMalloc(&p, bytes ? bytes : 16));
+    lk.lock();
     try {
         b.live[p] = Live{device, bytes ? bytes : 16, bytes};
     } catch (...) {
@@ -118,22 +113,25 @@ void output_free(void *p, size_t bytes) noexcept {
         cudaFree(p);
         return;
     }
-    size_t held = 0;
-    for (const Kept &k : b.kept) held += k.device == l.device ? k.size : 0;
-    for (auto k = b.kept.begin(); held > kOutputKeep;) {
+    size_t held = 0, count = 0;
+    for (const Kept &k : b.kept)
+        if (k.device == l.device) held += k.size, ++count;
+    for (auto k = b.kept.begin(); held > kOutputKeep || count > kOutputBlocks;) {
         if (k->device != l.device) {
             ++k;
             continue;
         }
         held -= k->size;
+        --count;
         cudaFree(k->p);
         k = b.kept.erase(k);
     }
 }
 
-void output_release(int device) noexcept {
+bool output_release(int device) noexcept {
     Blocks &b = blocks();
     std::lock_guard<std::mutex> lk(b.mu);
+    bool any = false;
     for (auto k = b.kept.begin(); k != b.kept.end();) {
         if (k->device != device) {
             ++k;
@@ -141,7 +139,16 @@ void output_release(int device) noexcept {
         }
         cudaFree(k->p);
         k = b.kept.erase(k);
+        any = true;
     }
+    return any;
+}
+
+bool reclaim_device_memory(cudaError_t e) {
+    if (e != cudaErrorMemoryAllocation) return false;
+    (void)cudaGetLastError();
+    int device = 0;
+    return cudaGetDevice(&device) == cudaSuccess && output_release(device);
 }
 
 }  // namespace hyt

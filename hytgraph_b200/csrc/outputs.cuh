@@ -4,10 +4,11 @@
 //
 // cudaMalloc and cudaFree of a renumbered graph cost more than the renumbering
 // (0.5 GB on R-MAT scale 22: 3.2 ms a call against 0.8), so freed blocks are
-// kept for the next call, up to kOutputKeep bytes per device.  A free waits for
-// the GPU first, as cudaFree does: the caller's own streams may still be reading,
-// and the next owner writes.  (Blocks of the graph pool in their place could be
-// handed on under such a reader, and could not be exported.)
+// kept for the next call, up to kOutputKeep bytes and kOutputBlocks blocks per
+// device, and returned when another allocation of this library finds no memory.  A
+// free waits for the GPU first, as cudaFree does: the caller's own streams may
+// still be reading, and the next owner writes.  (Blocks of the graph pool in their
+// place could be handed on under such a reader, and could not be exported.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,12 +19,13 @@
 namespace hyt {
 
 constexpr size_t kOutputKeep = size_t(1) << 30;
+constexpr size_t kOutputBlocks = 64;  // small results: a block is searched for by size
 
 // A cudaMalloc block of at least `bytes` on the current device.
 void *output_alloc(size_t bytes);
 // Frees a block that output_alloc(bytes) gave, or any other cudaMalloc memory.
 void output_free(void *p, size_t bytes) noexcept;
-// Returns a device's kept blocks to the driver.
-void output_release(int device) noexcept;
+// Returns a device's kept blocks to the driver; true when there were any.
+bool output_release(int device) noexcept;
 
 }  // namespace hyt

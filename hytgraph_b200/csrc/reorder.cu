@@ -619,7 +619,7 @@ void csr_reorder(const hyt_csr &csr, const uint32_t *vertex_order, bool on_devic
         if (on_device && pooled) {
             int dev = 0;
             HYT_CUDA(cudaGetDevice(&dev));
-            HYT_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, graph_pool(dev), cudaStreamLegacy));
+            HYT_ALLOC(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, graph_pool(dev), cudaStreamLegacy));
             HYT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         } else if (on_device) {
             p = output_alloc(bytes);

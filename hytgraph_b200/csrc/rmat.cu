@@ -141,9 +141,9 @@ void generate_device(const hyt_rmat_params &p, const RmatKey &k, hyt_csr_buffers
     const bool weighted = !(p.weight_min == 0 && p.weight_max == 0);
     uint64_t *off = nullptr;
     uint32_t *cols = nullptr, *w = nullptr;
-    HYT_CUDA(cudaMalloc(&off, (V + 1) * sizeof(uint64_t)));
-    HYT_CUDA(cudaMalloc(&cols, std::max<uint64_t>(E, 1) * sizeof(uint32_t) + 16));
-    if (weighted) HYT_CUDA(cudaMalloc(&w, std::max<uint64_t>(E, 1) * sizeof(uint32_t) + 16));
+    HYT_ALLOC(cudaMalloc(&off, (V + 1) * sizeof(uint64_t)));
+    HYT_ALLOC(cudaMalloc(&cols, std::max<uint64_t>(E, 1) * sizeof(uint32_t) + 16));
+    if (weighted) HYT_ALLOC(cudaMalloc(&w, std::max<uint64_t>(E, 1) * sizeof(uint32_t) + 16));
     const uint32_t span = p.weight_max - p.weight_min + 1u;
     csr_from_keys_kernel<<<grid_for(E + 1, 256, 148 * 16), 256, 0, s>>>(keys.get(), E, V, weight_seed(p.seed),
                                                                          p.weight_min, span ? span : 1u, off, cols, w);

@@ -43,7 +43,7 @@ struct Scratch {
     cudaStream_t s = nullptr;
     Scratch(size_t n, cudaStream_t st) : s(st) {
         void *q = nullptr;
-        HYT_CUDA(cudaMallocFromPoolAsync(&q, std::max<size_t>(n, 1) * sizeof(T) + 16, scratch_pool(), s));
+        HYT_ALLOC(cudaMallocFromPoolAsync(&q, std::max<size_t>(n, 1) * sizeof(T) + 16, scratch_pool(), s));
         p = static_cast<T *>(q);
     }
     ~Scratch() { release(); }

@@ -77,6 +77,16 @@ def test_blocks_are_reused_at_other_sizes(hyt, gpu):
         d.free()
 
 
+def test_many_small_results_at_once(hyt, gpu):
+    g, order = _graph(hyt, 1000, 8000, 2), _order(1000, 2)
+    want = hyt.reorder(g, order)
+    for _ in range(2):
+        held = [hyt.reorder(g, order, device=True) for _ in range(100)]  # 300 blocks
+        assert all(_same(d, want) for d in held)
+        for d in held[::2] + held[1::2]:
+            d.free()
+
+
 def test_kept_blocks_are_bounded_and_returned(hyt, gpu):
     import torch
 
