@@ -14,7 +14,8 @@
 // edge slots; sums are FP64, folded with shuffles in a fixed order, and
 // rows at or above the graph's long-row threshold use its chunk tasks
 // (chunk_edges edges each), summed per row in chunk order.  The thread layout
-// does not depend on how many lanes are in use, so a query's result is the same bit for bit alone or packed with others.
+// does not depend on how many lanes are in use, so a query's result is the same
+// bit for bit alone or packed with others.
 // A lane whose step met its tolerance stops (its values are carried
 // unchanged) while the others continue.
 #include <algorithm>
@@ -71,16 +72,6 @@ __global__ void ppr8_prep_kernel(const uint32_t *__restrict__ deg, const float *
     }
 }
 
-// Sums over in-edges [b, e) of c[u][4h .. 4h + 3], h = t % 2: thread t
-// takes edge slot t / 2 (16 slots) and adds its edges b + t/2, b + t/2 + 16,
-// ... in that order, four queries at a time from one 16-byte load
-// (kQuadInFlight edges loaded before any is added); the slots are then folded by
-// shuffles, so every thread of half h holds the four sums.
-#ifndef HYT_PPR_QUAD_INFLIGHT
-#define HYT_PPR_QUAD_INFLIGHT 6
-#endif
-constexpr int kQuadInFlight = HYT_PPR_QUAD_INFLIGHT;  // edges loaded per thread before any is added
-
 // The in-edges' source ids: the low bits of packed (id, weight) words where
 // the graph keeps them (no hot slots to look up: a dependent load for a third of
 // the edges of an R-MAT graph), else the tagged CSC.
@@ -92,33 +83,47 @@ struct Ids {
     __device__ __forceinline__ uint32_t vertex(uint32_t u) const { return (u & kHotTag) ? hot_vertex[u & ~kHotTag] : u; }
 };
 
+// One round of row_quad_sum: kN edges of a thread, all loaded before any is added.
+template <int kN>
+__device__ __forceinline__ void quad_round(const Ids &ids, const float4 *c4, uint64_t i0, uint64_t e, int h,
+                                           double (&acc)[4]) {
+    uint32_t u[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j) u[j] = (i0 + 16 * j < e) ? ids.load(i0 + 16 * j) : 0u;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) u[j] = ids.vertex(u[j]);
+    float4 v[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j)
+        v[j] = (i0 + 16 * j < e) ? c4[uint64_t(u[j]) * 2 + h] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+        if (i0 + 16 * j < e) {
+            acc[0] += double(v[j].x);
+            acc[1] += double(v[j].y);
+            acc[2] += double(v[j].z);
+            acc[3] += double(v[j].w);
+        }
+    }
+}
+
+// Sums over in-edges [b, e) of c[u][4h .. 4h + 3], h = t % 2: thread t
+// takes edge slot t / 2 (16 slots) and adds its edges b + t/2, b + t/2 + 16,
+// ... in that order, four queries at a time from one 16-byte load; the slots are
+// then folded by shuffles, so every thread of half h holds the four sums.  Rounds
+// of 6 edges a thread are the fastest for long spans (4: 8 % slower on R-MAT, 8
+// slower too); rows of up to 64 edges take one round of 4 (eight queries on 1 M
+// rows of 64 on average 8.5 -> 7.9 ms).
 __device__ __forceinline__ void row_quad_sum(const Ids &ids, const float *__restrict__ c,
                                              uint64_t b, uint64_t e, int t, double (&acc)[4]) {
     const int slot = t >> 1, h = t & 1;
     const float4 *c4 = reinterpret_cast<const float4 *>(c);
 #pragma unroll
     for (int k = 0; k < 4; ++k) acc[k] = 0.0;
-    for (uint64_t i0 = b + slot; i0 < e; i0 += 16 * kQuadInFlight) {
-        uint32_t u[kQuadInFlight];
-#pragma unroll
-        for (int j = 0; j < kQuadInFlight; ++j) u[j] = (i0 + 16 * j < e) ? ids.load(i0 + 16 * j) : 0u;
-#pragma unroll
-        for (int j = 0; j < kQuadInFlight; ++j)
-            u[j] = ids.vertex(u[j]);
-        float4 v[kQuadInFlight];
-#pragma unroll
-        for (int j = 0; j < kQuadInFlight; ++j)
-            v[j] = (i0 + 16 * j < e) ? c4[uint64_t(u[j]) * 2 + h] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < kQuadInFlight; ++j) {
-            if (i0 + 16 * j < e) {
-                acc[0] += double(v[j].x);
-                acc[1] += double(v[j].y);
-                acc[2] += double(v[j].z);
-                acc[3] += double(v[j].w);
-            }
-        }
-    }
+    if (e - b <= 64)
+        quad_round<4>(ids, c4, b + slot, e, h, acc);
+    else
+        for (uint64_t i0 = b + slot; i0 < e; i0 += 96) quad_round<6>(ids, c4, i0, e, h, acc);
 #pragma unroll
     for (int o = 2; o < 32; o <<= 1)
 #pragma unroll
@@ -529,33 +534,6 @@ __global__ void ppr8_lane_kernel(const float *__restrict__ x, uint64_t V, int la
 
 unsigned grid_sm(unsigned per_sm) { return static_cast<unsigned>(sm_count()) * per_sm; }
 
-// Two side streams of a call and the events that fork and join them.
-struct SideStreams {
-    cudaStream_t stream[2] = {};
-    cudaEvent_t fork = nullptr, join[2] = {};
-    SideStreams() = default;
-    SideStreams(const SideStreams &) = delete;
-    SideStreams &operator=(const SideStreams &) = delete;
-    void open() {
-        HYT_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-        for (int i = 0; i < 2; ++i) {
-            HYT_CUDA(cudaStreamCreateWithFlags(&stream[i], cudaStreamNonBlocking));
-            HYT_CUDA(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
-        }
-    }
-    // waits for its work: the buffers of a call that fails are freed after it
-    ~SideStreams() {
-        for (int i = 0; i < 2; ++i) {
-            if (stream[i]) {
-                cudaStreamSynchronize(stream[i]);
-                cudaStreamDestroy(stream[i]);
-            }
-            if (join[i]) cudaEventDestroy(join[i]);
-        }
-        if (fork) cudaEventDestroy(fork);
-    }
-};
-
 }  // namespace
 
 void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart, float tolerance, uint32_t max_iter,
@@ -600,11 +578,15 @@ void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart,
     const uint64_t chunks = g.num_long ? g.num_chunks : 0;
     const uint64_t long_from = g.num_long ? g.tile_cost : ~uint64_t(0);
     const unsigned long_grid = g.num_long ? grid_for(g.num_long * 32, 256) : 0;
-    // chunks cut into pieces until there are enough warp tasks to fill the
-    // GPU (a function of the graph alone, so results do not depend on it)
+    // chunks cut into pieces of 512 edges or more until there are enough warp
+    // tasks to fill the GPU, of 128 or more where there are few in all (a function
+    // of the graph alone, so results do not depend on it).  A row's partial sums
+    // are added one after another: with pieces of 128 edges throughout, eight
+    // queries on a star of 1 M edges took 61 ms; now 18.
     uint32_t pieces = 1;
     if (!staged)
-        while (pieces < 8 && chunks * pieces < 16384) pieces *= 2;
+        while (pieces < 8 && (chunks * pieces < 512 || (chunks * pieces < 16384 && g.chunk_edges / (2 * pieces) >= 512)))
+            pieces *= 2;
     // the graph's wide rows (once per graph)
     if (!staged && !g.ppr_wide_ready) {
         Scratch<uint8_t> flags(V, s);
@@ -638,8 +620,19 @@ void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart,
     EventTimer timer;
     timer.start(s);
     uint64_t launches = 1;
-    SideStreams side;
-    if (!staged) side.open();
+    // Row classes that have work to speak of run side by side; one alone, or a few
+    // rows beside it, is not worth the events (4 us an iteration).
+    const uint64_t short_rows = V - g.num_long - num_wide;
+    const bool some_long = chunks > 0, some_wide = num_wide >= 32, some_short = short_rows >= 1024;
+    const bool side_long = !staged && some_long && (some_wide || some_short);
+    const bool side_wide = !staged && some_wide && some_short;
+    const bool fork = side_long || side_wide;
+    SideStreams &side = g.side;
+    struct Settle {  // the buffers of a call that fails are freed after the side streams' work
+        SideStreams &s;
+        ~Settle() { s.settle(); }
+    } settle{side};
+    if (fork) side.open();
     for (uint32_t it = 0; it < max_iter && p.active; ++it) {
         ppr8_prep_kernel<<<kPartBlocks, 256, 0, s>>>(g.out_degree.get(), x, V, c.get(), dpart.get());
         ppr8_lane_sums_kernel<<<1, kSumThreads, 0, s>>>(dpart.get(), kPartBlocks, nullptr, 0, nullptr, 0, dm.get());
@@ -660,29 +653,27 @@ void ppr_multi(GraphImpl &g, const uint32_t *sources, uint32_t k, float restart,
             // on average, the wide rows 38, the short rows 44 of 64).  2.1 M
             // vertices, 32 M edges, 8 queries: 5.95 -> 5.46 ms (with 6 edges in flight
             // per thread instead of 4; 8 ran slower).
-            HYT_CUDA(cudaEventRecord(side.fork, s));
+            const cudaStream_t s_long = side_long ? side.stream[0] : s, s_wide = side_wide ? side.stream[1] : s;
+            if (fork) HYT_CUDA(cudaEventRecord(side.fork, s));
             if (chunks) {
-                HYT_CUDA(cudaStreamWaitEvent(side.stream[0], side.fork, 0));
-                ppr8_chunks_kernel<<<grid_sm(8), 256, 0, side.stream[0]>>>(g.in_offsets.get(), ids, c.get(),
-                                                                           g.long_rows.get(), g.chunk_tasks.get(),
-                                                                           chunks, g.chunk_edges, pieces,
-                                                                           chunk_sum.get());
-                ppr8_long_rows_kernel<<<long_grid, 256, 0, side.stream[0]>>>(g.long_rows.get(), g.num_long, pieces,
-                                                                             chunk_sum.get(), x, p, dm.get(), nx,
-                                                                             lpart.get());
+                if (side_long) HYT_CUDA(cudaStreamWaitEvent(s_long, side.fork, 0));
+                ppr8_chunks_kernel<<<grid_sm(8), 256, 0, s_long>>>(g.in_offsets.get(), ids, c.get(), g.long_rows.get(),
+                                                                   g.chunk_tasks.get(), chunks, g.chunk_edges, pieces,
+                                                                   chunk_sum.get());
+                ppr8_long_rows_kernel<<<long_grid, 256, 0, s_long>>>(g.long_rows.get(), g.num_long, pieces,
+                                                                     chunk_sum.get(), x, p, dm.get(), nx, lpart.get());
                 launches += 2;
             }
             if (num_wide) {
-                HYT_CUDA(cudaStreamWaitEvent(side.stream[1], side.fork, 0));
-                ppr8_wide_kernel<<<wide_grid, kRowThreads, 0, side.stream[1]>>>(g.ppr_wide.get(), num_wide,
-                                                                                g.in_offsets.get(), ids, c.get(), x, p,
-                                                                                dm.get(), nx, wpart.get());
+                if (side_wide) HYT_CUDA(cudaStreamWaitEvent(s_wide, side.fork, 0));
+                ppr8_wide_kernel<<<wide_grid, kRowThreads, 0, s_wide>>>(g.ppr_wide.get(), num_wide, g.in_offsets.get(),
+                                                                        ids, c.get(), x, p, dm.get(), nx, wpart.get());
                 ++launches;
             }
             ppr8_rows_kernel<<<rows_grid, kRowThreads, 0, s>>>(g.in_offsets.get(), ids, c.get(), x, V, long_from, p,
                                                                dm.get(), nx, rpart.get());
             for (int i = 0; i < 2; ++i)
-                if (i == 0 ? chunks > 0 : num_wide > 0) {
+                if (i == 0 ? side_long : side_wide) {
                     HYT_CUDA(cudaEventRecord(side.join[i], side.stream[i]));
                     HYT_CUDA(cudaStreamWaitEvent(s, side.join[i], 0));
                 }
