@@ -19,6 +19,7 @@
 // order otherwise), computed as stable radix sorts (item index where the items
 // do not ascend already, then contribution), with the plan metrics (reordered, zero, redundant,
 // log2(n) overhead).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -36,10 +37,11 @@ namespace {
 constexpr int kPartBlocks = 1024;
 
 // x[u] = current(u) / deg(u) in FP64 (0 for a dangling vertex), and the
-// per-block partial sums of the dangling ranks.
+// per-block partial sums of the dangling ranks; clears the task cursor.
 __global__ void source_shares_kernel(const uint32_t *__restrict__ deg, const float *__restrict__ rank, uint64_t V,
-                                     double *__restrict__ x, double *__restrict__ partial) {
+                                     double *__restrict__ x, double *__restrict__ partial, uint32_t *cursor) {
     __shared__ double warp_sum[8];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;
     double acc = 0.0;
     for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < V; v += uint64_t(gridDim.x) * blockDim.x) {
         const uint32_t d = deg[v];
@@ -372,24 +374,28 @@ void pagerank_contributions(GraphImpl &g, const float *ranks, float damping, dou
         oh = std::make_unique<Scratch<double>>(V, s);
         o = oh->get();
     }
-    Scratch<double> partial(kPartBlocks, s), x(V, s);
+    Scratch<double> partial(kPartBlocks + 1, s), x(V, s);
+    uint32_t *cursor = reinterpret_cast<uint32_t *>(partial.get() + kPartBlocks);
     const uint64_t chunks = g.num_long ? g.num_chunks : 0;
     Scratch<double> chunk_sum(chunks ? chunks : 1, s);
-    Scratch<uint32_t> cursor(1, s);
     const unsigned smem = static_cast<unsigned>(g.num_hot * sizeof(uint32_t));
-    HYT_CUDA(cudaFuncSetAttribute(pagerank_contrib_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kPRSmemMax)));
+    if (smem > 32 * 1024)  // beyond what every kernel may have
+        HYT_CUDA(cudaFuncSetAttribute(pagerank_contrib_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kPRSmemMax)));
+    // blocks beyond the vertices would add zeros
+    const int parts = static_cast<int>(std::min<uint64_t>(kPartBlocks, (V + 255) / 256));
     EventTimer t;
     t.start(s);
-    HYT_CUDA(cudaMemsetAsync(cursor.get(), 0, sizeof(uint32_t), s));
-    source_shares_kernel<<<kPartBlocks, 256, 0, s>>>(g.out_degree.get(), r, V, x.get(), partial.get());
-    pagerank_contrib_kernel<<<grid_sm(1), kContribThreads, smem, s>>>(
+    source_shares_kernel<<<parts, 256, 0, s>>>(g.out_degree.get(), r, V, x.get(), partial.get(), cursor);
+    // no more CTAs than have tasks: each loads the hot table
+    const uint64_t want = (g.num_chunks + g.num_tiles + kContribThreads / 32 - 1) / (kContribThreads / 32);
+    pagerank_contrib_kernel<<<static_cast<unsigned>(std::min<uint64_t>(grid_sm(1), want)), kContribThreads, smem, s>>>(
         g.in_offsets.get(), g.in_sources.get(), g.hot_vertex.get(), g.num_hot, g.pull_tasks.get(),
-        g.num_chunks + g.num_tiles, g.long_rows.get(), x.get(), r, V, double(damping), partial.get(), kPartBlocks,
-        cursor.get(), chunk_sum.get(), o);
+        g.num_chunks + g.num_tiles, g.long_rows.get(), x.get(), r, V, double(damping), partial.get(), parts,
+        cursor, chunk_sum.get(), o);
     if (chunks) {
         contrib_long_rows_kernel<<<grid_for(g.num_long * 32, 256), 256, 0, s>>>(
-            g.long_rows.get(), g.num_long, chunk_sum.get(), r, V, double(damping), partial.get(), kPartBlocks, o);
+            g.long_rows.get(), g.num_long, chunk_sum.get(), r, V, double(damping), partial.get(), parts, o);
     }
     HYT_CUDA(cudaGetLastError());
     t.stop(s);
