@@ -210,7 +210,8 @@ __device__ __forceinline__ double short_quotient(uint64_t n, uint64_t d) {
     return sure || r == 0.0 ? q : extended_quotient(n, d);
 }
 
-// Scores, ranking keys and which vertices have a score above 0.  The
+// Scores, ranking keys, and (each if asked for) which vertices have a score above
+// 0 and the vertices' ids.  The
 // denominator Do_max * Di_max is read from device memory (maxes[0..1]).
 // Products below 2^52 rank exactly as their quotients do (two that differ are
 // more than one unit in the last place apart after the division, so rounding
@@ -220,7 +221,8 @@ __device__ __forceinline__ bool rank_by_product(uint64_t denom) { return denom <
 
 __global__ void hub_scores_kernel(const uint64_t *__restrict__ outdeg, const uint32_t *__restrict__ indeg, uint64_t V,
                                   const unsigned long long *__restrict__ maxes, double *__restrict__ scores,
-                                  uint64_t *__restrict__ key, uint8_t *__restrict__ scored, uint32_t *__restrict__ bad) {
+                                  uint64_t *__restrict__ key, uint8_t *__restrict__ scored, uint32_t *__restrict__ id,
+                                  uint32_t *__restrict__ bad) {
     const uint64_t max_out = maxes[0], max_in = maxes[1];
     const bool overflow = max_in && max_out > ~uint64_t(0) / max_in;
     if (overflow && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(bad, kBadOverflow);
@@ -233,7 +235,8 @@ __global__ void hub_scores_kernel(const uint64_t *__restrict__ outdeg, const uin
         if (num && !overflow && (scores || !product)) sc = product ? short_quotient(num, denom) : extended_quotient(num, denom);
         if (scores) scores[v] = sc;
         key[v] = product ? num : static_cast<uint64_t>(__double_as_longlong(sc));
-        scored[v] = num && !overflow;
+        if (scored) scored[v] = num && !overflow;
+        if (id) id[v] = static_cast<uint32_t>(v);
     }
 }
 
@@ -424,6 +427,10 @@ __global__ void __launch_bounds__(kPermThreads) permute_edges_kernel(
     if (b) atomicOr(bad, b);
 }
 
+// Graphs of up to this many vertices are ranked by one sort of all of them; leaving
+// out those without a score first costs a selection and a read-back in mid-call.
+constexpr uint64_t kWholeSort = 2048;
+
 // Stable descending sort of (key, id) pairs on key bits [0, end_bit); the
 // result ends in *keys / *ids (which may swap with the alternate buffers).
 void sort_desc(uint64_t *&keys, uint64_t *keys_alt, uint32_t *&ids, uint32_t *ids_alt, uint64_t n, int end_bit,
@@ -522,29 +529,40 @@ void hub_sort(const hyt_csr &csr, double fraction, uint32_t *order_out, double *
     std::unique_ptr<Scratch<double>> sc;
     if (scores_out && !scores_dev) sc = std::make_unique<Scratch<double>>(V, s);
     double *scores_d = scores_dev ? scores_out : (sc ? sc->get() : nullptr);
+    auto check_flags = [&] {  // waits for s
+        const uint32_t h = read_flags(bad.get(), s);
+        fail_on_csr_flags(h);
+        if (h & kBadOverflow) fail(HYT_E_INVALID, "degree product exceeds 2^64");
+    };
+    const bool whole_sort = V <= kWholeSort;
     hub_scores_kernel<<<grid_sm(8), 256, 0, s>>>(outdeg.get(), indeg.get(), V, maxes.get(), scores_d, key.get(),
-                                                 is_other.get(), bad.get());
+                                                 whole_sort ? nullptr : is_other.get(),
+                                                 whole_sort ? ids.get() : nullptr, bad.get());
     HYT_CUDA(cudaGetLastError());
     if (scores_out && !scores_dev) HYT_CUDA(cudaMemcpyAsync(scores_out, scores_d, V * 8, cudaMemcpyDeviceToHost, s));
     // Only vertices with a score are ranked: the others tie at 0 and keep
-    // their id order, which is where the stable sort would leave them too.
-    select_index(is_other.get(), ids.get(), V, rest.get(), s);
-    uint64_t scored = 0;
-    unsigned long long h_max[2] = {0, 0};
-    HYT_CUDA(cudaMemcpyAsync(&scored, rest.get(), 8, cudaMemcpyDeviceToHost, s));
-    HYT_CUDA(cudaMemcpyAsync(h_max, maxes.get(), 16, cudaMemcpyDeviceToHost, s));
-    const uint32_t h = read_flags(bad.get(), s);
-    fail_on_csr_flags(h);
-    if (h & kBadOverflow) fail(HYT_E_INVALID, "degree product exceeds 2^64");
-    const uint64_t denom = uint64_t(h_max[0]) * h_max[1];
-    // products: the bits of the largest; scores in [0, 1]: 62 bits
-    const int bits = denom < (uint64_t(1) << 52) ? (denom ? 64 - __builtin_clzll(denom) : 1) : 62;
-    uint64_t *keys = key_srt.get();
+    // their id order, which is where the stable sort would leave them too.  A
+    // small graph is sorted whole, over the bits of any key.
+    uint64_t scored = V;
+    uint64_t *keys = key.get();
     uint32_t *ranked = ids.get();
-    if (scored) {
-        gather_keys_kernel<<<grid_for(scored, 256, 148u * 8u), 256, 0, s>>>(key.get(), ranked, scored, keys);
-        HYT_CUDA(cudaGetLastError());
-        sort_desc(keys, key_alt.get(), ranked, ids_alt.get(), scored, bits, s);
+    if (whole_sort) {
+        sort_desc(keys, key_alt.get(), ranked, ids_alt.get(), V, 62, s);
+    } else {
+        select_index(is_other.get(), ids.get(), V, rest.get(), s);
+        unsigned long long h_max[2] = {0, 0};
+        HYT_CUDA(cudaMemcpyAsync(&scored, rest.get(), 8, cudaMemcpyDeviceToHost, s));
+        HYT_CUDA(cudaMemcpyAsync(h_max, maxes.get(), 16, cudaMemcpyDeviceToHost, s));
+        check_flags();
+        const uint64_t denom = uint64_t(h_max[0]) * h_max[1];
+        // products: the bits of the largest; scores in [0, 1]: 62 bits
+        const int bits = denom < (uint64_t(1) << 52) ? (denom ? 64 - __builtin_clzll(denom) : 1) : 62;
+        keys = key_srt.get();
+        if (scored) {
+            gather_keys_kernel<<<grid_for(scored, 256, 148u * 8u), 256, 0, s>>>(key.get(), ranked, scored, keys);
+            HYT_CUDA(cudaGetLastError());
+            sort_desc(keys, key_alt.get(), ranked, ids_alt.get(), scored, bits, s);
+        }
     }
     const uint64_t hubs = hub_count_for(V, fraction);
     const uint64_t top = std::min(hubs, scored);
@@ -564,7 +582,10 @@ void hub_sort(const hyt_csr &csr, double fraction, uint32_t *order_out, double *
     whole.stop(s);
     uint64_t h_rest = 0;
     HYT_CUDA(cudaMemcpyAsync(&h_rest, rest.get(), 8, cudaMemcpyDeviceToHost, s));
-    HYT_CUDA(cudaStreamSynchronize(s));
+    if (whole_sort)
+        check_flags();
+    else
+        HYT_CUDA(cudaStreamSynchronize(s));
     if (h_rest + top != V) fail(HYT_E_INTERNAL, "hub ordering lost vertices");
     if (hub_count) *hub_count = hubs;
     if (stats) {
