@@ -1,5 +1,8 @@
 // Copies between pageable host memory and the device through pinned chunks
 // filled (or emptied) by several host threads; see staging.cuh.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -15,9 +18,29 @@ namespace hyt {
 namespace {
 
 constexpr size_t kChunk = size_t(1) << 20;      // per buffer
-constexpr size_t kMinBytes = size_t(4) << 20;   // below this the threads cost more than they save
 constexpr int kBuffers = 2;                     // per worker: one in flight, one being filled
 constexpr int kMaxWorkers = 8;
+// From these sizes on the threads, started on idle cores by each copy, save more than
+// they cost.  Plain copy / through chunks, a pause before each copy as a solve makes
+// one: to the device 2 MiB 0.23 / 0.24 ms, 4 MiB 0.41 / 0.29, 8 MiB 0.79 / 0.47, 128
+// MiB 12.0 / 3.6; to the host 4 MiB 0.24 / 0.35, 8 MiB 0.43 / 0.61, 12 MiB 0.64 / 0.72,
+// 16 MiB 0.83 / 0.74, 128 MiB 6.4 / 3.8, but into pages that nothing has touched yet
+// 4 MiB 2.1 / 1.2, 8 MiB 4.1 / 1.7, 128 MiB 65 / 18.
+constexpr size_t kMinBytes = size_t(4) << 20;
+constexpr size_t kMinToTouched = size_t(16) << 20;
+
+// True when most of the memory at p has no pages yet (a look at eight of them).
+bool untouched(const void *p, size_t bytes) {
+    const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+    const uintptr_t first = reinterpret_cast<uintptr_t>(p) / page * page;
+    int missing = 0;
+    for (size_t k = 0; k < 8; ++k) {
+        unsigned char resident = 1;
+        const uintptr_t at = first + (2 * k + 1) * bytes / 16 / page * page;
+        if (mincore(reinterpret_cast<void *>(at), page, &resident) == 0 && !(resident & 1)) ++missing;
+    }
+    return missing > 4;
+}
 
 // One worker's pinned buffers, stream and events on one device.
 struct Lane {
@@ -118,6 +141,7 @@ cudaError_t work(Lane &l, unsigned char *dst, const unsigned char *src, size_t b
 
 bool staged_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaStream_t s) {
     if (bytes < kMinBytes) return false;
+    if (!to_device && bytes < kMinToTouched && !untouched(dst, bytes)) return false;
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, to_device ? src : dst) != cudaSuccess) {
         (void)cudaGetLastError();

@@ -3,6 +3,7 @@
 // and events that know their device, as CUDA's do (an event recorded on a stream
 // of another device is an invalid handle), and streams that a capture spreads to.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cstdio>
 #include <cstdlib>
@@ -102,7 +103,7 @@ void expect(bool got, bool want, const char *what) {
 }  // namespace
 
 int main() {
-    constexpr size_t kLarge = (size_t(9) << 20) + 12345;
+    constexpr size_t kLarge = (size_t(33) << 20) + 12345;
     for (int current = 0; current < 2; ++current) {
         cudaSetDevice(current);
         cudaStream_t own = reinterpret_cast<cudaStream_t>(new Handle{current});
@@ -110,7 +111,9 @@ int main() {
         for (bool to_device : {true, false}) {
             expect(through_chunks(kLarge, to_device, own, "own stream"), true, "own stream");
             expect(through_chunks(kLarge, to_device, nullptr, "default stream"), true, "default stream");
-            expect(through_chunks(1000, to_device, own, "small copy"), false, "small copy");
+            const size_t least = size_t(to_device ? 4 : 16) << 20;  // `dst` has its pages
+            expect(through_chunks(least, to_device, own, "least copy"), true, "least copy");
+            expect(through_chunks(least - 1, to_device, own, "small copy"), false, "small copy");
             // the runtime copies on a stream of any device: so must the caller, by itself
             expect(through_chunks(kLarge, to_device, other, "another device's stream"), false,
                    "another device's stream");
@@ -123,6 +126,17 @@ int main() {
             cudaGetDevice(&d);
             expect(d == current, true, "current device kept");
         }
+    }
+    // memory that nothing has touched yet is worth the chunks from 4 MiB on
+    cudaSetDevice(0);
+    for (size_t n : {size_t(4) << 20, (size_t(4) << 20) - 1, (size_t(9) << 20) + 12345}) {
+        const std::vector<unsigned char> src(n, 5);
+        void *m = mmap(nullptr, n + 8192, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        unsigned char *dst = static_cast<unsigned char *>(m) + 4099;
+        const bool staged = hyt::staged_copy(dst, src.data(), n, false, nullptr);
+        expect(staged, n >= size_t(4) << 20, "fresh memory");
+        if (staged) expect(std::memcmp(dst, src.data(), n) == 0 && dst[-1] == 0 && dst[n] == 0, true, "fresh memory: bytes");
+        munmap(m, n + 8192);
     }
     hyt::staging_release(0);
     hyt::staging_release(1);
