@@ -653,8 +653,13 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
         a.num_hot = g.num_hot;
         a.tile_cost = g.tile_cost;
         a.chunk_edges = g.chunk_edges;
+        float *hot_contrib[2];
         for (int i = 0; i < 2; ++i) a.rank[i] = reinterpret_cast<float *>(take(V * 4 + 16));
-        for (int i = 0; i < 2; ++i) a.contrib[i] = reinterpret_cast<float *>(take(V * 4 + 16));
+        // a parity's hot table lies right behind its contributions (prc::Sources)
+        for (int i = 0; i < 2; ++i) {
+            a.contrib[i] = reinterpret_cast<float *>(take(V * 4 + 16));
+            hot_contrib[i] = reinterpret_cast<float *>(take(uint64_t(g.num_hot) * 4 + 16));
+        }
         a.partial = reinterpret_cast<float2 *>(take(g.num_chunks * 8 + 16));
         a.ticket = reinterpret_cast<uint32_t *>(take(g.num_long * 4 + 16));
         PRExtra x{};
@@ -667,7 +672,7 @@ int QueryEngine::admit(const hyt_query &q, uint64_t tag) {
         a.dangling = reinterpret_cast<double *>(take((it + 2) * 8));
         x.block_sums = reinterpret_cast<double2 *>(take(kEndBlocks * 16));
         x.end_ticket = reinterpret_cast<uint32_t *>(take(16));
-        for (int i = 0; i < 2; ++i) x.hot_contrib[i] = reinterpret_cast<float *>(take(uint64_t(g.num_hot) * 4 + 16));
+        for (int i = 0; i < 2; ++i) x.hot_contrib[i] = hot_contrib[i];
         a.num_tiles = g.num_tiles;
         a.num_chunks = static_cast<uint32_t>(g.num_chunks);
         a.V = static_cast<uint32_t>(V);

@@ -133,24 +133,25 @@ constexpr int kBatch = HYT_PR_BATCH;
 // Where a task reads its contributions: whole-vector array for untagged
 // sources (L2, evict-last), table of the hot sources for tagged ones.  Slot
 // num_hot of the table is 0: `none`, its tagged id, stands for "no edge".
-// kSmemHot: the table is in shared memory (else in global memory).
+// kSmemHot: the table is in shared memory; else in global memory, at most 2^31
+// elements behind the array, and `turn` makes a tagged id an index of it from there.
 struct Sources {
     const float *ccur;
     const float *hot;
-    uint32_t none;
+    uint32_t none, turn;
     uint64_t pol;
 };
 
 __device__ __forceinline__ Sources make_sources(const PRArgs &a, const float *ccur, const float *hot) {
-    return Sources{ccur, hot, kHotTag | a.num_hot, dev::policy_evict_last()};
+    return Sources{ccur, hot, kHotTag | a.num_hot, static_cast<uint32_t>(hot - ccur) - kHotTag, dev::policy_evict_last()};
 }
 
 // Loads one source's contribution: its bits end in `g | id`.  Not through the
 // read-only path: the persistent solver rewrites the vector between
-// iterations.  The two loads
-// are predicated on the tag and write registers of their own (the hot one
-// its id's), so that neither waits for the other and no branch splits a run
-// of gathers.
+// iterations.  With the table in shared memory the two loads are predicated on
+// the tag and write registers of their own (the hot one its id's), so that
+// neither waits for the other and no branch splits a run of gathers; in global
+// memory one load serves both.
 template <bool kSmemHot>
 __device__ __forceinline__ void load_contribution(uint32_t &id, uint32_t &g, const Sources &S) {
     g = 0;
@@ -164,13 +165,9 @@ __device__ __forceinline__ void load_contribution(uint32_t &id, uint32_t &g, con
             : "+r"(g), "+r"(id)
             : "l"(S.ccur + id), "l"(S.pol), "r"(at));
     } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, 0;\n\t"
-            "@!p ld.global.L2::cache_hint.b32 %0, [%2], %3;\n\t"
-            "@!p mov.b32 %1, 0;\n\t"
-            "@p ld.global.b32 %1, [%4];\n\t}"
-            : "+r"(g), "+r"(id)
-            : "l"(S.ccur + id), "l"(S.pol), "l"(S.hot + (id & ~kHotTag)));
+        const uint32_t at = (id & kHotTag) ? id + S.turn : id;
+        asm volatile("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(g) : "l"(S.ccur + at), "l"(S.pol));
+        id = 0;
     }
 }
 
