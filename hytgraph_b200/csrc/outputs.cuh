@@ -18,7 +18,7 @@
 
 namespace hyt {
 
-constexpr size_t kOutputKeep = size_t(1) << 30;
+constexpr size_t kOutputKeep = size_t(4) << 30;  // a result of R-MAT scale 24 is 2.2 GiB: 10.3 ms a step without, 5.9 with
 constexpr size_t kOutputBlocks = 64;  // small results: a block is searched for by size
 
 // A cudaMalloc block of at least `bytes` on the current device.

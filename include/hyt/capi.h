@@ -113,7 +113,7 @@ typedef struct hyt_graph_options {
  * per-device memory pools that keep freed memory mapped (graph arrays: up to
  * 16 GiB; scratch: up to 8 GiB), so repeated graph creation does not map
  * fresh memory each time; freed device outputs of hyt_csr_reorder are kept for
- * the next call too (up to 1 GiB).  This returns that cached memory of
+ * the next call too (up to 4 GiB).  This returns that cached memory of
  * `device` to the driver (after waiting for the device). */
 int hyt_trim_device_memory(int device);
 

@@ -96,9 +96,9 @@ def test_kept_blocks_are_bounded_and_returned(hyt, gpu):
     hyt.reorder(g, order, device=True).free()
     hyt.capi.check(hyt.capi.lib.hyt_trim_device_memory(0))
     free = torch.cuda.mem_get_info()[0]
-    for d in [hyt.reorder(g, order, device=True) for _ in range(10)]:
+    for d in [hyt.reorder(g, order, device=True) for _ in range(14)]:
         d.free()
-    # 1 GiB of results are kept, and the scratch of one call
-    assert torch.cuda.mem_get_info()[0] >= free - (3 << 30) - (64 << 20)
+    # 4 GiB of results are kept, and the scratch of one call
+    assert torch.cuda.mem_get_info()[0] >= free - (5 << 30)
     hyt.capi.check(hyt.capi.lib.hyt_trim_device_memory(0))
     assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)
