@@ -603,7 +603,7 @@ void pagerank_partitioned(GraphImpl &g, PullSource &src, bool personalized, uint
             // Pieces readable together, with consecutive tasks, share a launch: a
             // launch's time is that of its slowest task, not its size.  16 M
             // edges in 64 partitions, 32 MB on the device: 71 launches an
-            // iteration -> 40, 16 iterations 31.9 -> 22.8 ms (shorter chunks
+            // iteration -> 40, 16 iterations 31.9 -> 22.8 ms (shorter tasks
             // of long rows included).
             PullPart run = src.part(p);
             size_t last = p;
