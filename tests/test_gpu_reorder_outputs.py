@@ -45,7 +45,7 @@ def test_free_waits_for_readers(hyt, gpu):
     and another renumbering of the same sizes follows at once."""
     import torch
 
-    V, E = 1 << 16, 1 << 22
+    V, E = 1 << 16, 1 << 24
     a, b, order = _graph(hyt, V, E, 5), _graph(hyt, V, E, 6), _order(V, 5)
     want = hyt.reorder(a, order).column_indices
     d = hyt.reorder(a, order, device=True)
@@ -56,7 +56,7 @@ def test_free_waits_for_readers(hyt, gpu):
     s = torch.cuda.Stream()
     torch.cuda.synchronize()
     with torch.cuda.stream(s):
-        for _ in range(3000):  # 16 MiB each: tens of milliseconds in all
+        for _ in range(1500):  # 64 MiB each, longer on the GPU than to queue: tens of milliseconds in all
             dst.copy_(src)
     queued = not s.query()
     d.free()
